@@ -12,9 +12,10 @@
 //   compact   the new keys, then runs of new keys sharing a leaf (segments);
 //   leaf      one 8-lane group per touched leaf merges its new keys by rank scatter
 //             (each element computes its merged position by binary search in
-//             the other sequence) and cuts an overflowing leaf into
-//             p = ceil(m / leaf_fill) leaves of even size; the first keys of
-//             pieces 1..p-1 become separator entries for the parent;
+//             the other sequence); an overflowing leaf becomes
+//             p = ceil(m / leaf_fill) leaves of even size, one group per piece;
+//             the first keys of pieces 1..p-1 become separator entries for the
+//             parent;
 //   inner     one block applies the entries level by level the same way
 //             (children spread evenly over q = ceil((s+1)/(inner_fill+1))
 //             nodes, the key between two pieces moves up) and rebuilds an
@@ -55,6 +56,24 @@ constexpr uint64_t kNoPos = ~0ull;  // merge_locate_kernel: no value to update i
 constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
+
+// S slots of a row that this kernel also writes (plain loads: the read-only
+// path must not be used for it)
+template <int S>
+__device__ __forceinline__ void load_row16(const uint64_t* p, uint64_t (&x)[S]) {
+#pragma unroll
+  for (int i = 0; i < S; i += 2) {
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(p + i);
+    x[i] = w.x;
+    x[i + 1] = w.y;
+  }
+}
+
+template <int S>
+__device__ __forceinline__ void store_row16(uint64_t* p, const uint64_t (&x)[S]) {
+#pragma unroll
+  for (int i = 0; i < S; i += 2) *reinterpret_cast<ulonglong2*>(p + i) = make_ulonglong2(x[i], x[i + 1]);
+}
 
 // piece index and slot of merged position `pos` when m items are spread over p
 // pieces (the first m % p pieces hold one more)
@@ -350,143 +369,221 @@ __global__ void merge_fail_mark_kernel(const MergeCounts* __restrict__ mc, const
 }
 
 // ------------------------------------------------------------- leaf ----
-// One group of G lanes per touched leaf (segment); lane g holds slots
-// g*S .. g*S+S-1 of the row.  Several leaves per warp keep more row loads in
-// flight than a warp per leaf (the kernel is bound by the dependent chain
-// segment bounds -> leaf id -> row).
+// A touched leaf of sz keys that gets cnt new ones becomes p pieces of even
+// size (p = 1 while they fit one leaf).  Piece c holds the merged positions
+// [st, st + kc); a group of G lanes builds it whole: every old key's merged
+// position by a binary search in the new keys, every new key of the range by
+// one in the old row, the row put together in shared memory and written with
+// 16-byte stores.  A piece needs nothing of its neighbours: its right fence is
+// the key at merged position st + kc.
 template <int G>
-__global__ void __launch_bounds__(256) merge_leaf_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* mc,
+struct LeafSmem {
+  uint64_t old[256 / G][32];
+  __align__(16) uint64_t mk[256 / G][32];
+  __align__(16) uint64_t mv[256 / G][32];
+};
+
+template <int G>
+__device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<G>& sm, uint32_t grp, uint32_t g,
+                                               uint32_t gmask, uint32_t nd, uint32_t c, uint32_t p, uint32_t m,
+                                               uint32_t sz, uint64_t hdr, uint64_t fence,
+                                               const uint64_t (&ok)[32 / G], const uint64_t (&ov)[32 / G],
+                                               const uint64_t* __restrict__ nk, const uint64_t* __restrict__ nv,
+                                               uint32_t cnt) {
+  constexpr int S = 32 / G;
+  const uint32_t st = piece_start(c, m, p), kc = piece_size(c, m, p), end = st + kc;
+  uint64_t* mk = sm.mk[grp];
+  uint64_t* mv = sm.mv[grp];
+  const uint64_t* old = sm.old[grp];
+  // old keys of the piece to their slots; how many of them precede its two ends
+  uint32_t before = 0;  // old keys at merged positions below st, and (high half) below end
+  uint64_t right = 0;   // the key at position end when it is an old one
+  bool right_old = false;
+#pragma unroll
+  for (int i = 0; i < S; i++) {
+    const uint32_t slot = g * S + i;
+    if (slot < sz) {
+      const uint32_t pos = slot + count_less(nk, cnt, ok[i]);
+      before += (pos < st ? 1u : 0u) + (pos < end ? 0x10000u : 0u);
+      if (pos >= st && pos < end) {
+        mk[pos - st] = ok[i];
+        mv[pos - st] = ov[i];
+      } else if (pos == end) {
+        right = ok[i];
+        right_old = true;
+      }
+    }
+  }
+  before = group_sum<G>(before, gmask);
+  const uint32_t j0 = st - (before & 0xffffu), j1 = end - (before >> 16);
+  for (uint32_t j = j0 + g; j < j1; j += G) {
+    const uint64_t key = nk[j];
+    const uint32_t pos = j + count_less(old, sz, key);
+    mk[pos - st] = key;
+    mv[pos - st] = nv[j];
+  }
+  uint64_t rf = fence;
+  if (c + 1 < p) {  // the next piece's first key: an old one, or the next new one
+    const uint32_t who = __ballot_sync(gmask, right_old) & gmask;
+    if (who) rf = __shfl_sync(gmask, right, __ffs(who) - 1);
+    else rf = nk[j1];
+  }
+  __syncwarp(gmask);
+  uint64_t wk[S], wv[S];
+#pragma unroll
+  for (int i = 0; i < S; i++) {
+    const uint32_t slot = g * S + i;
+    wk[i] = slot < kc ? mk[slot] : kKeyMax;
+    wv[i] = slot < kc ? mv[slot] : 0;
+  }
+  const uint64_t first = mk[0];
+  if (g == G - 1) {
+    wk[S - 1] = make_hdr(kc, 0, c == 0 ? hdr_version(hdr) + 1 : 0, hdr_epoch(hdr));
+    wv[S - 1] = rf;
+  }
+  store_row16<S>(t.keys + (size_t)nd * 32 + g * S, wk);
+  store_row16<S>(t.vals + (size_t)nd * 32 + g * S, wv);
+  __syncwarp(gmask);  // the shared rows are reused by the group's next piece
+  return first;
+}
+
+// a touched leaf's row in registers and its keys in shared memory; kNc: no
+// other group writes the row in this launch (read-only path)
+template <int G, bool kNc>
+__device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<G>& sm, uint32_t grp, uint32_t g, uint32_t gmask,
+                                         uint32_t leaf, uint64_t (&ok)[32 / G], uint64_t (&ov)[32 / G], uint64_t& hdr,
+                                         uint64_t& fence) {
+  constexpr int S = 32 / G;
+  if (kNc) {
+    load_slots<S>(t.keys + (size_t)leaf * 32 + g * S, ok);
+    load_slots<S>(t.vals + (size_t)leaf * 32 + g * S, ov);
+  } else {
+    load_row16<S>(t.keys + (size_t)leaf * 32 + g * S, ok);
+    load_row16<S>(t.vals + (size_t)leaf * 32 + g * S, ov);
+  }
+  hdr = __shfl_sync(gmask, ok[S - 1], G - 1, G);
+  fence = __shfl_sync(gmask, ov[S - 1], G - 1, G);
+  const uint32_t sz = hdr_size(hdr);
+#pragma unroll
+  for (int i = 0; i < S; i++) {
+    const uint32_t slot = g * S + i;
+    sm.old[grp][slot] = slot < sz ? ok[i] : kKeyMax;
+  }
+  __syncwarp(gmask);
+}
+
+// Leaf merge: a grid-stride loop of groups of G lanes over two kinds of items.
+//   segments  a touched leaf whose merged row fits: rewritten in place by its
+//             group.  Several leaves per warp keep more row loads in flight
+//             than a warp per leaf (the kernel is bound by the dependent chain
+//             segment bounds -> leaf id -> row).
+//   entries   one new piece (1 .. p - 1) of a leaf that splits; its segment by a
+//             binary search in the entry offsets.  All pieces read the old row,
+//             and the group that finishes the leaf's last one (a count down of
+//             `extra`, no group waits) writes piece 0 in its place.
+// With all the pieces of a leaf in the hands of the leaf's one group, a batch
+// that puts 1.3 million keys into a tree of one leaf ran for 75 ms; spread over
+// the chip, a tree of 2^23 keys grown by seven such batches takes 6.5 ms, from
+// 81.2.  A launch of its own for the pieces cost batches that split nothing 4 %
+// (a 50/50 batch of 2^20), and so did 74 registers (three blocks an SM).
+template <int G>
+__global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* mc,
                                                          const uint32_t* __restrict__ seg_start,
                                                          const uint32_t* __restrict__ eoff,
+                                                         uint32_t* __restrict__ extra,
                                                          const uint64_t* __restrict__ newk,
                                                          const uint64_t* __restrict__ newv,
                                                          const uint32_t* __restrict__ nq,
                                                          const uint32_t* __restrict__ seg_leaf,
                                                          MergeEntry* __restrict__ ent) {
   constexpr int S = 32 / G;
-  __shared__ uint64_t s_keys[256 / G][32];
-  __shared__ __align__(16) uint64_t s_mk[256 / G][32];  // merged row when it fits one leaf
-  __shared__ __align__(16) uint64_t s_mv[256 / G][32];
+  __shared__ LeafSmem<G> sm;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t g = lane % G;
   const uint32_t grp = threadIdx.x / G;
   const uint32_t gmask = group_mask<G>(lane);
-  const uint32_t n_segs = mc->n_segs;
-  const bool fail = mc->cap_fail != 0;
+  const uint32_t n_segs = mc->n_segs, n_ent = mc->n_leaf_entries;
+  if (mc->cap_fail) return;  // merge_fail_mark_kernel answered the new keys
   const uint32_t base = mc->node_base;
   const uint32_t n_groups = (gridDim.x * blockDim.x) / G;
   unsigned long long added = 0, splits = 0;
-  for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / G; s < n_segs; s += n_groups) {
+  const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+  for (uint32_t s = gid; s < n_segs; s += n_groups) {
     uint32_t a, b;
     seg_bounds(mc, seg_start, s, a, b);
     const uint32_t leaf = seg_leaf[s];
     const uint32_t cnt = b - a;
-    if (fail) continue;  // merge_fail_mark_kernel answered these keys
-    uint64_t ok[S], ov[S];
-    load_slots<S>(t.keys + (size_t)leaf * 32 + g * S, ok);
-    load_slots<S>(t.vals + (size_t)leaf * 32 + g * S, ov);
-    const uint64_t h = __shfl_sync(gmask, ok[S - 1], G - 1, G);
-    const uint64_t fence = __shfl_sync(gmask, ov[S - 1], G - 1, G);
-    const uint32_t sz = hdr_size(h);
+    if (g == 0) added += cnt;
+    // a leaf that splits (it has entries) is written by their groups
+    if (eoff[s] != (s + 1 < n_segs ? eoff[s + 1] : n_ent)) continue;
+    uint64_t ok[S], ov[S], hdr, fence;
+    leaf_row<G, true>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
+    const uint32_t sz = hdr_size(hdr), m = sz + cnt;
 #pragma unroll
     for (int i = 0; i < S; i++) {
       const uint32_t slot = g * S + i;
-      s_keys[grp][slot] = slot < sz ? ok[i] : kKeyMax;
-    }
-    __syncwarp(gmask);
-    const uint32_t m = sz + cnt;
-    const uint32_t p = m <= (uint32_t)kMaxKeys ? 1u : ceil_div(m, leaf_fill);
-    if (p == 1) {
-      // no split (the common case): merge into shared memory, then write
-      // the row with one 16-byte store per lane and pair of slots
-#pragma unroll
-      for (int i = 0; i < S; i++) {
-        const uint32_t slot = g * S + i;
-        if (slot < sz) {
-          const uint32_t pos = slot + count_less(newk + a, cnt, ok[i]);
-          s_mk[grp][pos] = ok[i];
-          s_mv[grp][pos] = ov[i];
-        }
+      if (slot < sz) {
+        const uint32_t pos = slot + count_less(newk + a, cnt, ok[i]);
+        sm.mk[grp][pos] = ok[i];
+        sm.mv[grp][pos] = ov[i];
       }
-      for (uint32_t j = g; j < cnt; j += G) {
-        const uint64_t key = newk[a + j];
-        const uint32_t pos = j + count_less(s_keys[grp], sz, key);
-        s_mk[grp][pos] = key;
-        s_mv[grp][pos] = newv[a + j];
-      }
-      __syncwarp(gmask);
-      uint64_t wk[S], wv[S];
-#pragma unroll
-      for (int i = 0; i < S; i++) {
-        const uint32_t slot = g * S + i;
-        wk[i] = slot < m ? s_mk[grp][slot] : kKeyMax;
-        wv[i] = slot < m ? s_mv[grp][slot] : 0;
-      }
-      if (g == G - 1) {
-        wk[S - 1] = make_hdr(m, 0, hdr_version(h) + 1, hdr_epoch(h));
-        wv[S - 1] = fence;
-      }
-      uint64_t* kr = t.keys + (size_t)leaf * 32 + g * S;
-      uint64_t* vr = t.vals + (size_t)leaf * 32 + g * S;
-#pragma unroll
-      for (int i = 0; i < S; i += 2) {
-        *reinterpret_cast<ulonglong2*>(kr + i) = make_ulonglong2(wk[i], wk[i + 1]);
-        *reinterpret_cast<ulonglong2*>(vr + i) = make_ulonglong2(wv[i], wv[i + 1]);
-      }
-      __syncwarp(gmask);  // s_mk / s_mv are reused by the next segment
-      if (g == 0) added += cnt;
-      continue;
-    }
-    const uint32_t eo = eoff[s];
-    auto node_of = [&](uint32_t c) -> uint32_t { return c == 0 ? leaf : base + eo + c - 1; };
-    auto place = [&](uint32_t pos, uint64_t key, uint64_t val) {
-      uint32_t c, slot;
-      piece_of(pos, m, p, c, slot);
-      const uint32_t nd = node_of(c);
-      t.keys[(size_t)nd * 32 + slot] = key;
-      t.vals[(size_t)nd * 32 + slot] = val;
-      if (slot == 0 && c >= 1) {
-        t.low[nd] = key;
-        t.vals[(size_t)node_of(c - 1) * 32 + 31] = key;  // right fence of the piece before
-        MergeEntry e;
-        e.key = key;
-        e.child = nd;
-        e.rep = nq[a];
-        ent[eo + c - 1] = e;
-      }
-    };
-    // old keys and new keys to their merged positions (all reads happened above)
-#pragma unroll
-    for (int i = 0; i < S; i++) {
-      const uint32_t slot = g * S + i;
-      if (slot < sz) place(slot + count_less(newk + a, cnt, ok[i]), ok[i], ov[i]);
     }
     for (uint32_t j = g; j < cnt; j += G) {
       const uint64_t key = newk[a + j];
-      place(j + count_less(s_keys[grp], sz, key), key, newv[a + j]);
+      const uint32_t pos = j + count_less(sm.old[grp], sz, key);
+      sm.mk[grp][pos] = key;
+      sm.mv[grp][pos] = newv[a + j];
     }
     __syncwarp(gmask);
-    // padding, headers, last fence
-    for (uint32_t c = 0; c < p; c++) {
-      const uint32_t nd = node_of(c);
-      const uint32_t kc = piece_size(c, m, p);
+    uint64_t wk[S], wv[S];
 #pragma unroll
-      for (int i = 0; i < S; i++) {
-        const uint32_t slot = g * S + i;
-        if (slot >= kc && slot < 31) {
-          t.keys[(size_t)nd * 32 + slot] = kKeyMax;
-          t.vals[(size_t)nd * 32 + slot] = 0;
-        }
-      }
-      if (g == G - 1) {
-        t.keys[(size_t)nd * 32 + 31] = make_hdr(kc, 0, c == 0 ? hdr_version(h) + 1 : 0, hdr_epoch(h));
-        if (c == p - 1) t.vals[(size_t)nd * 32 + 31] = fence;
-      }
+    for (int i = 0; i < S; i++) {
+      const uint32_t slot = g * S + i;
+      wk[i] = slot < m ? sm.mk[grp][slot] : kKeyMax;
+      wv[i] = slot < m ? sm.mv[grp][slot] : 0;
     }
-    __syncwarp(gmask);
-    if (g == 0) {
-      added += cnt;
-      splits += p - 1;
+    if (g == G - 1) {
+      wk[S - 1] = make_hdr(m, 0, hdr_version(hdr) + 1, hdr_epoch(hdr));
+      wv[S - 1] = fence;
+    }
+    store_row16<S>(t.keys + (size_t)leaf * 32 + g * S, wk);
+    store_row16<S>(t.vals + (size_t)leaf * 32 + g * S, wv);
+    __syncwarp(gmask);  // the shared rows are reused by the next segment
+  }
+  for (uint32_t e = gid; e < n_ent; e += n_groups) {
+    // the last segment whose entries begin at or before e
+    uint32_t lo = 0, hi = n_segs;
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (eoff[mid] <= e) lo = mid;
+      else hi = mid;
+    }
+    uint32_t a, b;
+    seg_bounds(mc, seg_start, lo, a, b);
+    const uint32_t cnt = b - a, leaf = seg_leaf[lo];
+    uint64_t ok[S], ov[S], hdr, fence;
+    leaf_row<G, false>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
+    const uint32_t sz = hdr_size(hdr), m = sz + cnt, p = ceil_div(m, leaf_fill);
+    uint32_t c = e - eoff[lo] + 1, nd = base + e;
+    for (;;) {
+      const uint64_t first = leaf_piece<G>(t, sm, grp, g, gmask, nd, c, p, m, sz, hdr, fence, ok, ov, newk + a,
+                                           newv + a, cnt);
+      if (c == 0) break;
+      uint32_t left = 0;
+      if (g == 0) {
+        t.low[nd] = first;
+        MergeEntry x;
+        x.key = first;
+        x.child = nd;
+        x.rep = nq[a];
+        ent[e] = x;
+        splits++;
+        __threadfence();  // the old row was read before the count says so
+        left = atomicSub(extra + lo, 1u);
+      }
+      if (__shfl_sync(gmask, left, 0, G) != 1u) break;
+      c = 0;  // the leaf's other pieces are done: piece 0 takes the leaf's row
+      nd = leaf;
     }
   }
   if (g == 0 && (added | splits)) {
@@ -885,7 +982,7 @@ int merge_write_phase(Handle* h, cudaStream_t s) {
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
   const uint32_t entry_cap = (uint32_t)w.cap;
   merge_leaf_kernel<8><<<(unsigned)((size_t)h->sm_count * 8), 256, 0, s>>>(
-      h->tree, h->leaf_fill, mc, w.m_seg, w.m_pos, w.m_newk, w.m_newv, w.m_nq, w.m_leaf,
+      h->tree, h->leaf_fill, mc, w.m_seg, w.m_pos, w.m_isnew, w.m_newk, w.m_newv, w.m_nq, w.m_leaf,
       reinterpret_cast<MergeEntry*>(w.m_ent_a));
   count_launch();
   if (launch_inner(h, entry_cap, mc, s) != cudaSuccess) return -2;
