@@ -29,6 +29,7 @@ SOURCES = [
     "bt_serve.cu",
     "bt_shard.cu",
     "bt_front.cu",
+    "bt_small.cu",
     "bt_snapshot.cu",
     "bt_delete.cu",
 ]

@@ -177,7 +177,7 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   h.L.n_segments = cfg.n_segments ? cfg.n_segments : 4096;
   h.L.window = cfg.window ? cfg.window : 64;
   cudaDeviceGetAttribute(&h.sm_count, cudaDevAttrMultiProcessorCount, cfg.device);
-  bool ok = bt::sort_prepare() == cudaSuccess;
+  bool ok = bt::sort_prepare() == cudaSuccess && bt::small_prepare() == 0 && bt::small_write_prepare() == 0;
   h.tree.cap = (uint32_t)nodes;
   ok = ok && cudaMalloc(&h.tree.keys, nodes * 256) == cudaSuccess;
   ok = ok && cudaMalloc(&h.tree.vals, nodes * 256) == cudaSuccess;
@@ -293,8 +293,11 @@ int bt_execute_batches(bt_handle* H, size_t count, const uint64_t* const* keys, 
   const int base = mode & 0xF;
   if (base != BT_MODE_SORTED && base != BT_MODE_STM) return BT_ERR_INVALID_ARG;
   EntryGuard g(H);
-  if (base != BT_MODE_SORTED || h.front_end != 1) {
-    // only sorted batches with the hash front end have a front part to run ahead
+  // only sorted batches with the hash front end have a front part to run
+  // ahead, and for small ones the launches saved are worth more
+  bool small = true;
+  for (size_t j = 0; j < count && small; j++) small = bt::small_usable(&h, n[j]);
+  if (base != BT_MODE_SORTED || h.front_end != 1 || small) {
     for (size_t j = 0; j < count; j++) {
       const int rc = bt_execute_batch(H, keys[j], vals[j], ops[j], out_vals[j], out_status[j], n[j], mode, stream);
       if (rc != BT_OK) return rc;
@@ -454,7 +457,8 @@ static int host_submit(bt_handle* H, const uint64_t* keys, const uint64_t* vals,
   // the front part on its own stream once the op codes and keys are in,
   // beside the previous host batch's tree part; the merge passes once the
   // values are in (a full value array: beside the lookups instead)
-  const bool chained = base == BT_MODE_SORTED && h.front_end == 1 && h.host_front_overlap && !remote && !h.prof;
+  const bool chained = base == BT_MODE_SORTED && h.front_end == 1 && h.host_front_overlap && !remote && !h.prof &&
+                       !bt::small_usable(&h, n);
   if (chained) {
     h.ans_ready = st.ans_ev;
     rc = map_internal(bt::batch_chained(&h, st.keys, st.vals, st.ops, st.out_vals, st.out_st, n, engine, s,

@@ -392,6 +392,7 @@ int work_alloc(Work* w, size_t cap) {
   A((void**)&w->f_tv, cap * 4);
   A((void**)&w->lb_status, scan_lb_words(cap) * 8);
   A((void**)&w->lb_ctr, 8);
+  A((void**)&w->s_write, 3 * 16 * 4);
   ok = ok && cudaMemset(w->lb_status, 0, scan_lb_words(cap) * 8) == cudaSuccess &&
        cudaMemset(w->lb_ctr, 0, 8) == cudaSuccess;
   if (!ok) {
@@ -399,6 +400,10 @@ int work_alloc(Work* w, size_t cap) {
     return -3;
   }
   w->cap = cap;
+  if (small_alloc(w) != 0) {
+    work_free(w);
+    return -3;
+  }
   return 0;
 }
 
@@ -451,7 +456,8 @@ void work_free(Work* w) {
                 w->m_path,   w->m_vpos,   w->m_leaf,    w->m_isnew,   w->m_pos,     w->m_newk,       w->m_newv,  w->m_nq,
                 w->m_nleaf,  w->m_seg,     w->d_leaf,    w->d_slot,    w->m_ent_a,   w->m_ent_b,   w->m_counts,     w->m_sync,
                 w->ins_ops,  w->f_tab, w->f_flags,
-                w->f_pos,    w->f_list,    w->f_lk,      w->f_tk,      w->f_tv,      w->lb_status, w->lb_ctr};
+                w->f_pos,    w->f_list,    w->f_lk,      w->f_tk,      w->f_tv,      w->lb_status, w->lb_ctr,
+                w->s_tab,    w->s_sums,  w->s_write};
   for (void* p : ps)
     if (p) cudaFree(p);
   *w = Work{};
@@ -654,6 +660,50 @@ static int batch_hashed(Handle* h, const uint64_t* keys, const uint64_t* vals, c
   return hashed_tree(h, keys, vals, out_vals, out_st, n, engine, s, fp);
 }
 
+// A batch of up to kSmallMax requests (bt_small.cu), whole on `s`.  Taken with
+// the options that say how the general path works at their defaults, and
+// while no phases are recorded (it has none of the general path's).
+bool small_usable(const Handle* h, size_t n) {
+  return n <= kSmallMax && h->front_end == 1 && h->touch_sort == 2 && !h->prof && !h->vals_remote;
+}
+
+static int batch_small(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,
+                       uint8_t* out_st, size_t n, int engine, cudaStream_t s) {
+  Work& w = h->w;
+  const bool early = merge_usable(h, engine);
+  if (tree_join(h, s) != cudaSuccess || wait_vals(h, s) != 0) return -2;
+  const bool learned = batch_learned(h, h->batch_descent >= 0 ? h->batch_descent : h->descent, s);
+  if (small_front(h, keys, vals, ops, out_vals, out_st, n, early, s) != 0) return -2;
+  // the default plain lookups ride with the locates; every other form of them
+  // has a launch of its own
+  const bool ride = !learned && h->search_pairs == 2 && h->search_group == 4;
+  if (small_read(h, ride, early, out_vals, out_st, n, s) != 0) return -2;
+  cudaError_t e = cudaSuccess;
+  if (learned)
+    e = launch_learned_lookup(h, keys, w.f_list, &w.counts->n_lookup, n, out_vals, out_st, s, w.f_lk, true);
+  else if (!ride)
+    e = launch_search(h, keys, w.f_list, &w.counts->n_lookup, n, out_vals, out_st, s, w.f_lk);
+  if (e != cudaSuccess) return -2;
+  if (learned) learned_sample(h, s);
+  if (!early) {
+    if (delete_apply(h, n, s) != 0 ||
+        launch_stm(h, w.ukeys, w.uvals, nullptr, kOpInsert, w.ins_list, &w.counts->n_ins, n, w.uans, w.uans_st, s) !=
+            cudaSuccess)
+      return -2;
+    writeback_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w.v_a, w.pend, n, &w.counts->n_touch, w.uans,
+                                                                 w.uans_st, out_vals, out_st);
+    count_launch();
+    return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
+  }
+  if (small_write(h, out_vals, out_st, n, s) != 0 || answers_ready(h, s) != 0) return -2;
+  // a later call on any stream comes after this batch's writes
+  if (h->async_write) {
+    if (cudaEventRecord(h->tree_ev, s) != cudaSuccess) return -2;
+    h->tree_pending = true;
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
 static int front_stream_init(Handle* h) {
   if (h->front_stream) return 0;
   bool ok = cudaStreamCreateWithFlags(&h->front_stream, cudaStreamNonBlocking) == cudaSuccess &&
@@ -769,6 +819,7 @@ int batch_sorted(Handle* h, const uint64_t* keys, const uint64_t* vals, const ui
   if (n == 0) return 0;
   Work& w = h->w;
   if (n > w.cap || n > kIdxMask) return -6;
+  if (small_usable(h, n)) return batch_small(h, keys, vals, ops, out_vals, out_st, n, engine, s);
   if (h->front_end == 1) return batch_hashed(h, keys, vals, ops, out_vals, out_st, n, engine, s);
   if (tree_join(h, s) != cudaSuccess) return -2;
   const bool learned = batch_learned(h, h->batch_descent >= 0 ? h->batch_descent : h->descent, s);

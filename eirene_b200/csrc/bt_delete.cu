@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "bt_common.cuh"
+#include "bt_delete.cuh"
 #include "bt_internal.h"
 #include "bt_search.cuh"
 
@@ -28,7 +29,6 @@ namespace {
 
 constexpr int kG = 8;
 constexpr int kS = 32 / kG;
-constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 
 __global__ void __launch_bounds__(256) del_locate_kernel(DevTree t, const uint64_t* __restrict__ ukeys,
                                                          const uint32_t* __restrict__ del_list,
@@ -85,44 +85,8 @@ __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_
   const size_t n = *n_dev;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long removed = 0;
-  for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-    const uint32_t leaf = dleaf[i];
-    if (leaf == kNil || (i > 0 && dleaf[i - 1] == leaf)) continue;  // not the first entry of its leaf
-    // slots to remove: every found entry of this leaf (entries of a leaf are adjacent)
-    uint32_t gone = 0;
-    for (size_t j = i;; j += 32) {
-      const size_t x = j + lane;
-      const bool mine = x < n && dleaf[x] == leaf;
-      const uint32_t sl = mine ? dslot[x] : kNoSlot;
-      uint32_t bit = (mine && sl != kNoSlot) ? (1u << sl) : 0u;
-      bit = __reduce_or_sync(0xffffffffu, bit);
-      gone |= bit;
-      if (__ballot_sync(0xffffffffu, mine) != 0xffffffffu) break;
-    }
-    if (!gone) continue;
-    uint64_t* kr = t.keys + (size_t)leaf * 32;
-    uint64_t* vr = t.vals + (size_t)leaf * 32;
-    const uint64_t k = kr[lane];
-    const uint64_t v = vr[lane];
-    const uint64_t h = __shfl_sync(0xffffffffu, k, 31);
-    const uint32_t sz = hdr_size(h);
-    const bool keep = lane < sz && !((gone >> lane) & 1u);
-    const uint32_t keepm = __ballot_sync(0xffffffffu, keep);
-    const uint32_t nsz = __popc(keepm);
-    const uint32_t pos = __popc(keepm & ((1u << lane) - 1u));
-    __syncwarp();
-    if (keep) {
-      kr[pos] = k;
-      vr[pos] = v;
-    }
-    __syncwarp();
-    if (lane >= nsz && lane < 31) {
-      kr[lane] = kKeyMax;
-      vr[lane] = 0;
-    }
-    if (lane == 31) kr[31] = make_hdr(nsz, 0, hdr_version(h) + 1, hdr_epoch(h));
-    removed += sz - nsz;
-  }
+  for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps)
+    removed += del_apply_at(t, dleaf, dslot, i, n, lane);
   if (lane == 0 && removed) atomicAdd(&t.ctrl->n_keys, (unsigned long long)0 - removed);
 }
 

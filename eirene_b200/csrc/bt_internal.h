@@ -166,6 +166,10 @@ struct Work {
   uint64_t* lb_status = nullptr;
   uint32_t* lb_ctr = nullptr;
   uint32_t lb_epoch = 0;
+  // small batches (bt_small.cu)
+  void* s_tab = nullptr;          // hash table, every slot empty between batches
+  void* s_sums = nullptr;         // per block: its part of the segmented scan, its edge keys
+  uint32_t* s_write = nullptr;    // per block: totals of the write part's scans
   BatchSet alt;        // the second set (allocated by the first bt_execute_batches)
   bool alt_in = false; // Work's fields hold the second set
 };
@@ -473,6 +477,21 @@ int route_batch(Handle* h, const uint64_t* splitters, int n_shards, const uint64
                 uint32_t* out_perm, uint64_t* out_counts, cudaStream_t s);
 int unroute_results(Handle* h, const uint32_t* perm, const uint64_t* in_vals, const uint8_t* in_st, size_t n,
                     uint64_t* out_vals, uint8_t* out_st, cudaStream_t s);
+
+// ---- sorted batches of up to kSmallMax requests (bt_small.cu; the write part in bt_merge.cu) ----
+constexpr size_t kSmallMax = 65536;
+int small_prepare();
+int small_write_prepare();
+int small_alloc(Work* w);
+bool small_usable(const Handle* h, size_t n);
+// classification, sort, segmented scan: w.f_list/f_lk (lookups), w.v_a and w.pend (touched requests),
+// w.ukeys/uvals/ins_list/del_list and the counts; with ensure_root an empty tree gets its root leaf
+int small_front(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,
+                uint8_t* out_st, size_t n, bool ensure_root, cudaStream_t s);
+// reads of the tree: the plain lookups (gets), the locates of the DELETE keys and (locate_ins) INSERT keys
+int small_read(Handle* h, bool gets, bool locate_ins, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s);
+// writes: values, DELETE apply, grouping, reservation, write-back, leaf and inner merge
+int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s);
 
 // ---- sorted-merge batch (bt_batch.cu) ----
 int work_alloc(Work* w, size_t cap);

@@ -29,8 +29,10 @@
 
 #include "bt_block.cuh"
 #include "bt_common.cuh"
+#include "bt_delete.cuh"
 #include "bt_internal.h"
 #include "bt_search.cuh"
+#include "bt_small.cuh"
 
 namespace bt {
 
@@ -46,7 +48,8 @@ struct MergeCounts {
   uint32_t n_leaf_entries;
   uint32_t node_base;
   uint32_t cap_fail;
-  uint32_t pad[3];
+  uint32_t root_level;  // of the tree before the inner merge
+  uint32_t pad[2];
 };
 
 namespace {
@@ -109,24 +112,7 @@ __device__ __forceinline__ uint32_t count_less(const uint64_t* a, uint32_t n, ui
 }
 
 // ------------------------------------------------------------- root ----
-__global__ void merge_ensure_root_kernel(DevTree t) {
-  Ctrl* C = t.ctrl;
-  if (C->root != kNil) return;
-  const uint32_t id = atomicAdd(&C->n_nodes, 1u);
-  if (id >= t.cap) {
-    atomicOr(&C->error, kErrCapacity);
-    return;
-  }
-  for (int i = 0; i < 31; i++) {
-    t.keys[(size_t)id * 32 + i] = kKeyMax;
-    t.vals[(size_t)id * 32 + i] = 0;
-  }
-  t.vals[(size_t)id * 32 + 31] = kKeyMax;
-  t.keys[(size_t)id * 32 + 31] = make_hdr(0, 0, 0, C->epoch);
-  t.low[id] = 0;
-  C->root = id;
-  C->root_level = 0;
-}
+__global__ void merge_ensure_root_kernel(DevTree t) { ensure_root_leaf(t); }
 
 // ------------------------------------------------------------- locate ----
 template <int G>
@@ -345,8 +331,11 @@ __global__ void merge_leaf_count_kernel(DevTree t, uint32_t leaf_fill, const Mer
 // reserve the leaf pieces (and headroom for the inner levels) in one step;
 // all-or-nothing: on failure no leaf is touched and the new keys report
 // kNoCapacity.  entry_cap bounds the separator-entry buffers.
-__global__ void merge_alloc_kernel(DevTree t, MergeCounts* mc, uint32_t entry_cap) {
+__device__ __forceinline__ void reserve_pieces(const DevTree& t, MergeCounts* mc, uint32_t entry_cap) {
   const uint32_t T = mc->n_leaf_entries;
+  // the inner merge's blocks take the level from here: the block that rebuilds
+  // the root changes Ctrl::root_level while others may not have read it yet
+  mc->root_level = t.ctrl->root_level;
   const uint32_t need = T + T / 4 + 64;
   const uint32_t have = atomicAdd(&t.ctrl->n_nodes, 0u);
   if ((uint64_t)have + need > t.cap || T > entry_cap) {
@@ -357,6 +346,7 @@ __global__ void merge_alloc_kernel(DevTree t, MergeCounts* mc, uint32_t entry_ca
   mc->cap_fail = 0;
   mc->node_base = atomicAdd(&t.ctrl->n_nodes, T);
 }
+__global__ void merge_alloc_kernel(DevTree t, MergeCounts* mc, uint32_t entry_cap) { reserve_pieces(t, mc, entry_cap); }
 
 // a batch whose pieces did not fit answers kNoCapacity for all its new keys
 __global__ void merge_fail_mark_kernel(const MergeCounts* __restrict__ mc, const uint32_t* __restrict__ nq,
@@ -376,15 +366,15 @@ __global__ void merge_fail_mark_kernel(const MergeCounts* __restrict__ mc, const
 // one in the old row, the row put together in shared memory and written with
 // 16-byte stores.  A piece needs nothing of its neighbours: its right fence is
 // the key at merged position st + kc.
-template <int G>
+template <int N>  // groups of the block
 struct LeafSmem {
-  uint64_t old[256 / G][32];
-  __align__(16) uint64_t mk[256 / G][32];
-  __align__(16) uint64_t mv[256 / G][32];
+  uint64_t old[N][32];
+  __align__(16) uint64_t mk[N][32];
+  __align__(16) uint64_t mv[N][32];
 };
 
-template <int G>
-__device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<G>& sm, uint32_t grp, uint32_t g,
+template <int G, int N>
+__device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm, uint32_t grp, uint32_t g,
                                                uint32_t gmask, uint32_t nd, uint32_t c, uint32_t p, uint32_t m,
                                                uint32_t sz, uint64_t hdr, uint64_t fence,
                                                const uint64_t (&ok)[32 / G], const uint64_t (&ov)[32 / G],
@@ -449,8 +439,8 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<G>& sm
 
 // a touched leaf's row in registers and its keys in shared memory; kNc: no
 // other group writes the row in this launch (read-only path)
-template <int G, bool kNc>
-__device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<G>& sm, uint32_t grp, uint32_t g, uint32_t gmask,
+template <int G, bool kNc, int N>
+__device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<N>& sm, uint32_t grp, uint32_t g, uint32_t gmask,
                                          uint32_t leaf, uint64_t (&ok)[32 / G], uint64_t (&ov)[32 / G], uint64_t& hdr,
                                          uint64_t& fence) {
   constexpr int S = 32 / G;
@@ -472,7 +462,7 @@ __device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<G>& sm, uint
   __syncwarp(gmask);
 }
 
-// Leaf merge: a grid-stride loop of groups of G lanes over two kinds of items.
+// Leaf merge: a strided loop of the n_groups groups of G lanes over two kinds of items.
 //   segments  a touched leaf whose merged row fits: rewritten in place by its
 //             group.  Several leaves per warp keep more row loads in flight
 //             than a warp per leaf (the kernel is bound by the dependent chain
@@ -486,28 +476,20 @@ __device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<G>& sm, uint
 // the chip, a tree of 2^23 keys grown by seven such batches takes 6.5 ms, from
 // 81.2.  A launch of its own for the pieces cost batches that split nothing 4 %
 // (a 50/50 batch of 2^20), and so did 74 registers (three blocks an SM).
-template <int G>
-__global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* mc,
-                                                         const uint32_t* __restrict__ seg_start,
-                                                         const uint32_t* __restrict__ eoff,
-                                                         uint32_t* __restrict__ extra,
-                                                         const uint64_t* __restrict__ newk,
-                                                         const uint64_t* __restrict__ newv,
-                                                         const uint32_t* __restrict__ nq,
-                                                         const uint32_t* __restrict__ seg_leaf,
-                                                         MergeEntry* __restrict__ ent) {
+template <int G, int N, bool kNc>
+__device__ __forceinline__ void leaf_merge(const DevTree& t, uint32_t leaf_fill, const MergeCounts* mc,
+                                           const uint32_t* seg_start, const uint32_t* eoff, uint32_t* extra,
+                                           const uint64_t* newk, const uint64_t* newv, const uint32_t* nq,
+                                           const uint32_t* seg_leaf, MergeEntry* ent, LeafSmem<N>& sm, uint32_t gid,
+                                           uint32_t n_groups) {
   constexpr int S = 32 / G;
-  __shared__ LeafSmem<G> sm;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t g = lane % G;
   const uint32_t grp = threadIdx.x / G;
   const uint32_t gmask = group_mask<G>(lane);
   const uint32_t n_segs = mc->n_segs, n_ent = mc->n_leaf_entries;
-  if (mc->cap_fail) return;  // merge_fail_mark_kernel answered the new keys
   const uint32_t base = mc->node_base;
-  const uint32_t n_groups = (gridDim.x * blockDim.x) / G;
   unsigned long long added = 0, splits = 0;
-  const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   for (uint32_t s = gid; s < n_segs; s += n_groups) {
     uint32_t a, b;
     seg_bounds(mc, seg_start, s, a, b);
@@ -517,7 +499,7 @@ __global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t 
     // a leaf that splits (it has entries) is written by their groups
     if (eoff[s] != (s + 1 < n_segs ? eoff[s + 1] : n_ent)) continue;
     uint64_t ok[S], ov[S], hdr, fence;
-    leaf_row<G, true>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
+    leaf_row<G, kNc, N>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
     const uint32_t sz = hdr_size(hdr), m = sz + cnt;
 #pragma unroll
     for (int i = 0; i < S; i++) {
@@ -562,11 +544,11 @@ __global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t 
     seg_bounds(mc, seg_start, lo, a, b);
     const uint32_t cnt = b - a, leaf = seg_leaf[lo];
     uint64_t ok[S], ov[S], hdr, fence;
-    leaf_row<G, false>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
+    leaf_row<G, false, N>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
     const uint32_t sz = hdr_size(hdr), m = sz + cnt, p = ceil_div(m, leaf_fill);
     uint32_t c = e - eoff[lo] + 1, nd = base + e;
     for (;;) {
-      const uint64_t first = leaf_piece<G>(t, sm, grp, g, gmask, nd, c, p, m, sz, hdr, fence, ok, ov, newk + a,
+      const uint64_t first = leaf_piece<G, N>(t, sm, grp, g, gmask, nd, c, p, m, sz, hdr, fence, ok, ov, newk + a,
                                            newv + a, cnt);
       if (c == 0) break;
       uint32_t left = 0;
@@ -592,6 +574,22 @@ __global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t 
   }
 }
 
+template <int G>
+__global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* mc,
+                                                            const uint32_t* __restrict__ seg_start,
+                                                            const uint32_t* __restrict__ eoff,
+                                                            uint32_t* __restrict__ extra,
+                                                            const uint64_t* __restrict__ newk,
+                                                            const uint64_t* __restrict__ newv,
+                                                            const uint32_t* __restrict__ nq,
+                                                            const uint32_t* __restrict__ seg_leaf,
+                                                            MergeEntry* __restrict__ ent) {
+  __shared__ LeafSmem<256 / G> sm;
+  if (mc->cap_fail) return;  // merge_fail_mark_kernel answered the new keys
+  leaf_merge<G, 256 / G, true>(t, leaf_fill, mc, seg_start, eoff, extra, newk, newv, nq, seg_leaf, ent, sm,
+                               (blockIdx.x * blockDim.x + threadIdx.x) / G, (gridDim.x * blockDim.x) / G);
+}
+
 // ------------------------------------------------------------- inner ----
 // The separator entries are applied level by level by one cooperative grid
 // (all blocks resident), with a grid barrier between the steps of a level.
@@ -599,7 +597,6 @@ __global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t 
 // The barrier's wait is bounded: past kBarrierSpin it sets kErrSpin and every
 // block leaves.
 constexpr int kInnerThreads = 512;
-constexpr int kInnerWarps = kInnerThreads / 32;
 constexpr uint32_t kBarrierSpin = 1u << 24;
 
 struct InnerSync {
@@ -644,34 +641,52 @@ __device__ bool grid_sync(InnerSync* gs, uint32_t* err) {
   return s_ok != 0;
 }
 
-// grid-wide exclusive scan of f(i), i < n: out[i] and the total.  Each block
-// takes one contiguous chunk.  Contains two grid barriers.
-template <typename F>
-__device__ bool grid_scan_n(uint32_t n, F f, uint32_t* out, InnerSync* gs, uint32_t* err, uint32_t* ws,
-                            uint32_t* total) {
-  const uint32_t chunk = ceil_div(n, gridDim.x);
-  const uint32_t c0 = min(n, blockIdx.x * chunk), c1 = min(n, c0 + chunk);
+// The blocks that apply the entries: the cooperative grid, or the cluster of a
+// small batch (whose hardware barrier cannot fail).
+struct GridTeam {
+  InnerSync* gs;
+  uint32_t* err;
+  __device__ uint32_t rank() const { return blockIdx.x; }
+  __device__ uint32_t size() const { return gridDim.x; }
+  __device__ bool sync() const { return grid_sync(gs, err); }
+};
+struct ClusterTeam {
+  __device__ uint32_t rank() const { return cluster_rank(); }
+  __device__ uint32_t size() const { return cluster_size(); }
+  __device__ bool sync() const {
+    cluster_sync();
+    return true;
+  }
+};
+
+// exclusive scan over the team of f(i), i < n: out[i] and the total.  Each block
+// takes one contiguous chunk.  Contains two barriers.
+template <int NT, typename Team, typename F>
+__device__ bool team_scan(const Team& team, uint32_t n, F f, uint32_t* out, InnerSync* gs, uint32_t* ws,
+                          uint32_t* total) {
+  const uint32_t chunk = ceil_div(n, team.size());
+  const uint32_t c0 = min(n, team.rank() * chunk), c1 = min(n, c0 + chunk);
   uint32_t sum = 0;
-  for (uint32_t base = c0; base < c1; base += kInnerThreads) {
+  for (uint32_t base = c0; base < c1; base += NT) {
     const uint32_t i = base + threadIdx.x;
     uint32_t tot;
     blk_exclusive_sum(i < c1 ? f(i) : 0u, ws, &tot);
     sum += tot;
   }
-  if (threadIdx.x == 0) gs->partial[blockIdx.x] = sum;
-  if (!grid_sync(gs, err)) return false;
+  if (threadIdx.x == 0) gs->partial[team.rank()] = sum;
+  if (!team.sync()) return false;
   // this block's offset: sum of the lower blocks' partials
   uint32_t off = 0, all = 0;
-  for (uint32_t b = threadIdx.x; b < gridDim.x; b += kInnerThreads) {
+  for (uint32_t b = threadIdx.x; b < team.size(); b += NT) {
     const uint32_t v = gs->partial[b];
     all += v;
-    if (b < blockIdx.x) off += v;
+    if (b < team.rank()) off += v;
   }
   uint32_t t0, t1;
   blk_exclusive_sum(off, ws, &t0);
   blk_exclusive_sum(all, ws, &t1);
   uint32_t carry = t0;
-  for (uint32_t base = c0; base < c1; base += kInnerThreads) {
+  for (uint32_t base = c0; base < c1; base += NT) {
     const uint32_t i = base + threadIdx.x;
     const uint32_t v = i < c1 ? f(i) : 0u;
     uint32_t tot;
@@ -680,41 +695,41 @@ __device__ bool grid_scan_n(uint32_t n, F f, uint32_t* out, InnerSync* gs, uint3
     carry += tot;
   }
   *total = t1;
-  return grid_sync(gs, err);  // out[] complete before anyone reads it
+  return team.sync();  // out[] complete before anyone reads it
 }
 
-__global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, uint32_t inner_fill, uint32_t entry_cap,
-                                                                    MergeCounts* mc, InnerSync* gs,
-                                                                    MergeEntry* ea, MergeEntry* eb,
-                                                                    const uint32_t* __restrict__ path,
-                                                                    uint32_t* __restrict__ gstart,
-                                                                    uint32_t* __restrict__ goff,
-                                                                    uint32_t* __restrict__ kids_a,
-                                                                    uint32_t* __restrict__ kids_b) {
-  __shared__ uint32_t ws[32];
-  __shared__ uint32_t s_base;
-  __shared__ uint64_t s_keys[kInnerWarps][32];
-  if (mc->cap_fail) return;
+template <int NT>
+struct InnerSmem {
+  uint32_t ws[32];
+  uint32_t base;
+  uint64_t keys[NT / 32][32];
+};
+
+template <int NT, typename Team>
+__device__ __forceinline__ void inner_merge(const DevTree& t, uint32_t inner_fill, uint32_t entry_cap,
+                                            MergeCounts* mc, InnerSync* gs, MergeEntry* ea, MergeEntry* eb,
+                                            const uint32_t* path, uint32_t* gstart, uint32_t* goff, uint32_t* kids_a,
+                                            uint32_t* kids_b, const Team& team, InnerSmem<NT>& sm) {
+  constexpr int NW = NT / 32;
   Ctrl* C = t.ctrl;
-  uint32_t* err = &C->error;
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t gw = blockIdx.x * kInnerWarps + w, n_warps = gridDim.x * kInnerWarps;
+  const uint32_t gw = team.rank() * NW + w, n_warps = team.size() * NW;
   const uint32_t epoch = C->epoch;
   uint32_t n_e = mc->n_leaf_entries;
   MergeEntry* cur = ea;
   MergeEntry* nxt = eb;
   unsigned long long inner_new = 0, roots_new = 0;
+  const uint32_t root_level = mc->root_level;
   for (uint32_t lvl = 1; n_e > 0; lvl++) {
-    const uint32_t root_level = C->root_level;
     if (lvl > root_level) {
       // the root split: block 0 rebuilds upward from [root, pieces...] with the bulk rule
-      if (blockIdx.x != 0) break;
+      if (team.rank() != 0) break;
       uint32_t cnt = n_e + 1;
       if ((uint64_t)C->n_nodes + cnt > t.cap) {
         if (threadIdx.x == 0) atomicOr(&C->error, kErrCapacity);
         return;
       }
-      for (uint32_t i = threadIdx.x; i < cnt; i += kInnerThreads) kids_a[i] = i == 0 ? C->root : cur[i - 1].child;
+      for (uint32_t i = threadIdx.x; i < cnt; i += NT) kids_a[i] = i == 0 ? C->root : cur[i - 1].child;
       __syncthreads();
       uint32_t* ka = kids_a;
       uint32_t* kb = kids_b;
@@ -722,10 +737,10 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
       while (cnt > 1) {
         const uint32_t per = inner_fill + 1;
         const uint32_t nn = ceil_div(cnt, per);
-        if (threadIdx.x == 0) s_base = atomicAdd(&C->n_nodes, nn);
+        if (threadIdx.x == 0) sm.base = atomicAdd(&C->n_nodes, nn);
         __syncthreads();
-        const uint32_t nb = s_base;
-        for (uint32_t pidx = w; pidx < nn; pidx += kInnerWarps) {
+        const uint32_t nb = sm.base;
+        for (uint32_t pidx = w; pidx < nn; pidx += NW) {
           const uint32_t kc = piece_size(pidx, cnt, nn), cs = piece_start(pidx, cnt, nn);
           const uint32_t nd = nb + pidx;
           if (lane < 31) {
@@ -761,10 +776,10 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
     auto parent_of = [&](uint32_t i) { return path[(size_t)cur[i].rep * kPathLevels + lvl]; };
     auto is_head = [&](uint32_t i) -> uint32_t { return (i == 0 || parent_of(i) != parent_of(i - 1)) ? 1u : 0u; };
     uint32_t ng = 0;
-    if (!grid_scan_n(n_e, is_head, goff, gs, err, ws, &ng)) return;
-    for (uint32_t i = blockIdx.x * kInnerThreads + threadIdx.x; i < n_e; i += gridDim.x * kInnerThreads)
+    if (!team_scan<NT>(team, n_e, is_head, goff, gs, sm.ws, &ng)) return;
+    for (uint32_t i = team.rank() * NT + threadIdx.x; i < n_e; i += team.size() * NT)
       if (is_head(i)) gstart[goff[i]] = i;
-    if (!grid_sync(gs, err)) return;
+    if (!team.sync()) return;
     // pieces - 1 per group
     auto group_extra = [&](uint32_t gi) -> uint32_t {
       const uint32_t a = gstart[gi], b = gi + 1 < ng ? gstart[gi + 1] : n_e;
@@ -773,9 +788,9 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
       return tot <= (uint32_t)kMaxKeys ? 0u : ceil_div(tot + 1, inner_fill + 1) - 1;
     };
     uint32_t total = 0;
-    if (!grid_scan_n(ng, group_extra, goff, gs, err, ws, &total)) return;
+    if (!team_scan<NT>(team, ng, group_extra, goff, gs, sm.ws, &total)) return;
     // one thread checks the capacity and allocates; everyone reads the outcome
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (team.rank() == 0 && threadIdx.x == 0) {
       if (total > entry_cap || (uint64_t)C->n_nodes + total > t.cap) {
         // cannot happen with inner_fill >= 16 and the headroom reserved
         // above; stop before writing out of bounds and flag the error
@@ -786,7 +801,7 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
         gs->base = total ? atomicAdd(&C->n_nodes, total) : 0;
       }
     }
-    if (!grid_sync(gs, err)) return;
+    if (!team.sync()) return;
     if (gs->total) return;
     const uint32_t nb = gs->base;
     for (uint32_t gi = gw; gi < ng; gi += n_warps) {
@@ -797,7 +812,7 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
       const uint64_t pv = t.vals[(size_t)P * 32 + lane];
       const uint64_t h = __shfl_sync(kFull, pk, 31);
       const uint32_t sz = hdr_size(h);
-      s_keys[w][lane] = lane < sz ? pk : kKeyMax;
+      sm.keys[w][lane] = lane < sz ? pk : kKeyMax;
       const uint64_t child0 = __shfl_sync(kFull, pv, 0);
       __syncwarp();
       const uint32_t tot = sz + cnt;
@@ -838,7 +853,7 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
       __syncwarp();
       for (uint32_t j = lane; j < cnt; j += 32) {
         const MergeEntry e = cur[a + j];
-        place(j + count_less(s_keys[w], sz, e.key), e.key, e.child);
+        place(j + count_less(sm.keys[w], sz, e.key), e.key, e.child);
       }
       __syncwarp();
       for (uint32_t c = 0; c < q; c++) {
@@ -855,20 +870,195 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
       }
       __syncwarp();
     }
-    if (blockIdx.x == 0) inner_new += total;
-    if (!grid_sync(gs, err)) return;  // this level's nodes and the next entries are written
+    if (team.rank() == 0) inner_new += total;
+    if (!team.sync()) return;  // this level's nodes and the next entries are written
     n_e = total;
     MergeEntry* tmp = cur;
     cur = nxt;
     nxt = tmp;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && (inner_new | roots_new)) {
+  if (team.rank() == 0 && threadIdx.x == 0 && (inner_new | roots_new)) {
     atomicAdd(&C->inner_splits, inner_new + roots_new);
     atomicAdd(&C->new_roots, roots_new);
   }
 }
 
-inline unsigned nblk(size_t n, int per) { return (unsigned)((n + per - 1) / per); }
+__global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, uint32_t inner_fill, uint32_t entry_cap,
+                                                                    MergeCounts* mc, InnerSync* gs,
+                                                                    MergeEntry* ea, MergeEntry* eb,
+                                                                    const uint32_t* __restrict__ path,
+                                                                    uint32_t* __restrict__ gstart,
+                                                                    uint32_t* __restrict__ goff,
+                                                                    uint32_t* __restrict__ kids_a,
+                                                                    uint32_t* __restrict__ kids_b) {
+  __shared__ InnerSmem<kInnerThreads> sm;
+  if (mc->cap_fail) return;
+  inner_merge<kInnerThreads>(t, inner_fill, entry_cap, mc, gs, ea, eb, path, gstart, goff, kids_a, kids_b,
+                             GridTeam{gs, &t.ctrl->error}, sm);
+}
+
+// ------------------------------------------------- small batches: write ----
+// Everything of a small batch (bt_small.cu) that writes the tree, in one
+// cluster: the phases of the general path (merge_update .. merge_fail_mark,
+// writeback_kernel, merge_leaf, merge_inner) with a cluster barrier between
+// them.  Leaving the leaf and inner merge to their launches over the whole chip
+// costs 9 us more a batch up to 4096 requests, and gains only at 65,536 (254
+// against 271 us, all INSERTs).
+struct WriteSmem {
+  union {
+    LeafSmem<kSmallThreads / 8> leaf;
+    InnerSmem<kSmallThreads> inner;
+  };
+  uint32_t ws[32];
+  uint32_t before, total;
+};
+
+struct SmallWrite {
+  const BatchCounts* counts;
+  MergeCounts* mc;
+  InnerSync* gs;
+  const uint64_t *ukeys, *uvals, *uans;
+  uint8_t* uans_st;
+  const uint32_t *ins_list, *pend, *sv, *dleaf, *dslot, *path;
+  const uint64_t* vpos;
+  uint32_t *isnew, *pos, *leaf, *nq, *nleaf, *seg;
+  uint64_t *newk, *newv;
+  MergeEntry *ea, *eb;
+  uint32_t* sums;  // three sets of 16 block totals
+  uint32_t leaf_fill, inner_fill, entry_cap;
+};
+
+// exclusive prefix of v over the threads of the cluster and the total; one
+// cluster barrier (sums: a set of its own per use)
+__device__ __forceinline__ uint32_t cluster_scan(uint32_t v, uint32_t* sums, WriteSmem& S, uint32_t* total) {
+  uint32_t tot;
+  const uint32_t ex = blk_exclusive_sum(v, S.ws, &tot);
+  if (threadIdx.x == 0) sums[cluster_rank()] = tot;
+  cluster_sync();
+  if (threadIdx.x < 32) {
+    const uint32_t x = threadIdx.x < cluster_size() ? __ldcg(sums + threadIdx.x) : 0u;
+    const uint32_t before = __reduce_add_sync(kFull, threadIdx.x < cluster_rank() ? x : 0u);
+    const uint32_t all = __reduce_add_sync(kFull, x);
+    if (threadIdx.x == 0) {
+      S.before = before;
+      S.total = all;
+    }
+  }
+  __syncthreads();
+  const uint32_t r = S.before + ex;
+  *total = S.total;
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
+                                                                       uint8_t* out_st) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  WriteSmem& S = *reinterpret_cast<WriteSmem*>(raw);
+  const uint32_t rank = cluster_rank(), C = cluster_size();
+  const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
+  const uint32_t n_ins = a.counts->n_ins, n_del = a.counts->n_del, n_touch = a.counts->n_touch;
+  MergeCounts* mc = a.mc;
+  // new values of the keys found in the tree, then the DELETE keys (which move values)
+  for (uint32_t q = gt; q < n_ins; q += nt) {
+    const uint64_t p = a.vpos[q];
+    if (p != kNoPos) t.vals[p] = a.uvals[a.ins_list[q]];
+  }
+  if (n_del) {
+    cluster_sync();
+    uint32_t removed = 0;
+    for (uint32_t i = gt >> 5; i < n_del; i += nt >> 5)
+      removed += del_apply_at(t, a.dleaf, a.dslot, i, n_del, threadIdx.x & 31);
+    if ((threadIdx.x & 31) == 0 && removed) atomicAdd(&t.ctrl->n_keys, (unsigned long long)0 - removed);
+  }
+  // this thread's four consecutive items of n spread over the cluster
+  auto mine = [&](uint32_t n, uint32_t& i0, uint32_t& i1) {
+    const uint32_t per = (ceil_div(n, C) + 3u) & ~3u;
+    i0 = min(n, rank * per + threadIdx.x * 4);
+    i1 = min(min(n, (rank + 1) * per), i0 + 4);
+    if (i1 < i0) i1 = i0;
+  };
+  uint32_t n_new = 0, n_segs = 0, n_ent = 0;
+  if (n_ins) {
+    // the new keys, compacted
+    uint32_t i0, i1, v = 0;
+    mine(n_ins, i0, i1);
+    for (uint32_t i = i0; i < i1; i++) v += a.isnew[i];
+    uint32_t p = cluster_scan(v, a.sums, S, &n_new);
+    for (uint32_t i = i0; i < i1; i++) {
+      if (!a.isnew[i]) continue;
+      const uint32_t u = a.ins_list[i];
+      a.newk[p] = a.ukeys[u];
+      a.newv[p] = a.uvals[u];
+      a.nq[p] = i;
+      a.nleaf[p] = a.leaf[i];
+      p++;
+    }
+  }
+  if (n_new) {
+    cluster_sync();
+    // runs of new keys that share a leaf
+    uint32_t i0, i1, v = 0, heads = 0;
+    mine(n_new, i0, i1);
+    uint32_t lf[4];
+    for (uint32_t i = i0; i < i1; i++) {
+      lf[i - i0] = __ldcg(a.nleaf + i);
+      const bool h = i == 0 || (i > i0 ? lf[i - i0 - 1] : __ldcg(a.nleaf + i - 1)) != lf[i - i0];
+      heads |= (h ? 1u : 0u) << (i - i0);
+      v += h ? 1u : 0u;
+    }
+    uint32_t p = cluster_scan(v, a.sums + 16, S, &n_segs);
+    for (uint32_t i = i0; i < i1; i++)
+      if ((heads >> (i - i0)) & 1u) {
+        a.seg[p] = i;
+        a.leaf[p++] = lf[i - i0];
+      }
+    cluster_sync();
+    // new leaves per run
+    mine(n_segs, i0, i1);
+    uint32_t ex[4];
+    v = 0;
+    for (uint32_t i = i0; i < i1; i++) {
+      const uint32_t b = __ldcg(a.seg + i), e = i + 1 < n_segs ? __ldcg(a.seg + i + 1) : n_new;
+      const uint32_t m = hdr_size(__ldcg(t.keys + (size_t)__ldcg(a.leaf + i) * 32 + 31)) + (e - b);
+      ex[i - i0] = m <= (uint32_t)kMaxKeys ? 0u : ceil_div(m, a.leaf_fill) - 1;
+      v += ex[i - i0];
+    }
+    p = cluster_scan(v, a.sums + 32, S, &n_ent);
+    for (uint32_t i = i0; i < i1; i++) {
+      a.isnew[i] = ex[i - i0];
+      a.pos[i] = p;
+      p += ex[i - i0];
+    }
+  }
+  if (gt == 0) {
+    mc->n_new = n_new;
+    mc->n_segs = n_segs;
+    mc->n_leaf_entries = n_ent;
+    reserve_pieces(t, mc, a.entry_cap);
+  }
+  cluster_sync();
+  const bool fail = __ldcg(&mc->cap_fail) != 0;
+  if (fail) {  // a full pool: the new keys are answered kNoCapacity
+    for (uint32_t i = gt; i < n_new; i += nt) a.uans_st[a.ins_list[a.nq[i]]] = kNoCapacity;
+    cluster_sync();
+  }
+  for (uint32_t i = gt; i < n_touch; i += nt) {
+    const uint32_t u = a.pend[i];
+    if (u == 0xFFFFFFFFu) continue;  // answered by the front part
+    const uint32_t r = a.sv[i] & 0x3FFFFFFFu;
+    out_vals[r] = a.uans[u];
+    out_st[r] = __ldcg(a.uans_st + u);
+  }
+  if (fail) return;
+  leaf_merge<8, kSmallThreads / 8, false>(t, a.leaf_fill, mc, a.seg, a.pos, a.isnew, a.newk, a.newv, a.nq, a.leaf,
+                                          a.ea, S.leaf, gt / 8, nt / 8);
+  if (n_ent == 0) return;
+  cluster_sync();
+  inner_merge<kSmallThreads>(t, a.inner_fill, a.entry_cap, mc, a.gs, a.ea, a.eb, a.path, a.seg, a.nleaf, a.nq, a.pos,
+                             ClusterTeam{}, S.inner);
+}
+
 
 }  // namespace
 
@@ -987,6 +1177,52 @@ int merge_write_phase(Handle* h, cudaStream_t s) {
   count_launch();
   if (launch_inner(h, entry_cap, mc, s) != cudaSuccess) return -2;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int small_write_prepare() {
+  cudaError_t e =
+      cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e == cudaSuccess ? 0 : -2;
+}
+
+int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s) {
+  Work& w = h->w;
+  SmallWrite a;
+  a.counts = w.counts;
+  a.mc = reinterpret_cast<MergeCounts*>(w.m_counts);
+  a.gs = reinterpret_cast<InnerSync*>(w.m_sync);
+  a.ukeys = w.ukeys;
+  a.uvals = w.uvals;
+  a.uans = w.uans;
+  a.uans_st = w.uans_st;
+  a.ins_list = w.ins_list;
+  a.pend = w.pend;
+  a.sv = w.v_a;
+  a.dleaf = w.d_leaf;
+  a.dslot = w.d_slot;
+  a.path = w.m_path;
+  a.vpos = w.m_vpos;
+  a.isnew = w.m_isnew;
+  a.pos = w.m_pos;
+  a.leaf = w.m_leaf;
+  a.nq = w.m_nq;
+  a.nleaf = w.m_nleaf;
+  a.seg = w.m_seg;
+  a.newk = w.m_newk;
+  a.newv = w.m_newv;
+  a.ea = reinterpret_cast<MergeEntry*>(w.m_ent_a);
+  a.eb = reinterpret_cast<MergeEntry*>(w.m_ent_b);
+  a.sums = w.s_write;
+  a.leaf_fill = h->leaf_fill;
+  a.inner_fill = h->inner_fill;
+  a.entry_cap = (uint32_t)w.cap;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  small_config(cfg, at, small_cluster(n), sizeof(WriteSmem), s);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, small_write_kernel, h->tree, a, out_vals, out_st);
+  count_launch();
+  return e == cudaSuccess ? 0 : -2;
 }
 
 int merge_engine(Handle* h, size_t n_upper, cudaStream_t s) {

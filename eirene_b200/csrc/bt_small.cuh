@@ -1,0 +1,104 @@
+// Shared by the kernels of the small sorted batches (bt_small.cu, and the write
+// part in bt_merge.cu): sizes, cluster barrier, launch shape, argument blocks.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "bt_common.cuh"
+#include "bt_internal.h"
+
+namespace bt {
+
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallItems = 4;  // requests (and sorted pairs, and new keys) per thread
+// most requests per block of a cluster
+constexpr uint32_t kSmallPer = kSmallThreads * kSmallItems;
+static_assert(kSmallMax == 16 * kSmallPer, "the largest small batch fills sixteen blocks");
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// every thread of every block of the cluster; global writes before it are seen after it
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// an empty tree gets a leaf as its root (one thread)
+__device__ __forceinline__ void ensure_root_leaf(const DevTree& t) {
+  Ctrl* C = t.ctrl;
+  if (C->root != kNil) return;
+  const uint32_t id = atomicAdd(&C->n_nodes, 1u);
+  if (id >= t.cap) {
+    atomicOr(&C->error, kErrCapacity);
+    return;
+  }
+  for (int i = 0; i < 31; i++) {
+    t.keys[(size_t)id * 32 + i] = kKeyMax;
+    t.vals[(size_t)id * 32 + i] = 0;
+  }
+  t.vals[(size_t)id * 32 + 31] = kKeyMax;
+  t.keys[(size_t)id * 32 + 31] = make_hdr(0, 0, 0, C->epoch);
+  t.low[id] = 0;
+  C->root = id;
+  C->root_level = 0;
+}
+
+struct SmallFront {
+  BatchCounts* counts;
+  uint64_t* tk;
+  uint32_t* tv;
+  uint32_t* list;
+  uint64_t* lk;
+  uint64_t *k_a, *k_b;
+  uint32_t *v_a, *v_b;
+  uint64_t *ukeys, *uvals;
+  uint32_t *ins_list, *del_list, *pend;
+  void* sums;      // per block: its part of the scan
+  uint64_t* edge;  // per block: its first and last key
+};
+
+struct SmallRead {
+  const BatchCounts* counts;
+  const uint32_t* list;
+  const uint64_t* lk;
+  const uint64_t* ukeys;
+  const uint32_t *ins_list, *del_list;
+  uint32_t *path, *mleaf, *isnew;
+  uint64_t* vpos;
+  uint32_t *dleaf, *dslot;
+  uint64_t* uans;
+  uint8_t* uans_st;
+  int locate_ins;  // 0: the STM kernel inserts
+};
+
+// Blocks of the cluster for n requests: one per 128, up to sixteen.  A block's
+// leaf merges are what costs in a write-heavy batch, and the barrier of a
+// larger cluster costs little (us a batch of 2048 / 4096 all-INSERT requests
+// with one block per 4096: 126 / 224, per 1024: 90 / 95, per 128: 59 / 69; a
+// 95/5 batch of 4096: 52, 43, 43).
+inline unsigned small_cluster(size_t n) {
+  unsigned c = 1;
+  while ((size_t)c * 128 < n && c < 16) c <<= 1;
+  return c;
+}
+
+inline void small_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned C, size_t smem, cudaStream_t s) {
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+
+}  // namespace bt
