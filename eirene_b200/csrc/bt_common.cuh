@@ -89,10 +89,28 @@ struct DevTree {
   uint32_t cap;  // node capacity
   // [cap][32] high 32 bits of an inner node's separators (slot 31 unused):
   // the batch lookups compare these first and read the full keys of a row
-  // only when a prefix equals the key's.  Kept by the merge engine's inner
-  // merge; rebuilt from the rows after other writers (Handle::pfx_valid).
+  // only when a prefix equals the key's.
   uint32_t* pfx;
+  // [cap][32] bytes of a leaf: key_fp of the key in each slot (0: empty), and
+  // in byte 31 how often the leaf has split (kSplitMany: that often or more).
+  // A lookup reads this one 32-byte sector instead of the 256-byte key row,
+  // then only the key and the value of the slots whose byte matches.
+  // Every writer keeps both tables (a loaded pool image has them rebuilt,
+  // Handle::pfx_valid); only kernels that run without a writer read them.
+  uint8_t* fp;
 };
+
+constexpr uint32_t kSplitMany = 255;
+
+// fingerprint of a key, 1 .. 255: the top byte of a multiplicative hash of its
+// two halves (Knuth's golden-ratio multiplier and another odd constant).  Keys
+// of one leaf are neighbours, so its low bits have to spread over the byte.
+__host__ __device__ __forceinline__ uint32_t key_fp(uint64_t key) {
+  const uint32_t h = (uint32_t)key * 0x9E3779B1u + (uint32_t)(key >> 32) * 0x85EBCA77u;
+  const uint32_t f = h >> 24;
+  return f ? f : 1u;
+}
+__device__ __forceinline__ uint8_t slot_fp(uint64_t key) { return key == kKeyMax ? (uint8_t)0 : (uint8_t)key_fp(key); }
 
 // ---- memory-order helpers --------------------------------------------------
 __device__ __forceinline__ uint64_t ld_acquire(const uint64_t* p) {

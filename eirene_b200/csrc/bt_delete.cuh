@@ -38,14 +38,17 @@ __device__ __forceinline__ uint32_t del_apply_at(const DevTree& t, const uint32_
   const uint32_t nsz = __popc(keepm);
   const uint32_t pos = __popc(keepm & ((1u << lane) - 1u));
   __syncwarp();
+  uint8_t* fr = t.fp + (size_t)leaf * 32;
   if (keep) {
     kr[pos] = k;
     vr[pos] = v;
+    fr[pos] = slot_fp(k);
   }
   __syncwarp();
   if (lane >= nsz && lane < 31) {
     kr[lane] = kKeyMax;
     vr[lane] = 0;
+    fr[lane] = 0;
   }
   if (lane == 31) kr[31] = make_hdr(nsz, 0, hdr_version(h) + 1, hdr_epoch(h));
   return sz - nsz;

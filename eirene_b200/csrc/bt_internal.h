@@ -271,7 +271,7 @@ struct Handle {
   int front_end = 1;         // sorted batches: 1 = hash front end (sort only INSERT-coupled requests), 0 = full sort
   int top_cache = 1;         // unsorted searches descend the upper levels from shared memory
   int search_pairs = 2;      // unsorted searches: 2 pairs of requests per lane group, child ids only; 1 pairs; 0 single
-  bool pfx_valid = false;    // tree.pfx matches every inner row (false after bulk builds and STM writers)
+  bool pfx_valid = false;    // tree.pfx and tree.fp match the rows (false after a loaded pool image)
   int use_pfx = 1;           // paired searches compare the separators' 32-bit prefixes first
   void* top = nullptr;       // top cache (kTopNodes nodes) + TopInfo
   TopInfo* top_info = nullptr;
@@ -355,7 +355,7 @@ void prof_mark(Handle* h, int which, cudaStream_t s);
 void prof_set_layout(Handle* h, int layout);
 
 // ---- tree kernels (bt_tree.cu) ----
-// make tree.pfx match every inner row (a rebuild when stale), stream ordered
+// make tree.pfx and tree.fp match the rows (a rebuild when stale), stream ordered
 cudaError_t ensure_pfx(Handle* h, cudaStream_t s);
 cudaError_t tree_reset(Handle* h, cudaStream_t s);
 // header word of node rows [first, last) set to 0 (epoch 0: never written)
@@ -375,6 +375,11 @@ struct BuildScratch {
 };
 int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s,
                             const BuildScratch& sc);
+// Plain lookups of at least so many requests take the warp form, fewer the
+// pairs of requests per four lanes: those have the shorter chain while one
+// resident wave holds every request (us a call on 2^20 keys, warp / pairs:
+// 100 requests 8.3 / 6.3, 30,000: 10.4 / 8.3, 100,000: 10.4 / 13.5, 10^6: 53 / 89).
+constexpr size_t kWarpLookupMin = 65536;
 // ckeys (nullable): the keys of the listed requests compacted, ckeys[q] =
 // qkeys[list[q]], read instead of the indirection where the kernel supports it
 cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list, const uint32_t* n_dev, size_t n,

@@ -66,7 +66,7 @@ __global__ void leaf_table_kernel(DevTree t, const uint32_t* __restrict__ ids, s
   if (s < L) {
     const uint32_t id = ids[s];
     tab[s].low = t.low[id];
-    tab[s].id = id;
+    tab[s].id = (uint64_t)t.fp[(size_t)id * 32 + 31] << 32 | id;
   } else if (s == L) {
     tab[s].low = kKeyMax;
     tab[s].id = 0;
@@ -782,6 +782,119 @@ __global__ void __launch_bounds__(kPipeThreads) learned_pipe_kernel(DevTree t, L
   }
 }
 
+// Learned lookup, one thread per request (mode 3 with 4 lanes, the default).
+// The chain of a lookup: request key -> segment line -> eight leaf-table
+// entries around the predicted slot -> the slot's node id (a hit in L1) -> the
+// leaf's fingerprint row -> the key and the value of the matching slots.  A key
+// that no slot holds is absent if the leaf has not split since the fit (its
+// split count is still the leaf table's), else if it is below the leaf's live
+// right fence; everything else joins the miss list, as in
+// learned_lookup_kernel.
+// Bound by the instructions issued before: with four lanes to a request and
+// shuffles under a mask per group (49 warp instructions a request, half of the
+// issue slots and of the unit that resolves the masks), 2^22 lookups on 2^24
+// keys took 325 us with DRAM at 60 % of its copy rate.  Here no lane waits for
+// another, nothing is exchanged, and a leaf costs its 32-byte fingerprint row
+// (in L2 for up to about 3 million leaves) and, for a key that is there, two
+// sectors, instead of a 256-byte row and one: 175 us.  What bounds it now is the
+// L1 data pipe (75 %), one pass per request and load.  Tried: the low fences in
+// an array of their own (two loads and an id from L2 instead of four and one
+// from L1: 185 us), two requests per thread (116 registers: 215 us), 7 or 8
+// blocks an SM (199 us).
+template <bool kCompact>
+__global__ void __launch_bounds__(kPipeThreads) learned_thread_kernel(DevTree t, LearnedDev M,
+                                                             const uint64_t* __restrict__ qkeys,
+                                                             const uint32_t* __restrict__ list,
+                                                             const uint32_t* __restrict__ n_dev, size_t n_host,
+                                                             uint64_t* __restrict__ out_vals,
+                                                             uint8_t* __restrict__ out_st,
+                                                             uint32_t* __restrict__ miss,
+                                                             uint32_t* __restrict__ n_miss,
+                                                             const uint64_t* __restrict__ ckeys) {
+  constexpr int W = 8;  // probe width, from an even entry: four 32-byte loads
+  __shared__ float4 hid[kHidden];  // w1, b1, w2 of each hidden unit
+  if (threadIdx.x < kHidden)
+    hid[threadIdx.x] = make_float4(M.params[threadIdx.x], M.params[kHidden + threadIdx.x],
+                                   M.params[2 * kHidden + threadIdx.x], M.params[3 * kHidden]);
+  __syncthreads();
+  const size_t n = n_dev ? (size_t)*n_dev : n_host;
+  if (gate_pass_all(M, qkeys, list, ckeys, n, miss, n_miss)) return;
+  const int L = (int)M.n_leaves;
+  // the table holds L + 1 entries (sentinel last); an even start may reach one past it
+  const int p_hi = L + 2 - W > 0 ? (L + 2 - W) & ~1 : 0;
+  const uint64_t keep = l2_keep(), stream = l2_stream();
+  uint32_t hits = 0, falls = 0, probe = 0;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
+    const uint32_t r = list ? __ldg(list + q) : (uint32_t)q;
+    const uint64_t key = kCompact ? __ldg(ckeys + q) : __ldg(qkeys + r);
+    // stage 1, in the training's order of operations (mlp_fwd)
+    const float x = norm_x(key, M.kmin, M.inv_range);
+    float y = hid[0].w;
+#pragma unroll 8
+    for (int j = 0; j < kHidden; j++) {
+      const float4 u = hid[j];
+      const float h = fmaf(u.x, x, u.y);
+      y = h > 0.f ? fmaf(u.z, h, y) : y;
+    }
+    const SegParam sp = load_seg(M.seg, seg_of_y(y, M.n_seg));
+    bool ok = key != kKeyMax && sp.a == sp.a;  // NaN: no usable line
+    const float pred = seg_predict(sp, key);
+    const int pc = (pred > 0.f) ? (pred < (float)(L - 1) ? __float2int_rn(pred) : L - 1) : 0;
+    int p0 = (pc - (W / 2 - 1)) & ~1;
+    p0 = p0 > p_hi ? p_hi : p0;
+    p0 = p0 < 0 ? 0 : p0;
+    uint32_t c = 0;
+    if (ok) {
+      // entries past the sentinel are the allocation's headroom: masked
+#pragma unroll
+      for (int e = 0; e < W; e += 2) {
+        uint64_t w[4];
+        ldg32_hint(M.tab + p0 + e, w, keep);
+        c += (w[0] <= key && p0 + e <= L) ? 1u : 0u;
+        c += (w[2] <= key && p0 + e + 1 <= L) ? 1u : 0u;
+      }
+    }
+    // bracketed: tab[slot].low <= key < tab[slot + 1].low inside the probe
+    ok = ok && c >= 1 && c < (uint32_t)W;
+    uint64_t val = 0;
+    bool found = false;
+    const int slot = p0 + (int)c - 1;
+    if (ok) {
+      const uint64_t id = ldg_hint(&M.tab[slot].id, keep);
+      const uint32_t leaf = (uint32_t)id;
+      uint64_t row[4];
+      ldg32_hint(t.fp + (size_t)leaf * 32, row, keep);
+      const uint32_t splits = (uint32_t)(row[3] >> 56);
+      const bool moved = splits != (uint32_t)(id >> 32) || splits == kSplitMany;
+      uint64_t fence = kKeyMax;
+      if (moved) fence = ldg_hint(t.vals + (size_t)leaf * 32 + 31, stream);
+      found = leaf_pick(t, leaf, key, fp_match(row, key_fp(key)), stream, val);
+      ok = found || key < fence;
+    }
+    if (key == kKeyMax) {
+      out_vals[r] = 0;
+      out_st[r] = kRejected;
+    } else if (ok) {
+      out_vals[r] = val;
+      out_st[r] = found ? kFound : kAbsent;
+      hits++;
+      probe += (uint32_t)(pc > slot ? pc - slot : slot - pc);
+    } else {
+      falls++;
+      append_miss(miss, M.miss_keys, n_miss, r, key);
+    }
+  }
+  hits = __reduce_add_sync(0xffffffffu, hits);
+  falls = __reduce_add_sync(0xffffffffu, falls);
+  probe = __reduce_add_sync(0xffffffffu, probe);
+  if ((threadIdx.x & 31) == 0 && (hits | falls)) {
+    atomicAdd(&t.ctrl->learned_hits, (unsigned long long)hits);
+    atomicAdd(&t.ctrl->learned_fallbacks, (unsigned long long)falls);
+    atomicAdd(&t.ctrl->learned_probe_sum, (unsigned long long)probe);
+  }
+}
+
 inline unsigned nblk(size_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 }  // namespace
@@ -991,6 +1104,8 @@ int learned_retrain(Handle* h, cudaStream_t s, bool refit) {
   Learned& L = h->L;
   refit = refit && L.trained;
   L.valid = false;
+  // the leaf table takes the leaves' split counts: none may be rebuilt later
+  if (ensure_pfx(h, s) != cudaSuccess) return -2;
   uint32_t* ids = nullptr;
   size_t nl = 0;
   int rc = enumerate_leaves(h, s, &ids, &nl);
@@ -1120,6 +1235,32 @@ static LearnedDev dev_view(const Learned& L) {
   return M;
 }
 
+// the resident, grid-striding launch of `kfn` less the slots that
+// lookup_reserve (256-thread blocks) keeps for kernels beside it
+static size_t resident_blocks(Handle* h, const void* kfn, int threads, int& per) {
+  if (per == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, threads, 0) != cudaSuccess || per < 1))
+    per = 1;
+  const size_t resident = (size_t)h->sm_count * per;
+  const size_t reserve = (size_t)h->lookup_reserve * 256 / threads;
+  return resident > reserve + h->sm_count ? resident - reserve : (size_t)h->sm_count;
+}
+
+template <bool C>
+static cudaError_t thread_launch(Handle* h, const LearnedDev& M, const uint64_t* qkeys, const uint32_t* list,
+                                 const uint32_t* n_dev, size_t n, uint64_t* out_vals, uint8_t* out_st, cudaStream_t s,
+                                 const uint64_t* ckeys) {
+  static int per_sm[64] = {};
+  int none = 0;
+  const int dev = h->device;
+  const size_t cap = resident_blocks(h, (const void*)learned_thread_kernel<C>, kPipeThreads,
+                                     dev >= 0 && dev < 64 ? per_sm[dev] : none);
+  const size_t blocks = min((n + kPipeThreads - 1) / kPipeThreads, cap);
+  learned_thread_kernel<C><<<(unsigned)blocks, kPipeThreads, 0, s>>>(h->tree, M, qkeys, list, n_dev, n, out_vals,
+                                                                     out_st, h->L.miss, h->L.n_miss, ckeys);
+  count_launch();
+  return cudaGetLastError();
+}
+
 // R = 1 or 2: learned_lookup_kernel<G, R>; R = 0: learned_pipe_kernel<G, C>
 template <int G, int R, bool C>
 static cudaError_t lookup_launch(Handle* h, const LearnedDev& M, const uint64_t* qkeys, const uint32_t* list,
@@ -1128,20 +1269,10 @@ static cudaError_t lookup_launch(Handle* h, const LearnedDev& M, const uint64_t*
   const void* kfn =
       R == 0 ? (const void*)learned_pipe_kernel<G, C> : (const void*)learned_lookup_kernel<G, R ? R : 1>;
   const int threads = R == 0 ? kPipeThreads : 256;
-  // a resident, grid-striding launch that leaves `lookup_reserve` block slots
-  // free for kernels running beside it (the batch's overlapped locates)
   static int per_sm[64] = {};
+  int none = 0;
   const int dev = h->device;
-  int per = (dev >= 0 && dev < 64) ? per_sm[dev] : 0;
-  if (per == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, threads, 0) != cudaSuccess || per < 1)
-      per = 1;
-    if (dev >= 0 && dev < 64) per_sm[dev] = per;
-  }
-  const size_t resident = (size_t)h->sm_count * per;
-  // lookup_reserve counts 256-thread block slots
-  const size_t reserve = (size_t)h->lookup_reserve * 256 / threads;
-  const size_t cap = resident > reserve + h->sm_count ? resident - reserve : (size_t)h->sm_count;
+  const size_t cap = resident_blocks(h, kfn, threads, dev >= 0 && dev < 64 ? per_sm[dev] : none);
   // the pipelined form wants several requests per group to fill its rounds
   const size_t per_group = R == 0 ? 8 : R;
   size_t blocks = ((n + per_group - 1) / per_group * (size_t)G + threads - 1) / threads;
@@ -1188,7 +1319,9 @@ cudaError_t launch_learned_lookup(Handle* h, const uint64_t* qkeys, const uint32
   else if (G == 2) e = R == 3 ? BT_LL(2, 0) : BT_LL(2, 1);
   else if (G == 16) e = R == 3 ? BT_LL(16, 0) : BT_LL(16, 1);
   else if (G == 32) e = BT_LL(32, 1);
-  else e = R == 3 ? BT_LL(4, 0) : R == 2 ? BT_LL(4, 2) : BT_LL(4, 1);
+  else if (R == 3) e = ckeys ? thread_launch<true>(h, M, qkeys, list, n_dev, n, out_vals, out_st, s, ckeys)
+                            : thread_launch<false>(h, M, qkeys, list, n_dev, n, out_vals, out_st, s, nullptr);
+  else e = R == 2 ? BT_LL(4, 2) : BT_LL(4, 1);
 #undef BT_LL
   if (e != cudaSuccess) return e;
   // the misses: plain descent over the miss list (keys compacted beside it),

@@ -9,7 +9,7 @@ namespace bt {
 
 struct LeafEnt {
   uint64_t low;
-  uint64_t id;
+  uint64_t id;  // node id; high half: the leaf's split count (DevTree::fp, byte 31) at the fit
 };
 
 // Segment line, 16 B: predicted slot = a + slope * (key - base).  A segment

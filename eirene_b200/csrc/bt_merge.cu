@@ -72,6 +72,24 @@ __device__ __forceinline__ void load_row16(const uint64_t* p, uint64_t (&x)[S]) 
   }
 }
 
+// the fingerprints of a lane's four slots of leaf nd (G = 8); slot 31's byte,
+// the split count, is `splits` unless that is negative (then it stays)
+__device__ __forceinline__ void store_fp4(const DevTree& t, uint32_t nd, uint32_t g, const uint64_t (&k)[4],
+                                          int splits) {
+  uint8_t* p = t.fp + (size_t)nd * 32 + g * 4;
+  uint32_t w = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++) w |= (uint32_t)slot_fp(k[i]) << (8 * i);
+  if (g < 7) {
+    *reinterpret_cast<uint32_t*>(p) = w | (uint32_t)slot_fp(k[3]) << 24;
+  } else if (splits >= 0) {
+    *reinterpret_cast<uint32_t*>(p) = w | (uint32_t)splits << 24;
+  } else {
+    *reinterpret_cast<uint16_t*>(p) = (uint16_t)w;
+    p[2] = (uint8_t)(w >> 16);
+  }
+}
+
 template <int S>
 __device__ __forceinline__ void store_row16(uint64_t* p, const uint64_t (&x)[S]) {
 #pragma unroll
@@ -427,6 +445,13 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm
     wv[i] = slot < kc ? mv[slot] : 0;
   }
   const uint64_t first = mk[0];
+  static_assert(G == 8, "four slots per lane");
+  int splits = 0;
+  if (c == 0 && g == G - 1) {
+    splits = t.fp[(size_t)nd * 32 + 31];
+    splits = splits < (int)kSplitMany ? splits + 1 : splits;
+  }
+  store_fp4(t, nd, g, wk, splits);
   if (g == G - 1) {
     wk[S - 1] = make_hdr(kc, 0, c == 0 ? hdr_version(hdr) + 1 : 0, hdr_epoch(hdr));
     wv[S - 1] = rf;
@@ -524,6 +549,7 @@ __device__ __forceinline__ void leaf_merge(const DevTree& t, uint32_t leaf_fill,
       wk[i] = slot < m ? sm.mk[grp][slot] : kKeyMax;
       wv[i] = slot < m ? sm.mv[grp][slot] : 0;
     }
+    store_fp4(t, leaf, g, wk, -1);
     if (g == G - 1) {
       wk[S - 1] = make_hdr(m, 0, hdr_version(hdr) + 1, hdr_epoch(hdr));
       wv[S - 1] = fence;

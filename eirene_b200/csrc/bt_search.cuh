@@ -143,6 +143,147 @@ __device__ __forceinline__ uint32_t pfx_rank(const uint32_t (&p)[S], uint64_t ke
   return group_sum<G>(x, gmask);
 }
 
+// ---- leaf lookup by one thread (DevTree::fp) ----
+// 32 bytes in one load
+__device__ __forceinline__ void ldg32_hint(const void* p, uint64_t (&x)[4], uint64_t pol) {
+  asm("ld.global.nc.L2::cache_hint.v4.u64 {%0, %1, %2, %3}, [%4], %5;"
+      : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+      : "l"(p), "l"(pol));
+}
+
+// the slots of a fingerprint row whose byte equals q, as bits 0 .. 30
+__device__ __forceinline__ uint32_t fp_match(const uint64_t (&row)[4], uint32_t q) {
+  const uint32_t qq = q * 0x01010101u;
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const uint32_t x = (uint32_t)(row[i >> 1] >> (32 * (i & 1))) ^ qq;
+    // a byte's top bit set: the byte is zero (no carry leaves a byte)
+    const uint32_t z = ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) & 0x80808080u;
+    m |= ((z >> 7) * 0x10204080u >> 28) << (4 * i);
+  }
+  return m & 0x7fffffffu;
+}
+
+// The key in the matching slots m of leaf `node`: the first two candidates'
+// keys and values are loaded at once (a wrong first one: one lookup in ten;
+// a third one: one in 250).
+__device__ __forceinline__ bool leaf_pick(const DevTree& t, uint32_t node, uint64_t key, uint32_t m, uint64_t pol,
+                                          uint64_t& val) {
+  const uint64_t* kr = t.keys + (size_t)node * 32;
+  const uint64_t* vr = t.vals + (size_t)node * 32;
+  val = 0;
+  while (m) {
+    const uint32_t s0 = __ffs(m) - 1;
+    m &= m - 1;
+    const uint32_t s1 = m ? __ffs(m) - 1 : s0;
+    const uint64_t k0 = ldg_hint(kr + s0, pol), v0 = ldg_hint(vr + s0, pol);
+    uint64_t k1 = k0, v1 = v0;
+    if (s1 != s0) {
+      k1 = ldg_hint(kr + s1, pol);
+      v1 = ldg_hint(vr + s1, pol);
+    }
+    m &= m - 1;
+    if (k0 == key || k1 == key) {
+      val = k0 == key ? v0 : v1;
+      return true;
+    }
+  }
+  return false;
+}
+
+// ---- descent of 32 keys by one warp ----
+// Lane l owns key l and its node.  At each inner level the warp ranks the keys
+// eight at a time, four lanes to a key: a lane compares eight of the row's
+// separator prefixes by binary search in registers, the four turns' counts are
+// packed into one word (a byte each) and summed over the lanes together, and
+// the owner takes its byte and loads its child id.  All lanes stay in step
+// (the tree is of one height): full-mask shuffles, no divergence.  A prefix
+// equal to a key's (flagged in the byte's upper bits) makes the warp rank that
+// level with the full keys.
+constexpr uint32_t kEqBit = 0x20u;  // a lane's flag in its byte: four of them still fit
+
+// prefixes below kp among eight ascending ones, kEqBit added if one equals it
+__device__ __forceinline__ uint32_t rank8(const uint32_t (&p)[8], uint32_t kp) {
+  const bool c1 = p[3] < kp;
+  uint32_t ub = c1 ? p[7] : p[3];  // the smallest one seen that is not below kp (or p[7])
+  const uint32_t a = c1 ? p[5] : p[1], b0 = c1 ? p[4] : p[0], b1 = c1 ? p[6] : p[2];
+  const bool c2 = a < kp;
+  ub = c2 ? ub : a;
+  const uint32_t b = c2 ? b1 : b0;
+  const bool c3 = b < kp;
+  ub = c3 ? ub : b;
+  return (c1 ? 4u : 0u) + (c2 ? 2u : 0u) + (c3 ? 1u : 0u) + (p[7] < kp ? 1u : 0u) + (ub == kp ? kEqBit : 0u);
+}
+
+// every lane of the warp calls it, with any key; returns the lane's leaf
+__device__ __forceinline__ uint32_t warp_descend(const DevTree& t, uint32_t root, uint32_t root_level, uint64_t key) {
+  const uint32_t lane = threadIdx.x & 31, g = lane & 3u;
+  const uint64_t keep = l2_keep();
+  uint32_t kp[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) kp[j] = __shfl_sync(0xffffffffu, (uint32_t)(key >> 32), 8 * j + (lane >> 2));
+  uint32_t node = root;
+  for (uint32_t level = root_level; level > 0; level--) {
+    uint32_t sum = 0;
+    uint32_t p[4][8];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t nj = __shfl_sync(0xffffffffu, node, 8 * j + (lane >> 2));
+      // 32 bytes a lane: the row's line in one pass of the L1 data pipe (two
+      // 16-byte loads would take two)
+      uint64_t w[4];
+      ldg32_hint(t.pfx + (size_t)nj * 32 + g * 8, w, keep);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        p[j][2 * i] = (uint32_t)w[i];
+        p[j][2 * i + 1] = (uint32_t)(w[i] >> 32);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) sum += rank8(p[j], kp[j]) << (8 * j);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    const uint32_t mine = __shfl_sync(0xffffffffu, sum, (lane & 7u) * 4) >> (8 * (lane >> 3)) & 0xffu;
+    uint32_t cnt = mine & 31u;
+    if (__any_sync(0xffffffffu, mine >= kEqBit)) {
+      sum = 0;
+#pragma unroll 1
+      for (int j = 0; j < 4; j++) {
+        const uint32_t nj = __shfl_sync(0xffffffffu, node, 8 * j + (lane >> 2));
+        const uint64_t kj = __shfl_sync(0xffffffffu, key, 8 * j + (lane >> 2));
+        uint64_t k[8];
+        load_row_il<4>(t.keys + (size_t)nj * 32, g, k, keep);
+        if (g == 3) k[7] = kKeyMax;  // slot 31 holds the header
+        uint32_t c = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) c += (k[i] <= kj) ? 1u : 0u;
+        sum += c << (8 * j);
+      }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      cnt = __shfl_sync(0xffffffffu, sum, (lane & 7u) * 4) >> (8 * (lane >> 3)) & 0xffu;
+    }
+    node = (uint32_t)ldg_hint(t.vals + (size_t)node * 32 + cnt, keep);
+  }
+  return node;
+}
+
+// One lookup per lane, 32 by the warp (every lane calls it; `live` lanes get
+// an answer).  Descent as above, then the leaf's fingerprint row and the
+// candidates by the owner alone.
+__device__ __forceinline__ uint8_t warp_lookup(const DevTree& t, uint32_t root, uint32_t root_level, uint64_t key,
+                                               bool live, uint64_t& val) {
+  val = 0;
+  if (root == kNil) return key == kKeyMax ? kRejected : kAbsent;
+  const bool usable = live && key != kKeyMax;
+  const uint32_t leaf = warp_descend(t, root, root_level, usable ? key : 0);
+  if (!usable) return kRejected;
+  uint64_t row[4];
+  ldg32_hint(t.fp + (size_t)leaf * 32, row, l2_keep());
+  return leaf_pick(t, leaf, key, fp_match(row, key_fp(key)), l2_stream(), val) ? kFound : kAbsent;
+}
+
 // Look `key` up in leaf `node` (slots loaded by the group); returns the status
 // and the value (deferred 32 B load of the one matching slot).
 template <int G, bool kLeafVals>

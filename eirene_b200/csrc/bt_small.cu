@@ -587,8 +587,8 @@ __device__ __forceinline__ uint32_t locate_key(const DevTree& t, uint32_t root, 
 
 constexpr int kReadThreads = 256;
 constexpr int kLocG = 8;                                  // lanes per located key
-constexpr int kGetG = 4;                                  // lanes per pair of lookups
 constexpr uint32_t kLocPer = kReadThreads / kLocG;        // keys per block turn
+constexpr int kGetG = 4;                                  // lanes per pair of lookups (a few thousand: kWarpLookupMin)
 constexpr uint32_t kGetPer = 2 * kReadThreads / kGetG;
 
 // Blocks take turns of three kinds: 32 INSERT keys, 32 DELETE keys, or 128

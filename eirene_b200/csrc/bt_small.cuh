@@ -44,6 +44,7 @@ __device__ __forceinline__ void ensure_root_leaf(const DevTree& t) {
   }
   t.vals[(size_t)id * 32 + 31] = kKeyMax;
   t.keys[(size_t)id * 32 + 31] = make_hdr(0, 0, 0, C->epoch);
+  for (int i = 0; i < 32; i++) t.fp[(size_t)id * 32 + i] = 0;
   t.low[id] = 0;
   C->root = id;
   C->root_level = 0;

@@ -80,16 +80,28 @@ __device__ uint32_t alloc_nodes(const DevTree& t, uint32_t cnt) {
   return __shfl_sync(kFull, base, 0);
 }
 
-// lane-parallel row write; the header slot (keys[31]) is written only for new
-// nodes (write_hdr), existing nodes publish their header with a release store.
-__device__ __forceinline__ void write_row(const DevTree& t, uint32_t n, uint64_t k, uint64_t v, bool write_hdr,
-                                          uint64_t hdr) {
+// lane-parallel row write under the node's lock (or to a node no one can reach
+// yet), with the row's prefixes or fingerprints; the header slot (keys[31]) is
+// published afterwards with a release store.  A new leaf has never split;
+// rewriting an old one is its split.
+__device__ __forceinline__ void write_row(const DevTree& t, uint32_t n, uint64_t k, uint64_t v, uint32_t level,
+                                          bool fresh) {
   const uint32_t lane = lane_id();
   uint64_t* kr = t.keys + (size_t)n * 32;
   uint64_t* vr = t.vals + (size_t)n * 32;
   if (lane < 31) kr[lane] = k;
-  else if (write_hdr) kr[31] = hdr;
   vr[lane] = v;
+  if (level > 0) {
+    t.pfx[(size_t)n * 32 + lane] = lane < 31 ? (uint32_t)(k >> 32) : 0xffffffffu;
+  } else {
+    volatile uint8_t* f = t.fp + (size_t)n * 32 + lane;
+    uint32_t x = slot_fp(k);
+    if (lane == 31) {
+      x = fresh ? 0u : (uint32_t)*f;
+      if (!fresh && x < kSplitMany) x++;
+    }
+    *f = (uint8_t)x;
+  }
 }
 
 // Split commit shared by the leaf split and the early inner split.
@@ -121,20 +133,20 @@ __device__ int commit_split(const DevTree& t, uint32_t node, uint64_t h, uint64_
   }
   const uint32_t right = base;
   // new right node (unreachable until the parent / root is published)
-  write_row(t, right, rk, rv, false, 0);
+  write_row(t, right, rk, rv, level, true);
   if (lane == 0) t.low[right] = up;
-  write_row(t, node, lk, lv, false, 0);
+  write_row(t, node, lk, lv, level, false);
   uint32_t psize = 0;
   if (!new_root) {
     psize = hdr_size(ph);
     const uint64_t npk = lane < pslot ? pk : (lane == pslot ? up : upk);
     const uint64_t npv = lane <= pslot ? pv : (lane == pslot + 1 ? (uint64_t)right : upv);
-    write_row(t, parent, npk, npv, false, 0);
+    write_row(t, parent, npk, npv, level + 1, false);
   } else {
     const uint32_t nr = base + 1;
     const uint64_t nk = lane == 0 ? up : kKeyMax;
     const uint64_t nv = lane == 0 ? (uint64_t)node : (lane == 1 ? (uint64_t)right : 0);
-    write_row(t, nr, nk, nv, false, 0);
+    write_row(t, nr, nk, nv, level + 1, true);
     if (lane == 0) t.low[nr] = t.low[node];
   }
   // new nodes become valid with a release store of their header after their
@@ -187,6 +199,7 @@ __device__ int leaf_delete(const DevTree& t, uint32_t node, uint64_t h, uint64_t
     const bool last = lane + 1 == size;
     t.keys[(size_t)node * 32 + lane] = last ? kKeyMax : dk;
     t.vals[(size_t)node * 32 + lane] = last ? 0 : dv;
+    t.fp[(size_t)node * 32 + lane] = last ? (uint8_t)0 : slot_fp(dk);
   }
   __threadfence();
   __syncwarp();
@@ -230,7 +243,7 @@ __device__ int tx_attempt(const DevTree& t, const uint64_t key, const uint64_t v
       unlock_unchanged(t, kNil, 0, kNil, 0, true, rl);
       return TX_NOCAP;
     }
-    write_row(t, id, kKeyMax, lane == 31 ? kKeyMax : 0, false, 0);
+    write_row(t, id, kKeyMax, lane == 31 ? kKeyMax : 0, 0, true);
     if (lane == 0) t.low[id] = 0;
     __threadfence();
     __syncwarp();
@@ -329,6 +342,7 @@ __device__ int tx_attempt(const DevTree& t, const uint64_t key, const uint64_t v
     if (lane <= size && lane < 31) {
       t.keys[(size_t)node * 32 + lane] = nk;
       t.vals[(size_t)node * 32 + lane] = nv;
+      t.fp[(size_t)node * 32 + lane] = slot_fp(nk);
     }
     __threadfence();
     __syncwarp();
@@ -427,6 +441,7 @@ __device__ int fast_insert_locked(const DevTree& t, const uint32_t epoch, const 
   if (lane <= size && lane < 31) {
     t.keys[(size_t)node * 32 + lane] = nk;
     t.vals[(size_t)node * 32 + lane] = nv;
+    t.fp[(size_t)node * 32 + lane] = slot_fp(nk);
   }
   __threadfence();
   __syncwarp();
@@ -484,6 +499,7 @@ __device__ int fast_delete_locked(const DevTree& t, const uint32_t epoch, const 
     const bool last = lane + 1 == size;
     t.keys[(size_t)node * 32 + lane] = last ? kKeyMax : dk;
     t.vals[(size_t)node * 32 + lane] = last ? 0 : dv;
+    t.fp[(size_t)node * 32 + lane] = last ? (uint8_t)0 : slot_fp(dk);
   }
   __threadfence();
   __syncwarp();
@@ -985,7 +1001,6 @@ cudaError_t launch_serve(Handle* h, const ServeDev& S, cudaStream_t s) {
   const unsigned blocks = (unsigned)(h->sm_count * (h->device < 64 ? per_sm[h->device] : 2));
   LearnedDev lm{};
   const int use = learned_dev(h, &lm);
-  h->pfx_valid = false;  // STM writes inner rows without their prefixes
   serve_kernel<<<blocks, 256, 0, s>>>(h->tree, S, h->retry_limit, lm, use);
   count_launch();
   return cudaGetLastError();
@@ -1008,7 +1023,6 @@ cudaError_t launch_stm(Handle* h, const uint64_t* keys, const uint64_t* vals, co
   if (blocks > cap) blocks = cap;
   LearnedDev lm{};
   const int use = learned_dev(h, &lm);
-  h->pfx_valid = false;  // STM writes inner rows without their prefixes
   stm_kernel<<<(unsigned)blocks, threads, 0, s>>>(h->tree, keys, vals, ops, op_override, list, n_dev, n, out_vals,
                                                    out_st, h->retry_limit, lm, use, skip);
   count_launch();

@@ -70,6 +70,7 @@ __global__ void build_leaves_kernel(DevTree t, const uint64_t* __restrict__ uk, 
     kr[31] = make_hdr((uint32_t)k, 0, 0, epoch);
     vr[31] = (j + 1 < nl) ? uk[start + k] : kKeyMax;
   }
+  t.fp[j * 32 + lane] = lane < k ? slot_fp(uk[start + lane]) : (uint8_t)0;
   if (lane == 0) t.low[j] = j == 0 ? 0 : uk[start];
 }
 
@@ -86,8 +87,9 @@ __global__ void build_inner_kernel(DevTree t, uint32_t first_child, uint32_t n_c
   uint64_t* kr = t.keys + (size_t)id * 32;
   uint64_t* vr = t.vals + (size_t)id * 32;
   // key slot i (i < k-1) = low fence of child i+1
-  if (lane < 31) kr[lane] = (lane + 1 < k) ? t.low[c + lane + 1] : kKeyMax;
-  else kr[31] = make_hdr(k - 1, level, 0, epoch);
+  const uint64_t sep = (lane + 1 < k) ? t.low[c + lane + 1] : kKeyMax;
+  kr[lane] = lane < 31 ? sep : make_hdr(k - 1, level, 0, epoch);
+  t.pfx[(size_t)id * 32 + lane] = lane < 31 ? (uint32_t)(sep >> 32) : 0xffffffffu;
   vr[lane] = lane < k ? (uint64_t)(c + lane) : 0;
   if (lane == 0) t.low[id] = t.low[c];
 }
@@ -170,6 +172,36 @@ __global__ void __launch_bounds__(256) search2_kernel(DevTree t, const uint64_t*
         out_vals[rb] = ab;
         out_st[rb] = sb;
       }
+    }
+  }
+}
+
+// The default plain lookups (four lanes, child ids): a warp takes 32 requests
+// at a time (warp_lookup).  Four lanes to a request with two requests per
+// group, shuffles under a mask per group and a 256-byte leaf row issued 63 warp
+// instructions a request and took 384 us for 2^22 lookups on 2^24 keys (issue
+// 57 %, L1 data pipe 68 %); this form takes 228 us, bound by the L1 data pipe
+// (a pass for the row and one for the child id per request and level).
+__global__ void __launch_bounds__(256) search_warp_kernel(DevTree t, const uint64_t* __restrict__ qkeys,
+                                                          const uint32_t* __restrict__ list,
+                                                          const uint32_t* __restrict__ n_dev, size_t n_host,
+                                                          uint64_t* __restrict__ out_vals,
+                                                          uint8_t* __restrict__ out_st,
+                                                          const uint64_t* __restrict__ ckeys) {
+  const size_t n = n_dev ? (size_t)*n_dev : n_host;
+  const uint32_t root = t.ctrl->root, root_level = t.ctrl->root_level;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  // whole warps: the base index is the warp's
+  for (size_t b = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < n; b += stride) {
+    const size_t q = b + (threadIdx.x & 31u);
+    const bool live = q < n;
+    const uint32_t r = live && list ? __ldg(list + q) : (uint32_t)q;
+    const uint64_t key = live ? (ckeys ? __ldg(ckeys + q) : __ldg(qkeys + r)) : 0;
+    uint64_t val;
+    const uint8_t st = warp_lookup(t, root, root_level, key, live, val);
+    if (live) {
+      out_vals[r] = val;
+      out_st[r] = st;
     }
   }
 }
@@ -570,7 +602,7 @@ cudaError_t clear_headers(Handle* h, uint32_t first, uint32_t last, cudaStream_t
 }
 
 cudaError_t tree_reset(Handle* h, cudaStream_t s) {
-  h->pfx_valid = false;  // the bulk loader writes inner rows without prefixes
+  h->pfx_valid = true;  // no nodes: every writer from here on keeps the two tables
   // The epoch has 15 bits (1 .. 0x7fff; 0 marks never-written rows).  When
   // it comes round to 1 again, rows written by the trees of the last cycle
   // may still carry that number: clear every row's header first, so that a
@@ -751,8 +783,9 @@ cudaError_t launch_search_sorted(Handle* h, const uint64_t* qkeys, const uint32_
   return cudaGetLastError();
 }
 
-// Prefix rows of every inner node from its keys: one warp per 32 nodes reads
-// their headers (one sector each), then writes the rows of the inner ones.
+// Prefix rows of the inner nodes and fingerprint rows of the leaves from their
+// keys: one warp per 32 nodes reads their headers (one sector each), then
+// writes the rows one by one.
 __global__ void __launch_bounds__(256) pfx_rebuild_kernel(DevTree t) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t n_nodes = min(t.ctrl->n_nodes, t.cap);
@@ -760,12 +793,13 @@ __global__ void __launch_bounds__(256) pfx_rebuild_kernel(DevTree t) {
   for (uint32_t b = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; b < n_nodes; b += warps * 32) {
     const uint32_t mine = b + lane;
     const bool inner = mine < n_nodes && hdr_level(t.keys[(size_t)mine * 32 + 31]) > 0;
-    uint32_t todo = __ballot_sync(0xffffffffu, inner);
-    while (todo) {
-      const uint32_t nd = b + (uint32_t)(__ffs(todo) - 1);
-      todo &= todo - 1;
-      const uint64_t k = t.keys[(size_t)nd * 32 + lane];
-      t.pfx[(size_t)nd * 32 + lane] = lane < 31 ? (uint32_t)(k >> 32) : 0xffffffffu;
+    const uint32_t inners = __ballot_sync(0xffffffffu, inner);
+    const uint32_t m = min(32u, n_nodes - b);
+    for (uint32_t i = 0; i < m; i++) {
+      const size_t at = (size_t)(b + i) * 32 + lane;
+      const uint64_t k = t.keys[at];
+      if ((inners >> i) & 1u) t.pfx[at] = lane < 31 ? (uint32_t)(k >> 32) : 0xffffffffu;
+      else t.fp[at] = lane < 31 ? slot_fp(k) : (uint8_t)0;
     }
   }
 }
@@ -784,17 +818,27 @@ cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list
   if (h->search_pairs && (h->search_group == 8 || h->search_group == 4 || h->search_group == 16)) {
     const int threads = 256;
     const int G = h->search_group;
-    size_t blocks = ((n + 1) / 2 * (size_t)G + threads - 1) / threads;
+    const bool child = h->search_pairs == 2;
+    // the separators' prefixes and the leaves' fingerprints (child-id form only)
+    const int use_pfx = child && h->use_pfx ? 1 : 0;
+    if (use_pfx) {
+      const cudaError_t pe = ensure_pfx(h, s);
+      if (pe != cudaSuccess) return pe;
+    }
+    const bool warp = use_pfx && G == 4 && n >= kWarpLookupMin;
+    const size_t per_block = warp ? threads : 2 * threads / G;
+    size_t blocks = (n + per_block - 1) / per_block;
     size_t cap = (size_t)h->sm_count * 8 * 4;
     if (h->lookup_reserve > 0) {
       // a resident, grid-striding launch that leaves `lookup_reserve` block
       // slots free for kernels running beside it (the overlapped sort)
-      static int per_sm[64][3] = {};
-      const int gi = G == 4 ? 0 : G == 16 ? 2 : 1;
+      static int per_sm[64][4] = {};
+      const int gi = warp ? 3 : G == 4 ? 0 : G == 16 ? 2 : 1;
       const int dev = h->device;
       int per = (dev >= 0 && dev < 64) ? per_sm[dev][gi] : 0;
       if (per == 0) {
-        const void* k = G == 4 ? (const void*)search2_kernel<4, false, true>
+        const void* k = warp ? (const void*)search_warp_kernel
+                        : G == 4 ? (const void*)search2_kernel<4, false, true>
                         : G == 16 ? (const void*)search2_kernel<16, false, true>
                                   : (const void*)search2_kernel<8, false, true>;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, 0) != cudaSuccess || per < 1) per = 1;
@@ -805,12 +849,11 @@ cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list
     }
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    const bool child = h->search_pairs == 2;
-    // the separators' prefixes (child-id form only)
-    const int use_pfx = child && h->use_pfx ? 1 : 0;
-    if (use_pfx) {
-      const cudaError_t pe = ensure_pfx(h, s);
-      if (pe != cudaSuccess) return pe;
+    if (warp) {
+      search_warp_kernel<<<(unsigned)blocks, threads, 0, s>>>(h->tree, qkeys, list, n_dev, n, out_vals, out_st,
+                                                              list ? ckeys : nullptr);
+      count_launch();
+      return cudaGetLastError();
     }
 #define BT_S2(GG, CC) search2_kernel<GG, false, CC><<<(unsigned)blocks, threads, 0, s>>>(h->tree, qkeys, list, n_dev, n, out_vals, out_st, use_pfx, list ? ckeys : nullptr)
     if (G == 4) { if (child) BT_S2(4, true); else BT_S2(4, false); }
