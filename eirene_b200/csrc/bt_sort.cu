@@ -292,6 +292,10 @@ __global__ void __launch_bounds__(T) sort_onesweep_kernel(
     uint64_t key[kSortItems];
     uint32_t val[kSortItems];
     uint32_t rank[kSortItems];
+    // all loads first: between the rounds below, which hand counts on through
+    // shared memory, the compiler kept each round's loads behind the round
+    // before it (eight passes over 13,000 pairs, tiles of 256 threads: 96 -> 81 us;
+    // 2^19 and more: the same)
 #pragma unroll
     for (int r = 0; r < kSortItems; r++) {
       const size_t idx = warp_base + (size_t)r * 32 + lane;
@@ -299,6 +303,10 @@ __global__ void __launch_bounds__(T) sort_onesweep_kernel(
       key[r] = valid ? keys_in[idx] : 0;
       if (payload_mode == 0) val[r] = valid ? vals_in[idx] : 0;
       else val[r] = (uint32_t)idx | (ops && valid ? (op_code(ops[idx]) << 30) : 0u);
+    }
+#pragma unroll
+    for (int r = 0; r < kSortItems; r++) {
+      const bool valid = warp_base + (size_t)r * 32 + lane < n;
       const uint32_t d = valid ? digit_of(key[r], shift) : 0x1FFu;
       // lanes holding the same digit: AND of eight bit ballots (plus a validity bit)
       uint32_t peers = __ballot_sync(0xffffffffu, valid);
