@@ -171,6 +171,7 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   h.device = cfg.device;
   h.leaf_fill = cfg.leaf_fill;
   h.inner_fill = cfg.inner_fill;
+  h.inner_min = cfg.inner_fill;
   h.retry_limit = cfg.retry_limit ? cfg.retry_limit : (1u << 16);
   h.search_group = (int)cfg.search_group;
   h.L.seg_config = cfg.n_segments;
@@ -191,6 +192,7 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   ok = ok && cudaMemset(h.tree.low, 0, nodes * 8) == cudaSuccess;
   ok = ok && cudaMemset(h.tree.pfx, 0xff, nodes * 128) == cudaSuccess;
   ok = ok && cudaMemset(h.tree.fp, 0, nodes * 32) == cudaSuccess;
+  ok = ok && cudaMalloc(&h.geo, 256) == cudaSuccess && cudaMallocHost(&h.pin, 256) == cudaSuccess;
   ok = ok && bt::work_alloc(&h.w, cfg.max_batch) == 0;
   ok = ok && cudaStreamCreateWithFlags(&h.internal_stream, cudaStreamNonBlocking) == cudaSuccess;
   {
@@ -240,7 +242,10 @@ int bt_destroy(bt_handle* H) {
   cudaFree(h.enum_a);
   cudaFree(h.enum_b);
   cudaFree(h.enum_cnt);
-  cudaFree(h.enum_scan_scratch);
+  cudaFree(h.enum_lb);
+  cudaFree(h.geo);
+  if (h.pin) cudaFreeHost(h.pin);
+  if (h.build_pool) cudaMemPoolDestroy(h.build_pool);
   cudaFree(h.top);
   if (h.internal_stream) cudaStreamDestroy(h.internal_stream);
   if (h.hi_stream) cudaStreamDestroy(h.hi_stream);

@@ -256,6 +256,7 @@ struct Handle {
   DevTree tree{};
   uint32_t leaf_fill = 24;
   uint32_t inner_fill = 24;
+  uint32_t inner_min = 24;  // the inner fill that the handle was created with (bt_autotune_fill only raises it)
   uint32_t retry_limit = 1u << 16;
   int descent = 0;     // 0 plain, 1 learned
   uint32_t epoch = 0;  // tree epoch, bumped by every reset / bulk build
@@ -281,8 +282,13 @@ struct Handle {
   uint32_t* enum_a = nullptr;  // leaf enumeration buffers (node ids)
   uint32_t* enum_b = nullptr;
   uint32_t* enum_cnt = nullptr;
-  uint32_t* enum_scan_scratch = nullptr;
+  uint64_t* enum_lb = nullptr;  // look-back scan of the enumeration
+  size_t enum_lb_words = 0;
+  uint32_t enum_epoch = 0;
   size_t enum_cap = 0;
+  uint32_t* geo = nullptr;      // 256 bytes: the bulk build's geometry, the enumeration's counts
+  uint32_t* pin = nullptr;      // 256 bytes of page-locked memory: what the host reads back
+  cudaMemPool_t build_pool = nullptr;  // scratch of bulk builds of more than max_batch keys
   uint64_t level_counts[48] = {};  // filled by enumerate_leaves, leaf level first
   uint32_t n_levels = 0;
   cudaStream_t internal_stream = nullptr;

@@ -44,7 +44,7 @@ constexpr size_t kOffVb = kOffVa + up256(kStaticMaxKeys * 4);
 constexpr size_t kOffSort = kOffVb + up256(kStaticMaxKeys * 4);
 constexpr size_t kOffPos = kOffSort + up256(kSortWords * 4);
 constexpr size_t kOffUv = kOffPos + up256(kStaticMaxKeys * 4);
-constexpr size_t kOffTot = kOffUv + up256(kStaticMaxKeys * 8);
+constexpr size_t kOffTot = kOffUv + up256(kStaticMaxKeys * 8);  // 256 bytes: the build's geometry
 constexpr size_t kStaticBytes = kOffTot + 256;
 
 }  // namespace

@@ -35,70 +35,146 @@ __global__ void reset_kernel(Ctrl* c, uint32_t epoch) {
 }
 
 // ---------------------------------------------------------------- build ----
-__global__ void tail_flags_kernel(const uint64_t* __restrict__ sk, size_t n, uint32_t* __restrict__ flags) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) flags[i] = (i + 1 == n || sk[i + 1] != sk[i]) ? 1u : 0u;
+// The bulk loader reads nothing back until its end: how many distinct keys there
+// are, whether the last is the reserved one and how many nodes each level takes
+// is worked out on the device (BuildGeo), and the grids are sized for n distinct
+// keys.
+constexpr int kBuildLevels = 30;
+struct BuildGeo {
+  uint32_t m;       // distinct keys
+  uint32_t status;  // 0, or the kBuild* reason why the tree stays empty
+  uint32_t height, total;
+  uint32_t cnt[kBuildLevels];    // nodes per level, leaves first
+  uint32_t first[kBuildLevels];  // id of a level's first node
+};
+static_assert(sizeof(BuildGeo) <= 256, "the static build's scratch keeps 256 bytes for it");
+constexpr uint32_t kBuildCapacity = 4, kBuildReserved = 5;
+
+constexpr int kDedupeThreads = 1024;
+constexpr int kDedupeItems = 4;
+constexpr int kDedupeTile = kDedupeThreads * kDedupeItems;
+
+// the last pair of every run of equal keys stays (a repeated key's last value wins)
+__device__ __forceinline__ uint32_t tails_of(const uint64_t* __restrict__ sk, size_t n, size_t i0,
+                                             uint64_t (&k)[kDedupeItems + 1]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j <= kDedupeItems; j++) k[j] = i0 + j < n ? sk[i0 + j] : 0;
+#pragma unroll
+  for (int j = 0; j < kDedupeItems; j++)
+    if (i0 + j < n && (i0 + j + 1 == n || k[j + 1] != k[j])) m |= 1u << j;
+  return m;
 }
 
-__global__ void dedupe_kernel(const uint64_t* __restrict__ sk, const uint32_t* __restrict__ sidx,
-                              const uint64_t* __restrict__ vals, const uint32_t* __restrict__ flags,
-                              const uint32_t* __restrict__ pos, size_t n, uint64_t* __restrict__ uk,
-                              uint64_t* __restrict__ uv) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && flags[i]) {
-    uint32_t p = pos[i];
-    uk[p] = sk[i];
-    uv[p] = vals[sidx[i]];
+__global__ void __launch_bounds__(kDedupeThreads) tail_count_kernel(const uint64_t* __restrict__ sk, size_t n,
+                                                                    uint32_t* __restrict__ tile) {
+  __shared__ uint32_t ws[32];
+  uint64_t k[kDedupeItems + 1];
+  uint32_t total;
+  blk_exclusive_sum(__popc(tails_of(sk, n, (size_t)blockIdx.x * kDedupeTile + threadIdx.x * kDedupeItems, k)), ws,
+                    &total);
+  if (threadIdx.x == 0) tile[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kDedupeThreads) dedupe_kernel(const uint64_t* __restrict__ sk,
+                                                                const uint32_t* __restrict__ sidx,
+                                                                const uint64_t* __restrict__ vals, size_t n,
+                                                                const uint32_t* __restrict__ tile,
+                                                                uint64_t* __restrict__ uk, uint64_t* __restrict__ uv) {
+  __shared__ uint32_t ws[32];
+  const size_t i0 = (size_t)blockIdx.x * kDedupeTile + threadIdx.x * kDedupeItems;
+  uint64_t k[kDedupeItems + 1];
+  const uint32_t m = tails_of(sk, n, i0, k);
+  uint32_t p = tile[blockIdx.x] + blk_exclusive_sum(__popc(m), ws, nullptr);
+#pragma unroll
+  for (int j = 0; j < kDedupeItems; j++)
+    if ((m >> j) & 1u) {
+      uk[p] = k[j];
+      uv[p++] = vals[sidx[i0 + j]];
+    }
+}
+
+__global__ void build_geo_kernel(BuildGeo* g, const uint32_t* m, const uint64_t* last, uint32_t leaf_fill,
+                                 uint32_t per, uint32_t cap) {
+  g->m = *m;
+  uint64_t total = 0;
+  uint32_t cnt = (g->m + leaf_fill - 1) / leaf_fill, h = 0;
+  for (;; cnt = (cnt + per - 1) / per) {
+    g->cnt[h] = cnt;
+    g->first[h] = (uint32_t)total;
+    total += cnt;
+    h++;
+    if (cnt == 1 || h == (uint32_t)kBuildLevels) break;
   }
+  g->height = h;
+  g->total = (uint32_t)total;
+  g->status = *last == kKeyMax ? kBuildReserved : (total > cap || cnt != 1) ? kBuildCapacity : 0u;
 }
 
 // one warp per leaf; leaves get base or base+1 keys (the first `rem` get one more)
-__global__ void build_leaves_kernel(DevTree t, const uint64_t* __restrict__ uk, const uint64_t* __restrict__ uv,
-                                    size_t m, uint32_t nl, uint32_t epoch) {
+__global__ void __launch_bounds__(256) build_leaves_kernel(DevTree t, const uint64_t* __restrict__ uk,
+                                                           const uint64_t* __restrict__ uv,
+                                                           const BuildGeo* __restrict__ geo, uint32_t epoch) {
   const uint32_t lane = threadIdx.x & 31;
   const size_t j = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (j >= nl) return;
-  const size_t base = m / nl, rem = m % nl;
-  const size_t k = base + (j < rem ? 1 : 0);
+  const uint32_t nl = geo->cnt[0];
+  if (j >= nl || geo->status) return;
+  const uint32_t base = geo->m / nl, rem = geo->m % nl;
+  const uint32_t k = base + (j < rem ? 1 : 0);
   const size_t start = j * base + (j < rem ? j : rem);
+  const uint64_t key = lane < k ? uk[start + lane] : kKeyMax;
   uint64_t* kr = t.keys + j * 32;
   uint64_t* vr = t.vals + j * 32;
   if (lane < 31) {
-    kr[lane] = lane < k ? uk[start + lane] : kKeyMax;
+    kr[lane] = key;
     vr[lane] = lane < k ? uv[start + lane] : 0;
   } else {
-    kr[31] = make_hdr((uint32_t)k, 0, 0, epoch);
+    kr[31] = make_hdr(k, 0, 0, epoch);
     vr[31] = (j + 1 < nl) ? uk[start + k] : kKeyMax;
   }
-  t.fp[j * 32 + lane] = lane < k ? slot_fp(uk[start + lane]) : (uint8_t)0;
-  if (lane == 0) t.low[j] = j == 0 ? 0 : uk[start];
+  t.fp[j * 32 + lane] = lane < k ? slot_fp(key) : (uint8_t)0;
+  if (lane == 0) t.low[j] = j == 0 ? 0 : key;
 }
 
-// one warp per inner node of a level: node p groups children [c, c + k)
-__global__ void build_inner_kernel(DevTree t, uint32_t first_child, uint32_t n_children, uint32_t first_node,
-                                   uint32_t n_nodes_level, uint32_t level, uint32_t epoch) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t p = (uint32_t)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (p >= n_nodes_level) return;
-  const uint32_t base = n_children / n_nodes_level, rem = n_children % n_nodes_level;
+// one warp per inner node: node p of the level groups children [c, c + k)
+__device__ __forceinline__ void build_inner_node(const DevTree& t, const BuildGeo* geo, uint32_t level, uint32_t p,
+                                                 uint32_t lane, uint32_t epoch) {
+  const uint32_t n_children = geo->cnt[level - 1], nn = geo->cnt[level];
+  const uint32_t base = n_children / nn, rem = n_children % nn;
   const uint32_t k = base + (p < rem ? 1 : 0);
-  const uint32_t c = first_child + p * base + (p < rem ? p : rem);
-  const uint32_t id = first_node + p;
-  uint64_t* kr = t.keys + (size_t)id * 32;
-  uint64_t* vr = t.vals + (size_t)id * 32;
+  const uint32_t c = geo->first[level - 1] + p * base + (p < rem ? p : rem);
+  const uint32_t id = geo->first[level] + p;
   // key slot i (i < k-1) = low fence of child i+1
   const uint64_t sep = (lane + 1 < k) ? t.low[c + lane + 1] : kKeyMax;
-  kr[lane] = lane < 31 ? sep : make_hdr(k - 1, level, 0, epoch);
+  t.keys[(size_t)id * 32 + lane] = lane < 31 ? sep : make_hdr(k - 1, level, 0, epoch);
   t.pfx[(size_t)id * 32 + lane] = lane < 31 ? (uint32_t)(sep >> 32) : 0xffffffffu;
-  vr[lane] = lane < k ? (uint64_t)(c + lane) : 0;
+  t.vals[(size_t)id * 32 + lane] = lane < k ? (uint64_t)(c + lane) : 0;
   if (lane == 0) t.low[id] = t.low[c];
 }
 
-__global__ void set_root_kernel(Ctrl* c, uint32_t root, uint32_t root_level, uint32_t n_nodes, uint64_t n_keys) {
-  c->root = root;
-  c->root_level = root_level;
-  c->n_nodes = n_nodes;
-  c->n_keys = n_keys;
+__global__ void __launch_bounds__(256) build_inner_kernel(DevTree t, const BuildGeo* __restrict__ geo, uint32_t level,
+                                                          uint32_t epoch) {
+  const uint32_t p = (uint32_t)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (geo->status || level >= geo->height || p >= geo->cnt[level]) return;
+  build_inner_node(t, geo, level, p, threadIdx.x & 31, epoch);
+}
+
+// the levels from `level` up (a few hundred nodes at most) and the root, one block
+constexpr uint32_t kBuildTopNodes = 512;
+__global__ void __launch_bounds__(1024) build_top_kernel(DevTree t, const BuildGeo* geo, uint32_t level,
+                                                         uint32_t epoch) {
+  if (geo->status) return;
+  for (uint32_t l = level; l < geo->height; l++) {
+    for (uint32_t p = threadIdx.x >> 5; p < geo->cnt[l]; p += blockDim.x >> 5)
+      build_inner_node(t, geo, l, p, threadIdx.x & 31, epoch);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    t.ctrl->root = geo->total - 1;
+    t.ctrl->root_level = geo->height - 1;
+    t.ctrl->n_nodes = geo->total;
+    t.ctrl->n_keys = geo->m;
+  }
 }
 
 // --------------------------------------------------------------- search ----
@@ -307,37 +383,98 @@ __global__ void __launch_bounds__(256) search_sorted_kernel(DevTree t, const uin
 }
 
 // ---------------------------------------------------------- enumeration ----
-__global__ void child_count_kernel(DevTree t, const uint32_t* __restrict__ nodes, size_t n, uint32_t* cnt,
-                                   int leaf_sizes) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    uint64_t h = t.keys[(size_t)nodes[i] * 32 + 31];
-    cnt[i] = leaf_sizes ? hdr_size(h) : hdr_size(h) + 1;
+// Levels from the root down, their counts on the device (cnt[l]: nodes of
+// level l, leaves at 0).  The top levels, while they have few nodes, by one
+// block; each of the others by a count, a scan and a write.
+constexpr uint32_t kEnumTop = 512;
+
+__global__ void __launch_bounds__(1024) enum_top_kernel(DevTree t, uint32_t root_level, uint32_t* a, uint32_t* b,
+                                                        uint32_t* __restrict__ cnt) {
+  __shared__ uint32_t ws[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t n = 1;
+  if (threadIdx.x == 0) {
+    a[0] = t.ctrl->root;
+    cnt[root_level] = 1;
+  }
+  __syncthreads();
+  __shared__ uint32_t off[kEnumTop];
+  for (uint32_t l = root_level; l > 0 && n <= kEnumTop; l--) {
+    const uint32_t c = threadIdx.x < n ? hdr_size(t.keys[(size_t)a[threadIdx.x] * 32 + 31]) + 1 : 0u;
+    uint32_t total;
+    const uint32_t ex = blk_exclusive_sum(c, ws, &total);
+    if (threadIdx.x < n) off[threadIdx.x] = ex;
+    __syncthreads();
+    for (uint32_t i = warp; i < n; i += 32) {
+      const uint32_t node = a[i];
+      if (lane <= hdr_size(t.keys[(size_t)node * 32 + 31])) b[off[i] + lane] = (uint32_t)t.vals[(size_t)node * 32 + lane];
+    }
+    __syncthreads();
+    n = total;
+    if (threadIdx.x == 0) cnt[l - 1] = n;
+    uint32_t* x = a;
+    a = b;
+    b = x;
   }
 }
 
-__global__ void child_write_kernel(DevTree t, const uint32_t* __restrict__ nodes, size_t n,
-                                   const uint32_t* __restrict__ off, uint32_t* __restrict__ out) {
-  const uint32_t lane = threadIdx.x & 31;
-  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= n) return;
-  const uint32_t node = nodes[i];
-  const uint32_t sz = hdr_size(t.keys[(size_t)node * 32 + 31]);
-  if (lane <= sz) out[off[i] + lane] = (uint32_t)t.vals[(size_t)node * 32 + lane];
+// levels that enum_top_kernel has expanded (a node count up to kEnumTop) are skipped
+__device__ __forceinline__ bool enum_done(const uint32_t* cnt, uint32_t level, uint32_t root_level) {
+  for (uint32_t l = root_level; l > level; l--)
+    if (cnt[l] > kEnumTop) return false;  // the block stopped above this level
+  return cnt[level] <= kEnumTop;
 }
 
-__global__ void leaf_dump_kernel(DevTree t, const uint32_t* __restrict__ leaves, size_t n,
-                                 const uint32_t* __restrict__ off, uint64_t* __restrict__ ok,
-                                 uint64_t* __restrict__ ov) {
+// children per node of the level (or, `leaf_sizes`, keys per leaf); *n_out: how
+// many entries the scan and the write handle (0: done already)
+__global__ void __launch_bounds__(256) child_count_kernel(DevTree t, const uint32_t* __restrict__ nodes,
+                                                          const uint32_t* __restrict__ cnt, uint32_t level,
+                                                          uint32_t root_level, uint32_t* __restrict__ out,
+                                                          uint32_t* __restrict__ n_out, int leaf_sizes) {
+  const uint32_t n = !leaf_sizes && enum_done(cnt, level, root_level) ? 0u : cnt[level];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *n_out = n;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint64_t h = t.keys[(size_t)nodes[i] * 32 + 31];
+    out[i] = leaf_sizes ? hdr_size(h) : hdr_size(h) + 1;
+  }
+}
+
+// the children of the level's nodes in order; total: the scan's
+__global__ void __launch_bounds__(256) child_write_kernel(DevTree t, const uint32_t* __restrict__ nodes,
+                                                          const uint32_t* __restrict__ n_dev,
+                                                          const uint32_t* __restrict__ off,
+                                                          const uint32_t* __restrict__ total,
+                                                          uint32_t* __restrict__ out, uint32_t* __restrict__ cnt_below) {
   const uint32_t lane = threadIdx.x & 31;
-  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= n) return;
-  const uint32_t node = leaves[i];
-  const uint32_t sz = hdr_size(t.keys[(size_t)node * 32 + 31]);
-  if (lane < sz) {
-    size_t o = (size_t)off[i] + lane;
-    if (ok) ok[o] = t.keys[(size_t)node * 32 + lane];
-    if (ov) ov[o] = t.vals[(size_t)node * 32 + lane];
+  const uint32_t n = *n_dev;
+  if (n == 0) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cnt_below = *total;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const uint32_t node = nodes[i];
+    const uint32_t sz = hdr_size(t.keys[(size_t)node * 32 + 31]);
+    if (lane <= sz) out[off[i] + lane] = (uint32_t)t.vals[(size_t)node * 32 + lane];
+  }
+}
+
+// all pairs in order, unless there are more than `cap`
+__global__ void __launch_bounds__(256) leaf_dump_kernel(DevTree t, const uint32_t* __restrict__ leaves,
+                                                        const uint32_t* __restrict__ n_dev,
+                                                        const uint32_t* __restrict__ off,
+                                                        const uint32_t* __restrict__ total, size_t cap,
+                                                        uint64_t* __restrict__ ok, uint64_t* __restrict__ ov) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t n = *n_dev;
+  if (*total > cap) return;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const uint32_t node = leaves[i];
+    const uint32_t sz = hdr_size(t.keys[(size_t)node * 32 + 31]);
+    if (lane < sz) {
+      const size_t o = (size_t)off[i] + lane;
+      if (ok) ok[o] = t.keys[(size_t)node * 32 + lane];
+      if (ov) ov[o] = t.vals[(size_t)node * 32 + lane];
+    }
   }
 }
 
@@ -621,93 +758,8 @@ cudaError_t tree_reset(Handle* h, cudaStream_t s) {
 
 // Bulk loader: replaces the contents.  Same packing rule as the oracle
 // (bto_bulk_build): ceil(m/leaf_fill) leaves of even size, inner levels of
-// inner_fill+1 children per node, leaves first in id order.
-int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s) {
-  cudaError_t e = tree_reset(h, s);
-  if (e != cudaSuccess) return -2;
-  if (n == 0) return 0;
-  if (n > 0xFFFFFFFFull / 2) return -1;
-  // temporaries (stream ordered)
-  uint64_t *ka = nullptr, *kb = nullptr, *uk = nullptr, *uv = nullptr;
-  uint32_t *va = nullptr, *vb = nullptr, *flags = nullptr, *pos = nullptr, *scratch = nullptr, *tot = nullptr;
-  size_t scw = sort_scratch_words(n);
-  if (scan_scratch_words(n) > scw) scw = scan_scratch_words(n);
-  bool ok = cudaMallocAsync(&ka, n * 8, s) == cudaSuccess && cudaMallocAsync(&kb, n * 8, s) == cudaSuccess &&
-            cudaMallocAsync(&va, n * 4, s) == cudaSuccess && cudaMallocAsync(&vb, n * 4, s) == cudaSuccess &&
-            cudaMallocAsync(&scratch, scw * 4, s) == cudaSuccess && cudaMallocAsync(&tot, 64, s) == cudaSuccess;
-  int rc = 0;
-  uint64_t* sk = nullptr;
-  uint32_t* si = nullptr;
-  uint64_t last_key = 0;
-  uint32_t m32 = 0;
-  if (!ok) { rc = -3; goto done; }
-  if (radix_sort_pairs(keys, nullptr, nullptr, ka, va, kb, vb, n, 0, 64, scratch, s, &sk, &si, &h->tree.ctrl->error) !=
-      cudaSuccess) {
-    rc = -2;
-    goto done;
-  }
-  // reuse the other ping-pong buffers for flags / positions / unique pairs
-  flags = (si == va) ? vb : va;
-  uk = (sk == ka) ? kb : ka;
-  if (cudaMallocAsync(&pos, n * 4, s) != cudaSuccess || cudaMallocAsync(&uv, n * 8, s) != cudaSuccess) {
-    rc = -3;
-    goto done;
-  }
-  tail_flags_kernel<<<blocks_for(n, 256), 256, 0, s>>>(sk, n, flags);
-  count_launch();
-  if (scan_exclusive_u32(flags, pos, n, tot, scratch, s) != cudaSuccess) { rc = -2; goto done; }
-  dedupe_kernel<<<blocks_for(n, 256), 256, 0, s>>>(sk, si, vals, flags, pos, n, uk, uv);
-  count_launch();
-  cudaMemcpyAsync(&m32, tot, 4, cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&last_key, sk + (n - 1), 8, cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) { rc = -2; goto done; }
-  if (last_key == kKeyMax) { rc = -5; goto done; }
-  {
-    const size_t m = m32;
-    const uint32_t lf = h->leaf_fill, per = h->inner_fill + 1;
-    const uint32_t nl = (uint32_t)((m + lf - 1) / lf);
-    // count nodes first (capacity check)
-    uint64_t total = nl;
-    uint32_t cnt = nl, height = 1;
-    while (cnt > 1) {
-      cnt = (cnt + per - 1) / per;
-      total += cnt;
-      height++;
-    }
-    if (total > h->tree.cap) { rc = -4; goto done; }
-    build_leaves_kernel<<<blocks_for((size_t)nl * 32, 256), 256, 0, s>>>(h->tree, uk, uv, m, nl, h->epoch);
-    count_launch();
-    uint32_t first_child = 0, n_children = nl, next = nl, level = 1;
-    while (n_children > 1) {
-      uint32_t nn = (n_children + per - 1) / per;
-      build_inner_kernel<<<blocks_for((size_t)nn * 32, 256), 256, 0, s>>>(h->tree, first_child, n_children, next,
-                                                                          nn, level, h->epoch);
-      count_launch();
-      first_child = next;
-      next += nn;
-      n_children = nn;
-      level++;
-    }
-    set_root_kernel<<<1, 1, 0, s>>>(h->tree.ctrl, first_child, height - 1, (uint32_t)total, (uint64_t)m);
-    count_launch();
-    if (cudaGetLastError() != cudaSuccess) rc = -2;
-  }
-done:
-  cudaFreeAsync(ka, s);
-  cudaFreeAsync(kb, s);
-  cudaFreeAsync(va, s);
-  cudaFreeAsync(vb, s);
-  cudaFreeAsync(scratch, s);
-  cudaFreeAsync(tot, s);
-  if (pos) cudaFreeAsync(pos, s);
-  if (uv) cudaFreeAsync(uv, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess && rc == 0) rc = -2;
-  return rc;
-}
-
-// Same bulk build with the scratch supplied by the caller (nothing allocated
-// here); used by bt_bulk_build_static.  Packing rule identical to
-// tree_bulk_build above.
+// inner_fill+1 children per node, leaves first in id order.  The scratch is the
+// caller's; nothing is allocated.
 int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s,
                             const BuildScratch& sc) {
   if (n > sc.cap) return -6;
@@ -715,51 +767,98 @@ int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* val
   if (n == 0) return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -2;
   uint64_t* sk = nullptr;
   uint32_t* si = nullptr;
-  if (radix_sort_pairs(keys, nullptr, nullptr, sc.ka, sc.va, sc.kb, sc.vb, n, 0, 64, sc.sort_scratch, s, &sk, &si, &h->tree.ctrl->error) !=
-      cudaSuccess)
+  if (radix_sort_pairs(keys, nullptr, nullptr, sc.ka, sc.va, sc.kb, sc.vb, n, 0, 64, sc.sort_scratch, s, &sk, &si,
+                       &h->tree.ctrl->error) != cudaSuccess)
     return -2;
-  uint32_t* flags = (si == sc.va) ? sc.vb : sc.va;
   uint64_t* uk = (sk == sc.ka) ? sc.kb : sc.ka;
-  tail_flags_kernel<<<blocks_for(n, 256), 256, 0, s>>>(sk, n, flags);
+  BuildGeo* geo = reinterpret_cast<BuildGeo*>(sc.tot);
+  uint32_t* m = &geo->m;  // the scan's total
+  const unsigned tiles = blocks_for(n, kDedupeTile);
+  tail_count_kernel<<<tiles, kDedupeThreads, 0, s>>>(sk, n, sc.pos);
   count_launch();
-  if (scan_exclusive_u32(flags, sc.pos, n, sc.tot, sc.sort_scratch, s) != cudaSuccess) return -2;
-  dedupe_kernel<<<blocks_for(n, 256), 256, 0, s>>>(sk, si, vals, flags, sc.pos, n, uk, sc.uv);
+  if (scan_exclusive_u32(sc.pos, sc.pos, tiles, m, sc.sort_scratch, s) != cudaSuccess) return -2;
+  dedupe_kernel<<<tiles, kDedupeThreads, 0, s>>>(sk, si, vals, n, sc.pos, uk, sc.uv);
+  const uint32_t lf = h->leaf_fill, per = h->inner_fill + 1;
+  build_geo_kernel<<<1, 1, 0, s>>>(geo, m, sk + (n - 1), lf, per, h->tree.cap);
+  // the grids for n distinct keys
+  size_t nodes = (n + lf - 1) / lf;
+  build_leaves_kernel<<<blocks_for(nodes * 32, 256), 256, 0, s>>>(h->tree, uk, sc.uv, geo, h->epoch);
+  count_launch(3);
+  uint32_t level = 1;
+  for (nodes = (nodes + per - 1) / per; nodes > kBuildTopNodes; nodes = (nodes + per - 1) / per, level++) {
+    build_inner_kernel<<<blocks_for(nodes * 32, 256), 256, 0, s>>>(h->tree, geo, level, h->epoch);
+    count_launch();
+  }
+  build_top_kernel<<<1, 1024, 0, s>>>(h->tree, geo, level, h->epoch);
   count_launch();
-  uint32_t m32 = 0;
-  uint64_t last_key = 0;
-  if (cudaMemcpyAsync(&m32, sc.tot, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaMemcpyAsync(&last_key, sk + (n - 1), 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+  uint32_t* status = h->pin;
+  if (cudaGetLastError() != cudaSuccess ||
+      cudaMemcpyAsync(status, &geo->status, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return -2;
-  if (last_key == kKeyMax) return -5;
-  const size_t m = m32;
-  const uint32_t lf = h->leaf_fill, per = h->inner_fill + 1;
-  const uint32_t nl = (uint32_t)((m + lf - 1) / lf);
-  uint64_t total = nl;
-  uint32_t cnt = nl, height = 1;
-  while (cnt > 1) {
-    cnt = (cnt + per - 1) / per;
-    total += cnt;
-    height++;
+  return *status == kBuildReserved ? -5 : *status == kBuildCapacity ? -4 : 0;
+}
+
+// The same with the handle's scratch: up to max_batch keys in the batch work
+// buffers; more in one block of the handle's own pool, which keeps up to
+// kBuildKeep bytes between builds (a pool that gives its memory back at every
+// synchronisation maps and unmaps it per build: most of the 1.0 ms that a load
+// of 2^20 keys spent outside its kernels) and all of it until bt_destroy.
+constexpr uint64_t kBuildKeep = 1ull << 30;
+int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s) {
+  if (n == 0 || n > 0xFFFFFFFFull / 2) return tree_reset(h, s) != cudaSuccess ? -2 : n ? -1 : 0;
+  Work& w = h->w;
+  BuildScratch sc;
+  sc.tot = h->geo;
+  if (n <= w.cap) {
+    sc.ka = w.k_a;
+    sc.kb = w.k_b;
+    sc.va = w.v_a;
+    sc.vb = w.v_b;
+    sc.sort_scratch = w.sort_scratch;
+    sc.pos = w.f_pos;
+    sc.uv = w.uvals;
+    sc.cap = w.cap;
+    return tree_bulk_build_scratch(h, keys, vals, n, s, sc);
   }
-  if (total > h->tree.cap) return -4;
-  build_leaves_kernel<<<blocks_for((size_t)nl * 32, 256), 256, 0, s>>>(h->tree, uk, sc.uv, m, nl, h->epoch);
-  count_launch();
-  uint32_t first_child = 0, n_children = nl, next = nl, level = 1;
-  while (n_children > 1) {
-    const uint32_t nn = (n_children + per - 1) / per;
-    build_inner_kernel<<<blocks_for((size_t)nn * 32, 256), 256, 0, s>>>(h->tree, first_child, n_children, next, nn,
-                                                                        level, h->epoch);
-    count_launch();
-    first_child = next;
-    next += nn;
-    n_children = nn;
-    level++;
+  if (!h->build_pool) {
+    cudaMemPoolProps pp{};
+    pp.allocType = cudaMemAllocationTypePinned;
+    pp.handleTypes = cudaMemHandleTypeNone;
+    pp.location.type = cudaMemLocationTypeDevice;
+    pp.location.id = h->device;
+    uint64_t keep = kBuildKeep;
+    if (cudaMemPoolCreate(&h->build_pool, &pp) != cudaSuccess) {
+      h->build_pool = nullptr;
+      return -3;
+    }
+    cudaMemPoolSetAttribute(h->build_pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
-  set_root_kernel<<<1, 1, 0, s>>>(h->tree.ctrl, first_child, height - 1, (uint32_t)total, (uint64_t)m);
-  count_launch();
-  if (cudaGetLastError() != cudaSuccess) return -2;
-  return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -2;
+  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t kb = up(n * 8), vb = up(n * 4), pb = up((n / kDedupeTile + 2) * 4);
+  char* slab = nullptr;
+  if (cudaMallocFromPoolAsync((void**)&slab, 3 * kb + 2 * vb + pb + up(sort_scratch_words(n) * 4), h->build_pool, s) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return tree_reset(h, s) == cudaSuccess ? -3 : -2;
+  }
+  char* at = slab;
+  auto take = [&](size_t b) {
+    char* p = at;
+    at += b;
+    return p;
+  };
+  sc.ka = (uint64_t*)take(kb);
+  sc.kb = (uint64_t*)take(kb);
+  sc.uv = (uint64_t*)take(kb);
+  sc.va = (uint32_t*)take(vb);
+  sc.vb = (uint32_t*)take(vb);
+  sc.pos = (uint32_t*)take(pb);
+  sc.sort_scratch = (uint32_t*)at;
+  sc.cap = n;
+  const int rc = tree_bulk_build_scratch(h, keys, vals, n, s, sc);
+  cudaFreeAsync(slab, s);
+  return rc;
 }
 
 cudaError_t launch_search_sorted(Handle* h, const uint64_t* qkeys, const uint32_t* list, const uint32_t* n_dev,
@@ -903,83 +1002,118 @@ static int ensure_enum(Handle* h, size_t n) {
   cudaFree(h->enum_a);
   cudaFree(h->enum_b);
   cudaFree(h->enum_cnt);
-  cudaFree(h->enum_scan_scratch);
-  h->enum_a = h->enum_b = h->enum_cnt = h->enum_scan_scratch = nullptr;
+  cudaFree(h->enum_lb);
+  h->enum_a = h->enum_b = h->enum_cnt = nullptr;
+  h->enum_lb = nullptr;
   h->enum_cap = 0;
-  size_t c = n + 64;
+  const size_t c = n + 64, lb = scan_lb_words(c) + 1;  // the last word: the scan's two counters
   if (cudaMalloc(&h->enum_a, c * 4) != cudaSuccess || cudaMalloc(&h->enum_b, c * 4) != cudaSuccess ||
-      cudaMalloc(&h->enum_cnt, (c + 1) * 4) != cudaSuccess ||
-      cudaMalloc(&h->enum_scan_scratch, (scan_scratch_words(c) + 1) * 4) != cudaSuccess)
+      cudaMalloc(&h->enum_cnt, c * 4) != cudaSuccess || cudaMalloc(&h->enum_lb, lb * 8) != cudaSuccess ||
+      cudaMemset(h->enum_lb, 0, lb * 8) != cudaSuccess)
     return -3;
   h->enum_cap = c;
+  h->enum_lb_words = lb;
   return 0;
 }
 
-int enumerate_leaves(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_leaves) {
-  Ctrl c;
-  if (cudaMemcpyAsync(&c, h->tree.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -2;
+static cudaError_t enum_scan(Handle* h, uint32_t* x, const uint32_t* n_dev, size_t n_upper, uint32_t* total,
+                             cudaStream_t s) {
+  uint32_t* ctr = reinterpret_cast<uint32_t*>(h->enum_lb + h->enum_lb_words - 1);
+  return scan_exclusive_u32_lb(x, x, n_upper, n_dev, total, h->enum_lb, ctr, &h->enum_epoch, &h->tree.ctrl->error, s);
+}
+
+// words of the handle's small device block (h->geo) that the enumeration uses
+constexpr int kEnumWords = 64;  // [0, 48) counts per level, [48] entries of this level, [49] total
+
+// The leaves' ids in key order in *leaf_ids, their count in cnt[0] on the
+// device; one read back (the control block), no other wait.  *root_level < 0:
+// an empty tree.
+static int enumerate_queue(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_nodes, int* root_level) {
+  Ctrl* c = reinterpret_cast<Ctrl*>(h->pin);
+  if (cudaMemcpyAsync(c, h->tree.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -2;
   if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
-  *n_leaves = 0;
   *leaf_ids = nullptr;
+  *root_level = -1;
+  *n_nodes = 0;
   h->n_levels = 0;
-  if (c.root == kNil) return 0;
-  h->n_levels = c.root_level + 1;
-  if (h->n_levels <= 48) h->level_counts[c.root_level] = 1;
-  if (ensure_enum(h, c.n_nodes + 1) != 0) return -3;
+  if (c->root == kNil) return 0;
+  const uint32_t rl = c->root_level;
+  if (rl >= 48) return -2;
+  const size_t nn = c->n_nodes < h->tree.cap ? c->n_nodes : h->tree.cap;
+  h->n_levels = rl + 1;
+  if (ensure_enum(h, nn + 1) != 0) return -3;
+  uint32_t* cnt = h->geo;
   uint32_t* cur = h->enum_a;
   uint32_t* nxt = h->enum_b;
-  cudaMemcpyAsync(cur, &c.root, 4, cudaMemcpyHostToDevice, s);
-  size_t n = 1;
-  uint32_t* tot = h->enum_cnt + h->enum_cap;  // last word
-  for (uint32_t l = c.root_level; l > 0; l--) {
-    child_count_kernel<<<blocks_for(n, 256), 256, 0, s>>>(h->tree, cur, n, h->enum_cnt, 0);
-    count_launch();
-    if (scan_exclusive_u32(h->enum_cnt, h->enum_cnt, n, tot, h->enum_scan_scratch, s) != cudaSuccess) return -2;
-    child_write_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(h->tree, cur, n, h->enum_cnt, nxt);
-    count_launch();
-    uint32_t m = 0;
-    cudaMemcpyAsync(&m, tot, 4, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
-    n = m;
-    if (l - 1 < 48) h->level_counts[l - 1] = m;
-    uint32_t* t = cur;
+  enum_top_kernel<<<1, 1024, 0, s>>>(h->tree, rl, cur, nxt, cnt);
+  count_launch();
+  const unsigned grid = (unsigned)min((size_t)h->sm_count * 8, nn / 8 + 1);
+  for (uint32_t l = rl; l > 0; l--) {
+    // levels surely below the block's limit need no launches: every inner node
+    // has two children or more (unless the loader ever packed one per node)
+    size_t bound = nn;
+    for (uint32_t x = 0; x < l && h->inner_min >= 2; x++) bound = (bound + 1) / 2;
+    if (bound > kEnumTop) {
+      child_count_kernel<<<grid, 256, 0, s>>>(h->tree, cur, cnt, l, rl, h->enum_cnt, cnt + 48, 0);
+      count_launch();
+      if (enum_scan(h, h->enum_cnt, cnt + 48, bound, cnt + 49, s) != cudaSuccess) return -2;
+      child_write_kernel<<<grid, 256, 0, s>>>(h->tree, cur, cnt + 48, h->enum_cnt, cnt + 49, nxt, cnt + l - 1);
+      count_launch();
+    }
+    uint32_t* x = cur;
     cur = nxt;
-    nxt = t;
+    nxt = x;
   }
   *leaf_ids = cur;
-  *n_leaves = n;
+  *n_nodes = nn;
+  *root_level = (int)rl;
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int enumerate_leaves(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_leaves) {
+  size_t nn = 0;
+  int rl = -1;
+  *n_leaves = 0;
+  const int rc = enumerate_queue(h, s, leaf_ids, &nn, &rl);
+  if (rc || rl < 0) return rc;
+  if (cudaMemcpyAsync(h->pin, h->geo, kEnumWords * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
+    return -2;
+  for (int l = 0; l <= rl; l++) h->level_counts[l] = h->pin[l];
+  *n_leaves = h->pin[0];
   return 0;
 }
 
 cudaError_t leaf_sizes_device(Handle* h, const uint32_t* leaves, size_t n, uint32_t* out, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  child_count_kernel<<<blocks_for(n, 256), 256, 0, s>>>(h->tree, leaves, n, out, 1);
+  child_count_kernel<<<(unsigned)min((size_t)h->sm_count * 8, (n + 255) / 256), 256, 0, s>>>(
+      h->tree, leaves, h->geo, 0, 0, out, h->geo + 48, 1);
   count_launch();
   return cudaGetLastError();
 }
 
 int tree_dump(Handle* h, uint64_t* out_keys, uint64_t* out_vals, size_t cap, size_t* n_out, cudaStream_t s) {
   uint32_t* leaves = nullptr;
-  size_t nl = 0;
-  int rc = enumerate_leaves(h, s, &leaves, &nl);
-  if (rc) return rc;
+  size_t nn = 0;
+  int rl = -1;
   *n_out = 0;
-  if (nl == 0) return 0;
-  // leaves live in one enum buffer; use the other for sizes
-  uint32_t* sizes = (leaves == h->enum_a) ? h->enum_b : h->enum_a;
-  uint32_t* tot = h->enum_cnt + h->enum_cap;
-  child_count_kernel<<<blocks_for(nl, 256), 256, 0, s>>>(h->tree, leaves, nl, sizes, 1);
+  const int rc = enumerate_queue(h, s, &leaves, &nn, &rl);
+  if (rc || rl < 0) return rc;
+  uint32_t* cnt = h->geo;
+  const unsigned grid = (unsigned)min((size_t)h->sm_count * 8, nn / 8 + 1);
+  // the counts per parent are done with: the leaves' sizes take their place
+  child_count_kernel<<<grid, 256, 0, s>>>(h->tree, leaves, cnt, 0, 0, h->enum_cnt, cnt + 48, 1);
   count_launch();
-  if (scan_exclusive_u32(sizes, sizes, nl, tot, h->enum_scan_scratch, s) != cudaSuccess) return -2;
-  uint32_t total = 0;
-  cudaMemcpyAsync(&total, tot, 4, cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
-  *n_out = total;
-  if (total > cap) return -4;
-  leaf_dump_kernel<<<blocks_for(nl * 32, 256), 256, 0, s>>>(h->tree, leaves, nl, sizes, out_keys, out_vals);
+  if (enum_scan(h, h->enum_cnt, cnt + 48, nn, cnt + 49, s) != cudaSuccess) return -2;
+  leaf_dump_kernel<<<grid, 256, 0, s>>>(h->tree, leaves, cnt + 48, h->enum_cnt, cnt + 49, cap, out_keys, out_vals);
   count_launch();
-  if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
-  return 0;
+  if (cudaGetLastError() != cudaSuccess ||
+      cudaMemcpyAsync(h->pin, cnt, kEnumWords * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
+    return -2;
+  for (int l = 0; l <= rl; l++) h->level_counts[l] = h->pin[l];
+  *n_out = h->pin[49];
+  return *n_out > cap ? -4 : 0;
 }
 
 }  // namespace bt
