@@ -472,9 +472,12 @@ class BTree:
 
         n = lo.numel()
         dev_ = lo.device
-        keys = torch.zeros((n, max(max_per, 1)), dtype=torch.int64, device=dev_)[:, :max_per]
-        vals = torch.zeros((n, max(max_per, 1)), dtype=torch.int64, device=dev_)[:, :max_per]
-        counts = torch.zeros(max(n, 1), dtype=torch.int32, device=dev_)[:n]
+        w = max(max_per, 1)
+        # one zeroed block for the three results: one fill instead of three
+        buf = torch.zeros(2 * n * w + (n + 1) // 2 + 1, dtype=torch.int64, device=dev_)
+        keys = buf[: n * w].view(n, w)[:, :max_per]
+        vals = buf[n * w: 2 * n * w].view(n, w)[:, :max_per]
+        counts = buf[2 * n * w:].view(torch.int32)[:n]
         _check(lib().bt_range_batch(self._h, _ptr(lo), _ptr(hi), n, max_per, _ptr(keys), _ptr(vals), _ptr(counts),
                                     _stream_ptr(stream)), "bt_range_batch")
         return counts, keys, vals

@@ -620,19 +620,27 @@ __global__ void __launch_bounds__(512) search_top_kernel(DevTree t, const TopNod
   }
 }
 
-// Range scan, one warp per query: descend to the leaf that holds `lo`, take
-// the leaf's keys in [lo, hi] (lane i holds slot i; a ballot compacts them in
-// key order), and continue at the leaf that starts at this leaf's right fence
-// (found by a new descent: leaves carry no sibling pointer) until a leaf's
-// fence passes `hi`.  Read-only; runs only when no writer is active.
-__global__ void __launch_bounds__(256) range_kernel(DevTree t, const uint64_t* __restrict__ lo_keys,
+// Range scan, one warp per query.  The descent ends at the parent of the leaf
+// that holds `lo`: its separators say which of its children meet [lo, hi] (a
+// separator is the next child's low fence), so their rows are read one after
+// the other with the next one's loads ahead of the current one's work, and only
+// past the parent's last child does a new descent follow, from that leaf's
+// right fence.  A lane holds one slot; a ballot compacts the keys in [lo, hi] in
+// key order.  Inner levels are ranked by the separators' prefixes.  Read-only;
+// runs only when no writer is active.
+// 20,000 scans of about 100 keys on 2^24 keys, with the zero fill of the
+// results: 58.5 us with a descent per leaf (a dependent row and child id per
+// level), 42.2 with this at 46 registers, 39.4 at the 36 of seven blocks an SM.
+__global__ void __launch_bounds__(256, 7) range_kernel(DevTree t, const uint64_t* __restrict__ lo_keys,
                                                    const uint64_t* __restrict__ hi_keys, size_t n, uint32_t max_per,
                                                    uint64_t* __restrict__ out_keys, uint64_t* __restrict__ out_vals,
                                                    uint32_t* __restrict__ out_counts) {
+  constexpr unsigned kAll = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t root = t.ctrl->root;
   const uint32_t root_level = t.ctrl->root_level;
   const uint64_t cap_nodes = t.cap;
+  const uint64_t keep = l2_keep(), stream = l2_stream();
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t q = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n; q += warps) {
     const uint64_t lo = __ldg(lo_keys + q), hi = __ldg(hi_keys + q);
@@ -640,27 +648,52 @@ __global__ void __launch_bounds__(256) range_kernel(DevTree t, const uint64_t* _
     uint64_t from = lo;
     bool more = root != kNil && lo <= hi && lo != kKeyMax;  // UINT64_MAX is never a stored key
     for (uint64_t visited = 0; more && visited <= cap_nodes; visited++) {
-      // descend to the leaf holding `from`
+      // descend to the parent of the leaf holding `from`
       uint32_t node = root;
-      for (uint32_t level = root_level; level > 0; level--) {
-        const uint64_t k = __ldg(t.keys + (size_t)node * 32 + lane);
-        const uint32_t c = __popc(__ballot_sync(0xffffffffu, lane < 31 && k <= from));
-        node = (uint32_t)__ldg(t.vals + (size_t)node * 32 + c);
-      }
-      const uint64_t k = __ldg(t.keys + (size_t)node * 32 + lane);
-      const uint64_t v = __ldg(t.vals + (size_t)node * 32 + lane);
-      const uint32_t size = hdr_size(__shfl_sync(0xffffffffu, k, 31));
-      const uint64_t fence = __shfl_sync(0xffffffffu, v, 31);
-      const bool in = lane < size && lane < 31 && k >= lo && k <= hi;
-      const uint32_t m = __ballot_sync(0xffffffffu, in);
-      if (in) {
-        const uint32_t pos = count + __popc(m & ((1u << lane) - 1u));
-        if (pos < max_per) {
-          out_keys[q * max_per + pos] = k;
-          out_vals[q * max_per + pos] = v;
+      for (uint32_t level = root_level; level > 1; level--) {
+        const uint32_t p = __ldg(t.pfx + (size_t)node * 32 + lane), kp = (uint32_t)(from >> 32);
+        uint32_t c = __popc(__ballot_sync(kAll, p < kp));
+        if (__any_sync(kAll, p == kp)) {  // a separator shares the key's prefix: the full keys
+          const uint64_t k = ldg_hint(t.keys + (size_t)node * 32 + lane, keep);
+          c = __popc(__ballot_sync(kAll, lane < 31 && k <= from));
         }
+        node = (uint32_t)ldg_hint(t.vals + (size_t)node * 32 + c, keep);
       }
-      count += __popc(m);
+      // its children c0 .. c1 meet [from, hi]; a tree of one leaf is its only child
+      uint32_t c0 = 0, c1 = 0;
+      uint64_t kids = node;
+      if (root_level > 0) {
+        const uint64_t k = ldg_hint(t.keys + (size_t)node * 32 + lane, keep);
+        kids = ldg_hint(t.vals + (size_t)node * 32 + lane, keep);
+        c0 = __popc(__ballot_sync(kAll, lane < 31 && k <= from));
+        c1 = __popc(__ballot_sync(kAll, lane < 31 && k <= hi && k != kKeyMax));  // slots past the size hold kKeyMax
+      }
+      uint32_t leaf = (uint32_t)__shfl_sync(kAll, kids, c0);
+      uint64_t k = ldg_hint(t.keys + (size_t)leaf * 32 + lane, stream);
+      uint64_t v = ldg_hint(t.vals + (size_t)leaf * 32 + lane, stream);
+      uint64_t fence = kKeyMax;
+      for (uint32_t c = c0; c <= c1; c++) {
+        uint64_t k2 = 0, v2 = 0;
+        if (c < c1) {
+          leaf = (uint32_t)__shfl_sync(kAll, kids, c + 1);
+          k2 = ldg_hint(t.keys + (size_t)leaf * 32 + lane, stream);
+          v2 = ldg_hint(t.vals + (size_t)leaf * 32 + lane, stream);
+        }
+        const uint32_t size = hdr_size(__shfl_sync(kAll, k, 31));
+        if (c == c1) fence = __shfl_sync(kAll, v, 31);
+        const bool in = lane < size && lane < 31 && k >= lo && k <= hi;
+        const uint32_t m = __ballot_sync(kAll, in);
+        if (in) {
+          const uint32_t pos = count + __popc(m & ((1u << lane) - 1u));
+          if (pos < max_per) {
+            out_keys[q * max_per + pos] = k;
+            out_vals[q * max_per + pos] = v;
+          }
+        }
+        count += __popc(m);
+        k = k2;
+        v = v2;
+      }
       // the next leaf starts at the fence; stop when it lies past hi
       more = fence != kKeyMax && fence <= hi && fence > from;
       from = fence;
@@ -668,7 +701,6 @@ __global__ void __launch_bounds__(256) range_kernel(DevTree t, const uint64_t* _
     if (lane == 0) out_counts[q] = count;
   }
 }
-
 
 }  // namespace
 
@@ -985,6 +1017,8 @@ cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list
 cudaError_t launch_range(Handle* h, const uint64_t* lo, const uint64_t* hi, size_t n, uint32_t max_per,
                          uint64_t* out_keys, uint64_t* out_vals, uint32_t* out_counts, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
+  const cudaError_t pe = ensure_pfx(h, s);
+  if (pe != cudaSuccess) return pe;
   size_t blocks = (n * 32 + 255) / 256;
   const size_t cap = (size_t)h->sm_count * 16;
   if (blocks > cap) blocks = cap;
