@@ -30,6 +30,7 @@ SOURCES = [
     "bt_shard.cu",
     "bt_front.cu",
     "bt_small.cu",
+    "bt_sample.cu",
     "bt_snapshot.cu",
     "bt_delete.cu",
 ]

@@ -25,6 +25,7 @@
 #include "bt_block.cuh"
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_sort.cuh"
 
 namespace bt {
 
@@ -323,13 +324,13 @@ __global__ void __launch_bounds__(kThreads) merge_pass3(
 __global__ void writeback_kernel(const uint32_t* __restrict__ sv, const uint32_t* __restrict__ pend, size_t n,
                                  const uint32_t* __restrict__ n_dev, const uint64_t* __restrict__ uans,
                                  const uint8_t* __restrict__ uans_st, uint64_t* __restrict__ out_vals,
-                                 uint8_t* __restrict__ out_st) {
+                                 uint8_t* __restrict__ out_st, int pairs) {
   if (n_dev) n = min(n, (size_t)*n_dev);
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const uint32_t u = pend[i];
     if (u != kResolved) {
-      const uint32_t r = sv[i] & kIdxMask;
+      const uint32_t r = pairs ? pair_idx(sv[i]) : sv[i] & kIdxMask;  // the payload's form: the sort's
       out_vals[r] = uans[u];
       out_st[r] = uans_st[u];
     }
@@ -393,6 +394,8 @@ int work_alloc(Work* w, size_t cap) {
   A((void**)&w->lb_status, scan_lb_words(cap) * 8);
   A((void**)&w->lb_ctr, 8);
   A((void**)&w->s_write, 3 * 16 * 4);
+  A((void**)&w->s_split, kSsBuckets * 16);
+  A(&w->s_sum, sample_sum_bytes());
   ok = ok && cudaMemset(w->lb_status, 0, scan_lb_words(cap) * 8) == cudaSuccess &&
        cudaMemset(w->lb_ctr, 0, 8) == cudaSuccess;
   if (!ok) {
@@ -408,7 +411,7 @@ int work_alloc(Work* w, size_t cap) {
 }
 
 // the fields of Work that make up a BatchSet
-#define BT_SET_FIELDS(X) X(tiles) X(counts) X(f_list) X(f_lk) X(ukeys) X(uvals) X(ins_list) X(get_list) X(del_list) X(pend) \
+#define BT_SET_FIELDS(X) X(s_sum) X(tiles) X(counts) X(f_list) X(f_lk) X(ukeys) X(uvals) X(ins_list) X(get_list) X(del_list) X(pend) \
   X(k_a) X(k_b) X(v_a) X(v_b)
 
 void work_swap_set(Work* w) {
@@ -424,6 +427,7 @@ int work_alt_alloc(Work* w) {
   BatchSet& a = w->alt;
   bool ok = cudaMalloc((void**)&a.tiles, pass_tiles(cap) * sizeof(TileSummary)) == cudaSuccess &&
             cudaMalloc((void**)&a.counts, sizeof(BatchCounts)) == cudaSuccess &&
+            cudaMalloc(&a.s_sum, sample_sum_bytes()) == cudaSuccess &&
             cudaMalloc((void**)&a.f_list, cap * 4) == cudaSuccess && cudaMalloc((void**)&a.f_lk, cap * 8) == cudaSuccess &&
             cudaMalloc((void**)&a.ukeys, cap * 8) == cudaSuccess && cudaMalloc((void**)&a.uvals, cap * 8) == cudaSuccess &&
             cudaMalloc((void**)&a.ins_list, cap * 4) == cudaSuccess &&
@@ -457,7 +461,7 @@ void work_free(Work* w) {
                 w->m_nleaf,  w->m_seg,     w->d_leaf,    w->d_slot,    w->m_ent_a,   w->m_ent_b,   w->m_counts,     w->m_sync,
                 w->ins_ops,  w->f_tab, w->f_flags,
                 w->f_pos,    w->f_list,    w->f_lk,      w->f_tk,      w->f_tv,      w->lb_status, w->lb_ctr,
-                w->s_tab,    w->s_sums,  w->s_write};
+                w->s_tab,    w->s_sums,  w->s_write,   w->s_split,  w->s_sum};
   for (void* p : ps)
     if (p) cudaFree(p);
   *w = Work{};
@@ -519,40 +523,50 @@ struct FrontPart {
   uint64_t* sk = nullptr;
   uint32_t* sv = nullptr;
   uint32_t n_tiles = 0;
+  bool sample = false;  // sorted by the sample sort (its buckets' sums instead of tile passes)
   bool passes_done = false;
 };
+
+// the segmented scan over the sorted touched requests
+static int hashed_passes(Handle* h, const FrontPart& fp, const uint64_t* vals, uint64_t* out_vals, uint8_t* out_st,
+                         size_t n, cudaStream_t s) {
+  Work& w = h->w;
+  const uint32_t* n_touch = &w.counts->n_touch;
+  if (fp.sample) return sample_resolve(h, vals, out_vals, out_st, n, s);
+  merge_pass1<<<fp.n_tiles, kThreads, 0, s>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles);
+  merge_pass2<<<1, 1024, 0, s>>>(w.tiles, fp.n_tiles, n_touch, w.counts);
+  merge_pass3<<<fp.n_tiles, kThreads, 0, s>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles, w.ukeys, w.uvals, w.ins_list,
+                                              w.get_list, w.del_list, w.pend, out_vals, out_st);
+  count_launch(3);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 
 static int hashed_front(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,
                         uint8_t* out_st, size_t n, cudaStream_t s, bool passes, FrontPart& fp,
                         cudaEvent_t vals_ready = nullptr) {
   Work& w = h->w;
-  BatchCounts* c = w.counts;
-  const uint32_t* n_touch = &c->n_touch;
-  if (front_classify(h, keys, ops, n, s) != 0) return -2;
+  const uint32_t* n_touch = &w.counts->n_touch;
   // the touched requests' sort and merge passes need no tree: they run at
-  // full width (beside the previous batch's deferred merge)
-  // the merge sort while the touched counts are small (the count of a batch
-  // that ran before: a hint, both sorts give the same order)
-  bool merge = h->touch_sort == 1;
+  // full width (beside the previous batch's deferred merge).  The sample sort
+  // while the touched counts are small (the count of a batch that ran before:
+  // a hint, both sorts give the same order)
+  fp.sample = h->touch_sort == 1;
   if (h->touch_sort == 2 && h->touch_hint)
-    merge = *reinterpret_cast<volatile const uint32_t*>(h->touch_hint) <= kMergeSortMax;
-  const cudaError_t se =
-      merge
-          ? merge_sort_pairs(w.f_tk, w.f_tv, w.k_a, w.v_a, w.k_b, w.v_b, n, n_touch, h->sm_count, s, &fp.sk, &fp.sv)
-          : radix_sort_pairs(w.f_tk, w.f_tv, nullptr, w.k_a, w.v_a, w.k_b, w.v_b, n, 0, 64, w.sort_scratch, s,
-                             &fp.sk, &fp.sv, &h->tree.ctrl->error, n_touch, h->sort_threads_touch);
-  if (se != cudaSuccess) return -2;
+    fp.sample = *reinterpret_cast<volatile const uint32_t*>(h->touch_hint) <= kSampleSortMax;
+  if (front_classify(h, keys, ops, n, !fp.sample, s) != 0) return -2;
+  if (fp.sample) {
+    if (sample_sort(h, n, s) != 0) return -2;
+    fp.sk = w.k_a;
+    fp.sv = w.v_a;
+  } else if (radix_sort_pairs(w.f_tk, w.f_tv, nullptr, w.k_a, w.v_a, w.k_b, w.v_b, n, 0, 64, w.sort_scratch, s, &fp.sk,
+                              &fp.sv, &h->tree.ctrl->error, n_touch, h->sort_threads_touch) != cudaSuccess) {
+    return -2;
+  }
   fp.n_tiles = (uint32_t)pass_tiles(n);
   prof_mark(h, h->overlap != 0 ? kEvSortEnd : 1, s);
   if (passes) {
     if (vals_ready && cudaStreamWaitEvent(s, vals_ready, 0) != cudaSuccess) return -2;
-    merge_pass1<<<fp.n_tiles, kThreads, 0, s>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles);
-    count_launch();
-    merge_pass2<<<1, 1024, 0, s>>>(w.tiles, fp.n_tiles, n_touch, c);
-    count_launch();
-    merge_pass3<<<fp.n_tiles, kThreads, 0, s>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles, w.ukeys, w.uvals,
-                                                w.ins_list, w.get_list, w.del_list, w.pend, out_vals, out_st);
-    count_launch();
+    if (hashed_passes(h, fp, vals, out_vals, out_st, n, s) != 0) return -2;
     fp.passes_done = true;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -580,14 +594,7 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   if (!fp.passes_done) {
     cudaStream_t sp = ov ? s2 : s;
     if ((ov && !fork()) || wait_vals(h, sp) != 0) return -2;
-    merge_pass1<<<fp.n_tiles, kThreads, 0, sp>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles);
-    count_launch();
-    merge_pass2<<<1, 1024, 0, sp>>>(w.tiles, fp.n_tiles, n_touch, c);
-    count_launch();
-    merge_pass3<<<fp.n_tiles, kThreads, 0, sp>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles, w.ukeys, w.uvals,
-                                                 w.ins_list, w.get_list, w.del_list, w.pend, out_vals, out_st);
-    count_launch();
-    if (cudaGetLastError() != cudaSuccess) return -2;
+    if (hashed_passes(h, fp, vals, out_vals, out_st, n, sp) != 0) return -2;
   } else if (ov && !fork()) {
     return -2;
   }
@@ -622,7 +629,8 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   if (!early) {
     if (insert_phase(h, n, engine, s) != 0) return -2;
     prof_mark(h, 4, s);
-    writeback_kernel<<<wb_blocks, 256, 0, s>>>(fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st);
+    writeback_kernel<<<wb_blocks, 256, 0, s>>>(fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st,
+                                              fp.sample ? 1 : 0);
     count_launch();
     prof_mark(h, 5, s);
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
@@ -630,7 +638,8 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   if (merge_update_phase(h, n, s) != 0 || delete_apply(h, n, s) != 0 || merge_reserve_phase(h, n, s) != 0)
     return -2;
   prof_mark(h, kEvWbStart, s);
-  writeback_kernel<<<wb_blocks, 256, 0, s>>>(fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st);
+  writeback_kernel<<<wb_blocks, 256, 0, s>>>(fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st,
+                                              fp.sample ? 1 : 0);
   count_launch();
   prof_mark(h, 4, s);
   if (answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess) return -2;
@@ -691,7 +700,7 @@ static int batch_small(Handle* h, const uint64_t* keys, const uint64_t* vals, co
             cudaSuccess)
       return -2;
     writeback_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w.v_a, w.pend, n, &w.counts->n_touch, w.uans,
-                                                                 w.uans_st, out_vals, out_st);
+                                                                 w.uans_st, out_vals, out_st, 1);
     count_launch();
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
   }
@@ -856,7 +865,7 @@ int batch_sorted(Handle* h, const uint64_t* keys, const uint64_t* vals, const ui
   if (insert_phase(h, n, engine, s) != 0) return -2;
   prof_mark(h, 4, s);
   const unsigned wb_blocks = (unsigned)min((size_t)h->sm_count * 8, (n + 255) / 256);
-  writeback_kernel<<<wb_blocks, 256, 0, s>>>(sv, w.pend, n, nullptr, w.uans, w.uans_st, out_vals, out_st);
+  writeback_kernel<<<wb_blocks, 256, 0, s>>>(sv, w.pend, n, nullptr, w.uans, w.uans_st, out_vals, out_st, 0);
   count_launch();
   prof_mark(h, 5, s);
   if (answers_ready(h, s) != 0) return -2;

@@ -32,6 +32,7 @@
 #include "bt_block.cuh"
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_sort.cuh"
 
 namespace bt {
 
@@ -141,18 +142,14 @@ constexpr int kTileItems = 8;
 constexpr int kTile = kTileThreads * kTileItems;  // 2048
 constexpr int kTileWarps = kTileThreads / 32;
 
-__global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t* __restrict__ keys,
-                                                                  const uint8_t* __restrict__ ops, size_t n,
-                                                                  const Slot* __restrict__ tab,
-                                                                  const BatchCounts* __restrict__ counts,
-                                                                  uint8_t* __restrict__ flags,
-                                                                  uint32_t* __restrict__ tile_cnt) {
-  __shared__ uint32_t wsum[kTileWarps];
+// The thread's items of a tile (item j: base + j * kTileThreads + threadIdx.x),
+// their keys and op codes, and a bit per item: touched.
+__device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ keys, const uint8_t* __restrict__ ops,
+                                                   size_t n, const Slot* __restrict__ tab,
+                                                   const BatchCounts* __restrict__ counts, size_t base,
+                                                   uint64_t (&k)[kTileItems], uint8_t (&op)[kTileItems]) {
   const uint32_t mask = counts->cap - 1;
   const bool any = counts->n_ins_req != 0;
-  const size_t base = (size_t)blockIdx.x * kTile;
-  uint64_t k[kTileItems];
-  uint8_t op[kTileItems];
   uint64_t sk[kTileItems];
   uint32_t sf[kTileItems], sh[kTileItems];
   // loads first, then every item's first probe slot (independent loads in
@@ -204,18 +201,36 @@ __global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t
       }
     }
   }
-  uint32_t c = 0;
+  uint32_t touched = 0;
 #pragma unroll
   for (int j = 0; j < kTileItems; j++) {
     const size_t i = base + (size_t)j * kTileThreads + threadIdx.x;
     if (i < n) {
       bool f = op[j] > 2;  // invalid op codes are rejected on the sorted path
       if (!f && any && k[j] != kKeyMax) f = first[j] != kNone && (uint32_t)i >= first[j];
-      flags[i] = f ? 1 : 0;
-      c += f ? 1u : 0u;
+      touched |= (f ? 1u : 0u) << j;
     }
   }
-  c = __reduce_add_sync(0xffffffffu, c);
+  return touched;
+}
+
+__global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t* __restrict__ keys,
+                                                                  const uint8_t* __restrict__ ops, size_t n,
+                                                                  const Slot* __restrict__ tab,
+                                                                  const BatchCounts* __restrict__ counts,
+                                                                  uint8_t* __restrict__ flags,
+                                                                  uint32_t* __restrict__ tile_cnt) {
+  __shared__ uint32_t wsum[kTileWarps];
+  const size_t base = (size_t)blockIdx.x * kTile;
+  uint64_t k[kTileItems];
+  uint8_t op[kTileItems];
+  const uint32_t touched = classify_items(keys, ops, n, tab, counts, base, k, op);
+#pragma unroll
+  for (int j = 0; j < kTileItems; j++) {
+    const size_t i = base + (size_t)j * kTileThreads + threadIdx.x;
+    if (i < n) flags[i] = (touched >> j) & 1u;
+  }
+  const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(touched));
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = c;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -223,6 +238,69 @@ __global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t
 #pragma unroll
     for (int w = 0; w < kTileWarps; w++) t += wsum[w];
     tile_cnt[blockIdx.x] = t;
+  }
+}
+
+// Classify and compact in one launch, for the sample sort, which orders equal
+// keys by their request index: each tile takes its places in the two lists
+// with one atomic each, so the tiles come in any order (requests of a tile stay
+// together and in order).  `flags`-free: the class is used where it is found.
+__global__ void __launch_bounds__(kTileThreads) front_split_kernel(const uint64_t* __restrict__ keys,
+                                                                   const uint8_t* __restrict__ ops, size_t n,
+                                                                   const Slot* __restrict__ tab,
+                                                                   BatchCounts* __restrict__ counts,
+                                                                   uint64_t* __restrict__ tk,
+                                                                   uint32_t* __restrict__ tv,
+                                                                   uint32_t* __restrict__ list,
+                                                                   uint64_t* __restrict__ lk) {
+  __shared__ uint32_t cnt[kTileItems][kTileWarps];
+  __shared__ uint32_t at_touch, at_lookup;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const size_t base = (size_t)blockIdx.x * kTile;
+  uint64_t k[kTileItems];
+  uint8_t op[kTileItems];
+  uint32_t bal[kTileItems];
+  const uint32_t touched = classify_items(keys, ops, n, tab, counts, base, k, op);
+#pragma unroll
+  for (int j = 0; j < kTileItems; j++) {
+    bal[j] = __ballot_sync(0xffffffffu, (touched >> j) & 1u);
+    if (lane == 0) cnt[j][warp] = __popc(bal[j]);
+  }
+  __syncthreads();
+  // exclusive prefix over (item, warp) in index order
+  if (warp == 0) {
+    uint32_t carry = 0;
+#pragma unroll
+    for (int j = 0; j < kTileItems; j++) {
+      const uint32_t c = lane < kTileWarps ? cnt[j][lane] : 0u;
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < kTileWarps; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane < kTileWarps) cnt[j][lane] = carry + incl - c;
+      carry += __shfl_sync(0xffffffffu, incl, kTileWarps - 1);
+    }
+    const uint32_t here = (uint32_t)min((size_t)kTile, n - base);
+    if (lane == 0) at_touch = carry ? atomicAdd(&counts->n_touch, carry) : 0u;
+    if (lane == 1) at_lookup = here > carry ? atomicAdd(&counts->n_lookup, here - carry) : 0u;
+  }
+  __syncthreads();
+  const uint32_t t0 = at_touch, l0 = at_lookup;
+#pragma unroll
+  for (int j = 0; j < kTileItems; j++) {
+    const uint32_t i = (uint32_t)j * kTileThreads + threadIdx.x;
+    if (base + i >= n) continue;
+    const uint32_t p = cnt[j][warp] + __popc(bal[j] & lt);  // touched before it in the tile
+    if ((bal[j] >> lane) & 1u) {
+      tk[t0 + p] = k[j];
+      tv[t0 + p] = pair_payload((uint32_t)(base + i), op[j]);
+    } else {
+      list[l0 + i - p] = (uint32_t)(base + i);
+      lk[l0 + i - p] = k[j];
+    }
   }
 }
 
@@ -649,10 +727,10 @@ cudaError_t pack_expand(const uint8_t* ops, size_t n, const uint64_t* packed, si
   return cudaGetLastError();
 }
 
-// Fills w.f_tk/w.f_tv (touched requests, input order, count counts->n_touch)
-// and w.f_list/w.f_lk (plain lookups and their keys, input order, count
-// counts->n_lookup).
-int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n, cudaStream_t s) {
+// Fills w.f_tk/w.f_tv (touched requests, count counts->n_touch) and
+// w.f_list/w.f_lk (plain lookups and their keys, count counts->n_lookup), in
+// input order when `ordered`.
+int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n, bool ordered, cudaStream_t s) {
   Work& w = h->w;
   BatchCounts* c = w.counts;
   const size_t n_tiles = (n + kTile - 1) / kTile;
@@ -664,6 +742,12 @@ int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n
   front_count_kernel<<<(unsigned)h->sm_count * 2, kThreads, 0, s>>>(ops, n, c);
   front_clear_kernel<<<(unsigned)h->sm_count * 4, kThreads, 0, s>>>(tab, w.f_tab_cap, c);
   front_insert_kernel<<<g, kThreads, 0, s>>>(keys, ops, n, tab, c);
+  if (!ordered) {
+    front_split_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(keys, ops, n, tab, c, w.f_tk, w.f_tv, w.f_list,
+                                                                  w.f_lk);
+    count_launch(4);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   front_flag_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(keys, ops, n, tab, c, flags, tile);
   front_tile_scan_kernel<<<1, 1024, 0, s>>>(tile, (uint32_t)n_tiles, n, c, h->touch_hint_dev);
   front_scatter_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(keys, ops, n, flags, tile, w.f_tk, w.f_tv,

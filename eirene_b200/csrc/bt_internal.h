@@ -57,17 +57,22 @@ cudaError_t radix_sort_pairs(const uint64_t* keys_in, const uint32_t* vals_in, c
                              uint32_t* scratch, cudaStream_t s, uint64_t** k_out, uint32_t** v_out, uint32_t* err,
                              const uint32_t* n_dev = nullptr, int tile_threads = 512);
 
-// Stable sort by key of (key, payload) pairs whose payload carries the
-// request index in its low 30 bits, indices increasing in input order (the
-// hash front end's touched requests): tile sort plus merge rounds; the
-// result is always in (k_a, v_a).  n is the capacity, n_dev the count.
-// touched counts up to which BT_OPT_TOUCH_SORT 2 takes the merge sort
-// (2^18 touched requests: 92 against 126 us for the radix sort; the merge
-// rounds grow with the count, the radix passes with its bytes)
-constexpr uint32_t kMergeSortMax = 1u << 19;
-cudaError_t merge_sort_pairs(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* k_a, uint32_t* v_a,
-                             uint64_t* k_b, uint32_t* v_b, size_t n, const uint32_t* n_dev, int sm_count,
-                             cudaStream_t s, uint64_t** k_out, uint32_t** v_out);
+// ---- sample sort of the touched requests (bt_sample.cu) ----
+// touched counts up to which BT_OPT_TOUCH_SORT 2 takes the sample sort (us a
+// batch of INSERTs on 2^22 keys, sample / radix sort: 2^18 requests 364 / 417,
+// 2^19 487 / 518, 10^6 712 / 726, 1.5 * 10^6 979 / 948: its 512 buckets outgrow a
+// block's shared memory)
+constexpr uint32_t kSampleSortMax = 1u << 20;
+constexpr size_t kSsBuckets = 512;
+struct Handle;
+struct Work;
+size_t sample_sum_bytes();
+int sample_prepare();
+// w.f_tk / w.f_tv (count counts->n_touch, at most n, in any order) sorted by key,
+// then request index, into w.k_a / w.v_a, with the buckets' parts of the
+// segmented scan in w.s_sum; sample_resolve turns those into what merge_pass1 .. 3 write
+int sample_sort(Handle* h, size_t n, cudaStream_t s);
+int sample_resolve(Handle* h, const uint64_t* vals, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s);
 
 // ---- per-batch work buffers, sized for max_batch requests ----
 struct BatchCounts {
@@ -112,6 +117,7 @@ struct BatchSet {
   uint64_t* k_b = nullptr;
   uint32_t* v_a = nullptr;
   uint32_t* v_b = nullptr;
+  void* s_sum = nullptr;
 };
 
 struct Work {
@@ -166,6 +172,9 @@ struct Work {
   uint64_t* lb_status = nullptr;
   uint32_t* lb_ctr = nullptr;
   uint32_t lb_epoch = 0;
+  // sample sort of the touched requests (bt_sample.cu)
+  uint64_t* s_split = nullptr;    // splitters, bucket totals
+  void* s_sum = nullptr;          // per bucket: its part of the segmented scan, its start
   // small batches (bt_small.cu)
   void* s_tab = nullptr;          // hash table, every slot empty between batches
   void* s_sums = nullptr;         // per block: its part of the segmented scan, its edge keys
@@ -316,9 +325,9 @@ struct Handle {
   bool chain_open = false;
   int chain_set = 0;
   int host_front_overlap = 1;  // BT_OPT_HOST_FRONT_OVERLAP
-  // BT_OPT_TOUCH_SORT: 0 onesweep radix sort, 1 tile sort + merge rounds, 2 the
-  // second while the touched count last seen (touch_hint, page-locked and
-  // mapped, written by front_tile_scan_kernel) is at most kMergeSortMax
+  // BT_OPT_TOUCH_SORT: 0 onesweep radix sort, 1 sample sort, 2 the second
+  // while the touched count last seen (touch_hint, page-locked and mapped,
+  // written by either sort's first kernels) is at most kSampleSortMax
   int touch_sort = 2;
   uint32_t* touch_hint = nullptr;
   uint32_t* touch_hint_dev = nullptr;
@@ -451,7 +460,9 @@ cudaError_t gen_sample_requests(uint64_t seed, const uint64_t* sample, size_t n_
                                 uint64_t* keys, uint64_t* vals, uint8_t* ops, cudaStream_t s);
 
 // ---- hash front end of the sorted batch (bt_front.cu) ----
-int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n, cudaStream_t s);
+// ordered: both lists in input order (the radix sort keeps equal keys in it);
+// otherwise tile by tile as the blocks come, in two launches less
+int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n, bool ordered, cudaStream_t s);
 // a whole BT_MODE_STM batch: its GETs first, by the lookup kernels, then its
 // writes as STM transactions (bt_stm.cu)
 int batch_stm(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,

@@ -33,6 +33,7 @@
 #include "bt_internal.h"
 #include "bt_search.cuh"
 #include "bt_small.cuh"
+#include "bt_sort.cuh"
 
 namespace bt {
 
@@ -1072,7 +1073,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
   for (uint32_t i = gt; i < n_touch; i += nt) {
     const uint32_t u = a.pend[i];
     if (u == 0xFFFFFFFFu) continue;  // answered by the front part
-    const uint32_t r = a.sv[i] & 0x3FFFFFFFu;
+    const uint32_t r = pair_idx(a.sv[i]);
     out_vals[r] = a.uans[u];
     out_st[r] = __ldcg(a.uans_st + u);
   }

@@ -29,13 +29,13 @@
 #include "bt_internal.h"
 #include "bt_search.cuh"
 #include "bt_small.cuh"
+#include "bt_sort.cuh"
 
 namespace bt {
 
 namespace {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;
-constexpr uint32_t kIdxMask = 0x3FFFFFFFu;
 constexpr uint32_t kResolved = 0xFFFFFFFFu;
 constexpr int kItems = kSmallItems;
 
@@ -52,142 +52,6 @@ __device__ __forceinline__ uint64_t slot_hash(uint64_t x) {
   x ^= x >> 27;
   x *= 0x94D049BB133111EBull;
   return x ^ (x >> 31);
-}
-
-__device__ __forceinline__ bool pair_less(uint64_t ka, uint32_t va, uint64_t kb, uint32_t vb) {
-  return (ka < kb) | ((ka == kb) & ((va & kIdxMask) < (vb & kIdxMask)));
-}
-
-// bitonic exchange of this lane's element i with its partner i ^ j
-__device__ __forceinline__ void keep(uint64_t& k, uint32_t& v, uint64_t pk, uint32_t pv, int i, int j, int kk) {
-  const bool asc = (i & kk) == 0, lower = (i & j) == 0;
-  const bool p_lt = pair_less(pk, pv, k, v);
-  const bool m_lt = pair_less(k, v, pk, pv);
-  const bool take = (lower == asc) ? p_lt : m_lt;
-  k = take ? pk : k;
-  v = take ? pv : v;
-}
-
-__device__ __forceinline__ void exchange(uint64_t& ka, uint32_t& va, uint64_t& kb, uint32_t& vb, bool asc) {
-  const bool sw = pair_less(kb, vb, ka, va) == asc;
-  const uint64_t k0 = sw ? kb : ka, k1 = sw ? ka : kb;
-  const uint32_t v0 = sw ? vb : va, v1 = sw ? va : vb;
-  ka = k0;
-  kb = k1;
-  va = v0;
-  vb = v1;
-}
-
-// 128 pairs of a warp, four consecutive ones per lane, in ascending order
-__device__ __forceinline__ void warp_sort(uint64_t (&K)[4], uint32_t (&V)[4]) {
-  const int base = (threadIdx.x & 31) * 4;
-#pragma unroll
-  for (int kk = 2; kk <= 128; kk <<= 1) {
-#pragma unroll
-    for (int j = kk >> 1; j >= 4; j >>= 1) {
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const uint64_t pk = __shfl_xor_sync(0xffffffffu, K[e], j / 4);
-        const uint32_t pv = __shfl_xor_sync(0xffffffffu, V[e], j / 4);
-        keep(K[e], V[e], pk, pv, base + e, j, kk);
-      }
-    }
-    if (kk >= 4) {
-      exchange(K[0], V[0], K[2], V[2], (base & kk) == 0);
-      exchange(K[1], V[1], K[3], V[3], ((base + 1) & kk) == 0);
-    }
-    exchange(K[0], V[0], K[1], V[1], (base & kk) == 0);
-    exchange(K[2], V[2], K[3], V[3], ((base + 2) & kk) == 0);
-  }
-}
-
-// this thread's four outputs [d, d + 4) of the merge of the sorted runs
-// (ka, va)[0, la) and (kb, vb)[0, lb) in shared memory
-__device__ __forceinline__ void merge4(const uint64_t* ka, const uint32_t* va, int la, const uint64_t* kb,
-                                       const uint32_t* vb, int lb, int d, uint64_t (&ok)[4], uint32_t (&ov)[4]) {
-  int lo = d > lb ? d - lb : 0, hi = min(d, la);
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (pair_less(ka[mid], va[mid], kb[d - 1 - mid], vb[d - 1 - mid])) lo = mid + 1;
-    else hi = mid;
-  }
-  int ia = lo, ib = d - lo;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (ia + ib >= la + lb) break;
-    const bool take_a = ib >= lb || (ia < la && pair_less(ka[ia], va[ia], kb[ib], vb[ib]));
-    ok[j] = take_a ? ka[ia] : kb[ib];
-    ov[j] = take_a ? va[ia] : vb[ib];
-    ia += take_a ? 1 : 0;
-    ib += take_a ? 0 : 1;
-  }
-}
-
-// The first cnt of a block's pairs in shared memory, sorted: 128-pair runs by
-// warp (registers and shuffles), then merged pairwise.  The bitonic network
-// over the whole tile (ms_tile_kernel) takes 26 us for 2048 pairs, whatever
-// their count; this takes what the count needs.
-__device__ __forceinline__ void block_sort(uint64_t* sk, uint32_t* sv, int cnt) {
-  int P = 128;
-  while (P < cnt) P <<= 1;
-  const int d = threadIdx.x * 4;
-  uint64_t K[4];
-  uint32_t V[4];
-  if (d < P) {
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      K[e] = d + e < cnt ? sk[d + e] : ~0ull;
-      V[e] = d + e < cnt ? sv[d + e] : 0xFFFFFFFFu;  // behind every request
-    }
-    warp_sort(K, V);
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      sk[d + e] = K[e];
-      sv[d + e] = V[e];
-    }
-  }
-  __syncthreads();
-  for (int L = 128; L < P; L <<= 1) {
-    if (d < P) {
-      const int ps = d & ~(2 * L - 1);
-      merge4(sk + ps, sv + ps, L, sk + ps + L, sv + ps + L, L, d - ps, K, V);
-    }
-    __syncthreads();
-    if (d < P) {
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        sk[d + e] = K[e];
-        sv[d + e] = V[e];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// elements of A among the first d of merge(A, B), A = k[a0, a0 + na), B = k[b0, b0 + nb)
-// in global memory; one warp, 32 candidates per step
-__device__ __forceinline__ uint32_t split_of(const uint64_t* k, const uint32_t* v, uint32_t a0, uint32_t na,
-                                             uint32_t b0, uint32_t nb, uint32_t d) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t lo = d > nb ? d - nb : 0, hi = min(d, na);
-  while (lo < hi) {
-    const uint32_t stride = (hi - lo + 31) / 32;
-    const uint32_t a = lo + lane * stride;
-    bool p = false;
-    if (a < hi) {
-      const uint32_t b = b0 + d - 1 - a;
-      p = pair_less(__ldcg(k + a0 + a), __ldcg(v + a0 + a), __ldcg(k + b), __ldcg(v + b));
-    }
-    const uint32_t c = __popc(__ballot_sync(0xffffffffu, p));
-    if (c == 0) {
-      hi = lo;
-    } else {
-      const uint32_t top = lo + c * stride;
-      lo += (c - 1) * stride + 1;
-      hi = min(hi, top);
-    }
-  }
-  return lo;
 }
 
 struct alignas(16) FrontSum {  // one block's part of the segmented scan (read in 16-byte pieces)
@@ -294,7 +158,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       if (i >= n) continue;
       if ((touched >> j) & 1u) {
         f.tk[pt] = k[j];
-        f.tv[pt++] = i | ((op[j] <= 2 ? op[j] : 3u) << 30);
+        f.tv[pt++] = pair_payload(i, op[j]);
       } else {
         f.list[pl] = i;
         f.lk[pl++] = k[j];
@@ -391,8 +255,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     valid |= 1u << j;
     kk[j] = S.k[i];
     const uint32_t p = S.v[i];
-    r[j] = p & kIdxMask;
-    o[j] = p >> 30;
+    r[j] = pair_idx(p);
+    o[j] = pair_op(p);
     const bool h = i > 0 ? S.k[i - 1] != kk[j] : (rank == 0 || k_prev != kk[j]);
     const bool tl = i + 1 < cnt ? S.k[i + 1] != kk[j] : (o0 + i + 1 == m || k_next != kk[j]);
     head |= (h ? 1u : 0u) << j;

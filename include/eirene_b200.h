@@ -310,20 +310,20 @@ int bt_set_search_group(bt_handle *h, uint32_t lanes);
                                       * per-batch buffers (as bt_execute_batches); any other call on the handle
                                       * in between makes the next one wait for it.  0 runs each batch whole on
                                       * `stream`.  Same answers and tree */
-#define BT_OPT_TOUCH_SORT 18 /* hash front end: the sort of the requests whose key a write touches.  1 sorts
-                              * tiles of 2048 pairs on chip, then merges sorted runs pairwise (merge path)
-                              * until one is left: a few rounds for the few hundred thousand such requests
-                              * of a read-mostly batch; 0 the onesweep radix sort (eight passes of 8 bits,
-                              * BT_OPT_SORT_TILE), better for many; 2 (default) the first while the touched
-                              * count of the batch seen last was at most 2^19, else the second (the first
-                              * batch: the second).  Same order in every case (by key, then request order) */
+#define BT_OPT_TOUCH_SORT 18 /* hash front end: the sort of the requests whose key a write touches.  1 splits
+                              * them into buckets of a block's size by sampled splitters and sorts each on
+                              * chip (up to about a million of them); 0 the onesweep radix sort (eight passes
+                              * of 8 bits, BT_OPT_SORT_TILE), better for more; 2 (default) the first while the
+                              * touched count of the batch seen last was at most 2^20, else the second (the
+                              * first batch: the second), and batches of up to 65,536 requests whole in three
+                              * kernels.  Same order in every case (by key, then request order) */
 #define BT_OPT_SORT_TILE 14     /* radix sort tile of sorted batches: 256, 512 (default) or 1024 threads x 8 keys,
                                  * for whole batches and for the hash front end's touched requests alike
                                  * (bt_autotune picks the two separately) */
 #define BT_OPT_LEARNED_MODE 12 /* unsorted learned lookups: 1 one request per lane group, 2 two requests per
-                                * group in lock step, 3 (default) software-pipelined: a group carries up to five
-                                * requests, one in each round of loads (list entry, key, leaf-table probe, leaf
-                                * row, value); bt_autotune picks */
+                                * group in lock step, 3 (default) with 4 lanes one thread per request over the
+                                * leaves' fingerprints, with others software-pipelined: a group carries up to
+                                * five requests, one in each round of loads; bt_autotune picks */
 int bt_set_option(bt_handle *h, int option, int64_t value);
 /* Orders work after every batch issued so far on this handle, its deferred
  * leaf/inner merge included (BT_OPT_ASYNC_WRITE): with a stream, the stream
