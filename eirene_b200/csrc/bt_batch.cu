@@ -479,8 +479,7 @@ static bool merge_usable(const Handle* h, int engine) {
 static int insert_phase(Handle* h, size_t n, int engine, cudaStream_t s) {
   Work& w = h->w;
   // the DELETE runs first: their keys differ from the INSERT runs' keys
-  if (delete_locate(h, n, s) != 0) return -2;
-  if (delete_apply(h, n, s) != 0) return -2;
+  if (locate_phase(h, kLocateDel, n, s) != 0 || delete_apply(h, n, s) != 0) return -2;
   if (merge_usable(h, engine)) return merge_engine(h, n, s) != 0 ? -2 : 0;
   const cudaError_t e =
       launch_stm(h, w.ukeys, w.uvals, nullptr, kOpInsert, w.ins_list, &w.counts->n_ins, n, w.uans, w.uans_st, s);
@@ -524,6 +523,7 @@ struct FrontPart {
   uint32_t* sv = nullptr;
   uint32_t n_tiles = 0;
   bool sample = false;  // sorted by the sample sort (its buckets' sums instead of tile passes)
+  bool cluster = false;  // few enough of them for one cluster to write
   bool passes_done = false;
 };
 
@@ -551,8 +551,11 @@ static int hashed_front(Handle* h, const uint64_t* keys, const uint64_t* vals, c
   // while the touched counts are small (the count of a batch that ran before:
   // a hint, both sorts give the same order)
   fp.sample = h->touch_sort == 1;
-  if (h->touch_sort == 2 && h->touch_hint)
-    fp.sample = *reinterpret_cast<volatile const uint32_t*>(h->touch_hint) <= kSampleSortMax;
+  if (h->touch_sort == 2 && h->touch_hint) {
+    const uint32_t seen = *reinterpret_cast<volatile const uint32_t*>(h->touch_hint);
+    fp.sample = seen <= kSampleSortMax;
+    fp.cluster = seen <= kClusterWriteMax && !h->prof;
+  }
   if (front_classify(h, keys, ops, n, !fp.sample, s) != 0) return -2;
   if (fp.sample) {
     if (sample_sort(h, n, s) != 0) return -2;
@@ -579,6 +582,8 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   const uint32_t* n_touch = &c->n_touch;
   const bool ov = h->overlap != 0;
   const bool early = merge_usable(h, engine);
+  // few touched requests (by the hint that chose the sample sort): the write part of the small batches
+  const bool cluster = early && fp.cluster;
   const bool defer = early && h->async_write != 0;
   const bool learned = batch_learned(h, h->batch_descent >= 0 ? h->batch_descent : h->descent, s);
   // the locates (side stream) run beside the lookups (`s`); so do the merge
@@ -599,8 +604,8 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
     return -2;
   }
   if (early) {
-    if (tree_join(h, s2) != cudaSuccess || delete_locate(h, n, s2) != 0 || merge_locate_phase(h, s2) != 0 ||
-        merge_group_phase(h, n, s2) != 0)
+    if (tree_join(h, s2) != cudaSuccess || locate_phase(h, kLocateIns | kLocateDel, n, s2) != 0 ||
+        (!cluster && merge_group_phase(h, n, s2) != 0))
       return -2;
   }
   prof_mark(h, 2, s2);
@@ -634,6 +639,14 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
     count_launch();
     prof_mark(h, 5, s);
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
+  }
+  if (cluster) {
+    if (small_write(h, out_vals, out_st, kSmallMax, s) != 0 || answers_ready(h, s) != 0) return -2;
+    if (defer) {  // a later call on any stream comes after this batch's writes
+      if (cudaEventRecord(h->tree_ev, s) != cudaSuccess) return -2;
+      h->tree_pending = true;
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   if (merge_update_phase(h, n, s) != 0 || delete_apply(h, n, s) != 0 || merge_reserve_phase(h, n, s) != 0)
     return -2;

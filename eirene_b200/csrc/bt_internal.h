@@ -139,7 +139,7 @@ struct Work {
   uint64_t* tile_carry = nullptr;  // scratch for the tile pass
   BatchCounts* counts = nullptr;
   // segmented leaf merge (bt_merge.cu)
-  uint32_t* m_path = nullptr;   // [cap][8] root-to-leaf path of each unique insert
+  uint32_t* m_path = nullptr;   // [8][cap] per level the node on each unique insert's path
   uint64_t* m_vpos = nullptr;   // [cap] value slot (node * 32 + slot) of an existing key, or ~0
   uint32_t* m_leaf = nullptr;
   uint32_t* m_isnew = nullptr;
@@ -281,6 +281,7 @@ struct Handle {
   int front_end = 1;         // sorted batches: 1 = hash front end (sort only INSERT-coupled requests), 0 = full sort
   int top_cache = 1;         // unsorted searches descend the upper levels from shared memory
   int search_pairs = 2;      // unsorted searches: 2 pairs of requests per lane group, child ids only; 1 pairs; 0 single
+  bool has_root = false;     // the tree surely has a root (false: it may have)
   bool pfx_valid = false;    // tree.pfx and tree.fp match the rows (false after a loaded pool image)
   int use_pfx = 1;           // paired searches compare the separators' 32-bit prefixes first
   void* top = nullptr;       // top cache (kTopNodes nodes) + TopInfo
@@ -450,8 +451,7 @@ cudaError_t launch_stm(Handle* h, const uint64_t* keys, const uint64_t* vals, co
                        cudaStream_t s, const uint8_t* skip = nullptr);
 
 // ---- delete phase of the sorted batch (bt_delete.cu) ----
-// locate: reads the tree only (answers the DELETE runs); apply: removes the keys
-int delete_locate(Handle* h, size_t n_upper, cudaStream_t s);
+// removes the DELETE keys that locate_phase found
 int delete_apply(Handle* h, size_t n_upper, cudaStream_t s);
 
 // ---- workload generators (bt_workload.cu) ----
@@ -502,6 +502,11 @@ int unroute_results(Handle* h, const uint32_t* perm, const uint64_t* in_vals, co
 
 // ---- sorted batches of up to kSmallMax requests (bt_small.cu; the write part in bt_merge.cu) ----
 constexpr size_t kSmallMax = 65536;
+// touched count (seen last) up to which a larger batch's write part is the small
+// batches' one too (us a batch on 2^23 keys, its own twelve launches / one: 100,000
+// requests with 1000 writes 133 / 102, 20,000 175 / 169; 400,000 with 20,000 196 /
+// 187, 40,000 222 / 237)
+constexpr uint32_t kClusterWriteMax = 20480;
 int small_prepare();
 int small_write_prepare();
 int small_alloc(Work* w);
@@ -540,8 +545,8 @@ int batch_chained(Handle* h, const uint64_t* keys, const uint64_t* vals, const u
 // ---- segmented leaf merge (bt_merge.cu) ----
 int merge_engine(Handle* h, size_t n_upper, cudaStream_t s);
 // the same in five parts:
-//   locate   descents of the pre-batch tree, answers of the INSERT runs
-//            (reads the tree only);
+//   locate   descents of the pre-batch tree, answers of the INSERT (and
+//            DELETE) runs (reads the tree only);
 //   update   new values of the existing keys, in place (after the batch's
 //            plain lookups, before its DELETE apply);
 //   group    the new keys and their runs per leaf (no tree access);
@@ -549,7 +554,9 @@ int merge_engine(Handle* h, size_t n_upper, cudaStream_t s);
 //            apply), node reservation, kNoCapacity answers when it fails;
 //   write    leaf merge and inner levels: reads only the merge scratch
 //            (m_*), so the next batch's front end and sort may run beside it.
-int merge_locate_phase(Handle* h, cudaStream_t s);
+// what: kLocateIns | kLocateDel
+constexpr int kLocateIns = 1, kLocateDel = 2;
+int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s);
 int merge_update_phase(Handle* h, size_t n_upper, cudaStream_t s);
 int merge_group_phase(Handle* h, size_t n_upper, cudaStream_t s);
 int merge_reserve_phase(Handle* h, size_t n_upper, cudaStream_t s);

@@ -31,6 +31,7 @@
 #include "bt_common.cuh"
 #include "bt_delete.cuh"
 #include "bt_internal.h"
+#include "bt_rows.cuh"
 #include "bt_search.cuh"
 #include "bt_small.cuh"
 #include "bt_sort.cuh"
@@ -60,42 +61,6 @@ constexpr uint64_t kNoPos = ~0ull;  // merge_locate_kernel: no value to update i
 constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
-
-// S slots of a row that this kernel also writes (plain loads: the read-only
-// path must not be used for it)
-template <int S>
-__device__ __forceinline__ void load_row16(const uint64_t* p, uint64_t (&x)[S]) {
-#pragma unroll
-  for (int i = 0; i < S; i += 2) {
-    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(p + i);
-    x[i] = w.x;
-    x[i + 1] = w.y;
-  }
-}
-
-// the fingerprints of a lane's four slots of leaf nd (G = 8); slot 31's byte,
-// the split count, is `splits` unless that is negative (then it stays)
-__device__ __forceinline__ void store_fp4(const DevTree& t, uint32_t nd, uint32_t g, const uint64_t (&k)[4],
-                                          int splits) {
-  uint8_t* p = t.fp + (size_t)nd * 32 + g * 4;
-  uint32_t w = 0;
-#pragma unroll
-  for (int i = 0; i < 3; i++) w |= (uint32_t)slot_fp(k[i]) << (8 * i);
-  if (g < 7) {
-    *reinterpret_cast<uint32_t*>(p) = w | (uint32_t)slot_fp(k[3]) << 24;
-  } else if (splits >= 0) {
-    *reinterpret_cast<uint32_t*>(p) = w | (uint32_t)splits << 24;
-  } else {
-    *reinterpret_cast<uint16_t*>(p) = (uint16_t)w;
-    p[2] = (uint8_t)(w >> 16);
-  }
-}
-
-template <int S>
-__device__ __forceinline__ void store_row16(uint64_t* p, const uint64_t (&x)[S]) {
-#pragma unroll
-  for (int i = 0; i < S; i += 2) *reinterpret_cast<ulonglong2*>(p + i) = make_ulonglong2(x[i], x[i + 1]);
-}
 
 // piece index and slot of merged position `pos` when m items are spread over p
 // pieces (the first m % p pieces hold one more)
@@ -134,139 +99,61 @@ __device__ __forceinline__ uint32_t count_less(const uint64_t* a, uint32_t n, ui
 __global__ void merge_ensure_root_kernel(DevTree t) { ensure_root_leaf(t); }
 
 // ------------------------------------------------------------- locate ----
-template <int G>
-__global__ void __launch_bounds__(256) merge_locate_kernel(DevTree t, const uint64_t* __restrict__ ukeys,
-                                                           const uint64_t* __restrict__ uvals,
-                                                           const uint32_t* __restrict__ ins_list,
-                                                           const uint32_t* __restrict__ n_dev,
-                                                           uint32_t* __restrict__ path, uint32_t* __restrict__ mleaf,
-                                                           uint32_t* __restrict__ isnew,
-                                                           uint64_t* __restrict__ vpos, uint64_t* __restrict__ uans,
-                                                           uint8_t* __restrict__ uans_st, int use_pfx) {
-  constexpr int S = 32 / G;
+// The batch's unique INSERT and DELETE keys in the pre-batch tree, 32 to a warp
+// (warp_descend): the leaf, the slot of a key that is there (by the leaf's
+// fingerprints) and its value, and for an INSERT key the inner nodes of its path.
+// Reads only.  A run of keys per 8-lane group with path reuse and whole rows took
+// 80 us for 2^19 INSERT keys on 2^24 keys and 140 for as many DELETE keys with a
+// descent each; this takes 40 for either.
+struct LocateArgs {
+  const BatchCounts* counts;
+  const uint64_t* ukeys;
+  const uint32_t *ins_list, *del_list;
+  uint32_t *path, *mleaf, *isnew;
+  uint64_t* vpos;
+  uint32_t *dleaf, *dslot;
+  uint64_t* uans;
+  uint8_t* uans_st;
+  size_t path_stride;
+};
+
+__global__ void __launch_bounds__(256) locate_kernel(DevTree t, LocateArgs a, int what) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t g = lane % G;
-  const uint32_t gmask = group_mask<G>(lane);
-  const size_t n = *n_dev;
-  const uint32_t root = t.ctrl->root;
-  const uint32_t root_level = t.ctrl->root_level;
-  const size_t n_groups = ((size_t)gridDim.x * blockDim.x) / G;
-  const size_t gid = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const size_t chunk = (n + n_groups - 1) / n_groups;
-  const size_t q0 = gid * chunk;
-  const size_t q1 = min(n, q0 + chunk);
-  const bool usable = root != kNil && root_level < (uint32_t)kPathLevels;
-  uint32_t c_node = root;
-  uint64_t c_hi = 0;
-  bool c_valid = (g == root_level);
-  if (c_valid) c_hi = kKeyMax;
-  uint64_t k[S];
-  uint64_t v[S];
-  uint32_t leaf = kNil;
-  for (size_t q = q0; q < q1; q++) {
-    const uint32_t u = ins_list[q];
-    const uint64_t key = ukeys[u];
-    if (!usable) {  // no root (pool exhausted) or a tree too tall for the path record
-      if (g == 0) {
-        uans[u] = 0;
-        uans_st[u] = kNoCapacity;
-        isnew[q] = 0;
-        vpos[q] = kNoPos;
-      }
-      continue;
+  const uint32_t n_ins = (what & kLocateIns) ? a.counts->n_ins : 0, n_del = (what & kLocateDel) ? a.counts->n_del : 0;
+  const uint32_t ti = ceil_div(n_ins, 32), td = ceil_div(n_del, 32);
+  const uint32_t root = t.ctrl->root, root_level = t.ctrl->root_level;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ti + td; w += warps) {
+    const bool del = w >= ti;
+    const uint32_t q = (del ? w - ti : w) * 32 + lane;
+    const bool live = q < (del ? n_del : n_ins);
+    const uint32_t u = live ? (del ? a.del_list : a.ins_list)[q] : 0;
+    const uint64_t key = live ? a.ukeys[u] : 0;
+    // no root (pool exhausted), or a tree too tall for the path record
+    const bool usable = root != kNil && (del || root_level < (uint32_t)kPathLevels);
+    uint32_t leaf = kNil, slot = kNoSlot;
+    uint64_t val = 0;
+    if (usable) {
+      leaf = warp_descend(t, root, root_level, key, [&](uint32_t level, uint32_t node) {
+        if (live && !del) a.path[level * a.path_stride + q] = node;
+      });
+      uint64_t row[4];
+      ldg32_hint(t.fp + (size_t)leaf * 32, row, l2_keep());
+      if (live) leaf_pick(t, leaf, key, fp_match(row, key_fp(key)), l2_stream(), val, slot);
     }
-    const uint32_t hit = (__ballot_sync(gmask, c_valid && key < c_hi) >> (lane - g)) & ((1u << G) - 1u);
-    uint32_t level = hit ? (uint32_t)(__ffs(hit) - 1) : root_level;
-    uint32_t node = __shfl_sync(gmask, c_node, level, G);
-    uint64_t hi = __shfl_sync(gmask, c_hi, level, G);
-    if (!hit) {
-      node = root;
-      hi = kKeyMax;
-    }
-    if (g < level) c_valid = false;
-    uint32_t cnt = 0;
-    if (level == 0 && node == leaf) {
-      uint32_t c = 0;
-#pragma unroll
-      for (int i = 0; i < S; i++) c += (k[i] <= key) ? 1u : 0u;
-      cnt = group_sum<G>(c, gmask);
+    if (!live) continue;
+    const bool found = slot != kNoSlot;
+    a.uans[u] = val;
+    a.uans_st[u] = found ? kFound : (del || usable) ? kAbsent : kNoCapacity;
+    if (del) {
+      a.dleaf[q] = leaf;
+      a.dslot[q] = slot;
     } else {
-      for (;;) {
-        const size_t row = (size_t)node * 32 + g * S;
-        if (use_pfx && level > 0) {
-          // inner level from the separators' prefixes, then the one separator
-          // (the child's upper bound) and the one child id
-          uint32_t pf[S];
-          load_pfx<S>(t.pfx + row, pf, l2_keep());
-          const uint32_t x = pfx_rank<G, S>(pf, key, g, gmask);
-          cnt = x & 0xffffu;
-          if (x >> 16) {  // a separator shares the key's prefix: rank with the full keys
-            load_slots<S>(t.keys + row, k);
-            if (g == G - 1) k[S - 1] = kKeyMax;
-            uint32_t c = 0;
-#pragma unroll
-            for (int i = 0; i < S; i++) c += (k[i] <= key) ? 1u : 0u;
-            cnt = group_sum<G>(c, gmask);
-          }
-          // the separator after the chosen child (slot 31 is the header: none)
-          const uint64_t sep = cnt < 31 ? t.keys[(size_t)node * 32 + cnt] : kKeyMax;
-          const uint64_t child_hi = sep < hi ? sep : hi;
-          node = (uint32_t)t.vals[(size_t)node * 32 + cnt];
-          hi = child_hi;
-          level--;
-          if (g == level) {
-            c_node = node;
-            c_hi = hi;
-            c_valid = true;
-          }
-          continue;
-        }
-        load_slots<S>(t.keys + row, k);
-        if (level > 0) load_slots<S>(t.vals + row, v);
-        if (g == G - 1) k[S - 1] = kKeyMax;
-        uint32_t c = 0;
-#pragma unroll
-        for (int i = 0; i < S; i++) c += (k[i] <= key) ? 1u : 0u;
-        cnt = group_sum<G>(c, gmask);
-        if (level == 0) break;
-        const uint64_t sep = __shfl_sync(gmask, pick<S>(k, cnt % S), cnt / S, G);
-        const uint64_t child_hi = sep < hi ? sep : hi;
-        node = (uint32_t)__shfl_sync(gmask, pick<S>(v, cnt % S), cnt / S, G);
-        hi = child_hi;
-        level--;
-        if (g == level) {
-          c_node = node;
-          c_hi = hi;
-          c_valid = true;
-        }
-      }
-      leaf = node;
-    }
-    // record the path: lane g holds level g
-    if (g <= root_level) path[q * kPathLevels + g] = c_node;
-    bool exists = false;
-    uint32_t slot = 0;
-    if (cnt > 0) {
-      slot = cnt - 1;
-      const uint64_t kk = __shfl_sync(gmask, pick<S>(k, slot % S), slot / S, G);
-      exists = kk == key;
-    }
-    if (g == 0) {
-      if (exists) {
-        // the new value goes in later (merge_update_kernel): a plain lookup
-        // of this key that comes before its first write must still see it
-        const uint64_t p = (uint64_t)leaf * 32 + slot;
-        uans[u] = t.vals[p];
-        uans_st[u] = kFound;
-        vpos[q] = p;
-        isnew[q] = 0;
-      } else {
-        uans[u] = 0;
-        uans_st[u] = kAbsent;
-        isnew[q] = 1;
-        vpos[q] = kNoPos;
-        mleaf[q] = leaf;
-      }
+      // an existing key's new value goes in later (merge_update_kernel): a plain
+      // lookup of it that comes before its first write must still see the old one
+      a.vpos[q] = found ? (uint64_t)leaf * 32 + slot : kNoPos;
+      a.isnew[q] = usable && !found ? 1u : 0u;
+      a.mleaf[q] = leaf;
     }
   }
 }
@@ -735,7 +622,7 @@ struct InnerSmem {
 template <int NT, typename Team>
 __device__ __forceinline__ void inner_merge(const DevTree& t, uint32_t inner_fill, uint32_t entry_cap,
                                             MergeCounts* mc, InnerSync* gs, MergeEntry* ea, MergeEntry* eb,
-                                            const uint32_t* path, uint32_t* gstart, uint32_t* goff, uint32_t* kids_a,
+                                            const uint32_t* path, size_t path_stride, uint32_t* gstart, uint32_t* goff, uint32_t* kids_a,
                                             uint32_t* kids_b, const Team& team, InnerSmem<NT>& sm) {
   constexpr int NW = NT / 32;
   Ctrl* C = t.ctrl;
@@ -800,7 +687,7 @@ __device__ __forceinline__ void inner_merge(const DevTree& t, uint32_t inner_fil
       break;
     }
     // groups of entries sharing a parent at this level
-    auto parent_of = [&](uint32_t i) { return path[(size_t)cur[i].rep * kPathLevels + lvl]; };
+    auto parent_of = [&](uint32_t i) { return path[lvl * path_stride + cur[i].rep]; };
     auto is_head = [&](uint32_t i) -> uint32_t { return (i == 0 || parent_of(i) != parent_of(i - 1)) ? 1u : 0u; };
     uint32_t ng = 0;
     if (!team_scan<NT>(team, n_e, is_head, goff, gs, sm.ws, &ng)) return;
@@ -914,13 +801,14 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
                                                                     MergeCounts* mc, InnerSync* gs,
                                                                     MergeEntry* ea, MergeEntry* eb,
                                                                     const uint32_t* __restrict__ path,
+                                                                    size_t path_stride,
                                                                     uint32_t* __restrict__ gstart,
                                                                     uint32_t* __restrict__ goff,
                                                                     uint32_t* __restrict__ kids_a,
                                                                     uint32_t* __restrict__ kids_b) {
   __shared__ InnerSmem<kInnerThreads> sm;
   if (mc->cap_fail) return;
-  inner_merge<kInnerThreads>(t, inner_fill, entry_cap, mc, gs, ea, eb, path, gstart, goff, kids_a, kids_b,
+  inner_merge<kInnerThreads>(t, inner_fill, entry_cap, mc, gs, ea, eb, path, path_stride, gstart, goff, kids_a, kids_b,
                              GridTeam{gs, &t.ctrl->error}, sm);
 }
 
@@ -953,6 +841,7 @@ struct SmallWrite {
   MergeEntry *ea, *eb;
   uint32_t* sums;  // three sets of 16 block totals
   uint32_t leaf_fill, inner_fill, entry_cap;
+  size_t path_stride;
 };
 
 // exclusive prefix of v over the threads of the cluster and the total; one
@@ -998,12 +887,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
       removed += del_apply_at(t, a.dleaf, a.dslot, i, n_del, threadIdx.x & 31);
     if ((threadIdx.x & 31) == 0 && removed) atomicAdd(&t.ctrl->n_keys, (unsigned long long)0 - removed);
   }
-  // this thread's four consecutive items of n spread over the cluster
+  // this thread's consecutive items of n spread over the cluster: one while there
+  // are threads enough (several would be that many chains of loads in a row)
   auto mine = [&](uint32_t n, uint32_t& i0, uint32_t& i1) {
-    const uint32_t per = (ceil_div(n, C) + 3u) & ~3u;
-    i0 = min(n, rank * per + threadIdx.x * 4);
-    i1 = min(min(n, (rank + 1) * per), i0 + 4);
-    if (i1 < i0) i1 = i0;
+    const uint32_t each = ceil_div(n, nt);
+    i0 = (uint32_t)min((uint64_t)n, (uint64_t)gt * each);
+    i1 = min(n, i0 + each);
   };
   uint32_t n_new = 0, n_segs = 0, n_ent = 0;
   if (n_ins) {
@@ -1025,37 +914,41 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
   if (n_new) {
     cluster_sync();
     // runs of new keys that share a leaf
-    uint32_t i0, i1, v = 0, heads = 0;
+    uint32_t i0, i1, v = 0;
     mine(n_new, i0, i1);
-    uint32_t lf[4];
+    const uint32_t before = i0 > 0 && i0 < i1 ? __ldcg(a.nleaf + i0 - 1) : kNil;  // kNil: no leaf
+    uint32_t prev = before;
     for (uint32_t i = i0; i < i1; i++) {
-      lf[i - i0] = __ldcg(a.nleaf + i);
-      const bool h = i == 0 || (i > i0 ? lf[i - i0 - 1] : __ldcg(a.nleaf + i - 1)) != lf[i - i0];
-      heads |= (h ? 1u : 0u) << (i - i0);
-      v += h ? 1u : 0u;
+      const uint32_t lf = __ldcg(a.nleaf + i);
+      v += lf != prev ? 1u : 0u;
+      prev = lf;
     }
     uint32_t p = cluster_scan(v, a.sums + 16, S, &n_segs);
-    for (uint32_t i = i0; i < i1; i++)
-      if ((heads >> (i - i0)) & 1u) {
+    prev = before;
+    for (uint32_t i = i0; i < i1; i++) {
+      const uint32_t lf = __ldcg(a.nleaf + i);
+      if (lf != prev) {
         a.seg[p] = i;
-        a.leaf[p++] = lf[i - i0];
+        a.leaf[p++] = lf;
       }
+      prev = lf;
+    }
     cluster_sync();
     // new leaves per run
     mine(n_segs, i0, i1);
-    uint32_t ex[4];
     v = 0;
     for (uint32_t i = i0; i < i1; i++) {
       const uint32_t b = __ldcg(a.seg + i), e = i + 1 < n_segs ? __ldcg(a.seg + i + 1) : n_new;
       const uint32_t m = hdr_size(__ldcg(t.keys + (size_t)__ldcg(a.leaf + i) * 32 + 31)) + (e - b);
-      ex[i - i0] = m <= (uint32_t)kMaxKeys ? 0u : ceil_div(m, a.leaf_fill) - 1;
-      v += ex[i - i0];
+      const uint32_t x = m <= (uint32_t)kMaxKeys ? 0u : ceil_div(m, a.leaf_fill) - 1;
+      a.isnew[i] = x;
+      v += x;
     }
     p = cluster_scan(v, a.sums + 32, S, &n_ent);
     for (uint32_t i = i0; i < i1; i++) {
-      a.isnew[i] = ex[i - i0];
+      const uint32_t x = a.isnew[i];
       a.pos[i] = p;
-      p += ex[i - i0];
+      p += x;
     }
   }
   if (gt == 0) {
@@ -1082,7 +975,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
                                           a.ea, S.leaf, gt / 8, nt / 8);
   if (n_ent == 0) return;
   cluster_sync();
-  inner_merge<kSmallThreads>(t, a.inner_fill, a.entry_cap, mc, a.gs, a.ea, a.eb, a.path, a.seg, a.nleaf, a.nq, a.pos,
+  inner_merge<kSmallThreads>(t, a.inner_fill, a.entry_cap, mc, a.gs, a.ea, a.eb, a.path, a.path_stride, a.seg, a.nleaf, a.nq, a.pos,
                              ClusterTeam{}, S.inner);
 }
 
@@ -1114,37 +1007,42 @@ static cudaError_t launch_inner(Handle* h, uint32_t entry_cap, MergeCounts* mc, 
   MergeEntry* ea = reinterpret_cast<MergeEntry*>(w.m_ent_a);
   MergeEntry* eb = reinterpret_cast<MergeEntry*>(w.m_ent_b);
   const uint32_t* path = w.m_path;
+  size_t path_stride = w.cap;
   uint32_t* gstart = w.m_seg;
   uint32_t* goff = w.m_nleaf;
   uint32_t* kids_a = w.m_nq;
   uint32_t* kids_b = w.m_pos;
-  void* args[] = {&tree, &fill, &entry_cap, &mc, &gs, &ea, &eb, &path, &gstart, &goff, &kids_a, &kids_b};
+  void* args[] = {&tree, &fill, &entry_cap, &mc, &gs, &ea, &eb, &path, &path_stride, &gstart, &goff, &kids_a, &kids_b};
   e = cudaLaunchCooperativeKernel((const void*)merge_inner_kernel, dim3(blocks), dim3(kInnerThreads), args, 0, s);
   count_launch();
   return e;
 }
 
-// Runs the merge engine for the unique INSERT keys of the current batch
-// (w.ins_list, count on the device).  n_upper bounds the count.
-int merge_locate_phase(Handle* h, cudaStream_t s) {
+int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
-  MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
-  const uint32_t* n_ins = &w.counts->n_ins;
-  merge_ensure_root_kernel<<<1, 1, 0, s>>>(h->tree);
-  count_launch();
-  const int use_pfx = h->use_pfx ? 1 : 0;
-  if (use_pfx && ensure_pfx(h, s) != cudaSuccess) return -2;
-  if (cudaMemsetAsync(mc, 0, sizeof(MergeCounts), s) != cudaSuccess) return -2;
-  static int per_sm[64] = {};
-  if (h->device < 64 && per_sm[h->device] == 0) {
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, merge_locate_kernel<8>, 256, 0) != cudaSuccess || b < 1)
-      b = 4;
-    per_sm[h->device] = b;
+  // the INSERT keys need a root; once there is one only a new tree takes it away
+  if ((what & kLocateIns) && !h->has_root) {
+    merge_ensure_root_kernel<<<1, 1, 0, s>>>(h->tree);
+    count_launch();
+    h->has_root = true;
   }
-  const size_t blocks = (size_t)h->sm_count * (h->device < 64 ? per_sm[h->device] : 4);
-  merge_locate_kernel<8><<<(unsigned)blocks, 256, 0, s>>>(h->tree, w.ukeys, w.uvals, w.ins_list, n_ins, w.m_path,
-                                                          w.m_leaf, w.m_isnew, w.m_vpos, w.uans, w.uans_st, use_pfx);
+  if (ensure_pfx(h, s) != cudaSuccess) return -2;
+  LocateArgs a;
+  a.counts = w.counts;
+  a.ukeys = w.ukeys;
+  a.ins_list = w.ins_list;
+  a.del_list = w.del_list;
+  a.path = w.m_path;
+  a.mleaf = w.m_leaf;
+  a.isnew = w.m_isnew;
+  a.vpos = w.m_vpos;
+  a.dleaf = w.d_leaf;
+  a.dslot = w.d_slot;
+  a.uans = w.uans;
+  a.uans_st = w.uans_st;
+  a.path_stride = w.cap;
+  const unsigned blocks = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256 + 1);
+  locate_kernel<<<blocks, 256, 0, s>>>(h->tree, a, what);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1229,6 +1127,7 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaSt
   a.dleaf = w.d_leaf;
   a.dslot = w.d_slot;
   a.path = w.m_path;
+  a.path_stride = w.cap;
   a.vpos = w.m_vpos;
   a.isnew = w.m_isnew;
   a.pos = w.m_pos;
@@ -1253,7 +1152,7 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaSt
 }
 
 int merge_engine(Handle* h, size_t n_upper, cudaStream_t s) {
-  if (merge_locate_phase(h, s) != 0 || merge_update_phase(h, n_upper, s) != 0 ||
+  if (locate_phase(h, kLocateIns, n_upper, s) != 0 || merge_update_phase(h, n_upper, s) != 0 ||
       merge_group_phase(h, n_upper, s) != 0 || merge_reserve_phase(h, n_upper, s) != 0)
     return -2;
   return merge_write_phase(h, s);

@@ -169,7 +169,7 @@ __device__ __forceinline__ uint32_t fp_match(const uint64_t (&row)[4], uint32_t 
 // keys and values are loaded at once (a wrong first one: one lookup in ten;
 // a third one: one in 250).
 __device__ __forceinline__ bool leaf_pick(const DevTree& t, uint32_t node, uint64_t key, uint32_t m, uint64_t pol,
-                                          uint64_t& val) {
+                                          uint64_t& val, uint32_t& slot) {
   const uint64_t* kr = t.keys + (size_t)node * 32;
   const uint64_t* vr = t.vals + (size_t)node * 32;
   val = 0;
@@ -186,10 +186,16 @@ __device__ __forceinline__ bool leaf_pick(const DevTree& t, uint32_t node, uint6
     m &= m - 1;
     if (k0 == key || k1 == key) {
       val = k0 == key ? v0 : v1;
+      slot = k0 == key ? s0 : s1;
       return true;
     }
   }
   return false;
+}
+__device__ __forceinline__ bool leaf_pick(const DevTree& t, uint32_t node, uint64_t key, uint32_t m, uint64_t pol,
+                                          uint64_t& val) {
+  uint32_t slot;
+  return leaf_pick(t, node, key, m, pol, val, slot);
 }
 
 // ---- descent of 32 keys by one warp ----
@@ -216,8 +222,11 @@ __device__ __forceinline__ uint32_t rank8(const uint32_t (&p)[8], uint32_t kp) {
   return (c1 ? 4u : 0u) + (c2 ? 2u : 0u) + (c3 ? 1u : 0u) + (p[7] < kp ? 1u : 0u) + (ub == kp ? kEqBit : 0u);
 }
 
-// every lane of the warp calls it, with any key; returns the lane's leaf
-__device__ __forceinline__ uint32_t warp_descend(const DevTree& t, uint32_t root, uint32_t root_level, uint64_t key) {
+// every lane of the warp calls it, with any key; returns the lane's leaf;
+// visit(level, node): the inner nodes on the lane's way
+template <typename F>
+__device__ __forceinline__ uint32_t warp_descend(const DevTree& t, uint32_t root, uint32_t root_level, uint64_t key,
+                                                 F visit) {
   const uint32_t lane = threadIdx.x & 31, g = lane & 3u;
   const uint64_t keep = l2_keep();
   uint32_t kp[4];
@@ -225,6 +234,7 @@ __device__ __forceinline__ uint32_t warp_descend(const DevTree& t, uint32_t root
   for (int j = 0; j < 4; j++) kp[j] = __shfl_sync(0xffffffffu, (uint32_t)(key >> 32), 8 * j + (lane >> 2));
   uint32_t node = root;
   for (uint32_t level = root_level; level > 0; level--) {
+    visit(level, node);
     uint32_t sum = 0;
     uint32_t p[4][8];
 #pragma unroll
@@ -277,7 +287,7 @@ __device__ __forceinline__ uint8_t warp_lookup(const DevTree& t, uint32_t root, 
   val = 0;
   if (root == kNil) return key == kKeyMax ? kRejected : kAbsent;
   const bool usable = live && key != kKeyMax;
-  const uint32_t leaf = warp_descend(t, root, root_level, usable ? key : 0);
+  const uint32_t leaf = warp_descend(t, root, root_level, usable ? key : 0, [](uint32_t, uint32_t) {});
   if (!usable) return kRejected;
   uint64_t row[4];
   ldg32_hint(t.fp + (size_t)leaf * 32, row, l2_keep());

@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kReadThreads) small_read_kernel(DevTree t, Sma
         slot = cnt ? cnt - 1 : 0;
         const uint64_t kk = __shfl_sync(gmask, pick<S>(k, slot % S), slot / S, kLocG);
         found = cnt > 0 && kk == key;
-        if (!del && g <= root_level) a.path[(size_t)q * kLocG + g] = path;
+        if (!del && g > 0 && g <= root_level) a.path[g * a.path_stride + q] = path;
       }
       if (g == 0) {
         a.uans[u] = found ? __ldg(t.vals + (size_t)leaf * 32 + slot) : 0;
@@ -589,6 +589,7 @@ int small_read(Handle* h, bool gets, bool locate_ins, uint64_t* out_vals, uint8_
   a.ins_list = w.ins_list;
   a.del_list = w.del_list;
   a.path = w.m_path;
+  a.path_stride = w.cap;
   a.mleaf = w.m_leaf;
   a.isnew = w.m_isnew;
   a.vpos = w.m_vpos;

@@ -75,6 +75,7 @@ struct SmallRead {
   uint32_t *dleaf, *dslot;
   uint64_t* uans;
   uint8_t* uans_st;
+  size_t path_stride;
   int locate_ins;  // 0: the STM kernel inserts
 };
 

@@ -261,6 +261,7 @@ int bt_load_image(bt_handle* h, const char* path) {
     H.epoch = c.epoch;  // the rows carry the saved tree's epoch
     H.L.valid = false;
     H.pfx_valid = false;
+    H.has_root = false;
   }
   if (prev >= 0) cudaSetDevice(prev);
   return rc;

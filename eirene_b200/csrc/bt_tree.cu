@@ -771,6 +771,7 @@ cudaError_t clear_headers(Handle* h, uint32_t first, uint32_t last, cudaStream_t
 }
 
 cudaError_t tree_reset(Handle* h, cudaStream_t s) {
+  h->has_root = false;
   h->pfx_valid = true;  // no nodes: every writer from here on keeps the two tables
   // The epoch has 15 bits (1 .. 0x7fff; 0 marks never-written rows).  When
   // it comes round to 1 again, rows written by the trees of the last cycle
@@ -828,6 +829,7 @@ int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* val
       cudaMemcpyAsync(status, &geo->status, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return -2;
+  h->has_root = *status == 0;
   return *status == kBuildReserved ? -5 : *status == kBuildCapacity ? -4 : 0;
 }
 
