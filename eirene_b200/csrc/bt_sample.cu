@@ -102,7 +102,8 @@ __device__ __forceinline__ uint32_t item_state(uint64_t k, uint32_t v, bool head
 }
 
 // one bucket per 1024 pairs while every SM has one at most, then whole waves of
-// at most 1536
+// at most 1536 (one per 1024 throughout, with a last wave a fraction full: 2^19
+// pairs 8 us more)
 __device__ __forceinline__ uint32_t bucket_count(uint32_t m, uint32_t sms) {
   uint32_t p = (m + 1023) / 1024;
   if (p > sms) p = sms * ((m + sms * 1536 - 1) / (sms * 1536));
@@ -129,8 +130,11 @@ __global__ void __launch_bounds__(1024, 1) ss_splitters_kernel(const uint64_t* _
   if (threadIdx.x < kBuckets) total[threadIdx.x] = 0;
   if (threadIdx.x == 0 && hint) *reinterpret_cast<volatile uint32_t*>(hint) = *n_dev;  // host memory: a later batch's sort choice
   if (p == 1) return;
-  uint32_t s = 512;  // eight samples per bucket or more: the largest bucket about twice the mean
-  while (s < 8 * p && s < (uint32_t)kCap) s <<= 1;
+  // four samples per bucket or more (the largest bucket about 2.5 times the mean),
+  // eight when the buckets are more than 3/8 full: this block's sort is the longest
+  // step of the splitting (34 us for 4096 samples, half for 2048)
+  uint32_t s = 512;
+  while (s < (m > p * 1536 ? 8 : 4) * p && s < (uint32_t)kCap) s <<= 1;
   const uint32_t step = m / s;
   for (uint32_t i = threadIdx.x; i < s; i += blockDim.x) {
     const uint32_t at = (uint32_t)((uint64_t)i * m / s) + (i * 0x9E3779B1u >> 8) % (step ? step : 1u);
@@ -417,7 +421,7 @@ __global__ void __launch_bounds__(1024, 1) ss_sort_kernel(uint32_t n_upper, cons
 }
 
 constexpr int kResThreads = 512;
-constexpr int kResItems = 8;
+constexpr int kResItems = 4;  // most buckets in one turn (eight idled two threads of three)
 constexpr int kResTile = kResThreads * kResItems;
 
 __global__ void __launch_bounds__(kResThreads) ss_resolve_kernel(
