@@ -147,6 +147,14 @@ __device__ __forceinline__ void st_relaxed(uint64_t* p, uint64_t v) {
 }
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
+// Programmatic dependent launch: dependents_may_launch lets the stream's next
+// kernel, launched with the attribute (launch_after), set up while this one runs;
+// that one waits in wait_for_previous until every kernel before it has ended and
+// its writes are visible.  Nothing but the kernel's own arguments may be used
+// before the wait.
+__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
 }  // namespace bt

@@ -871,6 +871,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
                                                                        uint8_t* out_st) {
   extern __shared__ __align__(16) unsigned char raw[];
   WriteSmem& S = *reinterpret_cast<WriteSmem*>(raw);
+  dependents_may_launch();
+  wait_for_previous();
   const uint32_t rank = cluster_rank(), C = cluster_size();
   const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
   const uint32_t n_ins = a.counts->n_ins, n_del = a.counts->n_del, n_touch = a.counts->n_touch;
@@ -1144,7 +1146,7 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaSt
   a.inner_fill = h->inner_fill;
   a.entry_cap = (uint32_t)w.cap;
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   small_config(cfg, at, small_cluster(n), sizeof(WriteSmem), s);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, small_write_kernel, h->tree, a, out_vals, out_st);
   count_launch();

@@ -81,6 +81,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                        uint64_t* __restrict__ out_vals, uint8_t* __restrict__ out_st, DevTree t, int ensure_root) {
   extern __shared__ __align__(16) unsigned char raw[];
   FrontSmem& S = *reinterpret_cast<FrontSmem*>(raw);
+  dependents_may_launch();
+  wait_for_previous();
   const uint32_t rank = cluster_rank(), C = cluster_size();
   const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
   BatchCounts* c = f.counts;
@@ -462,6 +464,8 @@ template <bool kGets>
 __global__ void __launch_bounds__(kReadThreads) small_read_kernel(DevTree t, SmallRead a, int use_pfx,
                                                                   uint64_t* __restrict__ out_vals,
                                                                   uint8_t* __restrict__ out_st) {
+  dependents_may_launch();
+  wait_for_previous();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t n_ins = a.locate_ins ? a.counts->n_ins : 0, n_del = a.counts->n_del;
   const uint32_t n_get = kGets ? a.counts->n_lookup : 0;
@@ -570,7 +574,7 @@ int small_front(Handle* h, const uint64_t* keys, const uint64_t* vals, const uin
   while (slots < 4 * n) slots <<= 1;
   const unsigned C = small_cluster(n);
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   small_config(cfg, at, C, sizeof(FrontSmem), s);
   const cudaError_t e =
       cudaLaunchKernelEx(&cfg, small_front_kernel, keys, vals, ops, (uint32_t)n, reinterpret_cast<Slot*>(w.s_tab),
@@ -602,10 +606,20 @@ int small_read(Handle* h, bool gets, bool locate_ins, uint64_t* out_vals, uint8_
   if (use_pfx && ensure_pfx(h, s) != cudaSuccess) return -2;
   const size_t turns = (n + kLocPer - 1) / kLocPer + 2;
   const unsigned grid = (unsigned)min(turns, (size_t)h->sm_count * 8);
-  if (gets) small_read_kernel<true><<<grid, kReadThreads, 0, s>>>(h->tree, a, use_pfx, out_vals, out_st);
-  else small_read_kernel<false><<<grid, kReadThreads, 0, s>>>(h->tree, a, use_pfx, out_vals, out_st);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kReadThreads);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e =
+      gets ? cudaLaunchKernelEx(&cfg, small_read_kernel<true>, h->tree, a, use_pfx, out_vals, out_st)
+           : cudaLaunchKernelEx(&cfg, small_read_kernel<false>, h->tree, a, use_pfx, out_vals, out_st);
   count_launch();
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return e == cudaSuccess ? 0 : -2;
 }
 
 }  // namespace bt

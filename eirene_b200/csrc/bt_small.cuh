@@ -90,6 +90,7 @@ inline unsigned small_cluster(size_t n) {
   return c;
 }
 
+// at: two attributes, the cluster and the dependent launch
 inline void small_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned C, size_t smem, cudaStream_t s) {
   cfg.gridDim = dim3(C);
   cfg.blockDim = dim3(kSmallThreads);
@@ -99,8 +100,10 @@ inline void small_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsig
   at[0].val.clusterDim.x = C;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
 }
 
 }  // namespace bt
