@@ -25,6 +25,7 @@
 #include "bt_block.cuh"
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_sort.cuh"
 
 namespace bt {
@@ -114,11 +115,9 @@ __device__ __forceinline__ Seg item_seg(const Item& x, const uint64_t* __restric
 
 // pass 1: per tile aggregate, head count, locally determined tail counts and
 // the state at the tail of the run continued from the previous tile
-__global__ void __launch_bounds__(kThreads) merge_pass1(const uint64_t* __restrict__ sk,
-                                                        const uint32_t* __restrict__ sv,
-                                                        const uint64_t* __restrict__ vals, size_t n,
-                                                        const uint32_t* __restrict__ n_dev,
-                                                        TileSummary* __restrict__ tiles) {
+__global__ void __launch_bounds__(kThreads) merge_pass1(const uint64_t* sk, const uint32_t* sv, const uint64_t* vals,
+                                                        size_t n, const uint32_t* n_dev, TileSummary* tiles) {
+  after_previous();
   if (n_dev) n = min(n, (size_t)*n_dev);
   if ((size_t)blockIdx.x * kTile >= n) return;  // grid sized for the host bound
   __shared__ uint32_t wsf[32];
@@ -183,9 +182,9 @@ __global__ void __launch_bounds__(kThreads) merge_pass1(const uint64_t* __restri
 }
 
 // pass 2 (one block): carries and prefix counts across tiles; writes totals
-__global__ void __launch_bounds__(1024) merge_pass2(TileSummary* __restrict__ tiles, uint32_t n_tiles,
-                                                    const uint32_t* __restrict__ n_dev,
-                                                    BatchCounts* __restrict__ counts) {
+__global__ void __launch_bounds__(1024) merge_pass2(TileSummary* tiles, uint32_t n_tiles, const uint32_t* n_dev,
+                                                    BatchCounts* counts) {
+  after_previous();
   if (n_dev) n_tiles = min(n_tiles, (uint32_t)(((size_t)*n_dev + kTile - 1) / kTile));
   __shared__ uint32_t wsf[32];
   __shared__ uint64_t wsv[32];
@@ -248,11 +247,10 @@ __global__ void __launch_bounds__(1024) merge_pass2(TileSummary* __restrict__ ti
 
 // pass 3: per request resolution, unique ops and the two work lists
 __global__ void __launch_bounds__(kThreads) merge_pass3(
-    const uint64_t* __restrict__ sk, const uint32_t* __restrict__ sv, const uint64_t* __restrict__ vals, size_t n,
-    const uint32_t* __restrict__ n_dev, const TileSummary* __restrict__ tiles, uint64_t* __restrict__ ukeys,
-    uint64_t* __restrict__ uvals, uint32_t* __restrict__ ins_list, uint32_t* __restrict__ get_list,
-    uint32_t* __restrict__ del_list, uint32_t* __restrict__ pend, uint64_t* __restrict__ out_vals,
-    uint8_t* __restrict__ out_st) {
+    const uint64_t* sk, const uint32_t* sv, const uint64_t* vals, size_t n, const uint32_t* n_dev,
+    const TileSummary* tiles, uint64_t* ukeys, uint64_t* uvals, uint32_t* ins_list, uint32_t* get_list,
+    uint32_t* del_list, uint32_t* pend, uint64_t* out_vals, uint8_t* out_st) {
+  after_previous();
   if (n_dev) n = min(n, (size_t)*n_dev);
   if ((size_t)blockIdx.x * kTile >= n) return;
   __shared__ uint32_t wsf[32];
@@ -321,10 +319,10 @@ __global__ void __launch_bounds__(kThreads) merge_pass3(
   }
 }
 
-__global__ void writeback_kernel(const uint32_t* __restrict__ sv, const uint32_t* __restrict__ pend, size_t n,
-                                 const uint32_t* __restrict__ n_dev, const uint64_t* __restrict__ uans,
-                                 const uint8_t* __restrict__ uans_st, uint64_t* __restrict__ out_vals,
-                                 uint8_t* __restrict__ out_st, int pairs) {
+__global__ void writeback_kernel(const uint32_t* sv, const uint32_t* pend, size_t n, const uint32_t* n_dev,
+                                 const uint64_t* uans, const uint8_t* uans_st, uint64_t* out_vals, uint8_t* out_st,
+                                 int pairs) {
+  after_previous();
   if (n_dev) n = min(n, (size_t)*n_dev);
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -533,10 +531,10 @@ static int hashed_passes(Handle* h, const FrontPart& fp, const uint64_t* vals, u
   Work& w = h->w;
   const uint32_t* n_touch = &w.counts->n_touch;
   if (fp.sample) return sample_resolve(h, vals, out_vals, out_st, n, s);
-  merge_pass1<<<fp.n_tiles, kThreads, 0, s>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles);
-  merge_pass2<<<1, 1024, 0, s>>>(w.tiles, fp.n_tiles, n_touch, w.counts);
-  merge_pass3<<<fp.n_tiles, kThreads, 0, s>>>(fp.sk, fp.sv, vals, n, n_touch, w.tiles, w.ukeys, w.uvals, w.ins_list,
-                                              w.get_list, w.del_list, w.pend, out_vals, out_st);
+  launch_after(merge_pass1, fp.n_tiles, kThreads, 0, s, fp.sk, fp.sv, vals, n, n_touch, w.tiles);
+  launch_after(merge_pass2, 1, 1024, 0, s, w.tiles, fp.n_tiles, n_touch, w.counts);
+  launch_after(merge_pass3, fp.n_tiles, kThreads, 0, s, fp.sk, fp.sv, vals, n, n_touch, w.tiles, w.ukeys, w.uvals,
+               w.ins_list, w.get_list, w.del_list, w.pend, out_vals, out_st);
   count_launch(3);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -634,8 +632,8 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   if (!early) {
     if (insert_phase(h, n, engine, s) != 0) return -2;
     prof_mark(h, 4, s);
-    writeback_kernel<<<wb_blocks, 256, 0, s>>>(fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st,
-                                              fp.sample ? 1 : 0);
+    launch_after(writeback_kernel, wb_blocks, 256, 0, s, fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals,
+                 out_st, fp.sample ? 1 : 0);
     count_launch();
     prof_mark(h, 5, s);
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
@@ -651,8 +649,8 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   if (merge_update_phase(h, n, s) != 0 || delete_apply(h, n, s) != 0 || merge_reserve_phase(h, n, s) != 0)
     return -2;
   prof_mark(h, kEvWbStart, s);
-  writeback_kernel<<<wb_blocks, 256, 0, s>>>(fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st,
-                                              fp.sample ? 1 : 0);
+  launch_after(writeback_kernel, wb_blocks, 256, 0, s, fp.sv, w.pend, n, n_touch, w.uans, w.uans_st, out_vals, out_st,
+               fp.sample ? 1 : 0);
   count_launch();
   prof_mark(h, 4, s);
   if (answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess) return -2;
@@ -712,8 +710,8 @@ static int batch_small(Handle* h, const uint64_t* keys, const uint64_t* vals, co
         launch_stm(h, w.ukeys, w.uvals, nullptr, kOpInsert, w.ins_list, &w.counts->n_ins, n, w.uans, w.uans_st, s) !=
             cudaSuccess)
       return -2;
-    writeback_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w.v_a, w.pend, n, &w.counts->n_touch, w.uans,
-                                                                 w.uans_st, out_vals, out_st, 1);
+    launch_after(writeback_kernel, (unsigned)((n + 255) / 256), 256, 0, s, w.v_a, w.pend, n, &w.counts->n_touch,
+                 w.uans, w.uans_st, out_vals, out_st, 1);
     count_launch();
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
   }
@@ -854,12 +852,12 @@ int batch_sorted(Handle* h, const uint64_t* keys, const uint64_t* vals, const ui
   const uint32_t n_tiles = (uint32_t)pass_tiles(n);
   prof_mark(h, 1, s);
   if (wait_vals(h, s) != 0) return -2;
-  merge_pass1<<<n_tiles, kThreads, 0, s>>>(sk, sv, vals, n, nullptr, w.tiles);
+  launch_after(merge_pass1, n_tiles, kThreads, 0, s, sk, sv, vals, n, nullptr, w.tiles);
   count_launch();
-  merge_pass2<<<1, 1024, 0, s>>>(w.tiles, n_tiles, nullptr, w.counts);
+  launch_after(merge_pass2, 1, 1024, 0, s, w.tiles, n_tiles, nullptr, w.counts);
   count_launch();
-  merge_pass3<<<n_tiles, kThreads, 0, s>>>(sk, sv, vals, n, nullptr, w.tiles, w.ukeys, w.uvals, w.ins_list,
-                                           w.get_list, w.del_list, w.pend, out_vals, out_st);
+  launch_after(merge_pass3, n_tiles, kThreads, 0, s, sk, sv, vals, n, nullptr, w.tiles, w.ukeys, w.uvals, w.ins_list,
+               w.get_list, w.del_list, w.pend, out_vals, out_st);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) return -2;
   // search phase on the pre-batch tree, then the insert phase
@@ -878,7 +876,7 @@ int batch_sorted(Handle* h, const uint64_t* keys, const uint64_t* vals, const ui
   if (insert_phase(h, n, engine, s) != 0) return -2;
   prof_mark(h, 4, s);
   const unsigned wb_blocks = (unsigned)min((size_t)h->sm_count * 8, (n + 255) / 256);
-  writeback_kernel<<<wb_blocks, 256, 0, s>>>(sv, w.pend, n, nullptr, w.uans, w.uans_st, out_vals, out_st, 0);
+  launch_after(writeback_kernel, wb_blocks, 256, 0, s, sv, w.pend, n, nullptr, w.uans, w.uans_st, out_vals, out_st, 0);
   count_launch();
   prof_mark(h, 5, s);
   if (answers_ready(h, s) != 0) return -2;

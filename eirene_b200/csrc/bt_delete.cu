@@ -14,6 +14,7 @@
 #include "bt_common.cuh"
 #include "bt_delete.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_rows.cuh"
 #include "bt_search.cuh"
 
@@ -29,9 +30,9 @@ constexpr int kS = 32 / kG;
 // their new places in shared memory, the row written back with 16-byte stores.
 // Bound by the rows' traffic and the chain entry -> leaf -> row: with a warp per
 // entry, one leaf at a time, 2^19 deletes on 2^24 keys took 131 us; this takes 113.
-__global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_t* __restrict__ n_dev,
-                                                        const uint32_t* __restrict__ dleaf,
-                                                        const uint32_t* __restrict__ dslot) {
+__global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_t* n_dev, const uint32_t* dleaf,
+                                                        const uint32_t* dslot) {
+  after_previous();
   __shared__ __align__(16) uint64_t mk[256 / kG][32];
   __shared__ __align__(16) uint64_t mv[256 / kG][32];
   const uint32_t lane = threadIdx.x & 31;
@@ -101,8 +102,8 @@ __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_
 // n_upper bounds the device count w.counts->n_del.
 int delete_apply(Handle* h, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
-  del_apply_kernel<<<(unsigned)min((size_t)h->sm_count * 8, (n_upper * kG + 255) / 256 + 1), 256, 0, s>>>(
-      h->tree, &w.counts->n_del, w.d_leaf, w.d_slot);
+  launch_after(del_apply_kernel, (unsigned)min((size_t)h->sm_count * 8, (n_upper * kG + 255) / 256 + 1), 256, 0, s,
+               h->tree, &w.counts->n_del, w.d_leaf, w.d_slot);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -32,6 +32,7 @@
 #include "bt_block.cuh"
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_sort.cuh"
 
 namespace bt {
@@ -66,8 +67,8 @@ __device__ __forceinline__ uint32_t table_cap(uint32_t n_ins, size_t cap_max) {
 }
 
 // INSERT and DELETE op codes (an upper bound of the keys to hold: reserved keys count too)
-__global__ void __launch_bounds__(kThreads) front_count_kernel(const uint8_t* __restrict__ ops, size_t n,
-                                                               BatchCounts* __restrict__ counts) {
+__global__ void __launch_bounds__(kThreads) front_count_kernel(const uint8_t* ops, size_t n, BatchCounts* counts) {
+  after_previous();
   uint32_t c = 0;
   // four op codes per load when the array is 4-byte aligned
   const size_t n4 = ((uintptr_t)ops & 3u) ? 0 : n / 4;
@@ -82,8 +83,8 @@ __global__ void __launch_bounds__(kThreads) front_count_kernel(const uint8_t* __
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(&counts->n_ins_req, c);
 }
 
-__global__ void __launch_bounds__(kThreads) front_clear_kernel(Slot* __restrict__ tab, size_t cap_max,
-                                                               BatchCounts* __restrict__ counts) {
+__global__ void __launch_bounds__(kThreads) front_clear_kernel(Slot* tab, size_t cap_max, BatchCounts* counts) {
+  after_previous();
   const uint32_t cap = table_cap(counts->n_ins_req, cap_max);
   if (blockIdx.x == 0 && threadIdx.x == 0) counts->cap = cap;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (size_t)gridDim.x * blockDim.x) {
@@ -94,10 +95,9 @@ __global__ void __launch_bounds__(kThreads) front_clear_kernel(Slot* __restrict_
 }
 
 // linear probing; the table holds at most 2/3 of its slots, so a probe ends
-__global__ void __launch_bounds__(kThreads) front_insert_kernel(const uint64_t* __restrict__ keys,
-                                                                const uint8_t* __restrict__ ops, size_t n,
-                                                                Slot* __restrict__ tab,
-                                                                const BatchCounts* __restrict__ counts) {
+__global__ void __launch_bounds__(kThreads) front_insert_kernel(const uint64_t* keys, const uint8_t* ops, size_t n,
+                                                                Slot* tab, const BatchCounts* counts) {
+  after_previous();
   const uint32_t mask = counts->cap - 1;
   auto put = [&](size_t i) {
     const uint64_t k = keys[i];
@@ -166,7 +166,7 @@ __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ 
     sk[j] = kKeyMax;
     sf[j] = kNone;
     if (any && k[j] != kKeyMax) {
-      const ulonglong2 e = __ldg(reinterpret_cast<const ulonglong2*>(tab + sh[j]));
+      const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(tab + sh[j]);
       sk[j] = e.x;
       sf[j] = (uint32_t)e.y;
     }
@@ -186,7 +186,7 @@ __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ 
     for (int j = 0; j < kTileItems; j++) {
       if (!((todo >> j) & 1u)) continue;
       sh[j] = (sh[j] + 1) & mask;
-      const ulonglong2 e = __ldg(reinterpret_cast<const ulonglong2*>(tab + sh[j]));
+      const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(tab + sh[j]);
       sk[j] = e.x;
       sf[j] = (uint32_t)e.y;
     }
@@ -214,12 +214,10 @@ __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ 
   return touched;
 }
 
-__global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t* __restrict__ keys,
-                                                                  const uint8_t* __restrict__ ops, size_t n,
-                                                                  const Slot* __restrict__ tab,
-                                                                  const BatchCounts* __restrict__ counts,
-                                                                  uint8_t* __restrict__ flags,
-                                                                  uint32_t* __restrict__ tile_cnt) {
+__global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t* keys, const uint8_t* ops, size_t n,
+                                                                  const Slot* tab, const BatchCounts* counts,
+                                                                  uint8_t* flags, uint32_t* tile_cnt) {
+  after_previous();
   __shared__ uint32_t wsum[kTileWarps];
   const size_t base = (size_t)blockIdx.x * kTile;
   uint64_t k[kTileItems];
@@ -245,14 +243,10 @@ __global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t
 // keys by their request index: each tile takes its places in the two lists
 // with one atomic each, so the tiles come in any order (requests of a tile stay
 // together and in order).  `flags`-free: the class is used where it is found.
-__global__ void __launch_bounds__(kTileThreads) front_split_kernel(const uint64_t* __restrict__ keys,
-                                                                   const uint8_t* __restrict__ ops, size_t n,
-                                                                   const Slot* __restrict__ tab,
-                                                                   BatchCounts* __restrict__ counts,
-                                                                   uint64_t* __restrict__ tk,
-                                                                   uint32_t* __restrict__ tv,
-                                                                   uint32_t* __restrict__ list,
-                                                                   uint64_t* __restrict__ lk) {
+__global__ void __launch_bounds__(kTileThreads) front_split_kernel(const uint64_t* keys, const uint8_t* ops, size_t n,
+                                                                   const Slot* tab, BatchCounts* counts, uint64_t* tk,
+                                                                   uint32_t* tv, uint32_t* list, uint64_t* lk) {
+  after_previous();
   __shared__ uint32_t cnt[kTileItems][kTileWarps];
   __shared__ uint32_t at_touch, at_lookup;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -305,9 +299,9 @@ __global__ void __launch_bounds__(kTileThreads) front_split_kernel(const uint64_
 }
 
 // exclusive offsets of n_tiles counts, in place, with one block
-__global__ void __launch_bounds__(1024) front_tile_scan_kernel(uint32_t* __restrict__ tile, uint32_t n_tiles,
-                                                               size_t n, BatchCounts* __restrict__ counts,
-                                                               uint32_t* hint) {
+__global__ void __launch_bounds__(1024) front_tile_scan_kernel(uint32_t* tile, uint32_t n_tiles, size_t n,
+                                                               BatchCounts* counts, uint32_t* hint) {
+  after_previous();
   __shared__ uint32_t wtot[32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t carry = 0;
@@ -344,14 +338,11 @@ __global__ void __launch_bounds__(1024) front_tile_scan_kernel(uint32_t* __restr
   }
 }
 
-__global__ void __launch_bounds__(kTileThreads) front_scatter_kernel(const uint64_t* __restrict__ keys,
-                                                                     const uint8_t* __restrict__ ops, size_t n,
-                                                                     const uint8_t* __restrict__ flags,
-                                                                     const uint32_t* __restrict__ tile_off,
-                                                                     uint64_t* __restrict__ tk,
-                                                                     uint32_t* __restrict__ tv,
-                                                                     uint32_t* __restrict__ list,
-                                                                     uint64_t* __restrict__ lk) {
+__global__ void __launch_bounds__(kTileThreads) front_scatter_kernel(const uint64_t* keys, const uint8_t* ops,
+                                                                     size_t n, const uint8_t* flags,
+                                                                     const uint32_t* tile_off, uint64_t* tk,
+                                                                     uint32_t* tv, uint32_t* list, uint64_t* lk) {
+  after_previous();
   __shared__ uint32_t cnt[kTileItems][kTileWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
@@ -515,12 +506,10 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t m, uint32_t* __restrict
   return base + incl - c;  // this lane's first slot
 }
 
-__global__ void __launch_bounds__(kThreads) stm_split_kernel(const uint64_t* __restrict__ keys,
-                                                             const uint8_t* __restrict__ ops, size_t n,
-                                                             uint32_t* __restrict__ get_list,
-                                                             uint64_t* __restrict__ get_keys,
-                                                             uint32_t* __restrict__ wr_list,
-                                                             BatchCounts* __restrict__ counts) {
+__global__ void __launch_bounds__(kThreads) stm_split_kernel(const uint64_t* keys, const uint8_t* ops, size_t n,
+                                                             uint32_t* get_list, uint64_t* get_keys,
+                                                             uint32_t* wr_list, BatchCounts* counts) {
+  after_previous();
   const uint32_t lane = threadIdx.x & 31;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   // whole warps iterate together (the appends are warp-aggregated); four
@@ -554,13 +543,11 @@ __global__ void __launch_bounds__(kThreads) stm_split_kernel(const uint64_t* __r
   }
 }
 
-__global__ void __launch_bounds__(kThreads) combine_arrive_kernel(const uint64_t* __restrict__ keys,
-                                                                  const uint8_t* __restrict__ ops,
-                                                                  const uint32_t* __restrict__ list,
-                                                                  Slot* __restrict__ tab,
-                                                                  const BatchCounts* __restrict__ counts,
-                                                                  uint32_t* __restrict__ pred,
-                                                                  uint32_t* __restrict__ slot_of) {
+__global__ void __launch_bounds__(kThreads) combine_arrive_kernel(const uint64_t* keys, const uint8_t* ops,
+                                                                  const uint32_t* list, Slot* tab,
+                                                                  const BatchCounts* counts, uint32_t* pred,
+                                                                  uint32_t* slot_of) {
+  after_previous();
   const uint32_t mask = counts->cap - 1;
   const size_t m = counts->n_ins_req;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += (size_t)gridDim.x * blockDim.x) {
@@ -593,18 +580,13 @@ __global__ void __launch_bounds__(kThreads) combine_arrive_kernel(const uint64_t
 
 // per INSERT: its value for the STM kernel, or (combined with an earlier one)
 // its answer and a skip mark
-__global__ void __launch_bounds__(kThreads) combine_mark_kernel(const uint64_t* __restrict__ keys,
-                                                                const uint64_t* __restrict__ vals,
-                                                                const uint8_t* __restrict__ ops,
-                                                                const uint32_t* __restrict__ list,
-                                                                const BatchCounts* __restrict__ counts,
-                                                                const Slot* __restrict__ tab,
-                                                                const uint32_t* __restrict__ pred,
-                                                                const uint32_t* __restrict__ slot_of,
-                                                                uint8_t* __restrict__ skip,
-                                                                uint64_t* __restrict__ cvals,
-                                                                uint64_t* __restrict__ out_vals,
-                                                                uint8_t* __restrict__ out_st) {
+__global__ void __launch_bounds__(kThreads) combine_mark_kernel(const uint64_t* keys, const uint64_t* vals,
+                                                                const uint8_t* ops, const uint32_t* list,
+                                                                const BatchCounts* counts, const Slot* tab,
+                                                                const uint32_t* pred, const uint32_t* slot_of,
+                                                                uint8_t* skip, uint64_t* cvals, uint64_t* out_vals,
+                                                                uint8_t* out_st) {
+  after_previous();
   const size_t m = counts->n_ins_req;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += (size_t)gridDim.x * blockDim.x) {
     const uint32_t i = list[q];
@@ -626,14 +608,11 @@ __global__ void __launch_bounds__(kThreads) combine_mark_kernel(const uint64_t* 
 
 // a representative that did not commit (retry limit, full node pool): the
 // INSERTs combined with it report the same status
-__global__ void __launch_bounds__(kThreads) combine_fixup_kernel(const uint8_t* __restrict__ ops,
-                                                                 const uint32_t* __restrict__ list,
-                                                                 const BatchCounts* __restrict__ counts,
-                                                                 const uint8_t* __restrict__ skip,
-                                                                 const Slot* __restrict__ tab,
-                                                                 const uint32_t* __restrict__ slot_of,
-                                                                 uint64_t* __restrict__ out_vals,
-                                                                 uint8_t* __restrict__ out_st) {
+__global__ void __launch_bounds__(kThreads) combine_fixup_kernel(const uint8_t* ops, const uint32_t* list,
+                                                                 const BatchCounts* counts, const uint8_t* skip,
+                                                                 const Slot* tab, const uint32_t* slot_of,
+                                                                 uint64_t* out_vals, uint8_t* out_st) {
+  after_previous();
   const size_t m = counts->n_ins_req;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < m; q += (size_t)gridDim.x * blockDim.x) {
     const uint32_t i = list[q];
@@ -653,7 +632,7 @@ int stm_split(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n, cud
   Work& w = h->w;
   const unsigned g = (unsigned)min((size_t)h->sm_count * 8, (n / 4 + kThreads) / kThreads);
   if (cudaMemsetAsync(w.counts, 0, sizeof(BatchCounts), s) != cudaSuccess) return -2;
-  stm_split_kernel<<<g, kThreads, 0, s>>>(keys, ops, n, w.get_list, w.ukeys, w.ins_list, w.counts);
+  launch_after(stm_split_kernel, g, kThreads, 0, s, keys, ops, n, w.get_list, w.ukeys, w.ins_list, w.counts);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -669,9 +648,10 @@ int stm_combine(Handle* h, const uint64_t* keys, const uint64_t* vals, const uin
   uint32_t* slot_of = w.f_pos;
   uint32_t* list = w.ins_list;
   const unsigned g = (unsigned)min((size_t)h->sm_count * 8, (n / 4 + kThreads) / kThreads);
-  front_clear_kernel<<<(unsigned)h->sm_count * 4, kThreads, 0, s>>>(tab, w.f_tab_cap, c);
-  combine_arrive_kernel<<<g, kThreads, 0, s>>>(keys, ops, list, tab, c, pred, slot_of);
-  combine_mark_kernel<<<g, kThreads, 0, s>>>(keys, vals, ops, list, c, tab, pred, slot_of, sk, cv, out_vals, out_st);
+  launch_after(front_clear_kernel, (unsigned)h->sm_count * 4, kThreads, 0, s, tab, w.f_tab_cap, c);
+  launch_after(combine_arrive_kernel, g, kThreads, 0, s, keys, ops, list, tab, c, pred, slot_of);
+  launch_after(combine_mark_kernel, g, kThreads, 0, s, keys, vals, ops, list, c, tab, pred, slot_of, sk, cv, out_vals,
+               out_st);
   count_launch(3);
   *skip = sk;
   *cvals = cv;
@@ -681,8 +661,9 @@ int stm_combine(Handle* h, const uint64_t* keys, const uint64_t* vals, const uin
 int stm_combine_fixup(Handle* h, const uint8_t* ops, size_t n, uint64_t* out_vals, uint8_t* out_st, cudaStream_t s) {
   Work& w = h->w;
   const unsigned g = (unsigned)min((size_t)h->sm_count * 8, (n / 4 + kThreads) / kThreads);
-  combine_fixup_kernel<<<g, kThreads, 0, s>>>(ops, w.ins_list, w.counts, reinterpret_cast<const uint8_t*>(w.f_flags),
-                                              reinterpret_cast<const Slot*>(w.f_tab), w.f_pos, out_vals, out_st);
+  launch_after(combine_fixup_kernel, g, kThreads, 0, s, ops, w.ins_list, w.counts,
+               reinterpret_cast<const uint8_t*>(w.f_flags), reinterpret_cast<const Slot*>(w.f_tab), w.f_pos, out_vals,
+               out_st);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -739,19 +720,19 @@ int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n
   Slot* tab = reinterpret_cast<Slot*>(w.f_tab);
   uint8_t* flags = reinterpret_cast<uint8_t*>(w.f_flags);
   uint32_t* tile = w.f_pos;  // per-tile counts, then offsets
-  front_count_kernel<<<(unsigned)h->sm_count * 2, kThreads, 0, s>>>(ops, n, c);
-  front_clear_kernel<<<(unsigned)h->sm_count * 4, kThreads, 0, s>>>(tab, w.f_tab_cap, c);
-  front_insert_kernel<<<g, kThreads, 0, s>>>(keys, ops, n, tab, c);
+  launch_after(front_count_kernel, (unsigned)h->sm_count * 2, kThreads, 0, s, ops, n, c);
+  launch_after(front_clear_kernel, (unsigned)h->sm_count * 4, kThreads, 0, s, tab, w.f_tab_cap, c);
+  launch_after(front_insert_kernel, g, kThreads, 0, s, keys, ops, n, tab, c);
   if (!ordered) {
-    front_split_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(keys, ops, n, tab, c, w.f_tk, w.f_tv, w.f_list,
-                                                                  w.f_lk);
+    launch_after(front_split_kernel, (unsigned)n_tiles, kTileThreads, 0, s, keys, ops, n, tab, c, w.f_tk, w.f_tv,
+                 w.f_list, w.f_lk);
     count_launch(4);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
-  front_flag_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(keys, ops, n, tab, c, flags, tile);
-  front_tile_scan_kernel<<<1, 1024, 0, s>>>(tile, (uint32_t)n_tiles, n, c, h->touch_hint_dev);
-  front_scatter_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(keys, ops, n, flags, tile, w.f_tk, w.f_tv,
-                                                                  w.f_list, w.f_lk);
+  launch_after(front_flag_kernel, (unsigned)n_tiles, kTileThreads, 0, s, keys, ops, n, tab, c, flags, tile);
+  launch_after(front_tile_scan_kernel, 1, 1024, 0, s, tile, (uint32_t)n_tiles, n, c, h->touch_hint_dev);
+  launch_after(front_scatter_kernel, (unsigned)n_tiles, kTileThreads, 0, s, keys, ops, n, flags, tile, w.f_tk, w.f_tv,
+               w.f_list, w.f_lk);
   count_launch(6);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

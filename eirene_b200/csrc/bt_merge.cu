@@ -31,6 +31,7 @@
 #include "bt_common.cuh"
 #include "bt_delete.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_rows.cuh"
 #include "bt_search.cuh"
 #include "bt_small.cuh"
@@ -160,9 +161,9 @@ __global__ void __launch_bounds__(256) locate_kernel(DevTree t, LocateArgs a, in
 
 // new values of the keys the batch finds in the tree, in place (keys do not
 // move); after the batch's plain lookups, before its DELETE apply
-__global__ void merge_update_kernel(DevTree t, const uint64_t* __restrict__ uvals,
-                                    const uint32_t* __restrict__ ins_list, const uint32_t* __restrict__ n_dev,
-                                    const uint64_t* __restrict__ vpos) {
+__global__ void merge_update_kernel(DevTree t, const uint64_t* uvals, const uint32_t* ins_list, const uint32_t* n_dev,
+                                    const uint64_t* vpos) {
+  after_previous();
   const size_t n = *n_dev;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
@@ -172,12 +173,11 @@ __global__ void merge_update_kernel(DevTree t, const uint64_t* __restrict__ uval
 }
 
 // ------------------------------------------------------------- compact ----
-__global__ void merge_compact_kernel(const uint32_t* __restrict__ ins_list, const uint32_t* __restrict__ n_dev,
-                                     const uint32_t* __restrict__ isnew, const uint32_t* __restrict__ pos,
-                                     const uint64_t* __restrict__ ukeys, const uint64_t* __restrict__ uvals,
-                                     const uint32_t* __restrict__ mleaf, uint64_t* __restrict__ newk,
-                                     uint64_t* __restrict__ newv, uint32_t* __restrict__ nq,
-                                     uint32_t* __restrict__ nleaf) {
+__global__ void merge_compact_kernel(const uint32_t* ins_list, const uint32_t* n_dev, const uint32_t* isnew,
+                                     const uint32_t* pos, const uint64_t* ukeys, const uint64_t* uvals,
+                                     const uint32_t* mleaf, uint64_t* newk, uint64_t* newv, uint32_t* nq,
+                                     uint32_t* nleaf) {
+  after_previous();
   const size_t n = *n_dev;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
@@ -191,8 +191,8 @@ __global__ void merge_compact_kernel(const uint32_t* __restrict__ ins_list, cons
   }
 }
 
-__global__ void merge_seg_flags_kernel(const MergeCounts* __restrict__ mc, const uint32_t* __restrict__ nleaf,
-                                       size_t n_upper, uint32_t* __restrict__ flags) {
+__global__ void merge_seg_flags_kernel(const MergeCounts* mc, const uint32_t* nleaf, size_t n_upper, uint32_t* flags) {
+  after_previous();
   const size_t n_new = min(n_upper, (size_t)mc->n_new);  // the scan reads n_new flags
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += stride)
@@ -201,9 +201,9 @@ __global__ void merge_seg_flags_kernel(const MergeCounts* __restrict__ mc, const
 
 // segment starts and each segment's leaf (so the leaf merge loads it without
 // a dependent hop through the segment start)
-__global__ void merge_seg_start_kernel(const MergeCounts* __restrict__ mc, const uint32_t* __restrict__ flags,
-                                       const uint32_t* __restrict__ idx, const uint32_t* __restrict__ nleaf,
-                                       uint32_t* __restrict__ seg_start, uint32_t* __restrict__ seg_leaf) {
+__global__ void merge_seg_start_kernel(const MergeCounts* mc, const uint32_t* flags, const uint32_t* idx,
+                                       const uint32_t* nleaf, uint32_t* seg_start, uint32_t* seg_leaf) {
+  after_previous();
   const uint32_t n_new = mc->n_new;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += stride)
@@ -220,9 +220,10 @@ __device__ __forceinline__ void seg_bounds(const MergeCounts* mc, const uint32_t
 }
 
 // pieces - 1 per segment (new leaves it creates)
-__global__ void merge_leaf_count_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* __restrict__ mc,
-                                        const uint32_t* __restrict__ seg_start, const uint32_t* __restrict__ nleaf,
-                                        size_t n_upper, uint32_t* __restrict__ extra) {
+__global__ void merge_leaf_count_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* mc,
+                                        const uint32_t* seg_start, const uint32_t* nleaf, size_t n_upper,
+                                        uint32_t* extra) {
+  after_previous();
   const size_t n_segs = min(n_upper, (size_t)mc->n_segs);  // the scan reads n_segs entries
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_segs; s += stride) {
@@ -252,11 +253,15 @@ __device__ __forceinline__ void reserve_pieces(const DevTree& t, MergeCounts* mc
   mc->cap_fail = 0;
   mc->node_base = atomicAdd(&t.ctrl->n_nodes, T);
 }
-__global__ void merge_alloc_kernel(DevTree t, MergeCounts* mc, uint32_t entry_cap) { reserve_pieces(t, mc, entry_cap); }
+__global__ void merge_alloc_kernel(DevTree t, MergeCounts* mc, uint32_t entry_cap) {
+  after_previous();
+  reserve_pieces(t, mc, entry_cap);
+}
 
 // a batch whose pieces did not fit answers kNoCapacity for all its new keys
-__global__ void merge_fail_mark_kernel(const MergeCounts* __restrict__ mc, const uint32_t* __restrict__ nq,
-                                       const uint32_t* __restrict__ ins_list, uint8_t* __restrict__ uans_st) {
+__global__ void merge_fail_mark_kernel(const MergeCounts* mc, const uint32_t* nq, const uint32_t* ins_list,
+                                       uint8_t* uans_st) {
+  after_previous();
   if (mc->cap_fail == 0) return;
   const uint32_t n_new = mc->n_new;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -871,8 +876,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
                                                                        uint8_t* out_st) {
   extern __shared__ __align__(16) unsigned char raw[];
   WriteSmem& S = *reinterpret_cast<WriteSmem*>(raw);
-  dependents_may_launch();
-  wait_for_previous();
+  after_previous();
   const uint32_t rank = cluster_rank(), C = cluster_size();
   const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
   const uint32_t n_ins = a.counts->n_ins, n_del = a.counts->n_del, n_touch = a.counts->n_touch;
@@ -1052,7 +1056,7 @@ int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s) {
 int merge_update_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
   const unsigned gb = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256);
-  merge_update_kernel<<<gb, 256, 0, s>>>(h->tree, w.uvals, w.ins_list, &w.counts->n_ins, w.m_vpos);
+  launch_after(merge_update_kernel, gb, 256, 0, s, h->tree, w.uvals, w.ins_list, &w.counts->n_ins, w.m_vpos);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1066,14 +1070,14 @@ int merge_group_phase(Handle* h, size_t n_upper, cudaStream_t s) {
                             s) != cudaSuccess)
     return -2;
   const unsigned gb = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256);
-  merge_compact_kernel<<<gb, 256, 0, s>>>(w.ins_list, n_ins, w.m_isnew, w.m_pos, w.ukeys, w.uvals, w.m_leaf, w.m_newk,
-                                          w.m_newv, w.m_nq, w.m_nleaf);
-  merge_seg_flags_kernel<<<gb, 256, 0, s>>>(mc, w.m_nleaf, n_upper, w.m_isnew);
+  launch_after(merge_compact_kernel, gb, 256, 0, s, w.ins_list, n_ins, w.m_isnew, w.m_pos, w.ukeys, w.uvals, w.m_leaf,
+               w.m_newk, w.m_newv, w.m_nq, w.m_nleaf);
+  launch_after(merge_seg_flags_kernel, gb, 256, 0, s, mc, w.m_nleaf, n_upper, w.m_isnew);
   count_launch(2);
   if (scan_exclusive_u32_lb(w.m_isnew, w.m_pos, n_upper, &mc->n_new, &mc->n_segs, w.lb_status, w.lb_ctr, &w.lb_epoch,
                             err, s) != cudaSuccess)
     return -2;
-  merge_seg_start_kernel<<<gb, 256, 0, s>>>(mc, w.m_isnew, w.m_pos, w.m_nleaf, w.m_seg, w.m_leaf);
+  launch_after(merge_seg_start_kernel, gb, 256, 0, s, mc, w.m_isnew, w.m_pos, w.m_nleaf, w.m_seg, w.m_leaf);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1082,14 +1086,15 @@ int merge_reserve_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
   const unsigned gb = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256);
-  merge_leaf_count_kernel<<<gb, 256, 0, s>>>(h->tree, h->leaf_fill, mc, w.m_seg, w.m_nleaf, n_upper, w.m_isnew);
+  launch_after(merge_leaf_count_kernel, gb, 256, 0, s, h->tree, h->leaf_fill, mc, w.m_seg, w.m_nleaf, n_upper,
+               w.m_isnew);
   count_launch();
   if (scan_exclusive_u32_lb(w.m_isnew, w.m_pos, n_upper, &mc->n_segs, &mc->n_leaf_entries, w.lb_status, w.lb_ctr,
                             &w.lb_epoch, &h->tree.ctrl->error, s) !=
       cudaSuccess)
     return -2;
-  merge_alloc_kernel<<<1, 1, 0, s>>>(h->tree, mc, (uint32_t)w.cap);
-  merge_fail_mark_kernel<<<gb, 256, 0, s>>>(mc, w.m_nq, w.ins_list, w.uans_st);
+  launch_after(merge_alloc_kernel, 1, 1, 0, s, h->tree, mc, (uint32_t)w.cap);
+  launch_after(merge_fail_mark_kernel, gb, 256, 0, s, mc, w.m_nq, w.ins_list, w.uans_st);
   count_launch(2);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

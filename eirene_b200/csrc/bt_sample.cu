@@ -30,6 +30,7 @@
 #include "bt_block.cuh"
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_sort.cuh"
 
 namespace bt {
@@ -118,11 +119,11 @@ struct SortSmem {
   uint32_t pre, pre_any;
 };
 
-__global__ void __launch_bounds__(1024, 1) ss_splitters_kernel(const uint64_t* __restrict__ tk,
-                                                               const uint32_t* __restrict__ tv, uint32_t n_upper,
-                                                               const uint32_t* __restrict__ n_dev, uint32_t sms,
-                                                               uint64_t* __restrict__ spk, uint32_t* __restrict__ spv,
-                                                               uint32_t* __restrict__ total, uint32_t* hint) {
+__global__ void __launch_bounds__(1024, 1) ss_splitters_kernel(const uint64_t* tk, const uint32_t* tv,
+                                                               uint32_t n_upper, const uint32_t* n_dev, uint32_t sms,
+                                                               uint64_t* spk, uint32_t* spv, uint32_t* total,
+                                                               uint32_t* hint) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char raw[];
   SortSmem& S = *reinterpret_cast<SortSmem*>(raw);
   const uint32_t m = min(n_upper, *n_dev);
@@ -150,13 +151,11 @@ __global__ void __launch_bounds__(1024, 1) ss_splitters_kernel(const uint64_t* _
   }
 }
 
-__global__ void __launch_bounds__(kTileThreads) ss_count_kernel(const uint64_t* __restrict__ tk,
-                                                                const uint32_t* __restrict__ tv, uint32_t n_upper,
-                                                                const uint32_t* __restrict__ n_dev, uint32_t sms,
-                                                                const uint64_t* __restrict__ spk,
-                                                                const uint32_t* __restrict__ spv,
-                                                                uint16_t* __restrict__ ids, uint32_t* __restrict__ off,
-                                                                uint32_t* __restrict__ total) {
+__global__ void __launch_bounds__(kTileThreads) ss_count_kernel(const uint64_t* tk, const uint32_t* tv,
+                                                                uint32_t n_upper, const uint32_t* n_dev, uint32_t sms,
+                                                                const uint64_t* spk, const uint32_t* spv,
+                                                                uint16_t* ids, uint32_t* off, uint32_t* total) {
+  after_previous();
   __shared__ uint64_t sk[kBuckets];
   __shared__ uint32_t sv[kBuckets];
   __shared__ uint32_t hist[kBuckets];
@@ -205,14 +204,12 @@ __global__ void __launch_bounds__(kTileThreads) ss_count_kernel(const uint64_t* 
   }
 }
 
-__global__ void __launch_bounds__(kTileThreads) ss_scatter_kernel(const uint64_t* __restrict__ tk,
-                                                                  const uint32_t* __restrict__ tv, uint32_t n_upper,
-                                                                  const uint32_t* __restrict__ n_dev, uint32_t sms,
-                                                                  const uint16_t* __restrict__ ids,
-                                                                  const uint32_t* __restrict__ off,
-                                                                  const uint32_t* __restrict__ total,
-                                                                  uint32_t* __restrict__ base,
-                                                                  uint64_t* __restrict__ kb, uint32_t* __restrict__ vb) {
+__global__ void __launch_bounds__(kTileThreads) ss_scatter_kernel(const uint64_t* tk, const uint32_t* tv,
+                                                                  uint32_t n_upper, const uint32_t* n_dev,
+                                                                  uint32_t sms, const uint16_t* ids,
+                                                                  const uint32_t* off, const uint32_t* total,
+                                                                  uint32_t* base, uint64_t* kb, uint32_t* vb) {
+  after_previous();
   __shared__ uint32_t ws[32];
   __shared__ uint32_t start[kBuckets], hist[kBuckets];
   const uint32_t m = min(n_upper, *n_dev);
@@ -329,10 +326,10 @@ __device__ __noinline__ void sort_large(SortSmem& S, uint64_t* ka, uint32_t* va,
   }
 }
 
-__global__ void __launch_bounds__(1024, 1) ss_sort_kernel(uint32_t n_upper, const uint32_t* __restrict__ n_dev,
-                                                          uint32_t sms, const uint32_t* __restrict__ base,
-                                                          uint64_t* ka, uint32_t* va, uint64_t* kb, uint32_t* vb,
-                                                          BucketSum* __restrict__ sums) {
+__global__ void __launch_bounds__(1024, 1) ss_sort_kernel(uint32_t n_upper, const uint32_t* n_dev, uint32_t sms,
+                                                          const uint32_t* base, uint64_t* ka, uint32_t* va,
+                                                          uint64_t* kb, uint32_t* vb, BucketSum* sums) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char raw[];
   SortSmem& S = *reinterpret_cast<SortSmem*>(raw);
   const uint32_t m = min(n_upper, *n_dev);
@@ -425,11 +422,10 @@ constexpr int kResItems = 4;  // most buckets in one turn (eight idled two threa
 constexpr int kResTile = kResThreads * kResItems;
 
 __global__ void __launch_bounds__(kResThreads) ss_resolve_kernel(
-    const uint64_t* __restrict__ sk, const uint32_t* __restrict__ sv, const uint64_t* __restrict__ vals,
-    uint32_t n_upper, const uint32_t* __restrict__ n_dev, uint32_t sms, const uint32_t* __restrict__ base,
-    const BucketSum* __restrict__ sums, uint64_t* __restrict__ ukeys, uint64_t* __restrict__ uvals,
-    uint32_t* __restrict__ ins_list, uint32_t* __restrict__ del_list, uint32_t* __restrict__ pend,
-    uint64_t* __restrict__ out_vals, uint8_t* __restrict__ out_st, BatchCounts* __restrict__ counts) {
+    const uint64_t* sk, const uint32_t* sv, const uint64_t* vals, uint32_t n_upper, const uint32_t* n_dev,
+    uint32_t sms, const uint32_t* base, const BucketSum* sums, uint64_t* ukeys, uint64_t* uvals, uint32_t* ins_list,
+    uint32_t* del_list, uint32_t* pend, uint64_t* out_vals, uint8_t* out_st, BatchCounts* counts) {
+  after_previous();
   __shared__ uint32_t ws[32];
   __shared__ uint32_t carry[kBuckets], hb[kBuckets], ib[kBuckets], db[kBuckets];
   static_assert(kResThreads == kBuckets, "one bucket per thread below");
@@ -599,11 +595,13 @@ int sample_sort(Handle* h, size_t n, cudaStream_t s) {
   uint32_t* base = sum_base(w.s_sum);
   BucketSum* sums = reinterpret_cast<BucketSum*>(w.s_sum);
   const unsigned tiles = (unsigned)min((n + kTile - 1) / kTile, (size_t)h->sm_count * 4);
-  ss_splitters_kernel<<<1, 1024, sizeof(SortSmem), s>>>(w.f_tk, w.f_tv, nu, m, sms, spk, spv, total, h->touch_hint_dev);
-  ss_count_kernel<<<tiles, kTileThreads, 0, s>>>(w.f_tk, w.f_tv, nu, m, sms, spk, spv, ids, off, total);
-  ss_scatter_kernel<<<tiles, kTileThreads, 0, s>>>(w.f_tk, w.f_tv, nu, m, sms, ids, off, total, base, w.k_b, w.v_b);
+  launch_after(ss_splitters_kernel, 1, 1024, sizeof(SortSmem), s, w.f_tk, w.f_tv, nu, m, sms, spk, spv, total,
+               h->touch_hint_dev);
+  launch_after(ss_count_kernel, tiles, kTileThreads, 0, s, w.f_tk, w.f_tv, nu, m, sms, spk, spv, ids, off, total);
+  launch_after(ss_scatter_kernel, tiles, kTileThreads, 0, s, w.f_tk, w.f_tv, nu, m, sms, ids, off, total, base, w.k_b,
+               w.v_b);
   const unsigned buckets = (unsigned)min((n + 1023) / 1024, (size_t)h->sm_count);
-  ss_sort_kernel<<<buckets, 1024, sizeof(SortSmem), s>>>(nu, m, sms, base, w.k_a, w.v_a, w.k_b, w.v_b, sums);
+  launch_after(ss_sort_kernel, buckets, 1024, sizeof(SortSmem), s, nu, m, sms, base, w.k_a, w.v_a, w.k_b, w.v_b, sums);
   count_launch(4);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -611,10 +609,9 @@ int sample_sort(Handle* h, size_t n, cudaStream_t s) {
 int sample_resolve(Handle* h, const uint64_t* vals, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s) {
   Work& w = h->w;
   const unsigned buckets = (unsigned)min((n + 1023) / 1024, kSsBuckets);
-  ss_resolve_kernel<<<buckets, kResThreads, 0, s>>>(
-      w.k_a, w.v_a, vals, (uint32_t)n, &w.counts->n_touch, (uint32_t)h->sm_count, sum_base(w.s_sum),
-      reinterpret_cast<const BucketSum*>(w.s_sum), w.ukeys, w.uvals, w.ins_list, w.del_list, w.pend, out_vals, out_st,
-      w.counts);
+  launch_after(ss_resolve_kernel, buckets, kResThreads, 0, s, w.k_a, w.v_a, vals, (uint32_t)n, &w.counts->n_touch,
+               (uint32_t)h->sm_count, sum_base(w.s_sum), reinterpret_cast<const BucketSum*>(w.s_sum), w.ukeys,
+               w.uvals, w.ins_list, w.del_list, w.pend, out_vals, out_st, w.counts);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

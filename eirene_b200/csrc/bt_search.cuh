@@ -1,8 +1,9 @@
 // Grouped lock-free descent shared by the plain search kernel and the learned
 // search's fallback.  A group of G lanes serves one request; each lane owns
-// S = 32/G consecutive slots of a node row and loads them with 16-byte loads
-// through the read-only path (valid only while no writer runs: the batch
-// executor never overlaps this with the STM insert phase).
+// S = 32/G consecutive slots of a node row and loads them with 16-byte loads.
+// Valid only while no writer runs (the batch executor never overlaps this with
+// the STM insert phase); the loads are ordinary ones, not ld.global.nc, because
+// a kernel may be resident before the one that wrote the rows has ended.
 #pragma once
 #include "bt_common.cuh"
 
@@ -17,19 +18,19 @@ __device__ __forceinline__ uint32_t group_mask(uint32_t lane) {
 template <int S>
 __device__ __forceinline__ void load_slots(const uint64_t* p, uint64_t (&x)[S]) {
   if constexpr (S == 1) {
-    x[0] = __ldg(p);
+    x[0] = *p;
   } else {
 #pragma unroll
     for (int i = 0; i < S; i += 2) {
-      ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(p + i));
+      ulonglong2 w = *reinterpret_cast<const ulonglong2*>(p + i);
       x[i] = w.x;
       x[i + 1] = w.y;
     }
   }
 }
 
-// L2 eviction priorities for the descent (createpolicy + ld.global.nc with
-// an L2 cache hint, PTX ISA 7.4+): inner rows are read by every lookup and
+// L2 eviction priorities for the descent (createpolicy + ld.global with an
+// L2 cache hint, PTX ISA 7.4+): inner rows are read by every lookup and
 // should stay in L2 (evict_last); a leaf row or value is read once per
 // lookup and should not push them out (evict_first).
 __device__ __forceinline__ uint64_t l2_keep() {
@@ -46,13 +47,13 @@ __device__ __forceinline__ uint64_t l2_stream() {
 
 __device__ __forceinline__ uint64_t ldg_hint(const uint64_t* p, uint64_t pol) {
   uint64_t r;
-  asm("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(pol));
+  asm("ld.global.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(pol));
   return r;
 }
 
 __device__ __forceinline__ ulonglong2 ldg2_hint(const void* p, uint64_t pol) {
   ulonglong2 r;
-  asm("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(r.x), "=l"(r.y) : "l"(p), "l"(pol));
+  asm("ld.global.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(r.x), "=l"(r.y) : "l"(p), "l"(pol));
   return r;
 }
 
@@ -63,7 +64,7 @@ __device__ __forceinline__ void load_slots_hint(const uint64_t* p, uint64_t (&x)
   } else {
 #pragma unroll
     for (int i = 0; i < S; i += 2)
-      asm("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;"
+      asm("ld.global.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;"
           : "=l"(x[i]), "=l"(x[i + 1])
           : "l"(p + i), "l"(pol));
   }
@@ -84,7 +85,7 @@ __device__ __forceinline__ void load_row_il(const uint64_t* row, uint32_t g, uin
   } else {
 #pragma unroll
     for (int i = 0; i < S / 2; i++)
-      asm("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;"
+      asm("ld.global.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;"
           : "=l"(x[2 * i]), "=l"(x[2 * i + 1])
           : "l"(row + 2 * (i * G + g)), "l"(pol));
   }
@@ -104,11 +105,11 @@ __device__ __forceinline__ uint32_t il_elem(uint32_t s) {
 template <int S>
 __device__ __forceinline__ void load_pfx(const uint32_t* p, uint32_t (&x)[S], uint64_t pol) {
   if constexpr (S == 2) {
-    asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(x[0]), "=r"(x[1]) : "l"(p), "l"(pol));
+    asm("ld.global.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(x[0]), "=r"(x[1]) : "l"(p), "l"(pol));
   } else {
 #pragma unroll
     for (int i = 0; i < S; i += 4)
-      asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+      asm("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
           : "=r"(x[i]), "=r"(x[i + 1]), "=r"(x[i + 2]), "=r"(x[i + 3])
           : "l"(p + i), "l"(pol));
   }
@@ -146,7 +147,7 @@ __device__ __forceinline__ uint32_t pfx_rank(const uint32_t (&p)[S], uint64_t ke
 // ---- leaf lookup by one thread (DevTree::fp) ----
 // 32 bytes in one load
 __device__ __forceinline__ void ldg32_hint(const void* p, uint64_t (&x)[4], uint64_t pol) {
-  asm("ld.global.nc.L2::cache_hint.v4.u64 {%0, %1, %2, %3}, [%4], %5;"
+  asm("ld.global.L2::cache_hint.v4.u64 {%0, %1, %2, %3}, [%4], %5;"
       : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
       : "l"(p), "l"(pol));
 }
@@ -308,7 +309,7 @@ __device__ __forceinline__ uint8_t group_leaf_lookup(const DevTree& t, uint32_t 
   const uint64_t kk = __shfl_sync(gmask, pick<S>(k, e), owner, G);
   if (kk != key) return kAbsent;
   if (kLeafVals) ans = __shfl_sync(gmask, pick<S>(v, e), owner, G);
-  else ans = (g == 0) ? __ldg(t.vals + (size_t)node * 32 + slot) : 0;
+  else ans = (g == 0) ? t.vals[(size_t)node * 32 + slot] : 0;
   return kFound;
 }
 
@@ -455,8 +456,8 @@ __device__ __forceinline__ void group_descend2(const DevTree& t, uint32_t node, 
     ans_a = fa ? xa : 0;
     ans_b = fb ? xb : 0;
   } else if (g == 0) {
-    if (fa) ans_a = kChild ? ldg_hint(t.vals + (size_t)na * 32 + sa, stream) : __ldg(t.vals + (size_t)na * 32 + sa);
-    if (fb) ans_b = kChild ? ldg_hint(t.vals + (size_t)nb * 32 + sb, stream) : __ldg(t.vals + (size_t)nb * 32 + sb);
+    if (fa) ans_a = kChild ? ldg_hint(t.vals + (size_t)na * 32 + sa, stream) : t.vals[(size_t)na * 32 + sa];
+    if (fb) ans_b = kChild ? ldg_hint(t.vals + (size_t)nb * 32 + sb, stream) : t.vals[(size_t)nb * 32 + sb];
   }
   st_a = fa ? kFound : kAbsent;
   st_b = fb ? kFound : kAbsent;

@@ -27,6 +27,7 @@
 #include "bt_block.cuh"
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_search.cuh"
 #include "bt_small.cuh"
 #include "bt_sort.cuh"
@@ -76,13 +77,11 @@ struct FrontSmem {
 };
 
 __global__ void __launch_bounds__(kSmallThreads, 1)
-    small_front_kernel(const uint64_t* __restrict__ keys, const uint64_t* __restrict__ vals,
-                       const uint8_t* __restrict__ ops, uint32_t n, Slot* tab, uint32_t mask, SmallFront f,
-                       uint64_t* __restrict__ out_vals, uint8_t* __restrict__ out_st, DevTree t, int ensure_root) {
+    small_front_kernel(const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint32_t n, Slot* tab,
+                       uint32_t mask, SmallFront f, uint64_t* out_vals, uint8_t* out_st, DevTree t, int ensure_root) {
   extern __shared__ __align__(16) unsigned char raw[];
   FrontSmem& S = *reinterpret_cast<FrontSmem*>(raw);
-  dependents_may_launch();
-  wait_for_previous();
+  after_previous();
   const uint32_t rank = cluster_rank(), C = cluster_size();
   const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
   BatchCounts* c = f.counts;
@@ -462,10 +461,8 @@ constexpr uint32_t kGetPer = 2 * kReadThreads / kGetG;
 // own).  All of them only read the tree.
 template <bool kGets>
 __global__ void __launch_bounds__(kReadThreads) small_read_kernel(DevTree t, SmallRead a, int use_pfx,
-                                                                  uint64_t* __restrict__ out_vals,
-                                                                  uint8_t* __restrict__ out_st) {
-  dependents_may_launch();
-  wait_for_previous();
+                                                                  uint64_t* out_vals, uint8_t* out_st) {
+  after_previous();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t n_ins = a.locate_ins ? a.counts->n_ins : 0, n_del = a.counts->n_del;
   const uint32_t n_get = kGets ? a.counts->n_lookup : 0;
@@ -494,7 +491,7 @@ __global__ void __launch_bounds__(kReadThreads) small_read_kernel(DevTree t, Sma
         if (!del && g > 0 && g <= root_level) a.path[g * a.path_stride + q] = path;
       }
       if (g == 0) {
-        a.uans[u] = found ? __ldg(t.vals + (size_t)leaf * 32 + slot) : 0;
+        a.uans[u] = found ? t.vals[(size_t)leaf * 32 + slot] : 0;
         a.uans_st[u] = found ? kFound : (del || usable) ? kAbsent : kNoCapacity;
         if (del) {
           a.dleaf[q] = leaf;

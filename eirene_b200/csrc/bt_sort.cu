@@ -20,6 +20,7 @@
 
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 
 namespace bt {
 
@@ -142,22 +143,25 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
 constexpr uint64_t kLbAgg = 1ull << 32, kLbInc = 2ull << 32;
 constexpr uint32_t kLbSpinLimit = 1u << 22;
 
-__global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* __restrict__ in,
-                                                               uint32_t* __restrict__ out, size_t n_upper,
-                                                               const uint32_t* __restrict__ n_dev,
-                                                               uint32_t* __restrict__ total_out,
-                                                               uint64_t* __restrict__ status,
-                                                               uint32_t* __restrict__ ctr, uint32_t epoch,
-                                                               uint32_t* __restrict__ err) {
+__global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* in, uint32_t* out, size_t n_upper,
+                                                               const uint32_t* n_dev, uint32_t* total_out,
+                                                               uint64_t* status, uint32_t* ctr, uint32_t epoch,
+                                                               uint32_t* err) {
+  after_previous();
   __shared__ uint32_t ws[32];
   __shared__ uint32_t tot, s_tile, s_prefix;
   const size_t n = n_dev ? min(n_upper, (size_t)*n_dev) : n_upper;
   const size_t n_tiles = (n + kScanTile - 1) / kScanTile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
-  __syncthreads();
-  const uint32_t tile = s_tile;
   const uint64_t tag = (uint64_t)epoch << 34;
-  if (tile < n_tiles) {
+  for (;;) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    __syncthreads();
+    if (tile >= n_tiles) {
+      if (tile == 0 && threadIdx.x == 0 && total_out) *total_out = 0;  // nothing to scan
+      break;
+    }
     const size_t base = (size_t)tile * kScanTile + (size_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t sum = 0;
@@ -200,8 +204,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* _
       if (base + i < n) out[base + i] = ex;
       ex += v[i];
     }
-  } else if (tile == 0 && threadIdx.x == 0 && total_out) {
-    *total_out = 0;  // nothing to scan
   }
   // the last block to finish makes the tile ids start at 0 again
   if (threadIdx.x == 0) {
@@ -222,10 +224,10 @@ constexpr uint32_t kValMask = (1u << 30) - 1u;
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 // all digit histograms in one read of the keys: hist[pass][256]
-__global__ void __launch_bounds__(kSortThreads) sort_upfront_hist_kernel(const uint64_t* __restrict__ keys,
-                                                                         size_t n, const uint32_t* __restrict__ n_dev,
-                                                                         int begin_bit, int passes,
-                                                                         uint32_t* __restrict__ hist) {
+__global__ void __launch_bounds__(kSortThreads) sort_upfront_hist_kernel(const uint64_t* keys, size_t n,
+                                                                         const uint32_t* n_dev, int begin_bit,
+                                                                         int passes, uint32_t* hist) {
+  after_previous();
   __shared__ uint32_t h[kMaxPasses][kRadix];
   if (n_dev) n = min(n, (size_t)*n_dev);
   for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kSortThreads) (&h[0][0])[i] = 0;
@@ -243,7 +245,8 @@ __global__ void __launch_bounds__(kSortThreads) sort_upfront_hist_kernel(const u
 }
 
 // exclusive scan of each pass's 256 counts -> global bucket starts
-__global__ void sort_digit_scan_kernel(uint32_t* __restrict__ hist, int passes) {
+__global__ void sort_digit_scan_kernel(uint32_t* hist, int passes) {
+  after_previous();
   __shared__ uint32_t ws[32];
   for (int p = 0; p < passes; p++) {
     const uint32_t c = hist[p * kRadix + threadIdx.x];
@@ -269,10 +272,10 @@ struct ScatterSmem {
 // any grid size is safe (the launcher uses at most the resident blocks).
 template <int T>
 __global__ void __launch_bounds__(T) sort_onesweep_kernel(
-    const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, const uint8_t* __restrict__ ops,
-    int payload_mode, uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, size_t n,
-    const uint32_t* __restrict__ n_dev, int shift, const uint32_t* __restrict__ gbase,
-    uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ status, uint32_t* __restrict__ err) {
+    const uint64_t* keys_in, const uint32_t* vals_in, const uint8_t* ops, int payload_mode, uint64_t* keys_out,
+    uint32_t* vals_out, size_t n, const uint32_t* n_dev, int shift, const uint32_t* gbase, uint32_t* tile_counter,
+    uint32_t* status, uint32_t* err) {
+  after_previous();
   static_assert(T >= kRadix, "one thread per digit");
   constexpr int kTile = T * kSortItems;
   constexpr int kWarps = T / 32;
@@ -445,14 +448,26 @@ cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, uint
 
 size_t scan_lb_words(size_t n_upper) { return (n_upper + kScanTile - 1) / kScanTile + 1; }
 
+// SMs of the current device
+static unsigned sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
+                                                cudaSuccess || sms < 1)
+    return 148;
+  return (unsigned)sms;
+}
+
 cudaError_t scan_exclusive_u32_lb(const uint32_t* in, uint32_t* out, size_t n_upper, const uint32_t* n_dev,
                                   uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* epoch,
                                   uint32_t* err, cudaStream_t s) {
   *epoch = (*epoch + 1) & ((1u << 30) - 1);
   if (*epoch == 0) *epoch = 1;  // zeroed status words carry epoch 0
-  const size_t blocks = n_upper ? (n_upper + kScanTile - 1) / kScanTile : 1;
-  scan_lb_kernel<<<(unsigned)blocks, kScanThreads, 0, s>>>(in, out, n_upper, n_dev, total_dev, status, ctr, *epoch,
-                                                           err);
+  // one block per SM, taking tiles until there are none: the bound is the batch's size, the live entries
+  // mostly under 2^19, and a block per tile of the bound was 1,024 blocks of 1,024 threads that found
+  // nothing to do (11 us a scan of a 2^22 batch)
+  const size_t blocks = n_upper ? min((n_upper + kScanTile - 1) / kScanTile, (size_t)sm_count()) : 1;
+  launch_after(scan_lb_kernel, (unsigned)blocks, kScanThreads, 0, s, in, out, n_upper, n_dev, total_dev, status, ctr,
+               *epoch, err);
   count_launch();
   return cudaGetLastError();
 }
@@ -477,13 +492,12 @@ static unsigned onesweep_resident() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
   if (!cache[dev]) {
-    int per = 0, sms = 0;
+    int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sort_onesweep_kernel<T>, T, sizeof(ScatterSmem<T>)) !=
             cudaSuccess ||
         per < 1)
       per = 1;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
-    cache[dev] = (unsigned)(per * sms);
+    cache[dev] = (unsigned)per * sm_count();
   }
   return cache[dev];
 }
@@ -494,8 +508,8 @@ static void onesweep_pass(const uint64_t* src_k, const uint32_t* src_v, const ui
                           uint32_t* dst_v, size_t n, const uint32_t* n_dev, int shift, const uint32_t* gbase,
                           uint32_t* counter, uint32_t* status, uint32_t* err, uint32_t n_tiles, cudaStream_t s) {
   const unsigned grid = min(n_tiles, onesweep_resident<T>());
-  sort_onesweep_kernel<T><<<grid, T, sizeof(ScatterSmem<T>), s>>>(src_k, src_v, ops, mode, dst_k, dst_v, n, n_dev,
-                                                                  shift, gbase, counter, status, err);
+  launch_after(sort_onesweep_kernel<T>, grid, T, sizeof(ScatterSmem<T>), s, src_k, src_v, ops, mode, dst_k, dst_v, n,
+               n_dev, shift, gbase, counter, status, err);
 }
 
 // scratch: hist[8][256] | tile counters[8] (+pad) | status[8][tiles][256]
@@ -544,9 +558,9 @@ cudaError_t radix_sort_pairs(const uint64_t* keys_in, const uint32_t* vals_in, c
                                   ((size_t)kMaxPasses * kRadix + 64 + (size_t)passes * n_tiles * kRadix) * 4, s);
   if (e != cudaSuccess) return e;
   unsigned hb = (unsigned)min((n + kSortThreads * kSortItems - 1) / (kSortThreads * kSortItems), (size_t)1024);
-  sort_upfront_hist_kernel<<<hb, kSortThreads, 0, s>>>(keys_in, n, n_dev, begin_bit, passes, hist);
+  launch_after(sort_upfront_hist_kernel, hb, kSortThreads, 0, s, keys_in, n, n_dev, begin_bit, passes, hist);
   count_launch();
-  sort_digit_scan_kernel<<<1, kRadix, 0, s>>>(hist, passes);
+  launch_after(sort_digit_scan_kernel, 1, kRadix, 0, s, hist, passes);
   count_launch();
   const uint64_t* src_k = keys_in;
   const uint32_t* src_v = vals_in;

@@ -16,6 +16,7 @@
 
 #include "bt_common.cuh"
 #include "bt_internal.h"
+#include "bt_launch.cuh"
 #include "bt_learned.cuh"
 
 namespace bt {
@@ -928,13 +929,12 @@ __device__ __forceinline__ void flush_counters(const DevTree& t, const TxCounter
   }
 }
 
-__global__ void __launch_bounds__(256, 4) stm_kernel(DevTree t, const uint64_t* __restrict__ keys,
-                                                     const uint64_t* __restrict__ vals, const uint8_t* __restrict__ ops,
-                                                     uint32_t op_override, const uint32_t* __restrict__ list,
-                                                     const uint32_t* __restrict__ n_dev, size_t n_host,
-                                                     uint64_t* __restrict__ out_vals, uint8_t* __restrict__ out_st,
-                                                     uint32_t retry_limit, LearnedDev lm, int use_learned,
-                                                     const uint8_t* __restrict__ skip) {
+__global__ void __launch_bounds__(256, 4) stm_kernel(DevTree t, const uint64_t* keys, const uint64_t* vals,
+                                                     const uint8_t* ops, uint32_t op_override, const uint32_t* list,
+                                                     const uint32_t* n_dev, size_t n_host, uint64_t* out_vals,
+                                                     uint8_t* out_st, uint32_t retry_limit, LearnedDev lm,
+                                                     int use_learned, const uint8_t* skip) {
+  after_previous();
   const uint32_t lane = lane_id();
   const size_t n = n_dev ? (size_t)*n_dev : n_host;
   const LearnedDev* M = use_learned ? &lm : nullptr;
@@ -1198,8 +1198,8 @@ cudaError_t launch_stm(Handle* h, const uint64_t* keys, const uint64_t* vals, co
   if (blocks > cap) blocks = cap;
   LearnedDev lm{};
   const int use = learned_dev(h, &lm);
-  stm_kernel<<<(unsigned)blocks, threads, 0, s>>>(h->tree, keys, vals, ops, op_override, list, n_dev, n, out_vals,
-                                                   out_st, h->retry_limit, lm, use, skip);
+  launch_after(stm_kernel, (unsigned)blocks, threads, 0, s, h->tree, keys, vals, ops, op_override, list, n_dev, n,
+               out_vals, out_st, h->retry_limit, lm, use, skip);
   count_launch();
   return cudaGetLastError();
 }
