@@ -389,12 +389,12 @@ int work_alloc(Work* w, size_t cap) {
   A((void**)&w->f_lk, cap * 8);
   A((void**)&w->f_tk, cap * 8);
   A((void**)&w->f_tv, cap * 4);
-  A((void**)&w->lb_status, scan_lb_words(cap) * 8);
+  A((void**)&w->lb_status, merge_lb_words(cap) * 8);
   A((void**)&w->lb_ctr, 8);
   A((void**)&w->s_write, 3 * 16 * 4);
   A((void**)&w->s_split, kSsBuckets * 16);
   A(&w->s_sum, sample_sum_bytes());
-  ok = ok && cudaMemset(w->lb_status, 0, scan_lb_words(cap) * 8) == cudaSuccess &&
+  ok = ok && cudaMemset(w->lb_status, 0, merge_lb_words(cap) * 8) == cudaSuccess &&
        cudaMemset(w->lb_ctr, 0, 8) == cudaSuccess;
   if (!ok) {
     work_free(w);

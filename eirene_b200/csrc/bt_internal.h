@@ -168,7 +168,7 @@ struct Work {
   uint32_t* f_tv = nullptr;      // [cap] index | op << 30 of the touched requests
   // all-INSERT op codes of bt_insert_batch
   uint8_t* ins_ops = nullptr;
-  // look-back scan of the merge engine (scan_exclusive_u32_lb)
+  // look-back words of the merge engine (bt_lookback.cuh)
   uint64_t* lb_status = nullptr;
   uint32_t* lb_ctr = nullptr;
   uint32_t lb_epoch = 0;
@@ -558,6 +558,7 @@ int merge_engine(Handle* h, size_t n_upper, cudaStream_t s);
 constexpr int kLocateIns = 1, kLocateDel = 2;
 int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s);
 int merge_update_phase(Handle* h, size_t n_upper, cudaStream_t s);
+size_t merge_lb_words(size_t n);  // words of Work::lb_status
 int merge_group_phase(Handle* h, size_t n_upper, cudaStream_t s);
 int merge_reserve_phase(Handle* h, size_t n_upper, cudaStream_t s);
 int merge_write_phase(Handle* h, cudaStream_t s);

@@ -1,0 +1,66 @@
+// Decoupled look-back over tiles that blocks take in turn (the one-launch scans
+// of bt_sort.cu and bt_merge.cu).
+//
+// status[t] = epoch << 34 | state << 32 | value, state 1 the tile's own sum, 2
+// its inclusive prefix; each call's epoch makes the words of earlier calls read
+// as not ready, so the array is never cleared.  ctr[0] hands tile ids out in
+// the order blocks take them (a tile waits only on tiles taken before it); the
+// last block to finish resets ctr.  The wait is bounded: past kLbSpinLimit it
+// sets kErrSpin in *err and goes on.
+#pragma once
+#include <cstdint>
+
+#include "bt_common.cuh"
+
+namespace bt {
+
+constexpr uint64_t kLbAgg = 1ull << 32, kLbInc = 2ull << 32;
+constexpr uint32_t kLbSpinLimit = 1u << 22;
+
+// Publish tile `tile`'s sum and return the sum of the tiles before it; one whole
+// warp, all lanes get the result.  32 tiles are read at a time: one after
+// another, the walk back to the last prefix bounded a scan of 320 tiles (18 us).
+__device__ __forceinline__ uint32_t look_back(uint64_t* status, uint32_t tile, uint32_t sum, uint32_t epoch,
+                                              uint32_t* err) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t tag = (uint64_t)epoch << 34;
+  if (tile == 0) {
+    if (lane == 0) st_release(&status[0], tag | kLbInc | sum);
+    return 0;
+  }
+  if (lane == 0) st_release(&status[tile], tag | kLbAgg | sum);
+  uint32_t prefix = 0, spins = 0;
+  int64_t t = (int64_t)tile - 1;
+  for (;;) {
+    const int64_t i = t - lane;
+    const uint64_t w = i >= 0 ? ld_acquire(&status[i]) : (tag | kLbInc);  // before tile 0: nothing
+    const uint32_t state = (uint32_t)(w >> 34) == epoch ? (uint32_t)(w >> 32) & 3u : 0u;
+    const uint32_t done = __ballot_sync(0xffffffffu, state == 2), wait = __ballot_sync(0xffffffffu, state == 0);
+    const uint32_t upto = done ? (done & (0u - done)) * 2u - 1u : 0xffffffffu;  // lanes up to the nearest prefix
+    if (wait & upto) {
+      if (++spins > kLbSpinLimit) {
+        if (lane == 0 && err) atomicOr(err, kErrSpin);
+        break;
+      }
+      if (spins > 64) __nanosleep(64);
+      continue;
+    }
+    prefix += __reduce_add_sync(0xffffffffu, (upto >> lane) & 1u ? (uint32_t)w : 0u);
+    if (done) break;
+    t -= 32;
+  }
+  if (lane == 0) st_release(&status[tile], tag | kLbInc | (uint64_t)(prefix + sum));
+  return prefix;
+}
+
+// one thread of every block, at its end: the last makes the tile ids start at 0 again
+__device__ __forceinline__ void tiles_done(uint32_t* ctr) {
+  __threadfence();
+  if (atomicAdd(&ctr[1], 1u) == gridDim.x - 1) {
+    ctr[0] = 0;
+    ctr[1] = 0;
+    __threadfence();
+  }
+}
+
+}  // namespace bt

@@ -32,6 +32,7 @@
 #include "bt_delete.cuh"
 #include "bt_internal.h"
 #include "bt_launch.cuh"
+#include "bt_lookback.cuh"
 #include "bt_rows.cuh"
 #include "bt_search.cuh"
 #include "bt_small.cuh"
@@ -173,66 +174,98 @@ __global__ void merge_update_kernel(DevTree t, const uint64_t* uvals, const uint
 }
 
 // ------------------------------------------------------------- compact ----
-__global__ void merge_compact_kernel(const uint32_t* ins_list, const uint32_t* n_dev, const uint32_t* isnew,
-                                     const uint32_t* pos, const uint64_t* ukeys, const uint64_t* uvals,
-                                     const uint32_t* mleaf, uint64_t* newk, uint64_t* newv, uint32_t* nq,
-                                     uint32_t* nleaf) {
-  after_previous();
-  const size_t n = *n_dev;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
-    if (!isnew[q]) continue;
-    const uint32_t p = pos[q];
-    const uint32_t u = ins_list[q];
-    newk[p] = ukeys[u];
-    newv[p] = uvals[u];
-    nq[p] = (uint32_t)q;
-    nleaf[p] = mleaf[q];
-  }
-}
+// The new keys, packed, and the segments: runs of new keys that share a leaf.
+// One launch over tiles of the INSERT keys (the look-back of bt_lookback.cuh
+// gives a tile its places): a new key begins a segment when no new key before
+// it has its leaf, which the flags and leaves just before it tell (at most 31
+// keys of a leaf are in the tree already), so new keys and segments are counted
+// in one pass.  It was five launches (scan, compact, flags, scan, starts).
+constexpr int kGroupThreads = 1024;
+constexpr uint32_t kGroupTile = 2 * kGroupThreads;
 
-__global__ void merge_seg_flags_kernel(const MergeCounts* mc, const uint32_t* nleaf, size_t n_upper, uint32_t* flags) {
+__global__ void __launch_bounds__(kGroupThreads)
+    merge_group_kernel(MergeCounts* mc, const uint32_t* ins_list, const uint32_t* n_dev, const uint32_t* isnew,
+                       const uint64_t* ukeys, const uint64_t* uvals, const uint32_t* mleaf, uint64_t* newk,
+                       uint64_t* newv, uint32_t* nq, uint32_t* nleaf, uint32_t* seg_start, uint32_t* seg_leaf,
+                       uint64_t* status, uint64_t* status_seg, uint32_t* ctr, uint32_t epoch, uint32_t* err) {
   after_previous();
-  const size_t n_new = min(n_upper, (size_t)mc->n_new);  // the scan reads n_new flags
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += stride)
-    flags[i] = (i == 0 || nleaf[i] != nleaf[i - 1]) ? 1u : 0u;
-}
-
-// segment starts and each segment's leaf (so the leaf merge loads it without
-// a dependent hop through the segment start)
-__global__ void merge_seg_start_kernel(const MergeCounts* mc, const uint32_t* flags, const uint32_t* idx,
-                                       const uint32_t* nleaf, uint32_t* seg_start, uint32_t* seg_leaf) {
-  after_previous();
-  const uint32_t n_new = mc->n_new;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += stride)
-    if (flags[i]) {
-      seg_start[idx[i]] = (uint32_t)i;
-      seg_leaf[idx[i]] = nleaf[i];
+  __shared__ uint32_t ws[32];
+  __shared__ uint32_t s_tile, s_pre[2];
+  const uint32_t n = *n_dev, n_tiles = ceil_div(n, kGroupTile);
+  for (;;) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    __syncthreads();
+    if (tile >= n_tiles) {
+      if (tile == 0 && threadIdx.x == 0) mc->n_new = mc->n_segs = 0;  // no INSERT
+      break;
     }
+    const uint32_t q = tile * kGroupTile + 2 * threadIdx.x;
+    uint2 is = make_uint2(0, 0), lf = make_uint2(kNil, kNil);
+    if (q + 1 < n) {
+      is = *reinterpret_cast<const uint2*>(isnew + q);
+      lf = *reinterpret_cast<const uint2*>(mleaf + q);
+    } else if (q < n) {
+      is.x = isnew[q];
+      lf.x = mleaf[q];
+    }
+    uint64_t k[2] = {0, 0}, v[2] = {0, 0};
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (j ? is.y : is.x) {
+        const uint32_t u = ins_list[q + j];
+        k[j] = ukeys[u];
+        v[j] = uvals[u];
+      }
+    uint32_t head_x = is.x, head_y = is.y;
+    if (head_y && is.x && lf.x == lf.y) head_y = 0;
+    if (head_x || (head_y && lf.x == lf.y)) {
+      bool seen = false;
+      for (uint32_t p = q; p > 0 && !seen && mleaf[p - 1] == lf.x; p--) seen = isnew[p - 1] != 0;
+      if (seen) {
+        head_x = 0;
+        if (lf.x == lf.y) head_y = 0;
+      }
+    }
+    // both counts in one sum: at most 2048 of each a tile
+    const uint32_t mine = is.x + is.y + ((head_x + head_y) << 16);
+    uint32_t tot;
+    const uint32_t ex = blk_exclusive_sum(mine, ws, &tot);
+    if (threadIdx.x < 64) {
+      const bool seg = threadIdx.x >= 32;
+      const uint32_t sum = seg ? tot >> 16 : tot & 0xffffu;
+      const uint32_t pre = look_back(seg ? status_seg : status, tile, sum, epoch, err);
+      if ((threadIdx.x & 31) == 0) {
+        s_pre[seg] = pre;
+        if (tile == n_tiles - 1) (seg ? mc->n_segs : mc->n_new) = pre + sum;
+      }
+    }
+    __syncthreads();
+    uint32_t p = s_pre[0] + (ex & 0xffffu), sg = s_pre[1] + (ex >> 16);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      if (!(j ? is.y : is.x)) continue;
+      const uint32_t leaf = j ? lf.y : lf.x;
+      newk[p] = k[j];
+      newv[p] = v[j];
+      nq[p] = q + j;
+      nleaf[p] = leaf;
+      if (j ? head_y : head_x) {
+        seg_start[sg] = p;
+        seg_leaf[sg] = leaf;
+        sg++;
+      }
+      p++;
+    }
+  }
+  if (threadIdx.x == 0) tiles_done(ctr);
 }
 
 __device__ __forceinline__ void seg_bounds(const MergeCounts* mc, const uint32_t* seg_start, uint32_t s,
                                            uint32_t& a, uint32_t& b) {
   a = seg_start[s];
   b = (s + 1 < mc->n_segs) ? seg_start[s + 1] : mc->n_new;
-}
-
-// pieces - 1 per segment (new leaves it creates)
-__global__ void merge_leaf_count_kernel(DevTree t, uint32_t leaf_fill, const MergeCounts* mc,
-                                        const uint32_t* seg_start, const uint32_t* nleaf, size_t n_upper,
-                                        uint32_t* extra) {
-  after_previous();
-  const size_t n_segs = min(n_upper, (size_t)mc->n_segs);  // the scan reads n_segs entries
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_segs; s += stride) {
-    uint32_t a, b;
-    seg_bounds(mc, seg_start, (uint32_t)s, a, b);
-    const uint32_t leaf = nleaf[a];
-    const uint32_t m = hdr_size(t.keys[(size_t)leaf * 32 + 31]) + (b - a);
-    extra[s] = m <= (uint32_t)kMaxKeys ? 0u : ceil_div(m, leaf_fill) - 1;
-  }
 }
 
 // reserve the leaf pieces (and headroom for the inner levels) in one step;
@@ -253,9 +286,57 @@ __device__ __forceinline__ void reserve_pieces(const DevTree& t, MergeCounts* mc
   mc->cap_fail = 0;
   mc->node_base = atomicAdd(&t.ctrl->n_nodes, T);
 }
-__global__ void merge_alloc_kernel(DevTree t, MergeCounts* mc, uint32_t entry_cap) {
+
+// New leaves per segment (pieces - 1), their places, and the reservation: one
+// launch over tiles of the segments; the last tile's block knows the total.  It
+// was three launches (count, scan, reserve).
+__global__ void __launch_bounds__(kGroupThreads)
+    merge_reserve_kernel(DevTree t, uint32_t leaf_fill, uint32_t entry_cap, MergeCounts* mc, const uint32_t* seg_start,
+                         const uint32_t* seg_leaf, uint32_t* extra, uint32_t* eoff, uint64_t* status, uint32_t* ctr,
+                         uint32_t epoch, uint32_t* err) {
   after_previous();
-  reserve_pieces(t, mc, entry_cap);
+  __shared__ uint32_t ws[32];
+  __shared__ uint32_t s_tile, s_pre;
+  const uint32_t n = mc->n_segs, n_tiles = ceil_div(n, (uint32_t)kGroupThreads);
+  for (;;) {
+    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    __syncthreads();
+    if (tile >= n_tiles) {
+      if (tile == 0 && threadIdx.x == 0) {
+        mc->n_leaf_entries = 0;
+        reserve_pieces(t, mc, entry_cap);
+      }
+      break;
+    }
+    const uint32_t i = tile * kGroupThreads + threadIdx.x;
+    uint32_t e = 0;
+    if (i < n) {
+      uint32_t a, b;
+      seg_bounds(mc, seg_start, i, a, b);
+      const uint32_t m = hdr_size(t.keys[(size_t)seg_leaf[i] * 32 + 31]) + (b - a);
+      e = m <= (uint32_t)kMaxKeys ? 0u : ceil_div(m, leaf_fill) - 1;
+    }
+    uint32_t tot;
+    const uint32_t ex = blk_exclusive_sum(e, ws, &tot);
+    if (threadIdx.x < 32) {
+      const uint32_t pre = look_back(status, tile, tot, epoch, err);
+      if (threadIdx.x == 0) {
+        s_pre = pre;
+        if (tile == n_tiles - 1) {
+          mc->n_leaf_entries = pre + tot;
+          reserve_pieces(t, mc, entry_cap);
+        }
+      }
+    }
+    __syncthreads();
+    if (i < n) {
+      extra[i] = e;
+      eoff[i] = s_pre + ex;
+    }
+  }
+  if (threadIdx.x == 0) tiles_done(ctr);
 }
 
 // a batch whose pieces did not fit answers kNoCapacity for all its new keys
@@ -1061,23 +1142,23 @@ int merge_update_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+// look-back words for a batch of up to n requests: new keys, segments | the
+// segments' new leaves reuse the first part
+size_t merge_lb_words(size_t n) { return 2 * ((n + kGroupThreads - 1) / kGroupThreads + 1); }
+
+static uint32_t next_epoch(uint32_t* epoch) {
+  *epoch = (*epoch + 1) & ((1u << 30) - 1);
+  if (*epoch == 0) *epoch = 1;  // zeroed status words carry epoch 0
+  return *epoch;
+}
+
 int merge_group_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
-  const uint32_t* n_ins = &w.counts->n_ins;
-  uint32_t* err = &h->tree.ctrl->error;
-  if (scan_exclusive_u32_lb(w.m_isnew, w.m_pos, n_upper, n_ins, &mc->n_new, w.lb_status, w.lb_ctr, &w.lb_epoch, err,
-                            s) != cudaSuccess)
-    return -2;
-  const unsigned gb = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256);
-  launch_after(merge_compact_kernel, gb, 256, 0, s, w.ins_list, n_ins, w.m_isnew, w.m_pos, w.ukeys, w.uvals, w.m_leaf,
-               w.m_newk, w.m_newv, w.m_nq, w.m_nleaf);
-  launch_after(merge_seg_flags_kernel, gb, 256, 0, s, mc, w.m_nleaf, n_upper, w.m_isnew);
-  count_launch(2);
-  if (scan_exclusive_u32_lb(w.m_isnew, w.m_pos, n_upper, &mc->n_new, &mc->n_segs, w.lb_status, w.lb_ctr, &w.lb_epoch,
-                            err, s) != cudaSuccess)
-    return -2;
-  launch_after(merge_seg_start_kernel, gb, 256, 0, s, mc, w.m_isnew, w.m_pos, w.m_nleaf, w.m_seg, w.m_leaf);
+  const unsigned gb = (unsigned)min((size_t)h->sm_count * 2, (n_upper + kGroupTile - 1) / kGroupTile);
+  launch_after(merge_group_kernel, gb, kGroupThreads, 0, s, mc, w.ins_list, &w.counts->n_ins, w.m_isnew, w.ukeys,
+               w.uvals, w.m_leaf, w.m_newk, w.m_newv, w.m_nq, w.m_nleaf, w.m_seg, w.m_pos, w.lb_status,
+               w.lb_status + merge_lb_words(w.cap) / 2, w.lb_ctr, next_epoch(&w.lb_epoch), &h->tree.ctrl->error);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1085,15 +1166,10 @@ int merge_group_phase(Handle* h, size_t n_upper, cudaStream_t s) {
 int merge_reserve_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
+  const unsigned rb = (unsigned)min((size_t)h->sm_count * 2, (n_upper + kGroupThreads - 1) / kGroupThreads);
+  launch_after(merge_reserve_kernel, rb, kGroupThreads, 0, s, h->tree, h->leaf_fill, (uint32_t)w.cap, mc, w.m_seg,
+               w.m_pos, w.m_isnew, w.m_leaf, w.lb_status, w.lb_ctr, next_epoch(&w.lb_epoch), &h->tree.ctrl->error);
   const unsigned gb = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256);
-  launch_after(merge_leaf_count_kernel, gb, 256, 0, s, h->tree, h->leaf_fill, mc, w.m_seg, w.m_nleaf, n_upper,
-               w.m_isnew);
-  count_launch();
-  if (scan_exclusive_u32_lb(w.m_isnew, w.m_pos, n_upper, &mc->n_segs, &mc->n_leaf_entries, w.lb_status, w.lb_ctr,
-                            &w.lb_epoch, &h->tree.ctrl->error, s) !=
-      cudaSuccess)
-    return -2;
-  launch_after(merge_alloc_kernel, 1, 1, 0, s, h->tree, mc, (uint32_t)w.cap);
   launch_after(merge_fail_mark_kernel, gb, 256, 0, s, mc, w.m_nq, w.ins_list, w.uans_st);
   count_launch(2);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1104,7 +1180,7 @@ int merge_write_phase(Handle* h, cudaStream_t s) {
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
   const uint32_t entry_cap = (uint32_t)w.cap;
   merge_leaf_kernel<8><<<(unsigned)((size_t)h->sm_count * 8), 256, 0, s>>>(
-      h->tree, h->leaf_fill, mc, w.m_seg, w.m_pos, w.m_isnew, w.m_newk, w.m_newv, w.m_nq, w.m_leaf,
+      h->tree, h->leaf_fill, mc, w.m_seg, w.m_leaf, w.m_isnew, w.m_newk, w.m_newv, w.m_nq, w.m_pos,
       reinterpret_cast<MergeEntry*>(w.m_ent_a));
   count_launch();
   if (launch_inner(h, entry_cap, mc, s) != cudaSuccess) return -2;

@@ -21,6 +21,7 @@
 #include "bt_common.cuh"
 #include "bt_internal.h"
 #include "bt_launch.cuh"
+#include "bt_lookback.cuh"
 
 namespace bt {
 
@@ -131,18 +132,9 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
   }
 }
 
-// Single-pass exclusive scan with decoupled look-back, for a count on the
-// device far below its bound (the merge engine's scans: about 2^18 live
-// entries under a 2^22 bound): one launch where the reduce / single / apply
-// form takes three.  status[t] = epoch << 34 | state << 32 | value, state 1
-// the tile's own sum, 2 its inclusive prefix; each call's epoch makes the
-// words of earlier calls read as not ready, so the array is never cleared.
-// ctr[0] hands tile ids out in the order blocks take them (a tile waits only
-// on tiles taken before it); the last block to finish resets ctr.  The
-// look-back spin is bounded: past kSpinLimit it sets kErrSpin in *err.
-constexpr uint64_t kLbAgg = 1ull << 32, kLbInc = 2ull << 32;
-constexpr uint32_t kLbSpinLimit = 1u << 22;
-
+// Single-pass exclusive scan with decoupled look-back (bt_lookback.cuh), for a
+// count on the device far below its bound: one launch where the reduce / single
+// / apply form takes three.
 __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* in, uint32_t* out, size_t n_upper,
                                                                const uint32_t* n_dev, uint32_t* total_out,
                                                                uint64_t* status, uint32_t* ctr, uint32_t epoch,
@@ -152,7 +144,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* i
   __shared__ uint32_t tot, s_tile, s_prefix;
   const size_t n = n_dev ? min(n_upper, (size_t)*n_dev) : n_upper;
   const size_t n_tiles = (n + kScanTile - 1) / kScanTile;
-  const uint64_t tag = (uint64_t)epoch << 34;
   for (;;) {
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
     __syncthreads();
@@ -171,31 +162,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* i
       sum += v[i];
     }
     uint32_t ex = block_exclusive_scan(sum, ws, &tot);
-    if (threadIdx.x == 0) {
-      uint32_t prefix = 0;
-      if (tile > 0) {
-        st_release(&status[tile], tag | kLbAgg | tot);
-        int64_t t = (int64_t)tile - 1;
-        uint32_t spins = 0;
-        while (t >= 0) {
-          const uint64_t w = ld_acquire(&status[t]);
-          const uint32_t state = (uint32_t)(w >> 32) & 3u;
-          if ((uint32_t)(w >> 34) != epoch || state == 0) {
-            if (++spins > kLbSpinLimit) {
-              if (err) atomicOr(err, kErrSpin);
-              break;
-            }
-            if (spins > 64) __nanosleep(64);
-            continue;
-          }
-          prefix += (uint32_t)w;
-          if (state == 2) break;
-          t--;
-        }
+    if (threadIdx.x < 32) {
+      const uint32_t prefix = look_back(status, tile, tot, epoch, err);
+      if (threadIdx.x == 0) {
+        s_prefix = prefix;
+        if (tile == n_tiles - 1 && total_out) *total_out = prefix + tot;
       }
-      st_release(&status[tile], tag | kLbInc | (uint64_t)(prefix + tot));
-      s_prefix = prefix;
-      if (tile == n_tiles - 1 && total_out) *total_out = prefix + tot;
     }
     __syncthreads();
     ex += s_prefix;
@@ -205,15 +177,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* i
       ex += v[i];
     }
   }
-  // the last block to finish makes the tile ids start at 0 again
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&ctr[1], 1u) == gridDim.x - 1) {
-      ctr[0] = 0;
-      ctr[1] = 0;
-      __threadfence();
-    }
-  }
+  if (threadIdx.x == 0) tiles_done(ctr);
 }
 
 // ---------------------------------------------------------------- sort ----

@@ -1,5 +1,6 @@
-"""The merge engine's scans when the live entries need more tiles (4096) than
-there are blocks: one batch of INSERTs into a small tree, read back whole."""
+"""The merge engine's look-back tiles: more of them than there are blocks, their
+edges (2048 INSERT keys, 1024 segments), runs of keys of one leaf, old and new
+mixed, across the edges."""
 import numpy as np
 import pytest
 
@@ -22,4 +23,17 @@ def test_inserts_of_many_scan_tiles(gpu, n):
     ak, av = np.concatenate([k, base]), np.concatenate([v, base])
     at = np.argsort(ak)
     assert (gk == ak[at]).all() and (gv == av[at]).all()
+    assert t.stats()["error"] == 0
+
+
+@pytest.mark.parametrize("n", [1, 2, 2047, 2048, 2049, 4097, 40_001, 300_000])
+@pytest.mark.parametrize("step", [2, 16, 31])
+def test_new_keys_among_old_ones_of_their_leaf(gpu, n, step):
+    old = np.arange(0, n, step, dtype=np.uint64) + np.uint64(1)
+    t = E.BTree(max_keys=2 * n + 4096, max_batch=max(n, 1024))
+    t.bulk_build(dev(old), dev(old))
+    k = np.random.default_rng(n).permutation(np.arange(n, dtype=np.uint64) + np.uint64(1))
+    run_batch(t, k, k + np.uint64(5), np.full(n, E.OP_INSERT, np.uint8), E.MODE_SORTED | E.MODE_MERGE_ENGINE)
+    gk, gv = dump(t)
+    assert (gk == np.sort(k)).all() and (gv == gk + np.uint64(5)).all()
     assert t.stats()["error"] == 0
