@@ -6,7 +6,7 @@
 // one that comes before the first write of its key, sees the pre-batch tree.  So instead
 // of sorting the whole batch, the front end
 //
-//   1. counts the write requests and sizes an open-addressing table for
+//   1. lists the write requests and sizes an open-addressing table for
 //      their keys (a power of two >= 4x the count, at least 1024 slots:
 //      most lookups ask for a key the table does not hold, and a linear probe
 //      for an absent key runs about (1 + 1/(1-a)^2)/2 slots at load a: 1.4
@@ -14,8 +14,9 @@
 //   2. records, per written key, the index of its first write,
 //   3. classifies every request: "touched" if its op code is invalid or its
 //      key has a write at or before it; otherwise it is a plain lookup,
-//      and compacts both classes in input order (a flag pass, a scan of
-//      the per-tile counts, a scatter pass).
+//      and compacts both classes: in one pass over tiles that take their
+//      places as they come when the sample sort follows, else in input
+//      order (a flag pass, a scan of the per-tile counts, a scatter pass).
 //
 // The touched requests go through the sort + segmented-scan path (their
 // runs all start with a write, so the pre-batch value reaches them from the
@@ -23,10 +24,10 @@
 // run on the pre-batch tree, unsorted, writing their answers in place.  For a
 // read-mostly batch the sort shrinks to the INSERTs.
 //
-// HBM traffic per request: count (1 B op), table insert (1 B op, plus the key
-// of a write), flag (8 B key + 1 B op + the probe, which is L2-resident for
-// small write counts, then a 1 B flag), scatter (1 B flag, then a 4 B list
-// entry, or 9 B read and a 12 B touched entry).
+// HBM traffic per request: gather (1 B op), table insert (the key of a write),
+// split (8 B key + 1 B op + the probe, which is L2-resident for small write
+// counts, then a 12 B list entry or touched entry); in input order: flag (the
+// same reads, then a 1 B flag), scatter (1 B flag, 9 B read, a 12 B entry).
 #include <cuda_runtime.h>
 
 #include "bt_block.cuh"
@@ -162,26 +163,27 @@ constexpr int kTileItems = 8;
 constexpr int kTile = kTileThreads * kTileItems;  // 2048
 constexpr int kTileWarps = kTileThreads / 32;
 
-// The thread's items of a tile (item j: base + j * kTileThreads + threadIdx.x),
+// The thread's items of a tile (item j: base + j * THREADS + threadIdx.x),
 // their keys and op codes, and a bit per item: touched.
+template <int THREADS, int ITEMS>
 __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ keys, const uint8_t* __restrict__ ops,
                                                    size_t n, const Slot* __restrict__ tab,
                                                    const BatchCounts* __restrict__ counts, size_t base,
-                                                   uint64_t (&k)[kTileItems], uint8_t (&op)[kTileItems]) {
+                                                   uint64_t (&k)[ITEMS], uint8_t (&op)[ITEMS]) {
   const uint32_t mask = counts->cap - 1;
   const bool any = counts->n_ins_req != 0;
-  uint64_t sk[kTileItems];
-  uint32_t sf[kTileItems], sh[kTileItems];
+  uint64_t sk[ITEMS];
+  uint32_t sf[ITEMS], sh[ITEMS];
   // loads first, then every item's first probe slot (independent loads in
   // flight), then the rare longer probes
 #pragma unroll
-  for (int j = 0; j < kTileItems; j++) {
-    const size_t i = base + (size_t)j * kTileThreads + threadIdx.x;
+  for (int j = 0; j < ITEMS; j++) {
+    const size_t i = base + (size_t)j * THREADS + threadIdx.x;
     k[j] = i < n ? keys[i] : kKeyMax;
     op[j] = i < n ? ops[i] : 0;
   }
 #pragma unroll
-  for (int j = 0; j < kTileItems; j++) {
+  for (int j = 0; j < ITEMS; j++) {
     sh[j] = (uint32_t)slot_hash(k[j]) & mask;
     sk[j] = kKeyMax;
     sf[j] = kNone;
@@ -193,17 +195,17 @@ __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ 
   }
   // the longer probes, all of this thread's unresolved items one slot per
   // round (their loads in flight together), instead of item after item
-  uint32_t first[kTileItems];
+  uint32_t first[ITEMS];
   uint32_t todo = 0;
 #pragma unroll
-  for (int j = 0; j < kTileItems; j++) {
+  for (int j = 0; j < ITEMS; j++) {
     first[j] = kNone;
     if (sk[j] == k[j] && k[j] != kKeyMax) first[j] = sf[j];
     else if (sk[j] != kKeyMax) todo |= 1u << j;
   }
   for (uint32_t probe = 0; todo && probe < mask; probe++) {
 #pragma unroll
-    for (int j = 0; j < kTileItems; j++) {
+    for (int j = 0; j < ITEMS; j++) {
       if (!((todo >> j) & 1u)) continue;
       sh[j] = (sh[j] + 1) & mask;
       const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(tab + sh[j]);
@@ -211,7 +213,7 @@ __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ 
       sf[j] = (uint32_t)e.y;
     }
 #pragma unroll
-    for (int j = 0; j < kTileItems; j++) {
+    for (int j = 0; j < ITEMS; j++) {
       if (!((todo >> j) & 1u)) continue;
       if (sk[j] == k[j]) {
         first[j] = sf[j];
@@ -223,8 +225,8 @@ __device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ 
   }
   uint32_t touched = 0;
 #pragma unroll
-  for (int j = 0; j < kTileItems; j++) {
-    const size_t i = base + (size_t)j * kTileThreads + threadIdx.x;
+  for (int j = 0; j < ITEMS; j++) {
+    const size_t i = base + (size_t)j * THREADS + threadIdx.x;
     if (i < n) {
       bool f = op[j] > 2;  // invalid op codes are rejected on the sorted path
       if (!f && any && k[j] != kKeyMax) f = first[j] != kNone && (uint32_t)i >= first[j];
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t
   const size_t base = (size_t)blockIdx.x * kTile;
   uint64_t k[kTileItems];
   uint8_t op[kTileItems];
-  const uint32_t touched = classify_items(keys, ops, n, tab, counts, base, k, op);
+  const uint32_t touched = classify_items<kTileThreads, kTileItems>(keys, ops, n, tab, counts, base, k, op);
 #pragma unroll
   for (int j = 0; j < kTileItems; j++) {
     const size_t i = base + (size_t)j * kTileThreads + threadIdx.x;
@@ -259,63 +261,90 @@ __global__ void __launch_bounds__(kTileThreads) front_flag_kernel(const uint64_t
   }
 }
 
-// Classify and compact in one launch, for the sample sort, which orders equal
-// keys by their request index: each tile takes its places in the two lists
-// with one atomic each, so the tiles come in any order (requests of a tile stay
-// together and in order).  `flags`-free: the class is used where it is found.
-__global__ void __launch_bounds__(kTileThreads) front_split_kernel(const uint64_t* keys, const uint8_t* ops, size_t n,
-                                                                   const Slot* tab, BatchCounts* counts, uint64_t* tk,
-                                                                   uint32_t* tv, uint32_t* list, uint64_t* lk) {
-  after_previous();
-  __shared__ uint32_t cnt[kTileItems][kTileWarps];
-  __shared__ uint32_t at_touch, at_lookup;
+// A tile's requests parted in two lists, each in index order: the tile takes its
+// places in both with one atomic each, so the tiles come in any order.
+// put(item, in the first list, place).  Two requests a thread and every warp slot
+// of an SM in use: what bounds these kernels is the latency of the request, its
+// hash slot and the places, not the bytes.  With eight a thread (90 registers,
+// two blocks an SM) the 2^22 split took 72 us (1.4 TB/s); a batch is 21 us
+// shorter with two (four a thread: 14).
+constexpr int kSplitThreads = 512;
+constexpr int kSplitItems = 2;
+constexpr int kSplitTile = kSplitThreads * kSplitItems;
+constexpr int kSplitWarps = kSplitThreads / 32;
+
+template <typename Put>
+__device__ __forceinline__ void split_tile(uint32_t here, uint32_t first, uint32_t* n_first, uint32_t* n_second,
+                                           Put put) {
+  constexpr int kCells = kSplitItems * kSplitWarps, kPer = kCells / 32;  // cells of a lane of the scanning warp
+  static_assert(kCells % 32 == 0, "whole lanes");
+  __shared__ uint32_t cnt[kCells];
+  __shared__ uint32_t at_first, at_second;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1u;
-  const size_t base = (size_t)blockIdx.x * kTile;
-  uint64_t k[kTileItems];
-  uint8_t op[kTileItems];
-  uint32_t bal[kTileItems];
-  const uint32_t touched = classify_items(keys, ops, n, tab, counts, base, k, op);
+  uint32_t bal[kSplitItems];
 #pragma unroll
-  for (int j = 0; j < kTileItems; j++) {
-    bal[j] = __ballot_sync(0xffffffffu, (touched >> j) & 1u);
-    if (lane == 0) cnt[j][warp] = __popc(bal[j]);
+  for (int j = 0; j < kSplitItems; j++) {
+    bal[j] = __ballot_sync(0xffffffffu, (first >> j) & 1u);
+    if (lane == 0) cnt[j * kSplitWarps + warp] = __popc(bal[j]);
   }
   __syncthreads();
   // exclusive prefix over (item, warp) in index order
   if (warp == 0) {
-    uint32_t carry = 0;
+    uint32_t c[kPer], sum = 0;
 #pragma unroll
-    for (int j = 0; j < kTileItems; j++) {
-      const uint32_t c = lane < kTileWarps ? cnt[j][lane] : 0u;
-      uint32_t incl = c;
-#pragma unroll
-      for (int o = 1; o < kTileWarps; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (lane < kTileWarps) cnt[j][lane] = carry + incl - c;
-      carry += __shfl_sync(0xffffffffu, incl, kTileWarps - 1);
+    for (int x = 0; x < kPer; x++) {
+      c[x] = cnt[lane * kPer + x];
+      sum += c[x];
     }
-    const uint32_t here = (uint32_t)min((size_t)kTile, n - base);
-    if (lane == 0) at_touch = carry ? atomicAdd(&counts->n_touch, carry) : 0u;
-    if (lane == 1) at_lookup = here > carry ? atomicAdd(&counts->n_lookup, here - carry) : 0u;
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if (lane == 0) at_first = total ? atomicAdd(n_first, total) : 0u;
+    if (lane == 1) at_second = here > total ? atomicAdd(n_second, here - total) : 0u;
+    uint32_t at = incl - sum;
+#pragma unroll
+    for (int x = 0; x < kPer; x++) {
+      cnt[lane * kPer + x] = at;
+      at += c[x];
+    }
   }
   __syncthreads();
-  const uint32_t t0 = at_touch, l0 = at_lookup;
+  const uint32_t f0 = at_first, s0 = at_second;
 #pragma unroll
-  for (int j = 0; j < kTileItems; j++) {
-    const uint32_t i = (uint32_t)j * kTileThreads + threadIdx.x;
-    if (base + i >= n) continue;
-    const uint32_t p = cnt[j][warp] + __popc(bal[j] & lt);  // touched before it in the tile
-    if ((bal[j] >> lane) & 1u) {
-      tk[t0 + p] = k[j];
-      tv[t0 + p] = pair_payload((uint32_t)(base + i), op[j]);
-    } else {
-      list[l0 + i - p] = (uint32_t)(base + i);
-      lk[l0 + i - p] = k[j];
-    }
+  for (int j = 0; j < kSplitItems; j++) {
+    const uint32_t i = (uint32_t)j * kSplitThreads + threadIdx.x;
+    if (i >= here) continue;
+    const uint32_t p = cnt[j * kSplitWarps + warp] + __popc(bal[j] & ((1u << lane) - 1u));  // first ones before it
+    const bool f = (bal[j] >> lane) & 1u;
+    put(j, f, f ? f0 + p : s0 + i - p);
   }
+}
+
+// Classify and compact in one launch, for the sample sort, which orders equal
+// keys by their request index.  `flags`-free: the class is used where it is found.
+__global__ void __launch_bounds__(kSplitThreads, 4)
+    front_split_kernel(const uint64_t* keys, const uint8_t* ops, size_t n, const Slot* tab, BatchCounts* counts,
+                       uint64_t* tk, uint32_t* tv, uint32_t* list, uint64_t* lk) {
+  after_previous();
+  const size_t base = (size_t)blockIdx.x * kSplitTile;
+  uint64_t k[kSplitItems];
+  uint8_t op[kSplitItems];
+  const uint32_t touched = classify_items<kSplitThreads, kSplitItems>(keys, ops, n, tab, counts, base, k, op);
+  split_tile((uint32_t)min((size_t)kSplitTile, n - base), touched, &counts->n_touch, &counts->n_lookup,
+             [&](int j, bool touch, uint32_t at) {
+               const uint32_t i = (uint32_t)base + (uint32_t)j * kSplitThreads + threadIdx.x;
+               if (touch) {
+                 tk[at] = k[j];
+                 tv[at] = pair_payload(i, op[j]);
+               } else {
+                 list[at] = i;
+                 lk[at] = k[j];
+               }
+             });
 }
 
 // exclusive offsets of n_tiles counts, in place, with one block
@@ -505,62 +534,36 @@ __global__ void __launch_bounds__(kThreads) pack_check_kernel(const uint32_t* __
 // index, and `pad` the representative's index (bit 31: the key has a DELETE).
 constexpr uint32_t kDelBit = 1u << 31;
 
-// The requests of an STM batch split in two lists, in no particular order,
-// with one atomic per warp and list: the valid GETs (with their keys, for
-// the lookup kernels) and the rest (INSERT, DELETE, invalid op codes and the
-// reserved key, which the STM kernel answers).  counts->n_lookup and
-// counts->n_ins_req end as the lists' lengths.
-__device__ __forceinline__ uint32_t warp_append(uint32_t m, uint32_t* __restrict__ counter) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t c = __popc(m);
-  uint32_t incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= (uint32_t)o) incl += y;
-  }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(0xffffffffu, base, 31);
-  return base + incl - c;  // this lane's first slot
-}
-
-__global__ void __launch_bounds__(kThreads) stm_split_kernel(const uint64_t* keys, const uint8_t* ops, size_t n,
-                                                             uint32_t* get_list, uint64_t* get_keys,
-                                                             uint32_t* wr_list, BatchCounts* counts) {
+// The requests of an STM batch split in two lists, in no particular order (the
+// tiles'): the valid GETs (with their keys, for the lookup kernels) and the rest
+// (INSERT, DELETE, invalid op codes and the reserved key, which the STM kernel
+// answers).  counts->n_lookup and counts->n_ins_req end as the lists' lengths.
+// One atomic a tile and list: one a warp and list, 16,000 on two words, bound a
+// 2^20 batch's split (22 us).
+__global__ void __launch_bounds__(kSplitThreads, 4)
+    stm_split_kernel(const uint64_t* keys, const uint8_t* ops, size_t n, uint32_t* get_list, uint64_t* get_keys,
+                     uint32_t* wr_list, BatchCounts* counts) {
   after_previous();
-  const uint32_t lane = threadIdx.x & 31;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  // whole warps iterate together (the appends are warp-aggregated); four
-  // requests per lane
-  const size_t warp0 = ((size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * 4;
-  for (size_t w = warp0; w < n; w += stride * 4) {
-    const size_t i0 = w + 4 * (size_t)lane;
-    uint32_t gm = 0, wm = 0;
-    uint64_t k[4];
+  const size_t base = (size_t)blockIdx.x * kSplitTile;
+  uint64_t k[kSplitItems];
+  uint32_t gets = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      k[j] = kKeyMax;
-      if (i0 + j < n) {
-        k[j] = keys[i0 + j];
-        const bool get = ops[i0 + j] == kOpGet && k[j] != kKeyMax;
-        gm |= (get ? 1u : 0u) << j;
-        wm |= (get ? 0u : 1u) << j;
-      }
-    }
-    uint32_t pg = warp_append(gm, &counts->n_lookup);
-    uint32_t pw = warp_append(wm, &counts->n_ins_req);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if ((gm >> j) & 1u) {
-        get_list[pg] = (uint32_t)(i0 + j);
-        get_keys[pg++] = k[j];
-      } else if ((wm >> j) & 1u) {
-        wr_list[pw++] = (uint32_t)(i0 + j);
-      }
-    }
+  for (int j = 0; j < kSplitItems; j++) {
+    const size_t i = base + (size_t)j * kSplitThreads + threadIdx.x;
+    k[j] = i < n ? keys[i] : kKeyMax;
+    const uint8_t op = i < n ? ops[i] : (uint8_t)kOpGet;
+    gets |= (op == kOpGet && k[j] != kKeyMax ? 1u : 0u) << j;
   }
+  split_tile((uint32_t)min((size_t)kSplitTile, n - base), gets, &counts->n_lookup, &counts->n_ins_req,
+             [&](int j, bool get, uint32_t at) {
+               const uint32_t i = (uint32_t)base + (uint32_t)j * kSplitThreads + threadIdx.x;
+               if (get) {
+                 get_list[at] = i;
+                 get_keys[at] = k[j];
+               } else {
+                 wr_list[at] = i;
+               }
+             });
 }
 
 __global__ void __launch_bounds__(kThreads) combine_arrive_kernel(const uint64_t* keys, const uint8_t* ops,
@@ -650,9 +653,9 @@ __global__ void __launch_bounds__(kThreads) combine_fixup_kernel(const uint8_t* 
 
 int stm_split(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n, cudaStream_t s) {
   Work& w = h->w;
-  const unsigned g = (unsigned)min((size_t)h->sm_count * 8, (n / 4 + kThreads) / kThreads);
+  const unsigned tiles = (unsigned)((n + kSplitTile - 1) / kSplitTile);
   if (cudaMemsetAsync(w.counts, 0, sizeof(BatchCounts), s) != cudaSuccess) return -2;
-  launch_after(stm_split_kernel, g, kThreads, 0, s, keys, ops, n, w.get_list, w.ukeys, w.ins_list, w.counts);
+  launch_after(stm_split_kernel, tiles, kSplitThreads, 0, s, keys, ops, n, w.get_list, w.ukeys, w.ins_list, w.counts);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -746,7 +749,8 @@ int front_classify(Handle* h, const uint64_t* keys, const uint8_t* ops, size_t n
   launch_after(front_clear_kernel, (unsigned)h->sm_count * 4, kThreads, 0, s, tab, w.f_tab_cap, c);
   launch_after(front_insert_kernel, g, kThreads, 0, s, keys, w.f_list, tab, c);
   if (!ordered) {
-    launch_after(front_split_kernel, (unsigned)n_tiles, kTileThreads, 0, s, keys, ops, n, tab, c, w.f_tk, w.f_tv,
+    const unsigned split_tiles = (unsigned)((n + kSplitTile - 1) / kSplitTile);
+    launch_after(front_split_kernel, split_tiles, kSplitThreads, 0, s, keys, ops, n, tab, c, w.f_tk, w.f_tv,
                  w.f_list, w.f_lk);
     count_launch(4);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
