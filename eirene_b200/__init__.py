@@ -101,7 +101,7 @@ EXPORTS = [
     "bt_profile", "bt_profile_read", "bt_launch_count", "bt_bulk_build_static",
     "bt_set_learned_group", "bt_learned_info", "bt_mlp_grad", "bt_set_option", "bt_autotune",
     "bt_serve_config_init", "bt_serve_start", "bt_submit", "bt_poll", "bt_wait", "bt_serve_get_stats", "bt_serve_stop",
-    "bt_route_batch", "bt_unroute_results", "bt_save", "bt_load", "bt_range_batch", "bt_sync", "bt_save_image", "bt_load_image",
+    "bt_route_batch", "bt_unroute_results", "bt_save", "bt_load", "bt_range_batch", "bt_range_batch_filled", "bt_sync", "bt_save_image", "bt_load_image",
     "bt_refit", "bt_execute_batch_host_async", "bt_host_wait", "bt_serve_batch_times", "bt_autotune_fill",
     "bt_execute_batch_host_packed_async", "bt_execute_batches",
 ]
@@ -192,6 +192,7 @@ def lib():
             "bt_unroute_results": [_P, _P, _P, _P, _SZ, _P, _P, _P],
             "bt_save": [_P, ctypes.c_char_p],
             "bt_range_batch": [_P, _P, _P, _SZ, ctypes.c_uint32, _P, _P, _P, _P],
+            "bt_range_batch_filled": [_P, _P, _P, _SZ, ctypes.c_uint32, _P, _P, _P, _P],
             "bt_sync": [_P, _P],
             "bt_save_image": [_P, ctypes.c_char_p],
             "bt_load_image": [_P, ctypes.c_char_p],
@@ -472,14 +473,12 @@ class BTree:
 
         n = lo.numel()
         dev_ = lo.device
-        w = max(max_per, 1)
-        # one zeroed block for the three results: one fill instead of three
-        buf = torch.zeros(2 * n * w + (n + 1) // 2 + 1, dtype=torch.int64, device=dev_)
-        keys = buf[: n * w].view(n, w)[:, :max_per]
-        vals = buf[n * w: 2 * n * w].view(n, w)[:, :max_per]
-        counts = buf[2 * n * w:].view(torch.int32)[:n]
-        _check(lib().bt_range_batch(self._h, _ptr(lo), _ptr(hi), n, max_per, _ptr(keys), _ptr(vals), _ptr(counts),
-                                    _stream_ptr(stream)), "bt_range_batch")
+        # uninitialised: the kernel writes every place
+        keys = torch.empty((n, max(max_per, 1)), dtype=torch.int64, device=dev_)[:, :max_per]
+        vals = torch.empty((n, max(max_per, 1)), dtype=torch.int64, device=dev_)[:, :max_per]
+        counts = torch.empty(max(n, 1), dtype=torch.int32, device=dev_)[:n]
+        _check(lib().bt_range_batch_filled(self._h, _ptr(lo), _ptr(hi), n, max_per, _ptr(keys), _ptr(vals),
+                                           _ptr(counts), _stream_ptr(stream)), "bt_range_batch_filled")
         return counts, keys, vals
 
     def save(self, path: str):

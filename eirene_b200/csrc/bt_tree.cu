@@ -628,9 +628,13 @@ __global__ void __launch_bounds__(512) search_top_kernel(DevTree t, const TopNod
 // right fence.  A lane holds one slot; a ballot compacts the keys in [lo, hi] in
 // key order.  Inner levels are ranked by the separators' prefixes.  Read-only;
 // runs only when no writer is active.
+// kFill: the places past a query's pairs are zeroed, so that the caller need
+// not clear 16 bytes a place ahead of a kernel that writes most of them again
+// (the same scans, pages of 128: 37.9 -> 32.3 us).
 // 20,000 scans of about 100 keys on 2^24 keys, with the zero fill of the
 // results: 58.5 us with a descent per leaf (a dependent row and child id per
 // level), 42.2 with this at 46 registers, 39.4 at the 36 of seven blocks an SM.
+template <bool kFill>
 __global__ void __launch_bounds__(256, 7) range_kernel(DevTree t, const uint64_t* __restrict__ lo_keys,
                                                    const uint64_t* __restrict__ hi_keys, size_t n, uint32_t max_per,
                                                    uint64_t* __restrict__ out_keys, uint64_t* __restrict__ out_vals,
@@ -699,6 +703,11 @@ __global__ void __launch_bounds__(256, 7) range_kernel(DevTree t, const uint64_t
       from = fence;
     }
     if (lane == 0) out_counts[q] = count;
+    if (kFill)
+      for (uint64_t pos = (uint64_t)count + lane; pos < max_per; pos += 32) {
+        out_keys[q * max_per + pos] = 0;
+        out_vals[q * max_per + pos] = 0;
+      }
   }
 }
 
@@ -1017,14 +1026,15 @@ cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list
 }
 
 cudaError_t launch_range(Handle* h, const uint64_t* lo, const uint64_t* hi, size_t n, uint32_t max_per,
-                         uint64_t* out_keys, uint64_t* out_vals, uint32_t* out_counts, cudaStream_t s) {
+                         uint64_t* out_keys, uint64_t* out_vals, uint32_t* out_counts, bool fill, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const cudaError_t pe = ensure_pfx(h, s);
   if (pe != cudaSuccess) return pe;
   size_t blocks = (n * 32 + 255) / 256;
   const size_t cap = (size_t)h->sm_count * 16;
   if (blocks > cap) blocks = cap;
-  range_kernel<<<(unsigned)blocks, 256, 0, s>>>(h->tree, lo, hi, n, max_per, out_keys, out_vals, out_counts);
+  const auto kernel = fill ? range_kernel<true> : range_kernel<false>;
+  kernel<<<(unsigned)blocks, 256, 0, s>>>(h->tree, lo, hi, n, max_per, out_keys, out_vals, out_counts);
   count_launch();
   return cudaGetLastError();
 }

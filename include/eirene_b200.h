@@ -218,6 +218,10 @@ int bt_insert_batch(bt_handle *h, const uint64_t *keys, const uint64_t *vals, ui
  * Device buffers; stream ordered; must not overlap a batch that writes. */
 int bt_range_batch(bt_handle *h, const uint64_t *lo, const uint64_t *hi, size_t n, uint32_t max_per,
                    uint64_t *out_keys, uint64_t *out_vals, uint32_t *out_counts, void *stream);
+/* The same, with the places past a query's pairs set to zero (bt_range_batch
+ * leaves them as they are). */
+int bt_range_batch_filled(bt_handle *h, const uint64_t *lo, const uint64_t *hi, size_t n, uint32_t max_per,
+                          uint64_t *out_keys, uint64_t *out_vals, uint32_t *out_counts, void *stream);
 
 /* Number of keys (synchronous).  No reference counterpart. */
 int bt_size(bt_handle *h, uint64_t *n_keys);
