@@ -185,14 +185,16 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   ok = ok && cudaMalloc(&h.tree.low, nodes * 8) == cudaSuccess;
   ok = ok && cudaMalloc(&h.tree.pfx, nodes * 128) == cudaSuccess;
   ok = ok && cudaMalloc(&h.tree.fp, nodes * 32) == cudaSuccess;
-  ok = ok && cudaMalloc(&h.tree.ctrl, sizeof(bt::Ctrl)) == cudaSuccess;
+  // the control block and, behind it, the small counts of builds and dumps
+  constexpr size_t kCtrlBytes = (sizeof(bt::Ctrl) + 255) / 256 * 256;
+  ok = ok && cudaMalloc(&h.tree.ctrl, kCtrlBytes + 256) == cudaSuccess;
+  if (ok) h.geo = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h.tree.ctrl) + kCtrlBytes);
   // zeroed rows read as epoch 0, which no tree uses (see hdr_epoch)
   ok = ok && cudaMemset(h.tree.keys, 0, nodes * 256) == cudaSuccess;
   ok = ok && cudaMemset(h.tree.vals, 0, nodes * 256) == cudaSuccess;
   ok = ok && cudaMemset(h.tree.low, 0, nodes * 8) == cudaSuccess;
   ok = ok && cudaMemset(h.tree.pfx, 0xff, nodes * 128) == cudaSuccess;
   ok = ok && cudaMemset(h.tree.fp, 0, nodes * 32) == cudaSuccess;
-  ok = ok && cudaMalloc(&h.geo, 256) == cudaSuccess && cudaMallocHost(&h.pin, 256) == cudaSuccess;
   ok = ok && bt::work_alloc(&h.w, cfg.max_batch) == 0;
   ok = ok && cudaStreamCreateWithFlags(&h.internal_stream, cudaStreamNonBlocking) == cudaSuccess;
   {
@@ -206,10 +208,14 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
          cudaEventCreateWithFlags(&h.ans_ev, cudaEventDisableTiming) == cudaSuccess;
   }
   // the touched-request count of the batches, written by the front end into
-  // page-locked mapped memory: the next batches' sort choice (BT_OPT_TOUCH_SORT 2)
-  ok = ok && cudaHostAlloc((void**)&h.touch_hint, sizeof(uint32_t), cudaHostAllocMapped) == cudaSuccess &&
+  // page-locked mapped memory: the next batches' sort choice (BT_OPT_TOUCH_SORT 2);
+  // behind it the host's copy of the small counts
+  ok = ok && cudaHostAlloc((void**)&h.touch_hint, 512, cudaHostAllocMapped) == cudaSuccess &&
        cudaHostGetDevicePointer((void**)&h.touch_hint_dev, h.touch_hint, 0) == cudaSuccess;
-  if (h.touch_hint) *h.touch_hint = UINT32_MAX;  // none seen yet
+  if (h.touch_hint) {
+    *h.touch_hint = UINT32_MAX;  // none seen yet
+    h.pin = h.touch_hint + 64;
+  }
   ok = ok && bt::tree_reset(&h, h.internal_stream) == cudaSuccess;
   ok = ok && cudaStreamSynchronize(h.internal_stream) == cudaSuccess;
   if (!ok) {
@@ -243,8 +249,6 @@ int bt_destroy(bt_handle* H) {
   cudaFree(h.enum_b);
   cudaFree(h.enum_cnt);
   cudaFree(h.enum_lb);
-  cudaFree(h.geo);
-  if (h.pin) cudaFreeHost(h.pin);
   if (h.build_pool) cudaMemPoolDestroy(h.build_pool);
   cudaFree(h.top);
   if (h.internal_stream) cudaStreamDestroy(h.internal_stream);

