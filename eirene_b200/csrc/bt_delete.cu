@@ -27,9 +27,10 @@ constexpr int kS = 32 / kG;
 
 // One 8-lane group per touched leaf (equal leaves are adjacent because the keys
 // ascend), as in the leaf merge: the slots to remove as bits, the kept slots to
-// their new places in shared memory, the row written back with 16-byte stores.
-// Bound by the rows' traffic and the chain entry -> leaf -> row: with a warp per
-// entry, one leaf at a time, 2^19 deletes on 2^24 keys took 131 us; this takes 113.
+// their new places in shared memory, the row written back with 32-byte stores.
+// Bound by the chain entry -> leaf -> row and by L1 (72 % of its rate with
+// 16-byte accesses and conflicting shared rows, row_at): with a warp per entry, one
+// leaf at a time, 2^19 deletes on 2^24 keys took 131 us; groups with such rows 106.
 __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_t* n_dev, const uint32_t* dleaf,
                                                         const uint32_t* dslot) {
   after_previous();
@@ -60,8 +61,8 @@ __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_
     if (!gone) continue;
     const size_t row = (size_t)leaf * 32 + g * kS;
     uint64_t k[kS], v[kS];
-    load_row16<kS>(t.keys + row, k);
-    load_row16<kS>(t.vals + row, v);
+    load_row(t.keys + row, k);
+    load_row(t.vals + row, v);
     const uint64_t h = __shfl_sync(gmask, k[kS - 1], kG - 1, kG);
     const uint32_t sz = hdr_size(h);
     const uint32_t keep = ((1u << sz) - 1u) & ~gone;  // sz <= 31
@@ -71,8 +72,8 @@ __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_
       const uint32_t s = g * kS + e;
       if ((keep >> s) & 1u) {
         const uint32_t pos = __popc(keep & ((1u << s) - 1u));
-        mk[grp][pos] = k[e];
-        mv[grp][pos] = v[e];
+        mk[grp][row_at(pos, grp)] = k[e];
+        mv[grp][row_at(pos, grp)] = v[e];
       }
     }
     __syncwarp(gmask);
@@ -80,16 +81,16 @@ __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_
 #pragma unroll
     for (int e = 0; e < kS; e++) {
       const uint32_t s = g * kS + e;
-      k[e] = s < nsz ? mk[grp][s] : kKeyMax;
-      v[e] = s < nsz ? mv[grp][s] : 0;
+      k[e] = s < nsz ? mk[grp][row_at(s, grp)] : kKeyMax;
+      v[e] = s < nsz ? mv[grp][row_at(s, grp)] : 0;
     }
     store_fp4(t, leaf, g, k, -1);
     if (g == kG - 1) {
       k[kS - 1] = make_hdr(nsz, 0, hdr_version(h) + 1, hdr_epoch(h));
       v[kS - 1] = fence;
     }
-    store_row16<kS>(t.keys + row, k);
-    store_row16<kS>(t.vals + row, v);
+    store_row(t.keys + row, k);
+    store_row(t.vals + row, v);
     __syncwarp(gmask);  // the shared rows are reused by the group's next leaf
     if (g == 0) removed += sz - nsz;
   }

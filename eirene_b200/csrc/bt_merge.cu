@@ -97,6 +97,17 @@ __device__ __forceinline__ uint32_t count_less(const uint64_t* a, uint32_t n, ui
   return lo;
 }
 
+// the same over the n keys of group grp's shared row (row_at)
+__device__ __forceinline__ uint32_t count_less_row(const uint64_t* row, uint32_t grp, uint32_t n, uint64_t key) {
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (row[row_at(mid, grp)] < key) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // ------------------------------------------------------------- root ----
 __global__ void merge_ensure_root_kernel(DevTree t) { ensure_root_leaf(t); }
 
@@ -356,7 +367,7 @@ __global__ void merge_fail_mark_kernel(const MergeCounts* mc, const uint32_t* nq
 // [st, st + kc); a group of G lanes builds it whole: every old key's merged
 // position by a binary search in the new keys, every new key of the range by
 // one in the old row, the row put together in shared memory and written with
-// 16-byte stores.  A piece needs nothing of its neighbours: its right fence is
+// 32-byte stores.  A piece needs nothing of its neighbours: its right fence is
 // the key at merged position st + kc.
 template <int N>  // groups of the block
 struct LeafSmem {
@@ -388,8 +399,8 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm
       const uint32_t pos = slot + count_less(nk, cnt, ok[i]);
       before += (pos < st ? 1u : 0u) + (pos < end ? 0x10000u : 0u);
       if (pos >= st && pos < end) {
-        mk[pos - st] = ok[i];
-        mv[pos - st] = ov[i];
+        mk[row_at(pos - st, grp)] = ok[i];
+        mv[row_at(pos - st, grp)] = ov[i];
       } else if (pos == end) {
         right = ok[i];
         right_old = true;
@@ -400,9 +411,9 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm
   const uint32_t j0 = st - (before & 0xffffu), j1 = end - (before >> 16);
   for (uint32_t j = j0 + g; j < j1; j += G) {
     const uint64_t key = nk[j];
-    const uint32_t pos = j + count_less(old, sz, key);
-    mk[pos - st] = key;
-    mv[pos - st] = nv[j];
+    const uint32_t pos = j + count_less_row(old, grp, sz, key);
+    mk[row_at(pos - st, grp)] = key;
+    mv[row_at(pos - st, grp)] = nv[j];
   }
   uint64_t rf = fence;
   if (c + 1 < p) {  // the next piece's first key: an old one, or the next new one
@@ -415,10 +426,10 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm
 #pragma unroll
   for (int i = 0; i < S; i++) {
     const uint32_t slot = g * S + i;
-    wk[i] = slot < kc ? mk[slot] : kKeyMax;
-    wv[i] = slot < kc ? mv[slot] : 0;
+    wk[i] = slot < kc ? mk[row_at(slot, grp)] : kKeyMax;
+    wv[i] = slot < kc ? mv[row_at(slot, grp)] : 0;
   }
-  const uint64_t first = mk[0];
+  const uint64_t first = mk[row_at(0, grp)];
   static_assert(G == 8, "four slots per lane");
   int splits = 0;
   if (c == 0 && g == G - 1) {
@@ -430,33 +441,33 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm
     wk[S - 1] = make_hdr(kc, 0, c == 0 ? hdr_version(hdr) + 1 : 0, hdr_epoch(hdr));
     wv[S - 1] = rf;
   }
-  store_row16<S>(t.keys + (size_t)nd * 32 + g * S, wk);
-  store_row16<S>(t.vals + (size_t)nd * 32 + g * S, wv);
+  store_row(t.keys + (size_t)nd * 32 + g * S, wk);
+  store_row(t.vals + (size_t)nd * 32 + g * S, wv);
   __syncwarp(gmask);  // the shared rows are reused by the group's next piece
   return first;
 }
 
-// a touched leaf's row in registers and its keys in shared memory; kNc: no
-// other group writes the row in this launch (read-only path)
-template <int G, bool kNc, int N>
-__device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<N>& sm, uint32_t grp, uint32_t g, uint32_t gmask,
-                                         uint32_t leaf, uint64_t (&ok)[32 / G], uint64_t (&ov)[32 / G], uint64_t& hdr,
+// a touched leaf's row in registers
+template <int G>
+__device__ __forceinline__ void leaf_row(const DevTree& t, uint32_t g, uint32_t gmask, uint32_t leaf,
+                                         uint64_t (&ok)[32 / G], uint64_t (&ov)[32 / G], uint64_t& hdr,
                                          uint64_t& fence) {
   constexpr int S = 32 / G;
-  if (kNc) {
-    load_slots<S>(t.keys + (size_t)leaf * 32 + g * S, ok);
-    load_slots<S>(t.vals + (size_t)leaf * 32 + g * S, ov);
-  } else {
-    load_row16<S>(t.keys + (size_t)leaf * 32 + g * S, ok);
-    load_row16<S>(t.vals + (size_t)leaf * 32 + g * S, ov);
-  }
+  load_row(t.keys + (size_t)leaf * 32 + g * S, ok);
+  load_row(t.vals + (size_t)leaf * 32 + g * S, ov);
   hdr = __shfl_sync(gmask, ok[S - 1], G - 1, G);
   fence = __shfl_sync(gmask, ov[S - 1], G - 1, G);
-  const uint32_t sz = hdr_size(hdr);
+}
+
+// its keys in shared memory, for searches
+template <int G, int N>
+__device__ __forceinline__ void leaf_keys(LeafSmem<N>& sm, uint32_t grp, uint32_t g, uint32_t gmask, uint32_t sz,
+                                          const uint64_t (&ok)[32 / G]) {
+  constexpr int S = 32 / G;
 #pragma unroll
   for (int i = 0; i < S; i++) {
     const uint32_t slot = g * S + i;
-    sm.old[grp][slot] = slot < sz ? ok[i] : kKeyMax;
+    sm.old[grp][row_at(slot, grp)] = slot < sz ? ok[i] : kKeyMax;
   }
   __syncwarp(gmask);
 }
@@ -465,7 +476,12 @@ __device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<N>& sm, uint
 //   segments  a touched leaf whose merged row fits: rewritten in place by its
 //             group.  Several leaves per warp keep more row loads in flight
 //             than a warp per leaf (the kernel is bound by the dependent chain
-//             segment bounds -> leaf id -> row).
+//             segment bounds -> leaf id -> row, and by L1: 63 % of its rate with
+//             16-byte accesses, conflicting shared rows and a binary search per
+//             key).  Most leaves get one to three keys: these are ranked in
+//             registers.  With del_apply_kernel's rows the same way, two batches
+//             of 2^20 at 50 % writes 863 -> 836 us, four of 2^22 at 5 % 2084 ->
+//             2014.
 //   entries   one new piece (1 .. p - 1) of a leaf that splits; its segment by a
 //             binary search in the entry offsets.  All pieces read the old row,
 //             and the group that finishes the leaf's last one (a count down of
@@ -475,7 +491,7 @@ __device__ __forceinline__ void leaf_row(const DevTree& t, LeafSmem<N>& sm, uint
 // the chip, a tree of 2^23 keys grown by seven such batches takes 6.5 ms, from
 // 81.2.  A launch of its own for the pieces cost batches that split nothing 4 %
 // (a 50/50 batch of 2^20), and so did 74 registers (three blocks an SM).
-template <int G, int N, bool kNc>
+template <int G, int N>
 __device__ __forceinline__ void leaf_merge(const DevTree& t, uint32_t leaf_fill, const MergeCounts* mc,
                                            const uint32_t* seg_start, const uint32_t* eoff, uint32_t* extra,
                                            const uint64_t* newk, const uint64_t* newv, const uint32_t* nq,
@@ -498,38 +514,61 @@ __device__ __forceinline__ void leaf_merge(const DevTree& t, uint32_t leaf_fill,
     // a leaf that splits (it has entries) is written by their groups
     if (eoff[s] != (s + 1 < n_segs ? eoff[s + 1] : n_ent)) continue;
     uint64_t ok[S], ov[S], hdr, fence;
-    leaf_row<G, kNc, N>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
+    leaf_row<G>(t, g, gmask, leaf, ok, ov, hdr, fence);
     const uint32_t sz = hdr_size(hdr), m = sz + cnt;
+    if (cnt <= 3) {  // every old key against every new one in registers, the new ones' ranks by one sum
+      const uint64_t n0 = newk[a], n1 = cnt > 1 ? newk[a + 1] : kKeyMax, n2 = cnt > 2 ? newk[a + 2] : kKeyMax;
+      uint32_t less = 0;  // old keys below n0, n1, n2: a byte each
 #pragma unroll
-    for (int i = 0; i < S; i++) {
-      const uint32_t slot = g * S + i;
-      if (slot < sz) {
-        const uint32_t pos = slot + count_less(newk + a, cnt, ok[i]);
-        sm.mk[grp][pos] = ok[i];
-        sm.mv[grp][pos] = ov[i];
+      for (int i = 0; i < S; i++) {
+        const uint32_t slot = g * S + i;
+        if (slot < sz) {
+          const uint32_t b = (n0 < ok[i] ? 1u : 0u) + (n1 < ok[i] ? 0x100u : 0u) + (n2 < ok[i] ? 0x10000u : 0u);
+          less += 0x10101u - b;
+          const uint32_t at = row_at(slot + (b & 1u) + (b >> 8 & 1u) + (b >> 16), grp);
+          sm.mk[grp][at] = ok[i];
+          sm.mv[grp][at] = ov[i];
+        }
       }
-    }
-    for (uint32_t j = g; j < cnt; j += G) {
-      const uint64_t key = newk[a + j];
-      const uint32_t pos = j + count_less(sm.old[grp], sz, key);
-      sm.mk[grp][pos] = key;
-      sm.mv[grp][pos] = newv[a + j];
+      less = group_sum<G>(less, gmask);
+      if (g < cnt) {
+        const uint32_t at = row_at(g + (less >> (8 * g) & 0xffu), grp);
+        sm.mk[grp][at] = g == 0 ? n0 : g == 1 ? n1 : n2;
+        sm.mv[grp][at] = newv[a + g];
+      }
+    } else {
+      leaf_keys<G, N>(sm, grp, g, gmask, sz, ok);
+#pragma unroll
+      for (int i = 0; i < S; i++) {
+        const uint32_t slot = g * S + i;
+        if (slot < sz) {
+          const uint32_t at = row_at(slot + count_less(newk + a, cnt, ok[i]), grp);
+          sm.mk[grp][at] = ok[i];
+          sm.mv[grp][at] = ov[i];
+        }
+      }
+      for (uint32_t j = g; j < cnt; j += G) {
+        const uint64_t key = newk[a + j];
+        const uint32_t at = row_at(j + count_less_row(sm.old[grp], grp, sz, key), grp);
+        sm.mk[grp][at] = key;
+        sm.mv[grp][at] = newv[a + j];
+      }
     }
     __syncwarp(gmask);
     uint64_t wk[S], wv[S];
 #pragma unroll
     for (int i = 0; i < S; i++) {
       const uint32_t slot = g * S + i;
-      wk[i] = slot < m ? sm.mk[grp][slot] : kKeyMax;
-      wv[i] = slot < m ? sm.mv[grp][slot] : 0;
+      wk[i] = slot < m ? sm.mk[grp][row_at(slot, grp)] : kKeyMax;
+      wv[i] = slot < m ? sm.mv[grp][row_at(slot, grp)] : 0;
     }
     store_fp4(t, leaf, g, wk, -1);
     if (g == G - 1) {
       wk[S - 1] = make_hdr(m, 0, hdr_version(hdr) + 1, hdr_epoch(hdr));
       wv[S - 1] = fence;
     }
-    store_row16<S>(t.keys + (size_t)leaf * 32 + g * S, wk);
-    store_row16<S>(t.vals + (size_t)leaf * 32 + g * S, wv);
+    store_row(t.keys + (size_t)leaf * 32 + g * S, wk);
+    store_row(t.vals + (size_t)leaf * 32 + g * S, wv);
     __syncwarp(gmask);  // the shared rows are reused by the next segment
   }
   for (uint32_t e = gid; e < n_ent; e += n_groups) {
@@ -544,8 +583,9 @@ __device__ __forceinline__ void leaf_merge(const DevTree& t, uint32_t leaf_fill,
     seg_bounds(mc, seg_start, lo, a, b);
     const uint32_t cnt = b - a, leaf = seg_leaf[lo];
     uint64_t ok[S], ov[S], hdr, fence;
-    leaf_row<G, false, N>(t, sm, grp, g, gmask, leaf, ok, ov, hdr, fence);
+    leaf_row<G>(t, g, gmask, leaf, ok, ov, hdr, fence);
     const uint32_t sz = hdr_size(hdr), m = sz + cnt, p = ceil_div(m, leaf_fill);
+    leaf_keys<G, N>(sm, grp, g, gmask, sz, ok);
     uint32_t c = e - eoff[lo] + 1, nd = base + e;
     for (;;) {
       const uint64_t first = leaf_piece<G, N>(t, sm, grp, g, gmask, nd, c, p, m, sz, hdr, fence, ok, ov, newk + a,
@@ -586,7 +626,7 @@ __global__ void __launch_bounds__(256, 4) merge_leaf_kernel(DevTree t, uint32_t 
                                                             MergeEntry* __restrict__ ent) {
   __shared__ LeafSmem<256 / G> sm;
   if (mc->cap_fail) return;  // merge_fail_mark_kernel answered the new keys
-  leaf_merge<G, 256 / G, true>(t, leaf_fill, mc, seg_start, eoff, extra, newk, newv, nq, seg_leaf, ent, sm,
+  leaf_merge<G, 256 / G>(t, leaf_fill, mc, seg_start, eoff, extra, newk, newv, nq, seg_leaf, ent, sm,
                                (blockIdx.x * blockDim.x + threadIdx.x) / G, (gridDim.x * blockDim.x) / G);
 }
 
@@ -1058,7 +1098,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
     out_st[r] = __ldcg(a.uans_st + u);
   }
   if (fail) return;
-  leaf_merge<8, kSmallThreads / 8, false>(t, a.leaf_fill, mc, a.seg, a.pos, a.isnew, a.newk, a.newv, a.nq, a.leaf,
+  leaf_merge<8, kSmallThreads / 8>(t, a.leaf_fill, mc, a.seg, a.pos, a.isnew, a.newk, a.newv, a.nq, a.leaf,
                                           a.ea, S.leaf, gt / 8, nt / 8);
   if (n_ent == 0) return;
   cluster_sync();

@@ -4,16 +4,26 @@
 
 namespace bt {
 
-// S slots of a row that this kernel also writes (plain loads: the read-only
-// path must not be used for it)
-template <int S>
-__device__ __forceinline__ void load_row16(const uint64_t* p, uint64_t (&x)[S]) {
-#pragma unroll
-  for (int i = 0; i < S; i += 2) {
-    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(p + i);
-    x[i] = w.x;
-    x[i + 1] = w.y;
-  }
+// A lane's four slots of a row in one 32-byte access: two of 16 bytes at a stride
+// of 32 each touch half of every sector, twice the wavefronts.  Plain accesses,
+// in order with the kernel's others: it also writes the rows.
+__device__ __forceinline__ void load_row(const uint64_t* p, uint64_t (&x)[4]) {
+  asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void store_row(uint64_t* p, const uint64_t (&x)[4]) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(x[0]), "l"(x[1]), "l"(x[2]), "l"(x[3])
+               : "memory");
+}
+
+// Place of slot s in the shared row of the block's 8-lane group grp, a row
+// being 256 bytes.  Lane g holds slots 4g .. 4g + 3; in slot order the lanes'
+// e-th slots share four of the sixteen bank pairs and the two groups of a half
+// warp the same ones (8 wavefronts an access), here they take all sixteen (2).
+__device__ __forceinline__ uint32_t row_at(uint32_t s, uint32_t grp) {
+  return ((s & 3u) << 3 | s >> 2) ^ (grp & 1u) << 3;
 }
 
 // the fingerprints of a lane's four slots of leaf nd (G = 8); slot 31's byte,
@@ -32,12 +42,6 @@ __device__ __forceinline__ void store_fp4(const DevTree& t, uint32_t nd, uint32_
     *reinterpret_cast<uint16_t*>(p) = (uint16_t)w;
     p[2] = (uint8_t)(w >> 16);
   }
-}
-
-template <int S>
-__device__ __forceinline__ void store_row16(uint64_t* p, const uint64_t (&x)[S]) {
-#pragma unroll
-  for (int i = 0; i < S; i += 2) *reinterpret_cast<ulonglong2*>(p + i) = make_ulonglong2(x[i], x[i + 1]);
 }
 
 }  // namespace bt
