@@ -117,6 +117,7 @@ struct SortSmem {
   uint32_t ws[32];
   uint32_t split[2];
   uint32_t pre, pre_any;
+  uint32_t sum[3];  // heads, ins, del of the bucket
 };
 
 __global__ void __launch_bounds__(1024, 1) ss_splitters_kernel(const uint64_t* tk, const uint32_t* tv,
@@ -356,6 +357,7 @@ __global__ void __launch_bounds__(1024, 1) ss_sort_kernel(uint32_t n_upper, cons
     if (threadIdx.x == 0) {
       S.pre = kNoWrite;
       S.pre_any = 0;
+      S.sum[0] = S.sum[1] = S.sum[2] = 0;
     }
     for (uint32_t c0 = 0; c0 < s; c0 += kCap) {
       const int cnt = (int)min((uint32_t)kCap, s - c0);
@@ -400,17 +402,23 @@ __global__ void __launch_bounds__(1024, 1) ss_sort_kernel(uint32_t n_upper, cons
       }
       run = st_combine(run, all);
     }
-    uint32_t th, ti, td;
-    blk_exclusive_sum(heads, S.ws, &th);
-    blk_exclusive_sum(ins, S.ws, &ti);
-    blk_exclusive_sum(del, S.ws, &td);
+    // (nothing to add where the loop did not run, so the zeroes above are seen)
+    heads = __reduce_add_sync(0xffffffffu, heads);
+    ins = __reduce_add_sync(0xffffffffu, ins);
+    del = __reduce_add_sync(0xffffffffu, del);
+    if ((threadIdx.x & 31) == 0) {
+      if (heads) atomicAdd(&S.sum[0], heads);
+      if (ins) atomicAdd(&S.sum[1], ins);
+      if (del) atomicAdd(&S.sum[2], del);
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
       BucketSum& o = sums[b];
       o.agg = run;
       o.pre = S.pre;
-      o.heads = th;
-      o.ins = ti;
-      o.del = td;
+      o.heads = S.sum[0];
+      o.ins = S.sum[1];
+      o.del = S.sum[2];
       o.multi = S.pre_any;
     }
     __syncthreads();

@@ -79,39 +79,75 @@ __device__ __forceinline__ void merge4(const uint64_t* ka, const uint32_t* va, i
     if (pair_less(ka[mid], va[mid], kb[d - 1 - mid], vb[d - 1 - mid])) lo = mid + 1;
     else hi = mid;
   }
+  // the runs' next pairs in registers: one pair read per output, no branches (the
+  // rounds wait on these loads; with the 16-byte accesses below, two batches of 2^20
+  // at 50 % writes 836 -> 812 us, two Zipf batches of 2^18 336 -> 329)
   int ia = lo, ib = d - lo;
+  uint64_t a = ia < la ? ka[ia] : 0, b = ib < lb ? kb[ib] : 0;
+  uint32_t x = ia < la ? va[ia] : 0, y = ib < lb ? vb[ib] : 0;
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    if (ia + ib >= la + lb) break;
-    const bool take_a = ib >= lb || (ia < la && pair_less(ka[ia], va[ia], kb[ib], vb[ib]));
-    ok[j] = take_a ? ka[ia] : kb[ib];
-    ov[j] = take_a ? va[ia] : vb[ib];
+  for (int j = 0; j < 4; j++) {  // (past the runs' end: pairs nobody uses)
+    const bool take_a = (ib >= lb) | ((ia < la) & pair_less(a, x, b, y));
+    ok[j] = take_a ? a : b;
+    ov[j] = take_a ? x : y;
     ia += take_a ? 1 : 0;
     ib += take_a ? 0 : 1;
+    if (j == 3) break;
+    const bool any = take_a ? ia < la : ib < lb;
+    const uint64_t* pk = take_a ? ka + ia : kb + ib;
+    const uint32_t* pv = take_a ? va + ia : vb + ib;
+    const uint64_t nk = any ? *pk : 0;
+    const uint32_t nv = any ? *pv : 0;
+    a = take_a ? nk : a;
+    x = take_a ? nv : x;
+    b = take_a ? b : nk;
+    y = take_a ? y : nv;
   }
 }
 
-// The first cnt of a block's pairs in shared memory, sorted: 128-pair runs by
-// warp (registers and shuffles), then merged pairwise; the threads past the
-// count's last run idle.  The bitonic network over a whole tile of 2048 pairs
-// took 26 us, whatever their count.
+// a thread's four pairs [d, d + 4) of a block's arrays (16-byte aligned): 16 bytes
+// an access, where four of 8 at a stride of 32 met in four of the sixteen bank pairs
+__device__ __forceinline__ void load_pairs(const uint64_t* sk, const uint32_t* sv, int d, uint64_t (&K)[4],
+                                           uint32_t (&V)[4]) {
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(sk + d), b = *reinterpret_cast<const ulonglong2*>(sk + d + 2);
+  const uint4 v = *reinterpret_cast<const uint4*>(sv + d);
+  K[0] = a.x;
+  K[1] = a.y;
+  K[2] = b.x;
+  K[3] = b.y;
+  V[0] = v.x;
+  V[1] = v.y;
+  V[2] = v.z;
+  V[3] = v.w;
+}
+__device__ __forceinline__ void store_pairs(uint64_t* sk, uint32_t* sv, int d, const uint64_t (&K)[4],
+                                            const uint32_t (&V)[4]) {
+  *reinterpret_cast<ulonglong2*>(sk + d) = make_ulonglong2(K[0], K[1]);
+  *reinterpret_cast<ulonglong2*>(sk + d + 2) = make_ulonglong2(K[2], K[3]);
+  *reinterpret_cast<uint4*>(sv + d) = make_uint4(V[0], V[1], V[2], V[3]);
+}
+
+// The first cnt of a block's pairs in shared memory, sorted; the arrays hold cnt
+// rounded up to 128, the threads past the count's last run idle.  128-pair runs
+// by warp (registers and shuffles), then merged pairwise.  The bitonic network
+// over a whole tile of 2048 pairs took 26 us, whatever their count; a search of
+// every pair's rank in the other run instead of merge4 made two batches of 2^20
+// at 50 % writes 30 us slower.
 __device__ __forceinline__ void block_sort(uint64_t* sk, uint32_t* sv, int cnt) {
   const int P = (cnt + 127) & ~127;
   const int d = threadIdx.x * 4;
   uint64_t K[4];
   uint32_t V[4];
   if (d < P) {
+    load_pairs(sk, sv, d, K, V);
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-      K[e] = d + e < cnt ? sk[d + e] : ~0ull;
-      V[e] = d + e < cnt ? sv[d + e] : 0xFFFFFFFFu;  // behind every request
+      if (d + e < cnt) continue;
+      K[e] = ~0ull;
+      V[e] = 0xFFFFFFFFu;  // behind every request
     }
     warp_sort(K, V);
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      sk[d + e] = K[e];
-      sv[d + e] = V[e];
-    }
+    store_pairs(sk, sv, d, K, V);
   }
   __syncthreads();
   for (int L = 128; L < P; L <<= 1) {
@@ -120,13 +156,7 @@ __device__ __forceinline__ void block_sort(uint64_t* sk, uint32_t* sv, int cnt) 
     const bool pair = d < P && lb > 0;  // a last run without a partner stays
     if (pair) merge4(sk + ps, sv + ps, L, sk + ps + L, sv + ps + L, lb, d - ps, K, V);
     __syncthreads();
-    if (pair) {
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        sk[d + e] = K[e];
-        sv[d + e] = V[e];
-      }
-    }
+    if (pair) store_pairs(sk, sv, d, K, V);
     __syncthreads();
   }
 }
