@@ -31,7 +31,7 @@ constexpr int kS = 32 / kG;
 // Bound by the chain entry -> leaf -> row and by L1 (72 % of its rate with
 // 16-byte accesses and conflicting shared rows, row_at): with a warp per entry, one
 // leaf at a time, 2^19 deletes on 2^24 keys took 131 us; groups with such rows 106.
-__global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_t* n_dev, const uint32_t* dleaf,
+__global__ void __launch_bounds__(256, 5) del_apply_kernel(DevTree t, const uint32_t* n_dev, const uint32_t* dleaf,
                                                         const uint32_t* dslot) {
   after_previous();
   __shared__ __align__(16) uint64_t mk[256 / kG][32];
@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(256) del_apply_kernel(DevTree t, const uint32_
   const uint32_t groups = (gridDim.x * blockDim.x) / kG;
   unsigned long long removed = 0;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kG; i < n; i += groups) {
-    const uint32_t leaf = dleaf[i];
+    const uint32_t leaf = dleaf[i], ahead = i + groups < n ? dleaf[i + groups] : kNil;
+    if (ahead != kNil) prefetch_row(t, ahead, g);
     if (leaf == kNil || (i > 0 && dleaf[i - 1] == leaf)) continue;  // not the first entry of its leaf
     uint32_t gone = 0;
     for (uint32_t j = i;; j += kG) {

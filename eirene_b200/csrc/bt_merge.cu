@@ -510,6 +510,7 @@ __device__ __forceinline__ void leaf_merge(const DevTree& t, uint32_t leaf_fill,
     seg_bounds(mc, seg_start, s, a, b);
     const uint32_t leaf = seg_leaf[s];
     const uint32_t cnt = b - a;
+    if (s + n_groups < n_segs) prefetch_row(t, seg_leaf[s + n_groups], g);
     if (g == 0) added += cnt;
     // a leaf that splits (it has entries) is written by their groups
     if (eoff[s] != (s + 1 < n_segs ? eoff[s + 1] : n_ent)) continue;
