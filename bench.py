@@ -1095,10 +1095,12 @@ def main():
             tune = R.get("tune") or {}
             if head == "learned":
                 m, g = tune.get("learned_mode", 3), tune.get("learned_lanes", 4)
-                kname = (f"search phase: learned_pipe_kernel<{g}> + search2_kernel over its misses" if m == 3 else
+                kname = ("search phase: learned_thread_kernel + search_warp_kernel over its misses" if m == 3 and g == 4 else
+                         f"search phase: learned_pipe_kernel<{g}> + search2_kernel over its misses" if m == 3 else
                          f"search phase: learned_lookup_kernel<{g},{m}> + search2_kernel over its misses")
             else:
-                kname = f"search phase: search2_kernel<{tune.get('plain_lanes', 4)},0,1>"
+                kname = ("search phase: search_warp_kernel" if tune.get('plain_lanes', 4) == 4 else
+                         f"search phase: search2_kernel<{tune.get('plain_lanes', 4)},0,1>")
         roof = {"kernel": kname, "bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                 "peak_source": peak_kind, "traffic": traffic, "alg_bytes_per_launch": dom_bytes,
                 "launch_ms": dom_ms}
