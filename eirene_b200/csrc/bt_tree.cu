@@ -849,7 +849,12 @@ int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* val
 // of 2^20 keys spent outside its kernels) and all of it until bt_destroy.
 constexpr uint64_t kBuildKeep = 1ull << 30;
 int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s) {
-  if (n == 0 || n > 0xFFFFFFFFull / 2) return tree_reset(h, s) != cudaSuccess ? -2 : n ? -1 : 0;
+  // the contents are gone in these cases too: a call on another stream may
+  // follow at once and has to meet the new tree, not the old one
+  auto emptied = [&](int rc) {
+    return tree_reset(h, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess ? rc : -2;
+  };
+  if (n == 0 || n > 0xFFFFFFFFull / 2) return emptied(n ? -1 : 0);
   Work& w = h->w;
   BuildScratch sc;
   sc.tot = h->geo;
@@ -883,7 +888,7 @@ int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_
   if (cudaMallocFromPoolAsync((void**)&slab, 3 * kb + 2 * vb + pb + up(sort_scratch_words(n) * 4), h->build_pool, s) !=
       cudaSuccess) {
     cudaGetLastError();
-    return tree_reset(h, s) == cudaSuccess ? -3 : -2;
+    return emptied(-3);
   }
   char* at = slab;
   auto take = [&](size_t b) {
