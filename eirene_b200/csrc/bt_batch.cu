@@ -597,9 +597,6 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   // lookups do not need them
   cudaStream_t s2 = ov ? h->hi_stream : s;
   auto fork = [&]() {
-    // a stale prefix table is rebuilt before the fork, so that the locates
-    // (side stream) and the lookups (`s`) both come after the rebuild
-    if (early && h->use_pfx && (tree_join(h, s) != cudaSuccess || ensure_pfx(h, s) != cudaSuccess)) return false;
     return cudaEventRecord(h->fork_ev, s) == cudaSuccess && cudaStreamWaitEvent(s2, h->fork_ev, 0) == cudaSuccess;
   };
   if (!fp.passes_done) {

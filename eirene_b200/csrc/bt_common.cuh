@@ -95,8 +95,10 @@ struct DevTree {
   // in byte 31 how often the leaf has split (kSplitMany: that often or more).
   // A lookup reads this one 32-byte sector instead of the 256-byte key row,
   // then only the key and the value of the slots whose byte matches.
-  // Every writer keeps both tables (a loaded pool image has them rebuilt,
-  // Handle::pfx_valid); only kernels that run without a writer read them.
+  // Every writer keeps both tables, and loading a pool image rebuilds them
+  // (rebuild_tables) before it returns: left to the first lookup, the rebuild was
+  // ordered before that one's stream only, and a call on another stream read
+  // empty tables.  Only kernels that run without a writer read them.
   uint8_t* fp;
 };
 

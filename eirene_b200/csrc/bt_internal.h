@@ -283,7 +283,6 @@ struct Handle {
   int top_cache = 1;         // unsorted searches descend the upper levels from shared memory
   int search_pairs = 2;      // unsorted searches: 2 pairs of requests per lane group, child ids only; 1 pairs; 0 single
   bool has_root = false;     // the tree surely has a root (false: it may have)
-  bool pfx_valid = false;    // tree.pfx and tree.fp match the rows (false after a loaded pool image)
   int use_pfx = 1;           // paired searches compare the separators' 32-bit prefixes first
   void* top = nullptr;       // top cache (kTopNodes nodes) + TopInfo
   TopInfo* top_info = nullptr;
@@ -372,8 +371,8 @@ void prof_mark(Handle* h, int which, cudaStream_t s);
 void prof_set_layout(Handle* h, int layout);
 
 // ---- tree kernels (bt_tree.cu) ----
-// make tree.pfx and tree.fp match the rows (a rebuild when stale), stream ordered
-cudaError_t ensure_pfx(Handle* h, cudaStream_t s);
+// tree.pfx and tree.fp from the rows, stream ordered (a loaded pool image holds neither)
+cudaError_t rebuild_tables(Handle* h, cudaStream_t s);
 cudaError_t tree_reset(Handle* h, cudaStream_t s);
 // header word of node rows [first, last) set to 0 (epoch 0: never written)
 cudaError_t clear_headers(Handle* h, uint32_t first, uint32_t last, cudaStream_t s);

@@ -1104,8 +1104,6 @@ int learned_retrain(Handle* h, cudaStream_t s, bool refit) {
   Learned& L = h->L;
   refit = refit && L.trained;
   L.valid = false;
-  // the leaf table takes the leaves' split counts: none may be rebuilt later
-  if (ensure_pfx(h, s) != cudaSuccess) return -2;
   uint32_t* ids = nullptr;
   size_t nl = 0;
   int rc = enumerate_leaves(h, s, &ids, &nl);

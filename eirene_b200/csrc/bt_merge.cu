@@ -1154,7 +1154,6 @@ int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s) {
     count_launch();
     h->has_root = true;
   }
-  if (ensure_pfx(h, s) != cudaSuccess) return -2;
   LocateArgs a;
   a.counts = w.counts;
   a.ukeys = w.ukeys;

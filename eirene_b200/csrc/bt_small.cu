@@ -597,7 +597,6 @@ int small_read(Handle* h, bool gets, bool locate_ins, uint64_t* out_vals, uint8_
   a.uans_st = w.uans_st;
   a.locate_ins = locate_ins ? 1 : 0;
   const int use_pfx = h->use_pfx ? 1 : 0;
-  if (use_pfx && ensure_pfx(h, s) != cudaSuccess) return -2;
   const size_t turns = (n + kLocPer - 1) / kLocPer + 2;
   const unsigned grid = (unsigned)min(turns, (size_t)h->sm_count * 8);
   cudaLaunchConfig_t cfg{};

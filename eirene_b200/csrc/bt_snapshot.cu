@@ -139,7 +139,7 @@ int bt_load(bt_handle* h, const char* path) {
 // layout and goes on exactly as the saved one would (the merge engine is
 // deterministic).  The loading handle needs a pool of at least n_nodes
 // nodes and the saving handle's leaf and inner fills (later splits follow
-// them); its learned model and separator prefixes are rebuilt on demand.
+// them); its learned model is rebuilt on demand.
 //
 // File layout (little endian):
 //   0   8 B  magic "EIRB2IMG"
@@ -254,13 +254,14 @@ int bt_load_image(bt_handle* h, const char* path) {
     rc = BT_ERR_CUDA;
   // rows past the loaded ones may hold an earlier tree's nodes; clear their
   // headers (epoch 0, never used) so that none can pass for a row of this tree
+  // (the separators' prefixes and the leaves' fingerprints are not in the file)
   if (rc == BT_OK && (bt::clear_headers(&H, (uint32_t)nn, H.tree.cap, H.internal_stream) != cudaSuccess ||
+                      bt::rebuild_tables(&H, H.internal_stream) != cudaSuccess ||
                       cudaStreamSynchronize(H.internal_stream) != cudaSuccess))
     rc = BT_ERR_CUDA;
   if (rc == BT_OK) {
     H.epoch = c.epoch;  // the rows carry the saved tree's epoch
     H.L.valid = false;
-    H.pfx_valid = false;
     H.has_root = false;
   }
   if (prev >= 0) cudaSetDevice(prev);

@@ -781,7 +781,6 @@ cudaError_t clear_headers(Handle* h, uint32_t first, uint32_t last, cudaStream_t
 
 cudaError_t tree_reset(Handle* h, cudaStream_t s) {
   h->has_root = false;
-  h->pfx_valid = true;  // no nodes: every writer from here on keeps the two tables
   // The epoch has 15 bits (1 .. 0x7fff; 0 marks never-written rows).  When
   // it comes round to 1 again, rows written by the trees of the last cycle
   // may still carry that number: clear every row's header first, so that a
@@ -951,11 +950,9 @@ __global__ void __launch_bounds__(256) pfx_rebuild_kernel(DevTree t) {
   }
 }
 
-cudaError_t ensure_pfx(Handle* h, cudaStream_t s) {
-  if (h->pfx_valid) return cudaSuccess;
+cudaError_t rebuild_tables(Handle* h, cudaStream_t s) {
   pfx_rebuild_kernel<<<(unsigned)h->sm_count * 8, 256, 0, s>>>(h->tree);
   count_launch();
-  h->pfx_valid = true;
   return cudaGetLastError();
 }
 
@@ -968,10 +965,6 @@ cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list
     const bool child = h->search_pairs == 2;
     // the separators' prefixes and the leaves' fingerprints (child-id form only)
     const int use_pfx = child && h->use_pfx ? 1 : 0;
-    if (use_pfx) {
-      const cudaError_t pe = ensure_pfx(h, s);
-      if (pe != cudaSuccess) return pe;
-    }
     const bool warp = use_pfx && G == 4 && n >= kWarpLookupMin;
     const size_t per_block = warp ? threads : 2 * threads / G;
     size_t blocks = (n + per_block - 1) / per_block;
@@ -1033,8 +1026,6 @@ cudaError_t launch_search(Handle* h, const uint64_t* qkeys, const uint32_t* list
 cudaError_t launch_range(Handle* h, const uint64_t* lo, const uint64_t* hi, size_t n, uint32_t max_per,
                          uint64_t* out_keys, uint64_t* out_vals, uint32_t* out_counts, bool fill, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  const cudaError_t pe = ensure_pfx(h, s);
-  if (pe != cudaSuccess) return pe;
   size_t blocks = (n * 32 + 255) / 256;
   const size_t cap = (size_t)h->sm_count * 16;
   if (blocks > cap) blocks = cap;
