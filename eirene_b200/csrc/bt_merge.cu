@@ -1148,11 +1148,16 @@ static cudaError_t launch_inner(Handle* h, uint32_t entry_cap, MergeCounts* mc, 
 
 int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
-  // the INSERT keys need a root; once there is one only a new tree takes it away
-  if ((what & kLocateIns) && !h->has_root) {
+  // the INSERT keys need a root; once there is one only a new tree takes it away.
+  // A launch that is captured has not run, and its graph may run on a later tree
+  // without a root: there it is always part of the batch and says nothing
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) return -2;
+  const bool captured = cap != cudaStreamCaptureStatusNone;
+  if ((what & kLocateIns) && (captured || !h->has_root)) {
     merge_ensure_root_kernel<<<1, 1, 0, s>>>(h->tree);
     count_launch();
-    h->has_root = true;
+    h->has_root = h->has_root || !captured;
   }
   LocateArgs a;
   a.counts = w.counts;
