@@ -26,6 +26,7 @@
 #include "bt_common.cuh"
 #include "bt_internal.h"
 #include "bt_launch.cuh"
+#include "bt_lookback.cuh"
 #include "bt_sort.cuh"
 
 namespace bt {
@@ -398,7 +399,7 @@ static size_t carve_work(Work* w, size_t cap, char* base) {
   A(w->f_tk, cap * 8);
   A(w->f_tv, cap * 4);
   A(w->lb_status, merge_lb_words(cap) * 8);
-  A(w->lb_ctr, 8);
+  A(w->lb_ctr, kLbCtrWords * 4);
   A(w->s_write, 3 * 16 * 4);
   A(w->s_split, kSsBuckets * 16);
   A(w->s_sum, sample_sum_bytes());
@@ -418,7 +419,7 @@ int work_alloc(Work* w, size_t cap) {
   carve_work(w, cap, static_cast<char*>(w->arena));
   // look-back words of no epoch, and a clean table (every slot empty between batches)
   if (cudaMemset(w->lb_status, 0, merge_lb_words(cap) * 8) != cudaSuccess ||
-      cudaMemset(w->lb_ctr, 0, 8) != cudaSuccess ||
+      cudaMemset(w->lb_ctr, 0, kLbCtrWords * 4) != cudaSuccess ||
       cudaMemset(w->s_tab, 0xff, small_tab_bytes(cap)) != cudaSuccess) {
     work_free(w);
     return -3;

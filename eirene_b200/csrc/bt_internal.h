@@ -43,12 +43,11 @@ cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, uint
                                cudaStream_t s,
                                const uint32_t* n_dev = nullptr);
 // one-launch scan with decoupled look-back (status: scan_lb_words(n_upper)
-// words; ctr: two words, zero before the first call; *epoch: the caller's
-// call counter)
+// words and ctr: kLbCtrWords, both zero before the first call)
 size_t scan_lb_words(size_t n_upper);
 cudaError_t scan_exclusive_u32_lb(const uint32_t* in, uint32_t* out, size_t n_upper, const uint32_t* n_dev,
-                                  uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* epoch,
-                                  uint32_t* err, cudaStream_t s);
+                                  uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* err,
+                                  cudaStream_t s);
 cudaError_t sort_prepare();
 size_t sort_scratch_words(size_t n);
 // tile_threads: 256, 512 or 1024 threads per onesweep tile of 8 items each
@@ -170,7 +169,6 @@ struct Work {
   // look-back words of the merge engine (bt_lookback.cuh)
   uint64_t* lb_status = nullptr;
   uint32_t* lb_ctr = nullptr;
-  uint32_t lb_epoch = 0;
   // sample sort of the touched requests (bt_sample.cu)
   uint64_t* s_split = nullptr;    // splitters, bucket totals
   void* s_sum = nullptr;          // per bucket: its part of the segmented scan, its start
@@ -294,7 +292,6 @@ struct Handle {
   uint32_t* enum_cnt = nullptr;
   uint64_t* enum_lb = nullptr;  // look-back scan of the enumeration
   size_t enum_lb_words = 0;
-  uint32_t enum_epoch = 0;
   size_t enum_cap = 0;
   uint32_t* geo = nullptr;      // 256 bytes: the bulk build's geometry, the enumeration's counts
   uint32_t* pin = nullptr;      // 256 bytes of page-locked memory: what the host reads back

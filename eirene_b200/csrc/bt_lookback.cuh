@@ -2,11 +2,13 @@
 // of bt_sort.cu and bt_merge.cu).
 //
 // status[t] = epoch << 34 | state << 32 | value, state 1 the tile's own sum, 2
-// its inclusive prefix; each call's epoch makes the words of earlier calls read
-// as not ready, so the array is never cleared.  ctr[0] hands tile ids out in
-// the order blocks take them (a tile waits only on tiles taken before it); the
-// last block to finish resets ctr.  The wait is bounded: past kLbSpinLimit it
-// sets kErrSpin in *err and goes on.
+// its inclusive prefix; each run's epoch makes the words of earlier runs read
+// as not ready, so the array is never cleared.  The epoch is counted on the
+// device (ctr[2]): as a launch argument it was fixed in a captured launch, and a
+// second replay took the first one's words for its own.  ctr[0] hands tile ids
+// out in the order blocks take them (a tile waits only on tiles taken before
+// it); the last block to finish resets both and counts the run.  The wait is
+// bounded: past kLbSpinLimit it sets kErrSpin in *err and goes on.
 #pragma once
 #include <cstdint>
 
@@ -16,6 +18,11 @@ namespace bt {
 
 constexpr uint64_t kLbAgg = 1ull << 32, kLbInc = 2ull << 32;
 constexpr uint32_t kLbSpinLimit = 1u << 22;
+constexpr uint32_t kLbEpochs = (1u << 30) - 1;  // epochs 1 .. kLbEpochs; zeroed words carry epoch 0
+constexpr int kLbCtrWords = 3;                  // words of ctr, zero before the first run
+
+// this run's epoch: no block counts the run before every block is done
+__device__ __forceinline__ uint32_t tiles_epoch(const uint32_t* ctr) { return ld_relaxed32(&ctr[2]) + 1; }
 
 // Publish tile `tile`'s sum and return the sum of the tiles before it; one whole
 // warp, all lanes get the result.  32 tiles are read at a time: one after
@@ -53,12 +60,14 @@ __device__ __forceinline__ uint32_t look_back(uint64_t* status, uint32_t tile, u
   return prefix;
 }
 
-// one thread of every block, at its end: the last makes the tile ids start at 0 again
+// one thread of every block, at its end: the last makes the tile ids start at 0
+// again and the next run's epoch another one
 __device__ __forceinline__ void tiles_done(uint32_t* ctr) {
   __threadfence();
   if (atomicAdd(&ctr[1], 1u) == gridDim.x - 1) {
     ctr[0] = 0;
     ctr[1] = 0;
+    ctr[2] = (ctr[2] + 1) % kLbEpochs;
     __threadfence();
   }
 }

@@ -198,8 +198,9 @@ __global__ void __launch_bounds__(kGroupThreads)
     merge_group_kernel(MergeCounts* mc, const uint32_t* ins_list, const uint32_t* n_dev, const uint32_t* isnew,
                        const uint64_t* ukeys, const uint64_t* uvals, const uint32_t* mleaf, uint64_t* newk,
                        uint64_t* newv, uint32_t* nq, uint32_t* nleaf, uint32_t* seg_start, uint32_t* seg_leaf,
-                       uint64_t* status, uint64_t* status_seg, uint32_t* ctr, uint32_t epoch, uint32_t* err) {
+                       uint64_t* status, uint64_t* status_seg, uint32_t* ctr, uint32_t* err) {
   after_previous();
+  const uint32_t epoch = tiles_epoch(ctr);
   __shared__ uint32_t ws[32];
   __shared__ uint32_t s_tile, s_pre[2];
   const uint32_t n = *n_dev, n_tiles = ceil_div(n, kGroupTile);
@@ -304,8 +305,9 @@ __device__ __forceinline__ void reserve_pieces(const DevTree& t, MergeCounts* mc
 __global__ void __launch_bounds__(kGroupThreads)
     merge_reserve_kernel(DevTree t, uint32_t leaf_fill, uint32_t entry_cap, MergeCounts* mc, const uint32_t* seg_start,
                          const uint32_t* seg_leaf, uint32_t* extra, uint32_t* eoff, uint64_t* status, uint32_t* ctr,
-                         uint32_t epoch, uint32_t* err) {
+                         uint32_t* err) {
   after_previous();
+  const uint32_t epoch = tiles_epoch(ctr);
   __shared__ uint32_t ws[32];
   __shared__ uint32_t s_tile, s_pre;
   const uint32_t n = mc->n_segs, n_tiles = ceil_div(n, (uint32_t)kGroupThreads);
@@ -1191,19 +1193,13 @@ int merge_update_phase(Handle* h, size_t n_upper, cudaStream_t s) {
 // segments' new leaves reuse the first part
 size_t merge_lb_words(size_t n) { return 2 * ((n + kGroupThreads - 1) / kGroupThreads + 1); }
 
-static uint32_t next_epoch(uint32_t* epoch) {
-  *epoch = (*epoch + 1) & ((1u << 30) - 1);
-  if (*epoch == 0) *epoch = 1;  // zeroed status words carry epoch 0
-  return *epoch;
-}
-
 int merge_group_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   Work& w = h->w;
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
   const unsigned gb = (unsigned)min((size_t)h->sm_count * 2, (n_upper + kGroupTile - 1) / kGroupTile);
   launch_after(merge_group_kernel, gb, kGroupThreads, 0, s, mc, w.ins_list, &w.counts->n_ins, w.m_isnew, w.ukeys,
                w.uvals, w.m_leaf, w.m_newk, w.m_newv, w.m_nq, w.m_nleaf, w.m_seg, w.m_pos, w.lb_status,
-               w.lb_status + merge_lb_words(w.cap) / 2, w.lb_ctr, next_epoch(&w.lb_epoch), &h->tree.ctrl->error);
+               w.lb_status + merge_lb_words(w.cap) / 2, w.lb_ctr, &h->tree.ctrl->error);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1213,7 +1209,7 @@ int merge_reserve_phase(Handle* h, size_t n_upper, cudaStream_t s) {
   MergeCounts* mc = reinterpret_cast<MergeCounts*>(w.m_counts);
   const unsigned rb = (unsigned)min((size_t)h->sm_count * 2, (n_upper + kGroupThreads - 1) / kGroupThreads);
   launch_after(merge_reserve_kernel, rb, kGroupThreads, 0, s, h->tree, h->leaf_fill, (uint32_t)w.cap, mc, w.m_seg,
-               w.m_pos, w.m_isnew, w.m_leaf, w.lb_status, w.lb_ctr, next_epoch(&w.lb_epoch), &h->tree.ctrl->error);
+               w.m_pos, w.m_isnew, w.m_leaf, w.lb_status, w.lb_ctr, &h->tree.ctrl->error);
   const unsigned gb = (unsigned)min((size_t)h->sm_count * 8, (n_upper + 255) / 256);
   launch_after(merge_fail_mark_kernel, gb, 256, 0, s, mc, w.m_nq, w.ins_list, w.uans_st);
   count_launch(2);

@@ -137,9 +137,9 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
 // / apply form takes three.
 __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* in, uint32_t* out, size_t n_upper,
                                                                const uint32_t* n_dev, uint32_t* total_out,
-                                                               uint64_t* status, uint32_t* ctr, uint32_t epoch,
-                                                               uint32_t* err) {
+                                                               uint64_t* status, uint32_t* ctr, uint32_t* err) {
   after_previous();
+  const uint32_t epoch = tiles_epoch(ctr);
   __shared__ uint32_t ws[32];
   __shared__ uint32_t tot, s_tile, s_prefix;
   const size_t n = n_dev ? min(n_upper, (size_t)*n_dev) : n_upper;
@@ -422,16 +422,14 @@ static unsigned sm_count() {
 }
 
 cudaError_t scan_exclusive_u32_lb(const uint32_t* in, uint32_t* out, size_t n_upper, const uint32_t* n_dev,
-                                  uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* epoch,
-                                  uint32_t* err, cudaStream_t s) {
-  *epoch = (*epoch + 1) & ((1u << 30) - 1);
-  if (*epoch == 0) *epoch = 1;  // zeroed status words carry epoch 0
+                                  uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* err,
+                                  cudaStream_t s) {
   // one block per SM, taking tiles until there are none: the bound is the batch's size, the live entries
   // mostly under 2^19, and a block per tile of the bound was 1,024 blocks of 1,024 threads that found
   // nothing to do (11 us a scan of a 2^22 batch)
   const size_t blocks = n_upper ? min((n_upper + kScanTile - 1) / kScanTile, (size_t)sm_count()) : 1;
   launch_after(scan_lb_kernel, (unsigned)blocks, kScanThreads, 0, s, in, out, n_upper, n_dev, total_dev, status, ctr,
-               *epoch, err);
+               err);
   count_launch();
   return cudaGetLastError();
 }

@@ -60,3 +60,35 @@ def test_root_of_an_empty_tree(gpu, n):
     gk, gv = dump(t)
     o = np.argsort(k)
     assert (gk == k[o]).all() and (gv == v[o]).all()
+
+
+@pytest.mark.parametrize("n", [3_000, 70_000, 131_072])
+@pytest.mark.parametrize("mode, engine", [(MERGE, O.ENGINE_MERGE), (E.MODE_SORTED, O.ENGINE_STM)])
+def test_replays_with_other_inputs(gpu, n, mode, engine):
+    # every replay meets the tree and the counts of its own turn: fresh keys (many
+    # tiles of new keys and segments, leaves that split), few writes, deletes
+    keys, vals, _ = inserts(1211, 150_000)
+    t = tree(max_keys=1 << 21)
+    t.bulk_build(dev(keys), dev(vals))
+    o = O.OracleTree()
+    o.bulk_build(keys, vals)
+    g = Captured(t, n, mode)
+    rng = np.random.default_rng(1212)
+    for turn, pct in enumerate([0, 20, 99, 0, 60]):
+        rk, rv, ro = O.gen_requests("uniform", 1220 + turn, keys, n, pct)
+        if turn == 0 or turn == 3:  # keys that are not there
+            rk = O.gen_keys("uniform", 1230 + turn, n)
+        if turn == 4:
+            ro[rng.random(n) < 0.3] = E.OP_DELETE
+        ov, os_ = o.execute_merged(rk, rv, ro, engine=engine)
+        gv, gs = g.run(rk, rv, ro)
+        assert (gs == os_).all() and (gv == ov).all(), turn
+        # and an uncaptured batch between two replays
+        rk, rv, ro = O.gen_requests("uniform", 1240 + turn, keys, 100_000, 50)
+        ov, os_ = o.execute_merged(rk, rv, ro, engine=engine)
+        gv, gs = run_batch(t, rk, rv, ro, mode)
+        assert (gs == os_).all() and (gv == ov).all(), turn
+    gk, gv = dump(t)
+    ok, ovv = o.dump()
+    assert (gk == ok).all() and (gv == ovv).all()
+    assert (t.leaf_sizes().sum() == gk.size) and t.stats()["error"] == 0
