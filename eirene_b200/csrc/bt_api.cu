@@ -189,14 +189,17 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   constexpr size_t kCtrlBytes = (sizeof(bt::Ctrl) + 255) / 256 * 256;
   ok = ok && cudaMalloc(&h.tree.ctrl, kCtrlBytes + 256) == cudaSuccess;
   if (ok) h.geo = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h.tree.ctrl) + kCtrlBytes);
-  // zeroed rows read as epoch 0, which no tree uses (see hdr_epoch)
-  ok = ok && cudaMemset(h.tree.keys, 0, nodes * 256) == cudaSuccess;
-  ok = ok && cudaMemset(h.tree.vals, 0, nodes * 256) == cudaSuccess;
-  ok = ok && cudaMemset(h.tree.low, 0, nodes * 8) == cudaSuccess;
-  ok = ok && cudaMemset(h.tree.pfx, 0xff, nodes * 128) == cudaSuccess;
-  ok = ok && cudaMemset(h.tree.fp, 0, nodes * 32) == cudaSuccess;
-  ok = ok && bt::work_alloc(&h.w, cfg.max_batch) == 0;
+  // everything that is cleared, on the stream that is waited for below: on the
+  // default stream it queues behind whatever that holds, and no batch on another
+  // stream would wait for it
   ok = ok && cudaStreamCreateWithFlags(&h.internal_stream, cudaStreamNonBlocking) == cudaSuccess;
+  auto fill = [&](void* p, int byte, size_t bytes) {
+    return cudaMemsetAsync(p, byte, bytes, h.internal_stream) == cudaSuccess;
+  };
+  // zeroed rows read as epoch 0, which no tree uses (see hdr_epoch)
+  ok = ok && fill(h.tree.keys, 0, nodes * 256) && fill(h.tree.vals, 0, nodes * 256) &&
+       fill(h.tree.low, 0, nodes * 8) && fill(h.tree.pfx, 0xff, nodes * 128) && fill(h.tree.fp, 0, nodes * 32);
+  ok = ok && bt::work_alloc(&h.w, cfg.max_batch, h.internal_stream) == 0;
   {
     int lo_prio = 0, hi_prio = 0;
     cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio);

@@ -408,7 +408,7 @@ static size_t carve_work(Work* w, size_t cap, char* base) {
   return A.at;
 }
 
-int work_alloc(Work* w, size_t cap) {
+int work_alloc(Work* w, size_t cap, cudaStream_t s) {
   work_free(w);
   if (cap == 0) cap = 1;
   const size_t bytes = carve_work(w, cap, nullptr);
@@ -418,9 +418,9 @@ int work_alloc(Work* w, size_t cap) {
   }
   carve_work(w, cap, static_cast<char*>(w->arena));
   // look-back words of no epoch, and a clean table (every slot empty between batches)
-  if (cudaMemset(w->lb_status, 0, merge_lb_words(cap) * 8) != cudaSuccess ||
-      cudaMemset(w->lb_ctr, 0, kLbCtrWords * 4) != cudaSuccess ||
-      cudaMemset(w->s_tab, 0xff, small_tab_bytes(cap)) != cudaSuccess) {
+  if (cudaMemsetAsync(w->lb_status, 0, merge_lb_words(cap) * 8, s) != cudaSuccess ||
+      cudaMemsetAsync(w->lb_ctr, 0, kLbCtrWords * 4, s) != cudaSuccess ||
+      cudaMemsetAsync(w->s_tab, 0xff, small_tab_bytes(cap), s) != cudaSuccess) {
     work_free(w);
     return -3;
   }

@@ -519,7 +519,7 @@ int small_read(Handle* h, bool gets, bool locate_ins, uint64_t* out_vals, uint8_
 int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s);
 
 // ---- sorted-merge batch (bt_batch.cu) ----
-int work_alloc(Work* w, size_t cap);
+int work_alloc(Work* w, size_t cap, cudaStream_t s);  // cleared in the order of s
 void work_free(Work* w);
 int batch_sorted(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,
                  uint8_t* out_st, size_t n, int engine, cudaStream_t s);

@@ -1059,13 +1059,13 @@ static int learned_reserve(Learned* L, size_t n_leaves, uint32_t n_seg) {
   return 0;
 }
 
-static int miss_reserve(Learned* L, size_t cap) {
+static int miss_reserve(Learned* L, size_t cap, cudaStream_t s) {
   if (!L->gate) {
     if (cudaMalloc(&L->gate, sizeof(LearnedGate)) != cudaSuccess) {
       L->gate = nullptr;
       return -3;
     }
-    if (cudaMemset(L->gate, 0, sizeof(LearnedGate)) != cudaSuccess) return -3;
+    if (cudaMemsetAsync(L->gate, 0, sizeof(LearnedGate), s) != cudaSuccess) return -3;
   }
   if (cap <= L->miss_cap) return 0;
   cudaFree(L->miss);
@@ -1124,7 +1124,7 @@ int learned_retrain(Handle* h, cudaStream_t s, bool refit) {
   if (refit && n_seg > L.seg_cap) refit = false;
   if (!refit) L.trained = false;
   if (learned_reserve(&L, nl, n_seg)) return -3;
-  if (miss_reserve(&L, h->w.cap > 65536 ? h->w.cap : 65536)) return -3;
+  if (miss_reserve(&L, h->w.cap > 65536 ? h->w.cap : 65536, s)) return -3;
   LeafEnt* tab = reinterpret_cast<LeafEnt*>(L.leaf_low);
   leaf_table_kernel<<<nblk(nl + 1, 256), 256, 0, s>>>(h->tree, ids, nl, tab);
   count_launch();

@@ -236,9 +236,10 @@ int bt_serve_start(bt_handle* H, const bt_serve_config* cfg_in, bt_server** out)
     std::memset(S->h_tclaim, 0, S->cap * 8);
     std::memset(S->h_tend, 0, S->cap * 8);
     std::memset(S->st_zero, 0, 64);
-    ok = cudaMemset(S->d_tail, 0, 256) == cudaSuccess &&
-         cudaMemset(S->d_claimed, 0xFF, S->cap * sizeof(unsigned long long)) == cudaSuccess &&
-         cudaMemset(S->d_done, 0, S->cap * 4) == cudaSuccess;
+    ok = cudaMemsetAsync(S->d_tail, 0, 256, S->s_k) == cudaSuccess &&
+         cudaMemsetAsync(S->d_claimed, 0xFF, S->cap * sizeof(unsigned long long), S->s_k) == cudaSuccess &&
+         cudaMemsetAsync(S->d_done, 0, S->cap * 4, S->s_k) == cudaSuccess &&
+         cudaStreamSynchronize(S->s_k) == cudaSuccess;
   }
   uint32_t* h_done_dev = nullptr;
   unsigned long long* h_tend_dev = nullptr;

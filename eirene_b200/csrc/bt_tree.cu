@@ -1040,7 +1040,7 @@ cudaError_t launch_range(Handle* h, const uint64_t* lo, const uint64_t* hi, size
 // and a reallocation (cudaFree synchronises the device) on every refit or
 // dump stalled the batches queued behind it
 constexpr size_t kEnumCtrWords = (kLbCtrWords + 1) / 2;  // in 64-bit words
-static int ensure_enum(Handle* h, size_t n) {
+static int ensure_enum(Handle* h, size_t n, cudaStream_t s) {
   if (n <= h->enum_cap) return 0;
   n += n / 4 + 4096;
   cudaFree(h->enum_a);
@@ -1053,7 +1053,7 @@ static int ensure_enum(Handle* h, size_t n) {
   const size_t c = n + 64, lb = scan_lb_words(c) + kEnumCtrWords;  // the last ones: the scan's counters
   if (cudaMalloc(&h->enum_a, c * 4) != cudaSuccess || cudaMalloc(&h->enum_b, c * 4) != cudaSuccess ||
       cudaMalloc(&h->enum_cnt, c * 4) != cudaSuccess || cudaMalloc(&h->enum_lb, lb * 8) != cudaSuccess ||
-      cudaMemset(h->enum_lb, 0, lb * 8) != cudaSuccess)
+      cudaMemsetAsync(h->enum_lb, 0, lb * 8, s) != cudaSuccess)
     return -3;
   h->enum_cap = c;
   h->enum_lb_words = lb;
@@ -1085,7 +1085,7 @@ static int enumerate_queue(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_
   if (rl >= 48) return -2;
   const size_t nn = c->n_nodes < h->tree.cap ? c->n_nodes : h->tree.cap;
   h->n_levels = rl + 1;
-  if (ensure_enum(h, nn + 1) != 0) return -3;
+  if (ensure_enum(h, nn + 1, s) != 0) return -3;
   uint32_t* cnt = h->geo;
   uint32_t* cur = h->enum_a;
   uint32_t* nxt = h->enum_b;

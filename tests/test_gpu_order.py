@@ -85,3 +85,27 @@ def test_loaded_image_is_whole_when_it_returns(gpu, tmp_path, call):
         check(b)
         torch.cuda.synchronize()
         assert (host_u8(st1) == E.ST_FOUND).all()
+
+
+@pytest.mark.parametrize("n, max_batch", [(1_000, 1_024), (70_000, 1 << 17)])
+def test_new_handle_beside_a_busy_default_stream(gpu, n, max_batch):
+    # everything that a new handle, its first dump and its first training clear is
+    # clear when they are used, whatever else the default stream holds
+    import torch
+
+    keys = np.sort(O.gen_keys("uniform", 1121, n))
+    k, v, op = dev(keys), dev(O.value_of(keys)), torch.full((n,), E.OP_INSERT, dtype=torch.uint8, device="cuda")
+    s = torch.cuda.Stream()
+    ov, os_ = empty_u64(n), empty_u8(n)
+    for _ in range(2):  # the first turn loads the kernels, which waits for the device
+        torch.cuda.synchronize()
+        busy(torch.cuda.default_stream())
+        t = E.BTree(max_keys=1 << 18, max_batch=max_batch)
+        t.execute(k, v, op, ov, os_, mode=E.MODE_SORTED | E.MODE_MERGE_ENGINE, stream=s)
+        t.sync(s)
+        t.retrain(stream=s)
+        s.synchronize()
+        assert (host_u8(os_) == E.ST_ABSENT).all()
+        gk, gv = t.dump()
+        assert (gk == k).all() and (gv == v).all()
+        t.close()
