@@ -399,7 +399,7 @@ static size_t carve_work(Work* w, size_t cap, char* base) {
   A(w->f_tk, cap * 8);
   A(w->f_tv, cap * 4);
   A(w->lb_status, merge_lb_words(cap) * 8);
-  A(w->lb_ctr, kLbCtrWords * 4);
+  A(w->lb_ctr, kLbCtrWords * 8);
   A(w->s_write, 3 * 16 * 4);
   A(w->s_split, kSsBuckets * 16);
   A(w->s_sum, sample_sum_bytes());
@@ -419,7 +419,7 @@ int work_alloc(Work* w, size_t cap, cudaStream_t s) {
   carve_work(w, cap, static_cast<char*>(w->arena));
   // look-back words of no epoch, and a clean table (every slot empty between batches)
   if (cudaMemsetAsync(w->lb_status, 0, merge_lb_words(cap) * 8, s) != cudaSuccess ||
-      cudaMemsetAsync(w->lb_ctr, 0, kLbCtrWords * 4, s) != cudaSuccess ||
+      cudaMemsetAsync(w->lb_ctr, 0, kLbCtrWords * 8, s) != cudaSuccess ||
       cudaMemsetAsync(w->s_tab, 0xff, small_tab_bytes(cap), s) != cudaSuccess) {
     work_free(w);
     return -3;

@@ -46,7 +46,7 @@ cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, uint
 // words and ctr: kLbCtrWords, both zero before the first call)
 size_t scan_lb_words(size_t n_upper);
 cudaError_t scan_exclusive_u32_lb(const uint32_t* in, uint32_t* out, size_t n_upper, const uint32_t* n_dev,
-                                  uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* err,
+                                  uint32_t* total_dev, uint64_t* status, uint64_t* ctr, uint32_t* err,
                                   cudaStream_t s);
 cudaError_t sort_prepare();
 size_t sort_scratch_words(size_t n);
@@ -168,7 +168,7 @@ struct Work {
   uint8_t* ins_ops = nullptr;
   // look-back words of the merge engine (bt_lookback.cuh)
   uint64_t* lb_status = nullptr;
-  uint32_t* lb_ctr = nullptr;
+  uint64_t* lb_ctr = nullptr;
   // sample sort of the touched requests (bt_sample.cu)
   uint64_t* s_split = nullptr;    // splitters, bucket totals
   void* s_sum = nullptr;          // per bucket: its part of the segmented scan, its start

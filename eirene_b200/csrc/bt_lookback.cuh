@@ -4,10 +4,12 @@
 // status[t] = epoch << 34 | state << 32 | value, state 1 the tile's own sum, 2
 // its inclusive prefix; each run's epoch makes the words of earlier runs read
 // as not ready, so the array is never cleared.  The epoch is counted on the
-// device (ctr[2]): as a launch argument it was fixed in a captured launch, and a
-// second replay took the first one's words for its own.  ctr[0] hands tile ids
-// out in the order blocks take them (a tile waits only on tiles taken before
-// it); the last block to finish resets both and counts the run.  The wait is
+// device: as a launch argument it was fixed in a captured launch, and a second
+// replay took the first one's words for its own.  ctr[0] hands out tile ids, in
+// the order blocks take them (a tile waits only on tiles taken before it), with
+// the runs so far in its high half: one atomic gives a block both, where a word
+// of its own for the epoch cost a scan 2 us.  ctr[1] counts the blocks that are
+// done; the last one starts the ids again and counts the run.  The wait is
 // bounded: past kLbSpinLimit it sets kErrSpin in *err and goes on.
 #pragma once
 #include <cstdint>
@@ -19,10 +21,13 @@ namespace bt {
 constexpr uint64_t kLbAgg = 1ull << 32, kLbInc = 2ull << 32;
 constexpr uint32_t kLbSpinLimit = 1u << 22;
 constexpr uint32_t kLbEpochs = (1u << 30) - 1;  // epochs 1 .. kLbEpochs; zeroed words carry epoch 0
-constexpr int kLbCtrWords = 3;                  // words of ctr, zero before the first run
+constexpr size_t kLbCtrWords = 2;               // words of ctr, zero before the first run
 
-// this run's epoch: no block counts the run before every block is done
-__device__ __forceinline__ uint32_t tiles_epoch(const uint32_t* ctr) { return ld_relaxed32(&ctr[2]) + 1; }
+// a tile (low half) and the run's epoch less one
+__device__ __forceinline__ uint64_t take_tile(uint64_t* ctr) {
+  return atomicAdd(reinterpret_cast<unsigned long long*>(ctr), 1ull);
+}
+__device__ __forceinline__ uint32_t tile_epoch(uint64_t ticket) { return (uint32_t)(ticket >> 32) + 1; }
 
 // Publish tile `tile`'s sum and return the sum of the tiles before it; one whole
 // warp, all lanes get the result.  32 tiles are read at a time: one after
@@ -60,14 +65,12 @@ __device__ __forceinline__ uint32_t look_back(uint64_t* status, uint32_t tile, u
   return prefix;
 }
 
-// one thread of every block, at its end: the last makes the tile ids start at 0
-// again and the next run's epoch another one
-__device__ __forceinline__ void tiles_done(uint32_t* ctr) {
+// one thread of every block, at its end
+__device__ __forceinline__ void tiles_done(uint64_t* ctr, uint32_t epoch) {
   __threadfence();
-  if (atomicAdd(&ctr[1], 1u) == gridDim.x - 1) {
-    ctr[0] = 0;
+  if (atomicAdd(reinterpret_cast<unsigned long long*>(ctr + 1), 1ull) == gridDim.x - 1) {
+    ctr[0] = (uint64_t)(epoch % kLbEpochs) << 32;
     ctr[1] = 0;
-    ctr[2] = (ctr[2] + 1) % kLbEpochs;
     __threadfence();
   }
 }

@@ -198,16 +198,18 @@ __global__ void __launch_bounds__(kGroupThreads)
     merge_group_kernel(MergeCounts* mc, const uint32_t* ins_list, const uint32_t* n_dev, const uint32_t* isnew,
                        const uint64_t* ukeys, const uint64_t* uvals, const uint32_t* mleaf, uint64_t* newk,
                        uint64_t* newv, uint32_t* nq, uint32_t* nleaf, uint32_t* seg_start, uint32_t* seg_leaf,
-                       uint64_t* status, uint64_t* status_seg, uint32_t* ctr, uint32_t* err) {
+                       uint64_t* status, uint64_t* status_seg, uint64_t* ctr, uint32_t* err) {
   after_previous();
-  const uint32_t epoch = tiles_epoch(ctr);
   __shared__ uint32_t ws[32];
-  __shared__ uint32_t s_tile, s_pre[2];
+  __shared__ uint32_t s_pre[2];
+  __shared__ uint64_t s_ticket;
+  uint32_t epoch;
   const uint32_t n = *n_dev, n_tiles = ceil_div(n, kGroupTile);
   for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+    if (threadIdx.x == 0) s_ticket = take_tile(ctr);
     __syncthreads();
-    const uint32_t tile = s_tile;
+    const uint32_t tile = (uint32_t)s_ticket;
+    epoch = tile_epoch(s_ticket);
     __syncthreads();
     if (tile >= n_tiles) {
       if (tile == 0 && threadIdx.x == 0) mc->n_new = mc->n_segs = 0;  // no INSERT
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(kGroupThreads)
       p++;
     }
   }
-  if (threadIdx.x == 0) tiles_done(ctr);
+  if (threadIdx.x == 0) tiles_done(ctr, epoch);
 }
 
 __device__ __forceinline__ void seg_bounds(const MergeCounts* mc, const uint32_t* seg_start, uint32_t s,
@@ -304,17 +306,19 @@ __device__ __forceinline__ void reserve_pieces(const DevTree& t, MergeCounts* mc
 // was three launches (count, scan, reserve).
 __global__ void __launch_bounds__(kGroupThreads)
     merge_reserve_kernel(DevTree t, uint32_t leaf_fill, uint32_t entry_cap, MergeCounts* mc, const uint32_t* seg_start,
-                         const uint32_t* seg_leaf, uint32_t* extra, uint32_t* eoff, uint64_t* status, uint32_t* ctr,
+                         const uint32_t* seg_leaf, uint32_t* extra, uint32_t* eoff, uint64_t* status, uint64_t* ctr,
                          uint32_t* err) {
   after_previous();
-  const uint32_t epoch = tiles_epoch(ctr);
   __shared__ uint32_t ws[32];
-  __shared__ uint32_t s_tile, s_pre;
+  __shared__ uint32_t s_pre;
+  __shared__ uint64_t s_ticket;
+  uint32_t epoch;
   const uint32_t n = mc->n_segs, n_tiles = ceil_div(n, (uint32_t)kGroupThreads);
   for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+    if (threadIdx.x == 0) s_ticket = take_tile(ctr);
     __syncthreads();
-    const uint32_t tile = s_tile;
+    const uint32_t tile = (uint32_t)s_ticket;
+    epoch = tile_epoch(s_ticket);
     __syncthreads();
     if (tile >= n_tiles) {
       if (tile == 0 && threadIdx.x == 0) {
@@ -349,7 +353,7 @@ __global__ void __launch_bounds__(kGroupThreads)
       eoff[i] = s_pre + ex;
     }
   }
-  if (threadIdx.x == 0) tiles_done(ctr);
+  if (threadIdx.x == 0) tiles_done(ctr, epoch);
 }
 
 // a batch whose pieces did not fit answers kNoCapacity for all its new keys

@@ -137,17 +137,19 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
 // / apply form takes three.
 __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* in, uint32_t* out, size_t n_upper,
                                                                const uint32_t* n_dev, uint32_t* total_out,
-                                                               uint64_t* status, uint32_t* ctr, uint32_t* err) {
+                                                               uint64_t* status, uint64_t* ctr, uint32_t* err) {
   after_previous();
-  const uint32_t epoch = tiles_epoch(ctr);
   __shared__ uint32_t ws[32];
-  __shared__ uint32_t tot, s_tile, s_prefix;
+  __shared__ uint32_t tot, s_prefix;
+  __shared__ uint64_t s_ticket;
+  uint32_t epoch;
   const size_t n = n_dev ? min(n_upper, (size_t)*n_dev) : n_upper;
   const size_t n_tiles = (n + kScanTile - 1) / kScanTile;
   for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+    if (threadIdx.x == 0) s_ticket = take_tile(ctr);
     __syncthreads();
-    const uint32_t tile = s_tile;
+    const uint32_t tile = (uint32_t)s_ticket;
+    epoch = tile_epoch(s_ticket);
     __syncthreads();
     if (tile >= n_tiles) {
       if (tile == 0 && threadIdx.x == 0 && total_out) *total_out = 0;  // nothing to scan
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_lb_kernel(const uint32_t* i
       ex += v[i];
     }
   }
-  if (threadIdx.x == 0) tiles_done(ctr);
+  if (threadIdx.x == 0) tiles_done(ctr, epoch);
 }
 
 // ---------------------------------------------------------------- sort ----
@@ -422,7 +424,7 @@ static unsigned sm_count() {
 }
 
 cudaError_t scan_exclusive_u32_lb(const uint32_t* in, uint32_t* out, size_t n_upper, const uint32_t* n_dev,
-                                  uint32_t* total_dev, uint64_t* status, uint32_t* ctr, uint32_t* err,
+                                  uint32_t* total_dev, uint64_t* status, uint64_t* ctr, uint32_t* err,
                                   cudaStream_t s) {
   // one block per SM, taking tiles until there are none: the bound is the batch's size, the live entries
   // mostly under 2^19, and a block per tile of the bound was 1,024 blocks of 1,024 threads that found

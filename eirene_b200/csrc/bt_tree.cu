@@ -1039,7 +1039,6 @@ cudaError_t launch_range(Handle* h, const uint64_t* lo, const uint64_t* hi, size
 // grown with a quarter of headroom: the tree grows a little with every batch,
 // and a reallocation (cudaFree synchronises the device) on every refit or
 // dump stalled the batches queued behind it
-constexpr size_t kEnumCtrWords = (kLbCtrWords + 1) / 2;  // in 64-bit words
 static int ensure_enum(Handle* h, size_t n, cudaStream_t s) {
   if (n <= h->enum_cap) return 0;
   n += n / 4 + 4096;
@@ -1050,7 +1049,7 @@ static int ensure_enum(Handle* h, size_t n, cudaStream_t s) {
   h->enum_a = h->enum_b = h->enum_cnt = nullptr;
   h->enum_lb = nullptr;
   h->enum_cap = 0;
-  const size_t c = n + 64, lb = scan_lb_words(c) + kEnumCtrWords;  // the last ones: the scan's counters
+  const size_t c = n + 64, lb = scan_lb_words(c) + kLbCtrWords;  // the last ones: the scan's counters
   if (cudaMalloc(&h->enum_a, c * 4) != cudaSuccess || cudaMalloc(&h->enum_b, c * 4) != cudaSuccess ||
       cudaMalloc(&h->enum_cnt, c * 4) != cudaSuccess || cudaMalloc(&h->enum_lb, lb * 8) != cudaSuccess ||
       cudaMemsetAsync(h->enum_lb, 0, lb * 8, s) != cudaSuccess)
@@ -1062,7 +1061,7 @@ static int ensure_enum(Handle* h, size_t n, cudaStream_t s) {
 
 static cudaError_t enum_scan(Handle* h, uint32_t* x, const uint32_t* n_dev, size_t n_upper, uint32_t* total,
                              cudaStream_t s) {
-  uint32_t* ctr = reinterpret_cast<uint32_t*>(h->enum_lb + h->enum_lb_words - kEnumCtrWords);
+  uint64_t* ctr = h->enum_lb + h->enum_lb_words - kLbCtrWords;
   return scan_exclusive_u32_lb(x, x, n_upper, n_dev, total, h->enum_lb, ctr, &h->tree.ctrl->error, s);
 }
 
