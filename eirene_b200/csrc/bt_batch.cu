@@ -400,7 +400,7 @@ static size_t carve_work(Work* w, size_t cap, char* base) {
   A(w->f_tv, cap * 4);
   A(w->lb_status, merge_lb_words(cap) * 8);
   A(w->lb_ctr, kLbCtrWords * 8);
-  A(w->s_write, 3 * 16 * 4);
+  A(w->s_write, small_write_words() * 4);
   A(w->s_split, kSsBuckets * 16);
   A(w->s_sum, sample_sum_bytes());
   A(w->s_tab, small_tab_bytes(cap));
@@ -530,7 +530,7 @@ struct FrontPart {
   uint32_t* sv = nullptr;
   uint32_t n_tiles = 0;
   bool sample = false;  // sorted by the sample sort (its buckets' sums instead of tile passes)
-  bool cluster = false;  // few enough of them for one cluster to write
+  uint32_t cluster = 0;  // one cluster writes this many of them (0: none)
   bool passes_done = false;
 };
 
@@ -548,8 +548,9 @@ static int hashed_passes(Handle* h, const FrontPart& fp, const uint64_t* vals, u
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+// beside: on its own stream, beside the tree part of the batch before
 static int hashed_front(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,
-                        uint8_t* out_st, size_t n, cudaStream_t s, bool passes, FrontPart& fp,
+                        uint8_t* out_st, size_t n, cudaStream_t s, bool beside, bool passes, FrontPart& fp,
                         cudaEvent_t vals_ready = nullptr) {
   Work& w = h->w;
   const uint32_t* n_touch = &w.counts->n_touch;
@@ -561,7 +562,8 @@ static int hashed_front(Handle* h, const uint64_t* keys, const uint64_t* vals, c
   if (h->touch_sort == 2 && h->touch_hint) {
     const uint32_t seen = *reinterpret_cast<volatile const uint32_t*>(h->touch_hint);
     fp.sample = seen <= kSampleSortMax;
-    fp.cluster = seen <= kClusterWriteMax && !h->prof;
+    const uint32_t limit = cluster_write_limit(n, beside);
+    if (seen <= limit && !h->prof) fp.cluster = limit;
   }
   if (front_classify(h, keys, ops, n, !fp.sample, s) != 0) return -2;
   if (fp.sample) {
@@ -589,8 +591,10 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
   const uint32_t* n_touch = &c->n_touch;
   const bool ov = h->overlap != 0;
   const bool early = merge_usable(h, engine);
-  // few touched requests (by the hint that chose the sample sort): the write part of the small batches
-  const bool cluster = early && fp.cluster;
+  // few touched requests (by the hint that chose the sample sort): the write part of the small
+  // batches.  The hint is another batch's count; what is too much for it this batch's count tells
+  // on the device (small_write)
+  const bool cluster = early && fp.cluster != 0;
   const bool defer = early && h->async_write != 0;
   const bool learned = batch_learned(h, h->batch_descent >= 0 ? h->batch_descent : h->descent, s);
   // the locates (side stream) run beside the lookups (`s`); so do the merge
@@ -645,7 +649,7 @@ static int hashed_tree(Handle* h, const uint64_t* keys, const uint64_t* vals, ui
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
   }
   if (cluster) {
-    if (small_write(h, out_vals, out_st, kSmallMax, s) != 0 || answers_ready(h, s) != 0) return -2;
+    if (small_write(h, out_vals, out_st, n, fp.cluster, s) != 0 || answers_ready(h, s) != 0) return -2;
     if (defer) {  // a later call on any stream comes after this batch's writes
       if (cudaEventRecord(h->tree_ev, s) != cudaSuccess) return -2;
       h->tree_pending = true;
@@ -682,7 +686,7 @@ static int batch_hashed(Handle* h, const uint64_t* keys, const uint64_t* vals, c
   prof_mark(h, 0, s);
   prof_set_layout(h, (ov ? kLayoutOverlap : 0) | (merge_usable(h, engine) ? kLayoutEarly : 0));
   FrontPart fp;
-  if (hashed_front(h, keys, vals, ops, out_vals, out_st, n, s, !pass_side, fp) != 0) return -2;
+  if (hashed_front(h, keys, vals, ops, out_vals, out_st, n, s, false, !pass_side, fp) != 0) return -2;
   return hashed_tree(h, keys, vals, out_vals, out_st, n, engine, s, fp);
 }
 
@@ -721,7 +725,7 @@ static int batch_small(Handle* h, const uint64_t* keys, const uint64_t* vals, co
     count_launch();
     return answers_ready(h, s) != 0 || cudaGetLastError() != cudaSuccess ? -2 : 0;
   }
-  if (small_write(h, out_vals, out_st, n, s) != 0 || answers_ready(h, s) != 0) return -2;
+  if (small_write(h, out_vals, out_st, n, (uint32_t)n, s) != 0 || answers_ready(h, s) != 0) return -2;
   // a later call on any stream comes after this batch's writes
   if (h->async_write) {
     if (cudaEventRecord(h->tree_ev, s) != cudaSuccess) return -2;
@@ -773,7 +777,7 @@ int batches_pipelined(Handle* h, size_t count, const uint64_t* const* keys, cons
       use(p);
       fp[p] = FrontPart{};
       if ((j >= 2 && cudaStreamWaitEvent(F, h->tree_done[p], 0) != cudaSuccess) ||
-          hashed_front(h, keys[j], vals[j], ops[j], out_vals[j], out_st[j], n[j], F, true, fp[p]) != 0 ||
+          hashed_front(h, keys[j], vals[j], ops[j], out_vals[j], out_st[j], n[j], F, true, true, fp[p]) != 0 ||
           cudaEventRecord(h->front_done[p], F) != cudaSuccess)
         rc = -2;
     }
@@ -825,7 +829,7 @@ int batch_chained(Handle* h, const uint64_t* keys, const uint64_t* vals, const u
   use(p);
   if ((!open && cudaEventRecord(h->chain_gate, s) != cudaSuccess) ||
       cudaStreamWaitEvent(F, h->chain_gate, 0) != cudaSuccess || cudaStreamWaitEvent(F, in_ready, 0) != cudaSuccess ||
-      hashed_front(h, keys, vals, ops, out_vals, out_st, n, F, !pass_tree, fp, vals_ready) != 0 ||
+      hashed_front(h, keys, vals, ops, out_vals, out_st, n, F, true, !pass_tree, fp, vals_ready) != 0 ||
       cudaEventRecord(h->front_done[p], F) != cudaSuccess || cudaEventRecord(h->chain_gate, s) != cudaSuccess ||
       cudaStreamWaitEvent(s, h->front_done[p], 0) != cudaSuccess)
     rc = -2;

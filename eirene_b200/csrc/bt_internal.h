@@ -500,10 +500,18 @@ int unroute_results(Handle* h, const uint32_t* perm, const uint64_t* in_vals, co
 // ---- sorted batches of up to kSmallMax requests (bt_small.cu; the write part in bt_merge.cu) ----
 constexpr size_t kSmallMax = 65536;
 // touched count (seen last) up to which a larger batch's write part is the small
-// batches' one too (us a batch on 2^23 keys, its own twelve launches / one: 100,000
-// requests with 1000 writes 133 / 102, 20,000 175 / 169; 400,000 with 20,000 196 /
-// 187, 40,000 222 / 237)
-constexpr uint32_t kClusterWriteMax = 20480;
+// batches' one too, with grid_write_kernel behind it for a batch that turns out
+// to have more (us a batch on 2^23 keys, cluster and that launch / the general
+// path's launches).  One batch after another: 150,000 requests with no write 50 /
+// 63, 1000 writes 81 / 82, 4000 102 / 103, 10,000 116 / 114, 20,000 137 / 128; 2^20
+// requests 107 / 118, 146 / 146, 165 / 163, 179 / 171, 204 / 186.  Four batches of a
+// call, whose front parts want the chip meanwhile: 150,000 requests 49 / 65, 66 /
+// 81, 82 / 95, 94 / 106, 117 / 120; 2^20 100 / 123, 127 / 138, 138 / 151, 142 / 156,
+// 163 / 168; but 70,000 requests with 8000 writes 86 / 80.
+constexpr uint32_t kClusterWriteAlone = 2048, kClusterWriteMax = 20480;
+inline uint32_t cluster_write_limit(size_t n, bool beside) {
+  return !beside ? kClusterWriteAlone : n / 8 < kClusterWriteMax ? (uint32_t)(n / 8) : kClusterWriteMax;
+}
 int small_prepare();
 int small_write_prepare();
 size_t small_tab_bytes(size_t cap);
@@ -515,8 +523,10 @@ int small_front(Handle* h, const uint64_t* keys, const uint64_t* vals, const uin
                 uint8_t* out_st, size_t n, bool ensure_root, cudaStream_t s);
 // reads of the tree: the plain lookups (gets), the locates of the DELETE keys and (locate_ins) INSERT keys
 int small_read(Handle* h, bool gets, bool locate_ins, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s);
-// writes: values, DELETE apply, grouping, reservation, write-back, leaf and inner merge
-int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s);
+// writes: values, DELETE apply, grouping, reservation, write-back, leaf and inner merge; a cluster
+// for n requests, or the whole chip when more than `limit` requests turn out to be touched
+int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, uint32_t limit, cudaStream_t s);
+size_t small_write_words();
 
 // ---- sorted-merge batch (bt_batch.cu) ----
 int work_alloc(Work* w, size_t cap, cudaStream_t s);  // cleared in the order of s

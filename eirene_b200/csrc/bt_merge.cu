@@ -952,6 +952,12 @@ __global__ void __launch_bounds__(kInnerThreads) merge_inner_kernel(DevTree t, u
 // them.  Leaving the leaf and inner merge to their launches over the whole chip
 // costs 9 us more a batch up to 4096 requests, and gains only at 65,536 (254
 // against 271 us, all INSERTs).
+//
+// A larger batch takes it when the batch before had few touched requests.  That
+// is a guess, and sixteen SMs would take 2.5 us for every further thousand, so
+// the batch's own count decides on the device: above the limit the cluster
+// returns at once and grid_write_kernel, queued behind it, does the same on
+// every SM; at or below it that one finds nothing to do.
 struct WriteSmem {
   union {
     LeafSmem<kSmallThreads / 8> leaf;
@@ -960,6 +966,8 @@ struct WriteSmem {
   uint32_t ws[32];
   uint32_t before, total;
 };
+
+constexpr uint32_t kWriteTeam = 1024;  // most blocks that write together
 
 struct SmallWrite {
   const BatchCounts* counts;
@@ -972,40 +980,46 @@ struct SmallWrite {
   uint32_t *isnew, *pos, *leaf, *nq, *nleaf, *seg;
   uint64_t *newk, *newv;
   MergeEntry *ea, *eb;
-  uint32_t* sums;  // three sets of 16 block totals
+  uint32_t* sums;  // three sets of kWriteTeam block totals
   uint32_t leaf_fill, inner_fill, entry_cap;
+  uint32_t limit;  // touched requests up to which the cluster writes
   size_t path_stride;
 };
 
-// exclusive prefix of v over the threads of the cluster and the total; one
-// cluster barrier (sums: a set of its own per use)
-__device__ __forceinline__ uint32_t cluster_scan(uint32_t v, uint32_t* sums, WriteSmem& S, uint32_t* total) {
+// exclusive prefix of v over the threads of the team and the total; one
+// barrier (sums: a set of its own per use)
+template <typename Team>
+__device__ __forceinline__ bool team_prefix(const Team& team, uint32_t v, uint32_t* sums, WriteSmem& S,
+                                            uint32_t* before, uint32_t* total) {
   uint32_t tot;
   const uint32_t ex = blk_exclusive_sum(v, S.ws, &tot);
-  if (threadIdx.x == 0) sums[cluster_rank()] = tot;
-  cluster_sync();
+  if (threadIdx.x == 0) sums[team.rank()] = tot;
+  if (!team.sync()) return false;
   if (threadIdx.x < 32) {
-    const uint32_t x = threadIdx.x < cluster_size() ? __ldcg(sums + threadIdx.x) : 0u;
-    const uint32_t before = __reduce_add_sync(kFull, threadIdx.x < cluster_rank() ? x : 0u);
-    const uint32_t all = __reduce_add_sync(kFull, x);
+    uint32_t lower = 0, all = 0;
+    for (uint32_t b = threadIdx.x; b < team.size(); b += 32) {
+      const uint32_t x = __ldcg(sums + b);
+      all += x;
+      lower += b < team.rank() ? x : 0u;
+    }
+    lower = __reduce_add_sync(kFull, lower);
+    all = __reduce_add_sync(kFull, all);
     if (threadIdx.x == 0) {
-      S.before = before;
+      S.before = lower;
       S.total = all;
     }
   }
   __syncthreads();
-  const uint32_t r = S.before + ex;
+  *before = S.before + ex;
   *total = S.total;
   __syncthreads();
-  return r;
+  return true;
 }
 
-__global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
-                                                                       uint8_t* out_st) {
-  extern __shared__ __align__(16) unsigned char raw[];
-  WriteSmem& S = *reinterpret_cast<WriteSmem*>(raw);
-  after_previous();
-  const uint32_t rank = cluster_rank(), C = cluster_size();
+template <typename Team>
+__device__ __forceinline__ void write_part(const DevTree& t, const SmallWrite& a, uint64_t* out_vals, uint8_t* out_st,
+                                           const Team& team, WriteSmem& S) {
+  const uint32_t rank = team.rank(), C = team.size();
   const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
   const uint32_t n_ins = a.counts->n_ins, n_del = a.counts->n_del, n_touch = a.counts->n_touch;
   MergeCounts* mc = a.mc;
@@ -1015,13 +1029,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
     if (p != kNoPos) t.vals[p] = a.uvals[a.ins_list[q]];
   }
   if (n_del) {
-    cluster_sync();
+    if (!team.sync()) return;
     uint32_t removed = 0;
     for (uint32_t i = gt >> 5; i < n_del; i += nt >> 5)
       removed += del_apply_at(t, a.dleaf, a.dslot, i, n_del, threadIdx.x & 31);
     if ((threadIdx.x & 31) == 0 && removed) atomicAdd(&t.ctrl->n_keys, (unsigned long long)0 - removed);
   }
-  // this thread's consecutive items of n spread over the cluster: one while there
+  // this thread's consecutive items of n spread over the team: one while there
   // are threads enough (several would be that many chains of loads in a row)
   auto mine = [&](uint32_t n, uint32_t& i0, uint32_t& i1) {
     const uint32_t each = ceil_div(n, nt);
@@ -1034,7 +1048,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
     uint32_t i0, i1, v = 0;
     mine(n_ins, i0, i1);
     for (uint32_t i = i0; i < i1; i++) v += a.isnew[i];
-    uint32_t p = cluster_scan(v, a.sums, S, &n_new);
+    uint32_t p;
+    if (!team_prefix(team, v, a.sums, S, &p, &n_new)) return;
     for (uint32_t i = i0; i < i1; i++) {
       if (!a.isnew[i]) continue;
       const uint32_t u = a.ins_list[i];
@@ -1046,7 +1061,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
     }
   }
   if (n_new) {
-    cluster_sync();
+    if (!team.sync()) return;
     // runs of new keys that share a leaf
     uint32_t i0, i1, v = 0;
     mine(n_new, i0, i1);
@@ -1057,7 +1072,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
       v += lf != prev ? 1u : 0u;
       prev = lf;
     }
-    uint32_t p = cluster_scan(v, a.sums + 16, S, &n_segs);
+    uint32_t p;
+    if (!team_prefix(team, v, a.sums + kWriteTeam, S, &p, &n_segs)) return;
     prev = before;
     for (uint32_t i = i0; i < i1; i++) {
       const uint32_t lf = __ldcg(a.nleaf + i);
@@ -1067,7 +1083,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
       }
       prev = lf;
     }
-    cluster_sync();
+    if (!team.sync()) return;
     // new leaves per run
     mine(n_segs, i0, i1);
     v = 0;
@@ -1078,7 +1094,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
       a.isnew[i] = x;
       v += x;
     }
-    p = cluster_scan(v, a.sums + 32, S, &n_ent);
+    if (!team_prefix(team, v, a.sums + 2 * kWriteTeam, S, &p, &n_ent)) return;
     for (uint32_t i = i0; i < i1; i++) {
       const uint32_t x = a.isnew[i];
       a.pos[i] = p;
@@ -1091,11 +1107,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
     mc->n_leaf_entries = n_ent;
     reserve_pieces(t, mc, a.entry_cap);
   }
-  cluster_sync();
+  if (!team.sync()) return;
   const bool fail = __ldcg(&mc->cap_fail) != 0;
   if (fail) {  // a full pool: the new keys are answered kNoCapacity
     for (uint32_t i = gt; i < n_new; i += nt) a.uans_st[a.ins_list[a.nq[i]]] = kNoCapacity;
-    cluster_sync();
+    if (!team.sync()) return;
   }
   for (uint32_t i = gt; i < n_touch; i += nt) {
     const uint32_t u = a.pend[i];
@@ -1108,30 +1124,48 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
   leaf_merge<8, kSmallThreads / 8>(t, a.leaf_fill, mc, a.seg, a.pos, a.isnew, a.newk, a.newv, a.nq, a.leaf,
                                           a.ea, S.leaf, gt / 8, nt / 8);
   if (n_ent == 0) return;
-  cluster_sync();
-  inner_merge<kSmallThreads>(t, a.inner_fill, a.entry_cap, mc, a.gs, a.ea, a.eb, a.path, a.path_stride, a.seg, a.nleaf, a.nq, a.pos,
-                             ClusterTeam{}, S.inner);
+  if (!team.sync()) return;
+  inner_merge<kSmallThreads>(t, a.inner_fill, a.entry_cap, mc, a.gs, a.ea, a.eb, a.path, a.path_stride, a.seg, a.nleaf,
+                             a.nq, a.pos, team, S.inner);
 }
 
+__global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
+                                                                       uint8_t* out_st) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  after_previous();
+  if (a.counts->n_touch > a.limit) {  // for grid_write_kernel, its barrier as new
+    if (cluster_rank() == 0 && threadIdx.x == 0) a.gs->count = a.gs->fail = 0;
+    return;
+  }
+  write_part(t, a, out_vals, out_st, ClusterTeam{}, *reinterpret_cast<WriteSmem*>(raw));
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1) grid_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
+                                                                      uint8_t* out_st) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  if (a.counts->n_touch <= a.limit) return;  // small_write_kernel wrote it
+  write_part(t, a, out_vals, out_st, GridTeam{a.gs, &t.ctrl->error}, *reinterpret_cast<WriteSmem*>(raw));
+}
 
 }  // namespace
+
+// blocks of a cooperative kernel that are resident at once, asked once per device
+static unsigned resident_blocks(const Handle* h, const void* kernel, int threads, size_t smem, unsigned (&known)[64]) {
+  const int dev = h->device;
+  if (dev < 0 || dev >= 64) return (unsigned)h->sm_count;
+  if (!known[dev]) {
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess || per < 1) per = 1;
+    known[dev] = (unsigned)per * (unsigned)h->sm_count;
+  }
+  return known[dev];
+}
 
 // cooperative launch of merge_inner_kernel: at most the resident blocks
 static cudaError_t launch_inner(Handle* h, uint32_t entry_cap, MergeCounts* mc, cudaStream_t s) {
   Work& w = h->w;
   static unsigned resident[64] = {};
-  const int dev = h->device;
-  unsigned blocks = (unsigned)h->sm_count;
-  if (dev >= 0 && dev < 64) {
-    if (!resident[dev]) {
-      int per = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, merge_inner_kernel, kInnerThreads, 0) != cudaSuccess ||
-          per < 1)
-        per = 1;
-      resident[dev] = (unsigned)per * (unsigned)h->sm_count;
-    }
-    blocks = resident[dev];
-  }
+  unsigned blocks = resident_blocks(h, (const void*)merge_inner_kernel, kInnerThreads, 0, resident);
   if (blocks > 1024) blocks = 1024;  // InnerSync::partial
   InnerSync* gs = reinterpret_cast<InnerSync*>(w.m_sync);
   cudaError_t e = cudaMemsetAsync(gs, 0, sizeof(InnerSync), s);
@@ -1232,14 +1266,18 @@ int merge_write_phase(Handle* h, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+size_t small_write_words() { return 3 * kWriteTeam; }
+
 int small_write_prepare() {
   cudaError_t e =
       cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(grid_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e == cudaSuccess ? 0 : -2;
 }
 
-int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaStream_t s) {
+int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, uint32_t limit, cudaStream_t s) {
   Work& w = h->w;
   SmallWrite a;
   a.counts = w.counts;
@@ -1274,8 +1312,19 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, cudaSt
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[2];
   small_config(cfg, at, small_cluster(n), sizeof(WriteSmem), s);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, small_write_kernel, h->tree, a, out_vals, out_st);
+  a.limit = limit;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, small_write_kernel, h->tree, a, out_vals, out_st);
   count_launch();
+  if (e == cudaSuccess && limit < n) {
+    static unsigned resident[64] = {};
+    void* args[] = {&h->tree, &a, &out_vals, &out_st};
+    e = cudaLaunchCooperativeKernel(
+        (const void*)grid_write_kernel,
+        dim3(min(resident_blocks(h, (const void*)grid_write_kernel, kSmallThreads, sizeof(WriteSmem), resident),
+                 kWriteTeam)),
+        dim3(kSmallThreads), args, sizeof(WriteSmem), s);
+    count_launch();
+  }
   return e == cudaSuccess ? 0 : -2;
 }
 
