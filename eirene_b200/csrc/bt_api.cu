@@ -179,6 +179,7 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   h.L.window = cfg.window ? cfg.window : 64;
   cudaDeviceGetAttribute(&h.sm_count, cudaDevAttrMultiProcessorCount, cfg.device);
   bool ok = bt::sort_prepare() == cudaSuccess && bt::small_prepare() == 0 && bt::small_write_prepare() == 0 && bt::sample_prepare() == 0;
+  if (ok) h.small_blocks = bt::small_blocks(cfg.device);
   h.tree.cap = (uint32_t)nodes;
   ok = ok && cudaMalloc(&h.tree.keys, nodes * 256) == cudaSuccess;
   ok = ok && cudaMalloc(&h.tree.vals, nodes * 256) == cudaSuccess;

@@ -563,7 +563,7 @@ static int hashed_front(Handle* h, const uint64_t* keys, const uint64_t* vals, c
     const uint32_t seen = *reinterpret_cast<volatile const uint32_t*>(h->touch_hint);
     fp.sample = seen <= kSampleSortMax;
     const uint32_t limit = cluster_write_limit(n, beside);
-    if (seen <= limit && !h->prof) fp.cluster = limit;
+    if (seen <= limit && !h->prof && h->small_blocks == kSmallBlocks) fp.cluster = limit;
   }
   if (front_classify(h, keys, ops, n, !fp.sample, s) != 0) return -2;
   if (fp.sample) {
@@ -694,7 +694,7 @@ static int batch_hashed(Handle* h, const uint64_t* keys, const uint64_t* vals, c
 // the options that say how the general path works at their defaults, and
 // while no phases are recorded (it has none of the general path's).
 bool small_usable(const Handle* h, size_t n) {
-  return n <= kSmallMax && h->front_end == 1 && h->touch_sort == 2 && !h->prof && !h->vals_remote;
+  return n <= small_limit(h->small_blocks) && h->front_end == 1 && h->touch_sort == 2 && !h->prof && !h->vals_remote;
 }
 
 static int batch_small(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,

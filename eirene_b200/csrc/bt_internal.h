@@ -284,6 +284,7 @@ struct Handle {
   int use_pfx = 1;           // paired searches compare the separators' 32-bit prefixes first
   void* top = nullptr;       // top cache (kTopNodes nodes) + TopInfo
   TopInfo* top_info = nullptr;
+  unsigned small_blocks = 0;  // largest cluster of the small batches (bt_small.cu)
   int sm_count = 148;
   Work w;
   Learned L;
@@ -512,7 +513,13 @@ constexpr uint32_t kClusterWriteAlone = 2048, kClusterWriteMax = 20480;
 inline uint32_t cluster_write_limit(size_t n, bool beside) {
   return !beside ? kClusterWriteAlone : n / 8 < kClusterWriteMax ? (uint32_t)(n / 8) : kClusterWriteMax;
 }
+constexpr unsigned kSmallBlocks = 16;  // blocks of the largest cluster
 int small_prepare();
+// the largest cluster that the device takes, by its two kernels; 0: batches take the general path
+unsigned small_blocks(int device);
+unsigned small_write_largest();
+unsigned small_cluster(size_t n, unsigned most);
+size_t small_limit(unsigned most);
 int small_write_prepare();
 size_t small_tab_bytes(size_t cap);
 size_t small_sum_bytes();

@@ -1268,6 +1268,8 @@ int merge_write_phase(Handle* h, cudaStream_t s) {
 
 size_t small_write_words() { return 3 * kWriteTeam; }
 
+unsigned small_write_largest() { return small_largest((const void*)small_write_kernel, sizeof(WriteSmem)); }
+
 int small_write_prepare() {
   cudaError_t e =
       cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
@@ -1311,7 +1313,7 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, uint32
   a.entry_cap = (uint32_t)w.cap;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[2];
-  small_config(cfg, at, small_cluster(n), sizeof(WriteSmem), s);
+  small_config(cfg, at, small_cluster(n, h->small_blocks), sizeof(WriteSmem), s);
   a.limit = limit;
   cudaError_t e = cudaLaunchKernelEx(&cfg, small_write_kernel, h->tree, a, out_vals, out_st);
   count_launch();

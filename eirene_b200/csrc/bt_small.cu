@@ -528,6 +528,44 @@ __global__ void __launch_bounds__(kReadThreads) small_read_kernel(DevTree t, Sma
 
 }  // namespace
 
+// Blocks of the cluster for n requests: one per 128, up to `most`.  A block's
+// leaf merges are what costs in a write-heavy batch, and the barrier of a
+// larger cluster costs little (us a batch of 2048 / 4096 all-INSERT requests
+// with one block per 4096: 126 / 224, per 1024: 90 / 95, per 128: 59 / 69; a
+// 95/5 batch of 4096: 52, 43, 43).
+unsigned small_cluster(size_t n, unsigned most) {
+  unsigned c = 1;
+  while ((size_t)c * 128 < n && c < most) c <<= 1;
+  return c;
+}
+
+// requests that such clusters take
+size_t small_limit(unsigned most) { return (size_t)most * kSmallPer; }
+
+// Sixteen blocks are more than every device has to offer (eight are), and how
+// many fit depends on the SMs that a partition leaves each group of them.
+unsigned small_largest(const void* kernel, size_t smem) {
+  for (unsigned c = kSmallBlocks; c; c >>= 1) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[2];
+    small_config(cfg, at, c, smem, nullptr);
+    cfg.numAttrs = 1;  // the cluster alone
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0) return c;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
+unsigned small_blocks(int device) {
+  static unsigned known[64] = {};  // one more than the answer
+  if (device >= 0 && device < 64 && known[device]) return known[device] - 1;
+  const unsigned front = small_largest((const void*)small_front_kernel, sizeof(FrontSmem)), write = small_write_largest();
+  const unsigned most = front < write ? front : write;
+  if (device >= 0 && device < 64) known[device] = most + 1;
+  return most;
+}
+
 size_t small_tab_bytes(size_t cap) {
   const size_t nmax = cap < kSmallMax ? cap : kSmallMax;
   size_t slots = 1024;
@@ -566,7 +604,7 @@ int small_front(Handle* h, const uint64_t* keys, const uint64_t* vals, const uin
   f.edge = reinterpret_cast<uint64_t*>(static_cast<char*>(w.s_sums) + 16 * sizeof(FrontSum));
   uint32_t slots = 1024;
   while (slots < 4 * n) slots <<= 1;
-  const unsigned C = small_cluster(n);
+  const unsigned C = small_cluster(n, h->small_blocks);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[2];
   small_config(cfg, at, C, sizeof(FrontSmem), s);

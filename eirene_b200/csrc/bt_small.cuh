@@ -12,7 +12,7 @@ constexpr int kSmallThreads = 1024;
 constexpr int kSmallItems = 4;  // requests (and sorted pairs, and new keys) per thread
 // most requests per block of a cluster
 constexpr uint32_t kSmallPer = kSmallThreads * kSmallItems;
-static_assert(kSmallMax == 16 * kSmallPer, "the largest small batch fills sixteen blocks");
+static_assert(kSmallMax == kSmallBlocks * kSmallPer, "the largest small batch fills sixteen blocks");
 
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -79,16 +79,8 @@ struct SmallRead {
   int locate_ins;  // 0: the STM kernel inserts
 };
 
-// Blocks of the cluster for n requests: one per 128, up to sixteen.  A block's
-// leaf merges are what costs in a write-heavy batch, and the barrier of a
-// larger cluster costs little (us a batch of 2048 / 4096 all-INSERT requests
-// with one block per 4096: 126 / 224, per 1024: 90 / 95, per 128: 59 / 69; a
-// 95/5 batch of 4096: 52, 43, 43).
-inline unsigned small_cluster(size_t n) {
-  unsigned c = 1;
-  while ((size_t)c * 128 < n && c < 16) c <<= 1;
-  return c;
-}
+// largest cluster of a kernel with `smem` bytes a block that the current device takes (0: none)
+unsigned small_largest(const void* kernel, size_t smem);
 
 // at: two attributes, the cluster and the dependent launch
 inline void small_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned C, size_t smem, cudaStream_t s) {
