@@ -253,7 +253,7 @@ int bt_destroy(bt_handle* H) {
   cudaFree(h.enum_b);
   cudaFree(h.enum_cnt);
   cudaFree(h.enum_lb);
-  if (h.build_pool) cudaMemPoolDestroy(h.build_pool);
+  bt::build_pool_drop(&h);
   cudaFree(h.top);
   if (h.internal_stream) cudaStreamDestroy(h.internal_stream);
   if (h.hi_stream) cudaStreamDestroy(h.hi_stream);

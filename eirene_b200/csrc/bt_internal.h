@@ -296,7 +296,7 @@ struct Handle {
   size_t enum_cap = 0;
   uint32_t* geo = nullptr;      // 256 bytes: the bulk build's geometry, the enumeration's counts
   uint32_t* pin = nullptr;      // 256 bytes of page-locked memory: what the host reads back
-  cudaMemPool_t build_pool = nullptr;  // scratch of bulk builds of more than max_batch keys
+  cudaMemPool_t build_pool = nullptr;  // scratch of bulk builds of more than max_batch keys (the device's, shared)
   uint64_t level_counts[48] = {};  // filled by enumerate_leaves, leaf level first
   uint32_t n_levels = 0;
   cudaStream_t internal_stream = nullptr;
@@ -387,6 +387,7 @@ struct BuildScratch {
   uint32_t* tot;  // one word
   size_t cap;     // keys
 };
+void build_pool_drop(Handle* h);
 int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s,
                             const BuildScratch& sc);
 // Plain lookups of at least so many requests take the warp form, fewer the

@@ -11,6 +11,7 @@
 // is active (the batch executor orders it before/after the insert phase), so
 // it needs no version checks and may use the read-only cache path.
 #include <cstdio>
+#include <mutex>
 #include <cuda_runtime.h>
 
 #include "bt_block.cuh"
@@ -842,12 +843,59 @@ int tree_bulk_build_scratch(Handle* h, const uint64_t* keys, const uint64_t* val
   return *status == kBuildReserved ? -5 : *status == kBuildCapacity ? -4 : 0;
 }
 
-// The same with the handle's scratch: up to max_batch keys in the batch work
-// buffers; more in one block of the handle's own pool, which keeps up to
-// kBuildKeep bytes between builds (a pool that gives its memory back at every
-// synchronisation maps and unmaps it per build: most of the 1.0 ms that a load
-// of 2^20 keys spent outside its kernels) and all of it until bt_destroy.
+// Scratch of the builds of more than max_batch keys: one pool per device, shared
+// by its handles, which keeps up to kBuildKeep bytes between builds (a pool that
+// gives its memory back at every synchronisation maps and unmaps it per build:
+// most of the 1.0 ms that a load of 2^20 keys spent outside its kernels).  With a
+// pool for each handle, as many times kBuildKeep stayed mapped as there were large
+// trees.  The last handle that used it gives it back; the allocator orders reuse
+// between streams and threads.
 constexpr uint64_t kBuildKeep = 1ull << 30;
+constexpr int kPoolDevices = 64;
+struct BuildPool {
+  cudaMemPool_t pool = nullptr;
+  unsigned users = 0;
+};
+static std::mutex g_pool_mu;
+static BuildPool g_pools[kPoolDevices];
+
+// the handle's share; the device's default pool where there is no table for it
+static bool build_pool_take(Handle* h) {
+  if (h->build_pool) return true;
+  if (h->device < 0 || h->device >= kPoolDevices) return cudaDeviceGetDefaultMemPool(&h->build_pool, h->device) == cudaSuccess;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  BuildPool& p = g_pools[h->device];
+  if (p.users == 0) {
+    cudaMemPoolProps pp{};
+    pp.allocType = cudaMemAllocationTypePinned;
+    pp.handleTypes = cudaMemHandleTypeNone;
+    pp.location.type = cudaMemLocationTypeDevice;
+    pp.location.id = h->device;
+    uint64_t keep = kBuildKeep;
+    if (cudaMemPoolCreate(&p.pool, &pp) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  p.users++;
+  h->build_pool = p.pool;
+  return true;
+}
+
+void build_pool_drop(Handle* h) {
+  if (!h->build_pool || h->device < 0 || h->device >= kPoolDevices) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  BuildPool& p = g_pools[h->device];
+  h->build_pool = nullptr;
+  if (--p.users == 0) {
+    cudaMemPoolDestroy(p.pool);
+    p.pool = nullptr;
+  }
+}
+
+// The same with the library's scratch: up to max_batch keys in the batch work
+// buffers, more in one block of the device's pool.
 int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s) {
   // the contents are gone in these cases too: a call on another stream may
   // follow at once and has to meet the new tree, not the old one
@@ -869,23 +917,11 @@ int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_
     sc.cap = w.cap;
     return tree_bulk_build_scratch(h, keys, vals, n, s, sc);
   }
-  if (!h->build_pool) {
-    cudaMemPoolProps pp{};
-    pp.allocType = cudaMemAllocationTypePinned;
-    pp.handleTypes = cudaMemHandleTypeNone;
-    pp.location.type = cudaMemLocationTypeDevice;
-    pp.location.id = h->device;
-    uint64_t keep = kBuildKeep;
-    if (cudaMemPoolCreate(&h->build_pool, &pp) != cudaSuccess) {
-      h->build_pool = nullptr;
-      return -3;
-    }
-    cudaMemPoolSetAttribute(h->build_pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  }
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t kb = up(n * 8), vb = up(n * 4), pb = up((n / kDedupeTile + 2) * 4);
   char* slab = nullptr;
-  if (cudaMallocFromPoolAsync((void**)&slab, 3 * kb + 2 * vb + pb + up(sort_scratch_words(n) * 4), h->build_pool, s) !=
+  if (!build_pool_take(h) ||
+      cudaMallocFromPoolAsync((void**)&slab, 3 * kb + 2 * vb + pb + up(sort_scratch_words(n) * 4), h->build_pool, s) !=
       cudaSuccess) {
     cudaGetLastError();
     return emptied(-3);

@@ -118,7 +118,10 @@ int bt_destroy(bt_handle *h);
 
 /* Replace the tree contents with the n pairs (the last value wins for a repeated
  * key).  Synchronous.  The reference builds by running gpu_work() over a file of
- * P lines (src/main.cpp:21-25, src/gpu-stm-tree-v39/bpt-gpustm.cpp:67-132). */
+ * P lines (src/main.cpp:21-25, src/gpu-stm-tree-v39/bpt-gpustm.cpp:67-132).
+ * More than max_batch keys need scratch of about 38 bytes a key.  It comes from
+ * one memory pool per device, which keeps up to 1 GiB for the next such build
+ * until the last handle that made one is destroyed. */
 int bt_bulk_build(bt_handle *h, const uint64_t *keys, const uint64_t *vals, size_t n, void *stream);
 
 /* bt_bulk_build without any allocation, for callers that must not allocate GPU
