@@ -1155,6 +1155,11 @@ int enumerate_leaves(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_l
   *n_leaves = 0;
   const int rc = enumerate_queue(h, s, leaf_ids, &nn, &rl);
   if (rc || rl < 0) return rc;
+  if (rl == 0) {  // the root is the only leaf: nothing to wait for
+    h->level_counts[0] = 1;
+    *n_leaves = 1;
+    return 0;
+  }
   if (cudaMemcpyAsync(h->pin, h->geo, kEnumWords * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return -2;
