@@ -691,6 +691,7 @@ __device__ bool grid_sync(InnerSync* gs, uint32_t* err) {
 // The blocks that apply the entries: the cooperative grid, or the cluster of a
 // small batch (whose hardware barrier cannot fail).
 struct GridTeam {
+  static constexpr uint32_t kMost = 1024;
   InnerSync* gs;
   uint32_t* err;
   __device__ uint32_t rank() const { return blockIdx.x; }
@@ -698,6 +699,7 @@ struct GridTeam {
   __device__ bool sync() const { return grid_sync(gs, err); }
 };
 struct ClusterTeam {
+  static constexpr uint32_t kMost = kSmallBlocks;
   __device__ uint32_t rank() const { return cluster_rank(); }
   __device__ uint32_t size() const { return cluster_size(); }
   __device__ bool sync() const {
@@ -967,7 +969,7 @@ struct WriteSmem {
   uint32_t before, total;
 };
 
-constexpr uint32_t kWriteTeam = 1024;  // most blocks that write together
+constexpr uint32_t kWriteTeam = GridTeam::kMost;  // most blocks that write together
 
 struct SmallWrite {
   const BatchCounts* counts;
@@ -1001,6 +1003,7 @@ __device__ __forceinline__ bool team_prefix(const Team& team, uint32_t v, uint32
       const uint32_t x = __ldcg(sums + b);
       all += x;
       lower += b < team.rank() ? x : 0u;
+      if (Team::kMost <= 32) break;
     }
     lower = __reduce_add_sync(kFull, lower);
     all = __reduce_add_sync(kFull, all);
@@ -1017,11 +1020,11 @@ __device__ __forceinline__ bool team_prefix(const Team& team, uint32_t v, uint32
 }
 
 template <typename Team>
-__device__ __forceinline__ void write_part(const DevTree& t, const SmallWrite& a, uint64_t* out_vals, uint8_t* out_st,
-                                           const Team& team, WriteSmem& S) {
+__device__ __forceinline__ void write_part(const DevTree& t, const SmallWrite& a, uint32_t n_ins, uint32_t n_del,
+                                           uint32_t n_touch, uint64_t* out_vals, uint8_t* out_st, const Team& team,
+                                           WriteSmem& S) {
   const uint32_t rank = team.rank(), C = team.size();
   const uint32_t nt = C * kSmallThreads, gt = rank * kSmallThreads + threadIdx.x;
-  const uint32_t n_ins = a.counts->n_ins, n_del = a.counts->n_del, n_touch = a.counts->n_touch;
   MergeCounts* mc = a.mc;
   // new values of the keys found in the tree, then the DELETE keys (which move values)
   for (uint32_t q = gt; q < n_ins; q += nt) {
@@ -1129,22 +1132,27 @@ __device__ __forceinline__ void write_part(const DevTree& t, const SmallWrite& a
                              a.nq, a.pos, team, S.inner);
 }
 
+// kGuess: a larger batch's, which may have more touched requests than the limit
+template <bool kGuess>
 __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
                                                                        uint8_t* out_st) {
   extern __shared__ __align__(16) unsigned char raw[];
   after_previous();
-  if (a.counts->n_touch > a.limit) {  // for grid_write_kernel, its barrier as new
+  const uint32_t n_ins = a.counts->n_ins, n_del = a.counts->n_del, n_touch = a.counts->n_touch;
+  if (kGuess && n_touch > a.limit) {  // for grid_write_kernel, its barrier as new
     if (cluster_rank() == 0 && threadIdx.x == 0) a.gs->count = a.gs->fail = 0;
     return;
   }
-  write_part(t, a, out_vals, out_st, ClusterTeam{}, *reinterpret_cast<WriteSmem*>(raw));
+  write_part(t, a, n_ins, n_del, n_touch, out_vals, out_st, ClusterTeam{}, *reinterpret_cast<WriteSmem*>(raw));
 }
 
 __global__ void __launch_bounds__(kSmallThreads, 1) grid_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
                                                                       uint8_t* out_st) {
   extern __shared__ __align__(16) unsigned char raw[];
-  if (a.counts->n_touch <= a.limit) return;  // small_write_kernel wrote it
-  write_part(t, a, out_vals, out_st, GridTeam{a.gs, &t.ctrl->error}, *reinterpret_cast<WriteSmem*>(raw));
+  const uint32_t n_touch = a.counts->n_touch;
+  if (n_touch <= a.limit) return;  // small_write_kernel wrote it
+  write_part(t, a, a.counts->n_ins, a.counts->n_del, n_touch, out_vals, out_st, GridTeam{a.gs, &t.ctrl->error},
+             *reinterpret_cast<WriteSmem*>(raw));
 }
 
 }  // namespace
@@ -1268,14 +1276,17 @@ int merge_write_phase(Handle* h, cudaStream_t s) {
 
 size_t small_write_words() { return 3 * kWriteTeam; }
 
-unsigned small_write_largest() { return small_largest((const void*)small_write_kernel, sizeof(WriteSmem)); }
+unsigned small_write_largest() { return small_largest((const void*)small_write_kernel<true>, sizeof(WriteSmem)); }
 
 int small_write_prepare() {
-  cudaError_t e =
-      cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(grid_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WriteSmem));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(small_write_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const auto wide = cudaFuncAttributeNonPortableClusterSizeAllowed;
+  const int bytes = (int)sizeof(WriteSmem);
+  cudaError_t e = cudaFuncSetAttribute(grid_write_kernel, smem, bytes);
+  for (auto k : {small_write_kernel<false>, small_write_kernel<true>}) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, smem, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, wide, 1);
+  }
   return e == cudaSuccess ? 0 : -2;
 }
 
@@ -1315,9 +1326,11 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, uint32
   cudaLaunchAttribute at[2];
   small_config(cfg, at, small_cluster(n, h->small_blocks), sizeof(WriteSmem), s);
   a.limit = limit;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, small_write_kernel, h->tree, a, out_vals, out_st);
+  const bool guess = limit < n;
+  cudaError_t e =
+      cudaLaunchKernelEx(&cfg, guess ? small_write_kernel<true> : small_write_kernel<false>, h->tree, a, out_vals, out_st);
   count_launch();
-  if (e == cudaSuccess && limit < n) {
+  if (e == cudaSuccess && guess) {
     static unsigned resident[64] = {};
     void* args[] = {&h->tree, &a, &out_vals, &out_st};
     e = cudaLaunchCooperativeKernel(
