@@ -66,7 +66,7 @@ struct Item {
   bool head, tail, valid, wr, del;  // wr: INSERT or DELETE of a usable key
 };
 
-__device__ __forceinline__ void load_items(const uint64_t* __restrict__ sk, const uint32_t* __restrict__ sv,
+__device__ __forceinline__ void load_items(const uint64_t* sk, const uint32_t* sv,
                                            size_t n, size_t i0, Item (&it)[kItems]) {
   uint64_t prev = (i0 > 0 && i0 - 1 < n) ? sk[i0 - 1] : 0;
 #pragma unroll
@@ -103,7 +103,7 @@ __device__ __forceinline__ void load_items(const uint64_t* __restrict__ sk, cons
   }
 }
 
-__device__ __forceinline__ Seg item_seg(const Item& x, const uint64_t* __restrict__ vals) {
+__device__ __forceinline__ Seg item_seg(const Item& x, const uint64_t* vals) {
   Seg s;
   s.f = x.head ? 1u : 0u;
   s.v = 0;

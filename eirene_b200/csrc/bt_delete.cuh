@@ -10,8 +10,8 @@ constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 // One warp at entry i of the n located DELETE keys: when i is the first of its
 // leaf, all of that leaf's found keys are removed (a ballot over the row keeps
 // the others in order).  Returns how many.
-__device__ __forceinline__ uint32_t del_apply_at(const DevTree& t, const uint32_t* __restrict__ dleaf,
-                                                 const uint32_t* __restrict__ dslot, size_t i, size_t n,
+__device__ __forceinline__ uint32_t del_apply_at(const DevTree& t, const uint32_t* dleaf,
+                                                 const uint32_t* dslot, size_t i, size_t n,
                                                  uint32_t lane) {
   const uint32_t leaf = dleaf[i];
   if (leaf == kNil || (i > 0 && dleaf[i - 1] == leaf)) return 0;  // not the first entry of its leaf

@@ -166,9 +166,9 @@ constexpr int kTileWarps = kTileThreads / 32;
 // The thread's items of a tile (item j: base + j * THREADS + threadIdx.x),
 // their keys and op codes, and a bit per item: touched.
 template <int THREADS, int ITEMS>
-__device__ __forceinline__ uint32_t classify_items(const uint64_t* __restrict__ keys, const uint8_t* __restrict__ ops,
-                                                   size_t n, const Slot* __restrict__ tab,
-                                                   const BatchCounts* __restrict__ counts, size_t base,
+__device__ __forceinline__ uint32_t classify_items(const uint64_t* keys, const uint8_t* ops,
+                                                   size_t n, const Slot* tab,
+                                                   const BatchCounts* counts, size_t base,
                                                    uint64_t (&k)[ITEMS], uint8_t (&op)[ITEMS]) {
   const uint32_t mask = counts->cap - 1;
   const bool any = counts->n_ins_req != 0;

@@ -7,12 +7,15 @@
 
 namespace bt {
 
-// First statement of a kernel that launch_after starts.  Such a kernel takes no
-// __restrict__ pointers and makes no ld.global.nc loads: the compiler may move a
-// load through a __restrict__ parameter ahead of the wait (the memory clobber
-// says nothing about it), and the non-coherent path is only for data that
-// nothing writes while the kernel is there, which here is before its wait too.
-// (With them, a probe took its table's size from before the size was written.)
+// First statement of a kernel that launch_after starts.  Such a kernel, and every
+// function that it calls, takes no __restrict__ pointers and makes no
+// ld.global.nc loads: the compiler may move a load through a __restrict__
+// parameter ahead of the wait (the memory clobber says nothing about it), and the
+// non-coherent path is only for data that nothing writes while the kernel is
+// there, which here is before its wait too.  (With them, a probe took its table's
+// size from before the size was written.)  The loads with an L2 hint
+// (bt_search.cuh) are asm without a memory clobber: their addresses have to come
+// from something loaded after the wait.
 __device__ __forceinline__ void after_previous() {
   dependents_may_launch();
   wait_for_previous();

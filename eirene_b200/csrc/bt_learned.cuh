@@ -48,9 +48,9 @@ __device__ __forceinline__ float seg_predict(const SegParam& sp, uint64_t key) {
   return fmaf(sp.slope, d, sp.a);
 }
 
-// one 16-byte load of segment j's line
+// one 16-byte load of segment j's line (an ordinary one: stm_kernel is a dependent launch)
 __device__ __forceinline__ SegParam load_seg(const SegParam* seg, uint32_t j) {
-  const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(seg + j));
+  const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(seg + j);
   SegParam sp;
   sp.base = w.x;
   sp.a = __uint_as_float((uint32_t)w.y);

@@ -387,7 +387,7 @@ __device__ __forceinline__ uint64_t leaf_piece(const DevTree& t, LeafSmem<N>& sm
                                                uint32_t gmask, uint32_t nd, uint32_t c, uint32_t p, uint32_t m,
                                                uint32_t sz, uint64_t hdr, uint64_t fence,
                                                const uint64_t (&ok)[32 / G], const uint64_t (&ov)[32 / G],
-                                               const uint64_t* __restrict__ nk, const uint64_t* __restrict__ nv,
+                                               const uint64_t* nk, const uint64_t* nv,
                                                uint32_t cnt) {
   constexpr int S = 32 / G;
   const uint32_t st = piece_start(c, m, p), kc = piece_size(c, m, p), end = st + kc;

@@ -647,10 +647,10 @@ __device__ bool group_get(const DevTree& t, const uint32_t epoch, const uint64_t
 // without a list), four at a time by 8-lane groups.  Returns the bits q - b0
 // of the requests left for the warp path: the writes, and the GETs whose
 // leaf check failed.  op_override as in stm_kernel.
-__device__ uint32_t get_pass(const DevTree& t, const uint32_t epoch, const uint64_t* __restrict__ keys,
-                             const uint8_t* __restrict__ ops, const uint32_t op_override,
-                             const uint32_t* __restrict__ list, const size_t b0, const size_t b1,
-                             uint64_t* __restrict__ out_vals, uint8_t* __restrict__ out_st) {
+__device__ uint32_t get_pass(const DevTree& t, const uint32_t epoch, const uint64_t* keys,
+                             const uint8_t* ops, const uint32_t op_override,
+                             const uint32_t* list, const size_t b0, const size_t b1,
+                             uint64_t* out_vals, uint8_t* out_st) {
   const uint32_t lane = lane_id();
   const uint32_t g = lane % kGetG, grp = lane / kGetG;
   const uint32_t gmask = group_mask<kGetG>(lane);
@@ -806,11 +806,11 @@ struct TxCounters {
 // The writes among requests [b0, b0 + 32) whose bits are set in `rest`, four at
 // a time by 8-lane groups; returns the bits left for the warp path (failed
 // checks, splits, GETs, invalid requests).
-__device__ uint32_t write_pass(const DevTree& t, const uint32_t epoch, const uint64_t* __restrict__ keys,
-                               const uint64_t* __restrict__ vals, const uint8_t* __restrict__ ops,
-                               const uint32_t op_override, const uint32_t* __restrict__ list, const size_t b0,
-                               uint32_t rest, const uint8_t* __restrict__ skip, uint64_t* __restrict__ out_vals,
-                               uint8_t* __restrict__ out_st, TxCounters& cnt) {
+__device__ uint32_t write_pass(const DevTree& t, const uint32_t epoch, const uint64_t* keys,
+                               const uint64_t* vals, const uint8_t* ops,
+                               const uint32_t op_override, const uint32_t* list, const size_t b0,
+                               uint32_t rest, const uint8_t* skip, uint64_t* out_vals,
+                               uint8_t* out_st, TxCounters& cnt) {
   const uint32_t lane = lane_id();
   const uint32_t g = lane % kGetG, grp = lane / kGetG;
   const uint32_t gmask = group_mask<kGetG>(lane);
