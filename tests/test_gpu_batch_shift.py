@@ -153,3 +153,50 @@ def test_heavy_batches_cost_the_same_after_light_ones(gpu):
                 after[kind].append(ms(k, op))
     steady, shifted = (np.median(after[x][4:]) for x in ("heavy", "light"))
     assert shifted < 1.6 * steady, (steady, shifted)
+
+
+def test_two_handles_at_a_time(gpu):
+    # two threads, each with a handle and a stream: light and heavy batches of both
+    # meet on the device
+    import threading
+
+    import torch
+
+    n, base = 130_000, O.gen_keys("uniform", 1421, 200_000)
+    kinds = ["light", "fresh", "light", "delete", "few", "half", "light", 2_049, "light", "fresh"]
+    reqs = [requests(1430 + 10 * i, base, n, k) for i, k in enumerate(kinds)]
+    o = O.OracleTree()
+    o.bulk_build(base, O.value_of(base))
+    expect = [o.execute_merged(*r, engine=O.ENGINE_MERGE) for r in reqs]
+    b = [tuple(dev(x) for x in r) for r in reqs]
+    k, v = dev(base), dev(O.value_of(base))
+    trees = [E.BTree(max_keys=1 << 21, max_batch=1 << 18) for _ in range(2)]
+    outs = [[(empty_u64(n), empty_u8(n)) for _ in b] for _ in trees]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(i):
+        try:
+            s = torch.cuda.Stream()
+            for turn in range(4):
+                trees[i].bulk_build(k, v, stream=s)
+                if (i + turn) % 2:
+                    for x, out in zip(b, outs[i]):
+                        trees[i].execute(*x, *out, mode=MERGE, stream=s)
+                else:
+                    trees[i].execute_many(b, outs[i], mode=MERGE, stream=s)
+                trees[i].sync(s)
+                s.synchronize()
+                for j, ((gv, gs), (ov, os_)) in enumerate(zip(outs[i], expect)):
+                    assert (host_u8(gs) == os_).all() and (host_u64(gv) == ov).all(), (turn, j, kinds[j])
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for t in trees:
+        same_tree(t, o)
