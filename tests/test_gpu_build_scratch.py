@@ -1,6 +1,8 @@
 """Device memory that bulk builds of more than max_batch keys keep: one share for
 all handles of a device, given back with the last of them; builds of several
 handles at a time, from several threads and streams."""
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -8,6 +10,7 @@ import pytest
 
 import eirene_b200 as E
 from oracle import oracle as O
+from tests.conftest import ROOT
 from tests.helpers import dev, dump, host_u64
 
 pytestmark = pytest.mark.gpu
@@ -27,6 +30,13 @@ def handle():
 
 
 def test_scratch_is_shared_and_given_back(gpu):
+    # in a process of its own: another test's handle may still hold the device's scratch
+    r = subprocess.run([sys.executable, "-c", "import tests.test_gpu_build_scratch as t; t.shared_and_given_back()"],
+                       capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def shared_and_given_back():
     n = 3_000_001  # about 110 MiB of scratch
     keys = O.gen_keys("uniform", 1501, n)
     k, v = dev(keys), dev(O.value_of(keys))
