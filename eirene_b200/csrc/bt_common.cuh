@@ -105,7 +105,7 @@ struct DevTree {
 constexpr uint32_t kSplitMany = 255;
 
 // fingerprint of a key, 1 .. 255: the top byte of a multiplicative hash of its
-// two halves (Knuth's golden-ratio multiplier and another odd constant).  Keys
+// two halves (Knuth's golden-ratio multiplier and a prime of Collet's xxHash32).  Keys
 // of one leaf are neighbours, so its low bits have to spread over the byte.
 __host__ __device__ __forceinline__ uint32_t key_fp(uint64_t key) {
   const uint32_t h = (uint32_t)key * 0x9E3779B1u + (uint32_t)(key >> 32) * 0x85EBCA77u;

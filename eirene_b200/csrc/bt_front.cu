@@ -45,7 +45,7 @@ constexpr int kThreads = 256;
 
 struct Slot {
   unsigned long long key;  // kKeyMax = empty
-  uint32_t first;          // index of the first INSERT of the key
+  uint32_t first;          // index of the first write of the key
   uint32_t pad;
 };
 
@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(kThreads) front_clear_kernel(Slot* tab, size_t
   }
 }
 
-// linear probing; the table holds at most 2/3 of its slots, so a probe ends
+// linear probing; the table is at most a quarter full (half, where the allocation
+// limits it: table_cap), so a probe ends
 __global__ void __launch_bounds__(kThreads) front_insert_kernel(const uint64_t* keys, const uint32_t* list, Slot* tab,
                                                                 const BatchCounts* counts) {
   after_previous();

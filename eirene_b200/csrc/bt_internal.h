@@ -162,8 +162,8 @@ struct Work {
   uint32_t* f_pos = nullptr;     // [cap] per-tile touched counts, then the tiles' exclusive offsets
   uint32_t* f_list = nullptr;    // [cap] requests for the plain lookup, in input order
   uint64_t* f_lk = nullptr;      // [cap] their keys, in the same order
-  uint64_t* f_tk = nullptr;      // [cap] keys of the touched requests, in input order
-  uint32_t* f_tv = nullptr;      // [cap] index | op << 30 of the touched requests
+  uint64_t* f_tk = nullptr;      // [cap] keys of the touched requests (in input order for the radix sort)
+  uint32_t* f_tv = nullptr;      // [cap] their payloads: index | op << 30 for the radix sort, index << 2 | op for the sample sort
   // all-INSERT op codes of bt_insert_batch
   uint8_t* ins_ops = nullptr;
   // look-back words of the merge engine (bt_lookback.cuh)

@@ -4,25 +4,26 @@
 // bpt-gpustm-kernel.cu:14-256); the batch meaning is still v38's.
 //
 // With the batch's unique INSERT keys in ascending order:
-//   locate    each 8-lane group walks a contiguous run of the keys (path reuse,
-//             as in the sorted search), records the root-to-leaf path, answers
-//             the previous value and records where an existing key's value
-//             lives;
+//   locate    a warp descends with 32 keys at a time (warp_descend), records each
+//             one's root-to-leaf path, finds it by the leaf's fingerprints,
+//             answers the previous value and records where it lies;
 //   update    writes the new values of the existing keys in place;
-//   compact   the new keys, then runs of new keys sharing a leaf (segments);
+//   group     the new keys, packed, and runs of new keys sharing a leaf (segments);
+//   reserve   the new leaves of the segments that split, all or none;
 //   leaf      one 8-lane group per touched leaf merges its new keys by rank scatter
 //             (each element computes its merged position by binary search in
 //             the other sequence); an overflowing leaf becomes
 //             p = ceil(m / leaf_fill) leaves of even size, one group per piece;
 //             the first keys of pieces 1..p-1 become separator entries for the
 //             parent;
-//   inner     one block applies the entries level by level the same way
+//   inner     a cooperative grid applies the entries level by level the same way
 //             (children spread evenly over q = ceil((s+1)/(inner_fill+1))
 //             nodes, the key between two pieces moves up) and rebuilds an
 //             overflowing root with the bulk-load rule.
 // Locate only reads the tree, so it may run beside the batch's plain
-// lookups (the hash front end does so); the in-place value update, compact,
-// leaf and inner run after them and alone, so no locks are taken.  The rules are
+// lookups (the hash front end does so, and the grouping, which reads no tree);
+// the in-place value update, reserve, leaf and inner run after them and alone, so
+// no locks are taken.  The rules are
 // restated by the CPU oracle (bto_execute_merged with BTO_ENGINE_MERGE) and
 // the resulting leaf layout is compared exactly.
 #include <cuda_runtime.h>
@@ -59,7 +60,7 @@ struct MergeCounts {
 namespace {
 
 constexpr int kPathLevels = 8;
-constexpr uint64_t kNoPos = ~0ull;  // merge_locate_kernel: no value to update in place
+constexpr uint64_t kNoPos = ~0ull;  // locate_kernel: no value to update in place
 constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }

@@ -9,7 +9,7 @@
 // independent descents, four times the memory-level parallelism of the
 // reference's warp-per-request layout.  This kernel runs only when no writer
 // is active (the batch executor orders it before/after the insert phase), so
-// it needs no version checks and may use the read-only cache path.
+// it needs no version checks.
 #include <cstdio>
 #include <mutex>
 #include <cuda_runtime.h>
