@@ -2,6 +2,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -181,26 +182,33 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   bool ok = bt::sort_prepare() == cudaSuccess && bt::small_prepare() == 0 && bt::small_write_prepare() == 0 && bt::sample_prepare() == 0;
   if (ok) h.small_blocks = bt::small_blocks(cfg.device);
   h.tree.cap = (uint32_t)nodes;
-  ok = ok && cudaMalloc(&h.tree.keys, nodes * 256) == cudaSuccess;
-  ok = ok && cudaMalloc(&h.tree.vals, nodes * 256) == cudaSuccess;
-  ok = ok && cudaMalloc(&h.tree.low, nodes * 8) == cudaSuccess;
-  ok = ok && cudaMalloc(&h.tree.pfx, nodes * 128) == cudaSuccess;
-  ok = ok && cudaMalloc(&h.tree.fp, nodes * 32) == cudaSuccess;
-  // the control block and, behind it, the small counts of builds and dumps
-  constexpr size_t kCtrlBytes = (sizeof(bt::Ctrl) + 255) / 256 * 256;
-  ok = ok && cudaMalloc(&h.tree.ctrl, kCtrlBytes + 256) == cudaSuccess;
-  if (ok) h.geo = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h.tree.ctrl) + kCtrlBytes);
-  // everything that is cleared, on the stream that is waited for below: on the
-  // default stream it queues behind whatever that holds, and no batch on another
-  // stream would wait for it
+  // The tree's arrays in one allocation: rows, tables, fences, the control block
+  // and, behind it, the small counts of builds and dumps.  One allocation each made
+  // bt_create 1.85 ms for 2^20 keys and 1024 requests (0.64 so), and lookups of
+  // several small trees in turn met more of the chip's page mappings (100 lookups
+  // on four trees in turn, median of twelve runs 6.75 -> 6.3 us).
+  {
+    auto up = [](size_t b) { return (b + 511) / 512 * 512; };
+    const size_t row = up(nodes * 256), low = up(nodes * 8), pfx = up(nodes * 128), fp = up(nodes * 32),
+                 ctrl = up(sizeof(bt::Ctrl));
+    ok = ok && cudaMalloc(&h.tree_arena, 2 * row + low + pfx + fp + ctrl + 256) == cudaSuccess;
+    if (ok) {
+      char* at = static_cast<char*>(h.tree_arena);
+      auto take = [&](auto& p, size_t b) {
+        p = reinterpret_cast<std::decay_t<decltype(p)>>(at);
+        at += b;
+      };
+      take(h.tree.keys, row);
+      take(h.tree.vals, row);
+      take(h.tree.pfx, pfx);
+      take(h.tree.fp, fp);
+      take(h.tree.low, low);
+      take(h.tree.ctrl, ctrl);
+      h.geo = reinterpret_cast<uint32_t*>(at);
+    }
+  }
+  ok = ok && bt::work_alloc(&h.w, cfg.max_batch) == 0;
   ok = ok && cudaStreamCreateWithFlags(&h.internal_stream, cudaStreamNonBlocking) == cudaSuccess;
-  auto fill = [&](void* p, int byte, size_t bytes) {
-    return cudaMemsetAsync(p, byte, bytes, h.internal_stream) == cudaSuccess;
-  };
-  // zeroed rows read as epoch 0, which no tree uses (see hdr_epoch)
-  ok = ok && fill(h.tree.keys, 0, nodes * 256) && fill(h.tree.vals, 0, nodes * 256) &&
-       fill(h.tree.low, 0, nodes * 8) && fill(h.tree.pfx, 0xff, nodes * 128) && fill(h.tree.fp, 0, nodes * 32);
-  ok = ok && bt::work_alloc(&h.w, cfg.max_batch, h.internal_stream) == 0;
   {
     int lo_prio = 0, hi_prio = 0;
     cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio);
@@ -220,6 +228,16 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
     *h.touch_hint = UINT32_MAX;  // none seen yet
     h.pin = h.touch_hint + 64;
   }
+  // everything that is cleared, on the stream that is waited for below: on the
+  // default stream it queues behind whatever that holds, and no batch on another
+  // stream would wait for it
+  auto fill = [&](void* p, int byte, size_t bytes) {
+    return cudaMemsetAsync(p, byte, bytes, h.internal_stream) == cudaSuccess;
+  };
+  // zeroed rows read as epoch 0, which no tree uses (see hdr_epoch)
+  ok = ok && fill(h.tree.keys, 0, nodes * 256) && fill(h.tree.vals, 0, nodes * 256) &&
+       fill(h.tree.low, 0, nodes * 8) && fill(h.tree.pfx, 0xff, nodes * 128) && fill(h.tree.fp, 0, nodes * 32);
+  ok = ok && bt::work_clear(&h.w, h.internal_stream) == cudaSuccess;
   ok = ok && bt::tree_reset(&h, h.internal_stream) == cudaSuccess;
   ok = ok && cudaStreamSynchronize(h.internal_stream) == cudaSuccess;
   if (!ok) {
@@ -235,12 +253,7 @@ int bt_destroy(bt_handle* H) {
   EntryGuard g(H);
   bt::Handle& h = H->h;
   cudaDeviceSynchronize();
-  cudaFree(h.tree.keys);
-  cudaFree(h.tree.vals);
-  cudaFree(h.tree.low);
-  cudaFree(h.tree.pfx);
-  cudaFree(h.tree.fp);
-  cudaFree(h.tree.ctrl);
+  cudaFree(h.tree_arena);
   bt::work_free(&h.w);
   bt::learned_free(&h.L);
   bt::learned_policy_free(&h.L);

@@ -408,7 +408,7 @@ static size_t carve_work(Work* w, size_t cap, char* base) {
   return A.at;
 }
 
-int work_alloc(Work* w, size_t cap, cudaStream_t s) {
+int work_alloc(Work* w, size_t cap) {
   work_free(w);
   if (cap == 0) cap = 1;
   const size_t bytes = carve_work(w, cap, nullptr);
@@ -417,15 +417,16 @@ int work_alloc(Work* w, size_t cap, cudaStream_t s) {
     return -3;
   }
   carve_work(w, cap, static_cast<char*>(w->arena));
-  // look-back words of no epoch, and a clean table (every slot empty between batches)
-  if (cudaMemsetAsync(w->lb_status, 0, merge_lb_words(cap) * 8, s) != cudaSuccess ||
-      cudaMemsetAsync(w->lb_ctr, 0, kLbCtrWords * 8, s) != cudaSuccess ||
-      cudaMemsetAsync(w->s_tab, 0xff, small_tab_bytes(cap), s) != cudaSuccess) {
-    work_free(w);
-    return -3;
-  }
   w->cap = cap;
   return 0;
+}
+
+// look-back words of no epoch, and a clean table (every slot empty between batches)
+cudaError_t work_clear(Work* w, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(w->lb_status, 0, merge_lb_words(w->cap) * 8, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(w->lb_ctr, 0, kLbCtrWords * 8, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(w->s_tab, 0xff, small_tab_bytes(w->cap), s);
+  return e;
 }
 
 // the fields of Work that make up a BatchSet

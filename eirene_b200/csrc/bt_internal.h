@@ -262,6 +262,7 @@ struct Learned {
 struct Handle {
   int device = 0;
   DevTree tree{};
+  void* tree_arena = nullptr;  // the allocation that holds the tree's arrays and geo
   uint32_t leaf_fill = 24;
   uint32_t inner_fill = 24;
   uint32_t inner_min = 24;  // the inner fill that the handle was created with (bt_autotune_fill only raises it)
@@ -537,7 +538,8 @@ int small_write(Handle* h, uint64_t* out_vals, uint8_t* out_st, size_t n, uint32
 size_t small_write_words();
 
 // ---- sorted-merge batch (bt_batch.cu) ----
-int work_alloc(Work* w, size_t cap, cudaStream_t s);  // cleared in the order of s
+int work_alloc(Work* w, size_t cap);
+cudaError_t work_clear(Work* w, cudaStream_t s);  // once, before the first batch
 void work_free(Work* w);
 int batch_sorted(Handle* h, const uint64_t* keys, const uint64_t* vals, const uint8_t* ops, uint64_t* out_vals,
                  uint8_t* out_st, size_t n, int engine, cudaStream_t s);
