@@ -32,8 +32,12 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "Mops/s at 2^26 keys, 95% search; learned vs plain descent; p99 batch latency"
-BYTES_SEARCH = 288  # leaf keys (256 B) + one 32 B value sector
-BYTES_INSERT = 864  # search bytes + leaf rewrite (512 B) + version acquire/release (64 B)
+# a lookup: key and answer (17 B), the leaf's fingerprint row (32 B) and, for the half of them that
+# find their key, a key and a value sector (32 B each)
+BYTES_SEARCH = 81
+# a new key: its request and answer (17 B), the fingerprint row read (32 B), the leaf's key and value
+# rows read and written (2 x 512 B), the fingerprint row written (32 B)
+BYTES_INSERT = 1105
 BYTES_SORT = 192  # 8 radix passes x (8 B key + 4 B index) x (read + write)
 FALLBACK_HBM_GBS = 6650.0
 

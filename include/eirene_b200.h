@@ -322,8 +322,9 @@ int bt_set_search_group(bt_handle *h, uint32_t lanes);
                               * chip (up to about a million of them); 0 the onesweep radix sort (eight passes
                               * of 8 bits, BT_OPT_SORT_TILE), better for more; 2 (default) the first while the
                               * touched count of the batch seen last was at most 2^20, else the second (the
-                              * first batch: the second), and batches of up to 65,536 requests whole in three
-                              * kernels.  Same order in every case (by key, then request order) */
+                              * first batch: the second), batches of up to 65,536 requests whole in three
+                              * kernels, and a larger batch's writes in one cluster when that count was a few
+                              * thousand (on every SM if the batch then has more).  Same order in every case (by key, then request order) */
 #define BT_OPT_SORT_TILE 14     /* radix sort tile of sorted batches: 256, 512 (default) or 1024 threads x 8 keys,
                                  * for whole batches and for the hash front end's touched requests alike
                                  * (bt_autotune picks the two separately) */
