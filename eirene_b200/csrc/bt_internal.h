@@ -27,6 +27,14 @@ constexpr int kEvSortEnd = kNumPhases + 1, kEvLookupEnd = kNumPhases + 2, kEvWbS
 constexpr int kLayoutOverlap = 1;  // sort and merge passes on the side stream, beside the lookups
 constexpr int kLayoutEarly = 2;    // answers written back before the leaf merge
 
+// work on s goes into a graph instead of running
+inline cudaError_t stream_captured(cudaStream_t s, bool* yes) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(s, &st);
+  *yes = st != cudaStreamCaptureStatusNone;
+  return e;
+}
+
 // ---- scan / sort (bt_sort.cu) ----
 // layout of the radix sort's scratch: kSortMaxPasses digit histograms of
 // kSortRadix counters, 64 tile counters, and one look-back table of

@@ -1200,9 +1200,8 @@ int locate_phase(Handle* h, int what, size_t n_upper, cudaStream_t s) {
   // the INSERT keys need a root; once there is one only a new tree takes it away.
   // A launch that is captured has not run, and its graph may run on a later tree
   // without a root: there it is always part of the batch and says nothing
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) return -2;
-  const bool captured = cap != cudaStreamCaptureStatusNone;
+  bool captured = false;
+  if (stream_captured(s, &captured) != cudaSuccess) return -2;
   if ((what & kLocateIns) && (captured || !h->has_root)) {
     merge_ensure_root_kernel<<<1, 1, 0, s>>>(h->tree);
     count_launch();

@@ -898,9 +898,12 @@ void build_pool_drop(Handle* h) {
 // buffers, more in one block of the device's pool.
 int tree_bulk_build(Handle* h, const uint64_t* keys, const uint64_t* vals, size_t n, cudaStream_t s) {
   // the contents are gone in these cases too: a call on another stream may
-  // follow at once and has to meet the new tree, not the old one
+  // follow at once and has to meet the new tree, not the old one (a captured
+  // reset has nothing to wait for)
   auto emptied = [&](int rc) {
-    return tree_reset(h, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess ? rc : -2;
+    bool captured = false;
+    if (tree_reset(h, s) != cudaSuccess || stream_captured(s, &captured) != cudaSuccess) return -2;
+    return captured || cudaStreamSynchronize(s) == cudaSuccess ? rc : -2;
   };
   if (n == 0 || n > 0xFFFFFFFFull / 2) return emptied(n ? -1 : 0);
   Work& w = h->w;

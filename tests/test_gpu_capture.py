@@ -92,3 +92,30 @@ def test_replays_with_other_inputs(gpu, n, mode, engine):
     ok, ovv = o.dump()
     assert (gk == ok).all() and (gv == ovv).all()
     assert (t.leaf_sizes().sum() == gk.size) and t.stats()["error"] == 0
+
+
+@pytest.mark.parametrize("n", [3_000, 70_000])
+def test_empty_build_in_a_graph(gpu, n):
+    # a graph that empties the tree and fills it again
+    import torch
+
+    t = tree()
+    t.bulk_build(dev(np.arange(1, 1000, dtype=np.uint64)), dev(np.arange(1, 1000, dtype=np.uint64)))
+    b = empty_u64(n), empty_u64(n), empty_u8(n), empty_u64(n), empty_u8(n)
+    none = empty_u64(0)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        s = torch.cuda.current_stream()
+        t.bulk_build(none, none, stream=s)
+        t.execute(*b, mode=MERGE, stream=s)
+    for turn in range(3):
+        k, v, op = inserts(1251 + turn, n)
+        for x, y in zip(b, (k, v, op)):
+            x.copy_(dev(y))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert (host_u8(b[4]) == E.ST_ABSENT).all(), turn
+        gk, gv = dump(t)
+        o = np.argsort(k)
+        assert (gk == k[o]).all() and (gv == v[o]).all(), turn
