@@ -670,7 +670,7 @@ int bt_leaf_sizes(bt_handle* H, uint32_t* sizes_host, size_t cap, size_t* n_leav
   bt::Handle& h = H->h;
   uint32_t* leaves = nullptr;
   size_t nl = 0;
-  int rc = bt::enumerate_leaves(&h, h.internal_stream, &leaves, &nl);
+  int rc = bt::enumerate_leaves(&h, h.internal_stream, sizes_host ? &leaves : nullptr, &nl);
   if (rc) return map_internal(rc);
   *n_leaves = nl;
   if (!sizes_host || nl == 0) return BT_OK;
@@ -686,9 +686,8 @@ int bt_level_counts(bt_handle* H, uint64_t* counts_host, uint32_t cap, uint32_t*
   if (!H || !height) return BT_ERR_INVALID_ARG;
   EntryGuard g(H);
   cudaDeviceSynchronize();
-  uint32_t* leaves = nullptr;
   size_t nl = 0;
-  int rc = bt::enumerate_leaves(&H->h, H->h.internal_stream, &leaves, &nl);
+  int rc = bt::enumerate_leaves(&H->h, H->h.internal_stream, nullptr, &nl);
   if (rc) return map_internal(rc);
   *height = H->h.n_levels;
   if (counts_host)
@@ -718,9 +717,8 @@ int bt_stats_get(bt_handle* H, bt_stats* st, int with_leaves) {
   st->learned_probe_sum = c.learned_probe_sum;
   st->capacity_nodes = H->h.tree.cap;
   if (with_leaves) {
-    uint32_t* leaves = nullptr;
     size_t nl = 0;
-    int rc = bt::enumerate_leaves(&H->h, H->h.internal_stream, &leaves, &nl);
+    int rc = bt::enumerate_leaves(&H->h, H->h.internal_stream, nullptr, &nl);
     if (rc) return map_internal(rc);
     st->n_leaves = nl;
   }

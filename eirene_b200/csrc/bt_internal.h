@@ -417,7 +417,8 @@ cudaError_t launch_search_top(Handle* h, const uint64_t* qkeys, const uint32_t* 
 // search over keys in ascending order (path reuse); needs root_level < 8
 cudaError_t launch_search_sorted(Handle* h, const uint64_t* qkeys, const uint32_t* list, const uint32_t* n_dev,
                                  size_t n, uint64_t* out_vals, uint8_t* out_st, cudaStream_t s);
-// ids of the leaves in key order; returns count (synchronises the stream)
+// ids of the leaves in key order (stream ordered; nullptr: only the counts), and their number; the caller
+// waits for the stream before another one may use the enumeration's buffers
 int enumerate_leaves(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_leaves);
 // leaf sizes in key order into a device buffer (after enumerate_leaves)
 cudaError_t leaf_sizes_device(Handle* h, const uint32_t* leaves, size_t n, uint32_t* out, cudaStream_t s);

@@ -1108,7 +1108,7 @@ int learned_retrain(Handle* h, cudaStream_t s, bool refit) {
   size_t nl = 0;
   int rc = enumerate_leaves(h, s, &ids, &nl);
   if (rc) return rc;
-  if (nl < 2) return -7;
+  if (nl < 2) return cudaStreamSynchronize(s) == cudaSuccess ? -7 : -2;
   // segments: as configured, else one per 64 leaves (a power of two, at
   // least 4096), fixed at the full training so that refits keep stage 1.
   // Measured on a 2^26-key tree grown by 16 M merged inserts (3.4 M leaves

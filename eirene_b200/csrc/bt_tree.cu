@@ -1109,8 +1109,9 @@ constexpr int kEnumWords = 64;  // [0, 48) counts per level, [48] entries of thi
 
 // The leaves' ids in key order in *leaf_ids, their count in cnt[0] on the
 // device; one read back (the control block), no other wait.  *root_level < 0:
-// an empty tree.
-static int enumerate_queue(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_nodes, int* root_level) {
+// an empty tree.  Without `ids` a tree of one leaf needs no kernel.
+static int enumerate_queue(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_nodes, int* root_level,
+                           bool ids = true) {
   Ctrl* c = reinterpret_cast<Ctrl*>(h->pin);
   if (cudaMemcpyAsync(c, h->tree.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -2;
   if (cudaStreamSynchronize(s) != cudaSuccess) return -2;
@@ -1123,6 +1124,10 @@ static int enumerate_queue(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_
   if (rl >= 48) return -2;
   const size_t nn = c->n_nodes < h->tree.cap ? c->n_nodes : h->tree.cap;
   h->n_levels = rl + 1;
+  if (rl == 0 && !ids) {
+    *root_level = 0;
+    return 0;
+  }
   if (ensure_enum(h, nn + 1, s) != 0) return -3;
   uint32_t* cnt = h->geo;
   uint32_t* cur = h->enum_a;
@@ -1156,9 +1161,10 @@ int enumerate_leaves(Handle* h, cudaStream_t s, uint32_t** leaf_ids, size_t* n_l
   size_t nn = 0;
   int rl = -1;
   *n_leaves = 0;
-  const int rc = enumerate_queue(h, s, leaf_ids, &nn, &rl);
+  uint32_t* none = nullptr;
+  const int rc = enumerate_queue(h, s, leaf_ids ? leaf_ids : &none, &nn, &rl, leaf_ids != nullptr);
   if (rc || rl < 0) return rc;
-  if (rl == 0) {  // the root is the only leaf: nothing to wait for
+  if (rl == 0) {  // the root is the only leaf: no counts to read
     h->level_counts[0] = 1;
     *n_leaves = 1;
     return 0;

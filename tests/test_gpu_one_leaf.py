@@ -21,3 +21,14 @@ def test_few_leaves(gpu, n):
         assert t.stats(with_leaves=True)["n_leaves"] == leaves
         gk, gv = dump(t)
         assert (gk == keys).all() and (gv == O.value_of(keys)).all()
+
+
+def test_counts_then_builds(gpu):
+    # nothing of a count is left running in the build's memory
+    keys = np.sort(O.gen_keys("uniform", 1611, 3_000))
+    t = E.BTree(max_keys=1 << 14, max_batch=4_096)
+    for n in (1, 3_000, 20, 2_999, 24, 25) * 20:
+        t.bulk_build(dev(keys[:n]), dev(O.value_of(keys[:n])))
+        assert t.level_counts()[0] == -(-n // 24) and t.size() == n
+    gk, gv = dump(t)
+    assert (gk == keys[:25]).all() and (gv == O.value_of(keys[:25])).all()
