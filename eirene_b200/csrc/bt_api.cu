@@ -56,6 +56,9 @@ int map_internal(int rc) {
 // any insert order; the bulk layout needs far fewer.
 uint64_t pool_nodes(uint64_t max_keys) { return max_keys / 7 + 4096; }
 
+// trees whose arrays share one allocation
+constexpr size_t kTreeArenaMax = 256u << 20;
+
 }  // namespace
 
 namespace bt {
@@ -182,30 +185,37 @@ int bt_create(const bt_config* cfg_in, bt_handle** out) {
   bool ok = bt::sort_prepare() == cudaSuccess && bt::small_prepare() == 0 && bt::small_write_prepare() == 0 && bt::sample_prepare() == 0;
   if (ok) h.small_blocks = bt::small_blocks(cfg.device);
   h.tree.cap = (uint32_t)nodes;
-  // The tree's arrays in one allocation: rows, tables, fences, the control block
-  // and, behind it, the small counts of builds and dumps.  One allocation each made
-  // bt_create 1.85 ms for 2^20 keys and 1024 requests (0.64 so), and lookups of
-  // several small trees in turn met more of the chip's page mappings (100 lookups
-  // on four trees in turn, median of twelve runs 6.75 -> 6.3 us).
+  // The tree's arrays and, behind the control block, the small counts of builds and
+  // dumps.  A small tree's in one allocation: one each made bt_create 1.85 ms for
+  // 2^20 keys and 1024 requests (0.64 so), and lookups of several such trees in turn
+  // met more of the chip's page mappings (100 lookups on four trees in turn, median
+  // of twelve runs 6.75 -> 6.3 us).  A large one's each: range scans on 2^24 keys
+  // 27.4 us, 27.6 from one allocation, whose mapping is then most of the cost anyway.
   {
     auto up = [](size_t b) { return (b + 511) / 512 * 512; };
     const size_t row = up(nodes * 256), low = up(nodes * 8), pfx = up(nodes * 128), fp = up(nodes * 32),
                  ctrl = up(sizeof(bt::Ctrl));
-    ok = ok && cudaMalloc(&h.tree_arena, 2 * row + low + pfx + fp + ctrl + 256) == cudaSuccess;
+    const size_t total = 2 * row + low + pfx + fp + ctrl + 256;
+    char* at = nullptr;
+    if (total <= kTreeArenaMax) {
+      ok = ok && cudaMalloc(&h.tree_arena, total) == cudaSuccess;
+      at = static_cast<char*>(h.tree_arena);
+    }
+    auto take = [&](auto& p, size_t b) {
+      void* q = at;
+      if (at) at += b;
+      else ok = ok && cudaMalloc(&q, b) == cudaSuccess;
+      if (ok) p = static_cast<std::decay_t<decltype(p)>>(q);
+    };
     if (ok) {
-      char* at = static_cast<char*>(h.tree_arena);
-      auto take = [&](auto& p, size_t b) {
-        p = reinterpret_cast<std::decay_t<decltype(p)>>(at);
-        at += b;
-      };
       take(h.tree.keys, row);
       take(h.tree.vals, row);
+      take(h.tree.low, low);
       take(h.tree.pfx, pfx);
       take(h.tree.fp, fp);
-      take(h.tree.low, low);
-      take(h.tree.ctrl, ctrl);
-      h.geo = reinterpret_cast<uint32_t*>(at);
+      take(h.tree.ctrl, ctrl + 256);
     }
+    if (ok) h.geo = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h.tree.ctrl) + ctrl);
   }
   ok = ok && bt::work_alloc(&h.w, cfg.max_batch) == 0;
   ok = ok && cudaStreamCreateWithFlags(&h.internal_stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -253,7 +263,16 @@ int bt_destroy(bt_handle* H) {
   EntryGuard g(H);
   bt::Handle& h = H->h;
   cudaDeviceSynchronize();
-  cudaFree(h.tree_arena);
+  if (h.tree_arena) {
+    cudaFree(h.tree_arena);
+  } else {
+    cudaFree(h.tree.keys);
+    cudaFree(h.tree.vals);
+    cudaFree(h.tree.low);
+    cudaFree(h.tree.pfx);
+    cudaFree(h.tree.fp);
+    cudaFree(h.tree.ctrl);
+  }
   bt::work_free(&h.w);
   bt::learned_free(&h.L);
   bt::learned_policy_free(&h.L);

@@ -270,7 +270,7 @@ struct Learned {
 struct Handle {
   int device = 0;
   DevTree tree{};
-  void* tree_arena = nullptr;  // the allocation that holds the tree's arrays and geo
+  void* tree_arena = nullptr;  // a small tree: the allocation that holds its arrays and geo
   uint32_t leaf_fill = 24;
   uint32_t inner_fill = 24;
   uint32_t inner_min = 24;  // the inner fill that the handle was created with (bt_autotune_fill only raises it)
