@@ -1147,6 +1147,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_write_kernel(DevTree t
   write_part(t, a, n_ins, n_del, n_touch, out_vals, out_st, ClusterTeam{}, *reinterpret_cast<WriteSmem*>(raw));
 }
 
+// The same over the chip, one block an SM.  Bound by its ten or so grid barriers, then
+// like merge_leaf_kernel by entry -> leaf -> row.  Batches of INSERTs behind a light one
+// on 2^23 keys: 100,000 185 us (cluster 305, the general path's launches 210), 2^18 255
+// (632, 282), 2^20 565 (1977, 585), 2^21 1040 (general 970), 2^22 2550 (6280, 1740: there
+// a thread's 28 consecutive items are as many loads in a row).  Four blocks of 256
+// threads an SM: 2^21 1110; one of 256: 1390.
 __global__ void __launch_bounds__(kSmallThreads, 1) grid_write_kernel(DevTree t, SmallWrite a, uint64_t* out_vals,
                                                                       uint8_t* out_st) {
   extern __shared__ __align__(16) unsigned char raw[];
